@@ -15,11 +15,11 @@
 //   each pass reads from one buffer and writes a complete copy to another
 //   (ping-pong through handle-owned work buffers); the stage sequence is laid
 //   out so the final stage lands in the caller's arrays.
-// * x-direction: a warp covers 32 consecutive cells of a row; each lane
-//   computes the flux through its east face and receives the west face from
-//   its neighbour with a shuffle (lane 0 computes one extra face).
-// * y-direction: a 32 x BY block; each thread computes its north face and the
-//   south face comes from shared memory (row 0 computes one extra face).
+// * x-direction: a warp covers 31 consecutive cells of a row (32 faces); each
+//   face is evaluated once and reaches its second cell by a shuffle.
+// * y-direction: blocks of 32 x 16 threads cover 15 rows with the faces
+//   exchanged through shared memory, or (float arithmetic, several layers)
+//   warps march north with the rows in registers.
 // * Vertical pass: one thread per water column, sweeping k with a register
 //   window (the per-column update is in place, as in the reference).  The
 //   adaptive sub-stepping (itersmax = 200, restart semantics of
@@ -200,27 +200,13 @@ extern "C" int getm_advection_get_status(getm_advection* a, cudaStream_t stream)
 }
 
 // ---- kernels (one pass per launch) ------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(256) hpass_x_kernel(HPassArgs<T> a)
-{
-    hpass_x_body<T>(a, blockIdx.x, (long long)blockIdx.y * blockDim.y + threadIdx.y, threadIdx.x);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(32 * GETM_V_BY) hpass_y_kernel(HPassArgs<T> a)
-{
-    __shared__ double sQ[GETM_V_BY][32];
-    __shared__ T sF[GETM_V_BY][32];
-    hpass_y_body<T>(a, blockIdx.x, blockIdx.y, blockIdx.z, threadIdx.x, threadIdx.y, sQ, sF);
-}
-
 // grid (segments, ceil(ny_ / 8), nk): warp (ty) of block (x, y, k) owns row j = 8 y + ty of layer k
-template <typename S, typename V = S>
+template <typename S, typename V, typename C>
 __global__ void __launch_bounds__(256) hpass_x_inc_kernel(HPassArgs<S, V> a)
 {
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     if (j >= a.ny_) return;  // whole warp
-    hpass_x_inc_rows<S, 1, NoEpi, V>(a, blockIdx.x, j, blockIdx.z, threadIdx.x);
+    hpass_x_inc_rows<S, 1, NoEpi, V, C>(a, blockIdx.x, j, blockIdx.z, threadIdx.x);
 }
 
 // grid (1, ceil(ny_ / rows), nk): warp (ty) of block (0, y, k) sweeps row j = rows y + ty of layer k
@@ -247,11 +233,11 @@ static bool xpass_vec_ok(const HPassArgs<S, V>& a)
     return true;
 }
 
-template <typename S, typename V = S>
+template <typename S, typename V, typename C>
 __global__ void __launch_bounds__(32 * HY_BY) hpass_y_inc_kernel(HPassArgs<S, V> a)
 {
-    __shared__ YIncSmem<S> sm;
-    hpass_y_inc_body<S, NoEpi, V>(a, blockIdx.x, blockIdx.y, blockIdx.z, threadIdx.x, threadIdx.y, sm);
+    __shared__ YIncSmem<S, C> sm;
+    hpass_y_inc_body<S, NoEpi, V, C>(a, blockIdx.x, blockIdx.y, blockIdx.z, threadIdx.x, threadIdx.y, sm);
 }
 
 template <typename S, int NT, typename V = S>
@@ -265,35 +251,45 @@ __global__ void __launch_bounds__(256) hpass_y_march_kernel(HPassArgs<S, V> a, i
         hpass_y_march_body<S, NT, V>(a, blockIdx.x, chunk, k, threadIdx.x, t0);
 }
 
-// Launch one horizontal pass in increment form (any storage type S,
-// velocity type V).
-template <typename S, typename V = S>
-static int launch_hpass_inc(int direction, HPassArgs<S, V>& a, cudaStream_t stream)
+// Launch one horizontal pass (storage type S, velocity type V, arithmetic C).
+template <typename S, typename V, typename C>
+static int launch_hpass_c(int direction, HPassArgs<S, V>& a, cudaStream_t stream)
 {
+    constexpr bool f64 = std::is_same<C, double>::value;
     if (direction == 1) {
         const int rows = getm_tune(GETM_TUNE_XPASS_ROWS);
         dim3 block(32, rows);
-        if (getm_tune(GETM_TUNE_XPASS_VEC) && xpass_vec_ok(a)) {
+        bool vec = false;
+        // four cells per lane: float arithmetic only.  The FP64 form is bound
+        // by its FP64 instructions, and the one-cell kernel forms a face's
+        // geometry once for all fields where the sweep repeats it per pair
+        if constexpr (!f64) vec = getm_tune(GETM_TUNE_XPASS_VEC) && xpass_vec_ok(a);
+        if (vec) {
             dim3 grid(1, getm_div_up(a.ny_, rows), a.nk);
-            hpass_x_vec_kernel<S, V><<<grid, block, 0, stream>>>(a);
+            if constexpr (!f64) hpass_x_vec_kernel<S, V><<<grid, block, 0, stream>>>(a);
         } else {
             // lane 0 of the first segment handles the face west of cell 0
             dim3 grid(getm_div_up(a.nx_ + 1, HX_STRIDE), getm_div_up(a.ny_, rows), a.nk);
-            hpass_x_inc_kernel<S, V><<<grid, block, 0, stream>>>(a);
+            hpass_x_inc_kernel<S, V, C><<<grid, block, 0, stream>>>(a);
         }
-    } else if (a.nk < 4) {
+    } else if (f64 || a.nk < 4) {
         // a single plane: too few columns x layers for marching warps to fill
-        // the GPU, so blocks of 32 x HY_BY threads cover tiles instead
+        // the GPU, so blocks of 32 x HY_BY threads cover tiles instead.  FP64
+        // form: the tile kernel forms a face's geometry once for all fields
+        // and has a block per 15 rows, where the marching kernel repeats the
+        // geometry per pair and had blocks for 90 of 152 SMs on 173 x 131 x 23
         dim3 block(32, HY_BY);
         dim3 grid(getm_div_up(a.nx_, 32), getm_div_up(a.ny_ + 1, HY_STRIDE), a.nk);
-        hpass_y_inc_kernel<S, V><<<grid, block, 0, stream>>>(a);
+        hpass_y_inc_kernel<S, V, C><<<grid, block, 0, stream>>>(a);
     } else {
         a.ych = getm_tune(GETM_TUNE_YMARCH_CHUNK);
         const int nchunk = getm_div_up(a.ny_, a.ych);
         dim3 block(32, 8);
         dim3 grid(getm_div_up(a.nx_, 32), getm_div_up((long long)nchunk * a.nk, 8));
-        if (a.ntracer >= 2) hpass_y_march_kernel<S, 2, V><<<grid, block, 0, stream>>>(a, nchunk);
-        else hpass_y_march_kernel<S, 1, V><<<grid, block, 0, stream>>>(a, nchunk);
+        if constexpr (!f64) {
+            if (a.ntracer >= 2) hpass_y_march_kernel<S, 2, V><<<grid, block, 0, stream>>>(a, nchunk);
+            else hpass_y_march_kernel<S, 1, V><<<grid, block, 0, stream>>>(a, nchunk);
+        }
     }
     GETM_CHECK_LAUNCH();
     return GETM_OK;
@@ -303,21 +299,10 @@ template <typename T, typename V = T>
 static int launch_hpass(int direction, HPassArgs<T, V>& a, cudaStream_t stream)
 {
     if constexpr (getm_increment_form<T> || !std::is_same<T, V>::value) {
-        return launch_hpass_inc<T, V>(direction, a, stream);
+        return launch_hpass_c<T, V, float>(direction, a, stream);
     } else {
-        if (a.increment) return launch_hpass_inc<T, V>(direction, a, stream);
-        if (direction == 1) {
-            const int BY = 8;
-            dim3 block(32, BY);
-            dim3 grid(getm_div_up(a.nx_, 32), getm_div_up((long long)a.ny_ * a.nk, BY));
-            hpass_x_kernel<T><<<grid, block, 0, stream>>>(a);
-        } else {
-            dim3 block(32, GETM_V_BY);
-            dim3 grid(getm_div_up(a.nx_, 32), getm_div_up(a.ny_, GETM_V_BY), a.nk);
-            hpass_y_kernel<T><<<grid, block, 0, stream>>>(a);
-        }
-        GETM_CHECK_LAUNCH();
-        return GETM_OK;
+        if (a.increment) return launch_hpass_c<T, V, float>(direction, a, stream);
+        return launch_hpass_c<T, V, double>(direction, a, stream);
     }
 }
 
@@ -559,7 +544,7 @@ __device__ void w_substep_inc(const WPassArgs<S, float>& a, long long c, const f
         wkn = (k + 1 < nz) ? ring.w[s2 * 32] : 0.f;
         stage(k + 2 + W_STAGE);  // into the slot of level k + 1, read at k - 1
         const float cfl = fabsf(W) * dtf / fminf(hkf, hk1f) * itf;
-        const TvdFaceF tf = getm_tvd_face_f(a.scheme, cfl);
+        const TvdFace<float> tf = getm_tvd_face_c(a.scheme, cfl);
         const float dh = dtkf * (wk - wkm1);
         const double hn = hk - getm_f2d(dh);
         hd[c + k * P] = hn;
@@ -572,8 +557,8 @@ __device__ void w_substep_inc(const WPassArgs<S, float>& a, long long c, const f
             if (k < nz - 1) {
                 const float d = dk[q];
                 float dev;
-                if (W > 0.f) dev = getm_tvd_dev_f(tf, d, dkm1[q]);
-                else dev = getm_tvd_dev_f(tf, -d, -dn);
+                if (W > 0.f) dev = getm_tvd_dev_c(tf, d, dkm1[q]);
+                else dev = getm_tvd_dev_c(tf, -d, -dn);
                 el = W * (W > 0.f ? dev : d + dev);
                 er = W * (W > 0.f ? dev - d : dev);
             }

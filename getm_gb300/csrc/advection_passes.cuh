@@ -7,7 +7,6 @@
 #include "getm_common.cuh"
 
 #define GETM_MAX_BATCH 32
-#define GETM_V_BY 16
 
 // ---------------------------------------------------------------------------
 // horizontal pass kernels
@@ -15,10 +14,8 @@
 // T is the type of the advected fields, V that of the velocities (T unless
 // given): double for the FP64 form, float for the mixed form; the mixed form
 // with FP64 tracer storage has T = double, V = float (its increments are
-// still formed in float).  Layer thicknesses, the transports QU that update
-// them and all grid metrics are double in every form.  For T = V = double
-// without increment form every expression below is the FP64 reference
-// arithmetic.
+// still formed in float).  Layer thicknesses and all grid metrics are double
+// in every form.
 template <typename T, typename V = T>
 struct HPassArgs {
     int nx_, ny_, nk;
@@ -38,7 +35,7 @@ struct HPassArgs {
     int scheme;
     int ntracer;
     // mixed form: float copies of dt and of the metrics above; increment != 0
-    // selects the increment-form kernels for double fields (2D momentum)
+    // selects float increments for double fields (2D momentum)
     int increment;
     float dtf;
     int ych;                    // rows a warp marches in the 3D y pass (launch-shape knob)
@@ -57,181 +54,160 @@ struct NoEpi {
     __device__ __forceinline__ void operator()(long long, int, double, double) const {}
 };
 
-template <typename T>
-struct FaceGeom {
-    double QU;
-    T cfl;
-    bool active, up, uu_ok;
-};
-
-// Face quantities that do not depend on the advected field
-// (template :63-65, :70, :77).
-template <typename T>
-__device__ __forceinline__ FaceGeom<T> face_geom(const HPassArgs<T>& a, long long p2, long long p3,
-                                                 long long s, bool in_range)
-{
-    FaceGeom<T> g;
-    g.QU = 0.0; g.cfl = T(0); g.active = false; g.up = false; g.uu_ok = false;
-    if (!in_range) return g;
-    int m = a.umask[p2];
-    if (!getm_flux_point(m)) return g;
-    T uu = a.u[p3];
-    g.active = true;
-    g.QU = (double)uu * a.hu[p3] * a.dy[p2];
-    g.cfl = fabs(uu * (T)a.dt * (T)a.idx[p2]);
-    g.up = uu > T(0);
-    g.uu_ok = getm_flux_point(g.up ? a.umask[p2 - s] : a.umask[p2 + s]);
-    return g;
-}
-
-// Tracer flux through one face (template :66-104).
-template <typename T>
-__device__ __forceinline__ T face_flux(const HPassArgs<T>& a, const FaceGeom<T>& g, const T* __restrict__ f,
-                                       long long p2, long long p3, long long s)
-{
-    if (!g.active) return T(0);
-    T fu, fuu, fd;
-    if (g.up) {
-        fu = f[p3];
-        fuu = g.uu_ok ? f[p3 - s] : fu;
-        fd = f[p3 + s];
-    } else {
-        fu = f[p3 + s];
-        fuu = g.uu_ok ? f[p3 + 2 * s] : fu;
-        fd = f[p3];
-    }
-    fu = getm_tvd_face<T>(a.scheme, fuu, fu, fd, g.cfl);
-    T flux = (T)g.QU * fu;
-    if (a.Ah) flux = flux - (T)a.Ah[p2] * (T)a.hu[p3] * (f[p3 + s] - f[p3]) * (T)a.idx[p2] * (T)a.dy[p2];
-    return flux;
-}
-
-// x-direction pass.  blockDim = (32, BYX); grid = (ceil(nx_/32), ceil(ny_*nk/BYX)).
-template <typename T, typename Epi = NoEpi>
-__device__ __forceinline__ void hpass_x_body(const HPassArgs<T>& a, int bx, long long row, int lane,
-                                             const Epi& epi = Epi())
-{
-    const int i = bx * 32 + lane;
-    if (row >= (long long)a.ny_ * a.nk) return;  // whole warp shares one row
-    const int k = (int)(row / a.ny_);
-    const int j = (int)(row - (long long)k * a.ny_);
-    const bool inx = i < a.nx_;
-    const long long p2 = (long long)j * a.nx_ + i;
-    const long long p3 = (long long)k * a.plane + p2;
-    const bool jrow = j >= a.jlo && j <= a.jhi;
-
-    FaceGeom<T> gr = face_geom(a, p2, p3, 1, inx && jrow && i >= a.ilo - 1 && i <= a.ihi);
-    FaceGeom<T> gl = face_geom(a, p2 - 1, p3 - 1, 1, lane == 0 && jrow && i - 1 >= a.ilo - 1 && i - 1 <= a.ihi);
-    double QUl = __shfl_up_sync(0xffffffffu, gr.QU, 1);
-    if (lane == 0) QUl = gl.QU;
-    const bool upd = inx && jrow && i >= a.ilo && i <= a.ihi && a.tmask[p2] == 1;
-
-    double hold = 0.0, hnew = 0.0, iA = 0.0;
-    if (inx) {
-        hold = a.h_in[p3];
-        hnew = hold;
-        if (upd) {
-            iA = a.iA[p2];
-            hnew = hold - a.dt * (gr.QU - QUl) * iA;
-        }
-        a.h_out[p3] = hnew;
-    }
-    for (int t = 0; t < a.ntracer; t++) {
-        const T* __restrict__ f = a.fin[t];
-        T fr = inx ? face_flux(a, gr, f, p2, p3, 1) : T(0);
-        T fl = __shfl_up_sync(0xffffffffu, fr, 1);
-        if (lane == 0) fl = face_flux(a, gl, f, p2 - 1, p3 - 1, 1);
-        if (inx) {
-            T fo = f[p3];
-            T fn = fo;
-            if (upd) {
-                T hfo = (T)hold * fo;
-                T advn = (fr - fl) * (T)iA;
-                fn = (hfo - (T)a.dt * advn) / (T)hnew;
-            }
-            a.fout[t][p3] = fn;
-            if (t == 0) epi(p3, j, (double)fn, hnew);
-        }
-    }
-}
-
-// y-direction pass.  blockDim = (32, GETM_V_BY); grid = (ceil(nx_/32), ceil(ny_/BY), nk).
-template <typename T, typename Epi = NoEpi>
-__device__ __forceinline__ void hpass_y_body(const HPassArgs<T>& a, int bx, int by, int k, int tx, int ty,
-                                             double (&sQ)[GETM_V_BY][32], T (&sF)[GETM_V_BY][32],
-                                             const Epi& epi = Epi())
-{
-    const int i = bx * 32 + tx;
-    const int j = by * GETM_V_BY + ty;
-    const bool in = i < a.nx_ && j < a.ny_;
-    const long long s = a.nx_;
-    const long long p2 = (long long)j * a.nx_ + i;
-    const long long p3 = (long long)k * a.plane + p2;
-    const bool icol = i >= a.ilo && i <= a.ihi;
-
-    FaceGeom<T> gt = face_geom(a, p2, p3, s, in && icol && j >= a.jlo - 1 && j <= a.jhi);
-    FaceGeom<T> gb = face_geom(a, p2 - s, p3 - s, s, in && ty == 0 && icol && j - 1 >= a.jlo - 1 && j - 1 <= a.jhi);
-    sQ[ty][tx] = gt.QU;
-    __syncthreads();
-    double QUb = ty > 0 ? sQ[ty - 1][tx] : gb.QU;
-    const bool upd = in && icol && j >= a.jlo && j <= a.jhi && a.tmask[p2] == 1;
-
-    double hold = 0.0, hnew = 0.0, iA = 0.0;
-    if (in) {
-        hold = a.h_in[p3];
-        hnew = hold;
-        if (upd) {
-            iA = a.iA[p2];
-            hnew = hold - a.dt * (gt.QU - QUb) * iA;
-        }
-        a.h_out[p3] = hnew;
-    }
-    for (int t = 0; t < a.ntracer; t++) {
-        const T* __restrict__ f = a.fin[t];
-        T ft = in ? face_flux(a, gt, f, p2, p3, s) : T(0);
-        T fb = (ty == 0 && in) ? face_flux(a, gb, f, p2 - s, p3 - s, s) : T(0);
-        __syncthreads();  // previous tracer's reads of sF are done
-        sF[ty][tx] = ft;
-        __syncthreads();
-        if (ty > 0) fb = sF[ty - 1][tx];
-        if (in) {
-            T fo = f[p3];
-            T fn = fo;
-            if (upd) {
-                T hfo = (T)hold * fo;
-                T advn = (ft - fb) * (T)iA;
-                fn = (hfo - (T)a.dt * advn) / (T)hnew;
-            }
-            a.fout[t][p3] = fn;
-            if (t == 0) epi(p3, j, (double)fn, hnew);
-        }
-    }
-}
-
 // ---------------------------------------------------------------------------
-// Mixed form (float fields): increment form of the same passes.
+// Increment form of the passes (template :61-116).
 //
 // With hold - hnew = dt iA (QU_e - QU_w), the reference update
 // (hold f - dt iA (QU_e f_e - QU_w f_w)) / hnew equals
 //     f - dt iA (QU_e (f_e - f) - QU_w (f_w - f)) / hnew
 // exactly, where f_e, f_w are the limited face values.  Each face therefore
-// provides QU (face - left cell) and QU (face - right cell), formed from
-// differences of neighbouring values, so float32 rounding scales with the
-// change of the field, a field at rest is reproduced exactly, and the only
-// FP64 operations per cell are the thickness update hnew = hold - dh.
+// provides el = QU (face - left cell) and er = QU (face - right cell), formed
+// from differences of neighbouring values, so rounding scales with the change
+// of the field and a field at rest is reproduced exactly.
+//
+// C: the arithmetic of the increments.
+// * C = float (mixed form): float32 rounding scales with the change, and the
+//   only FP64 operations per cell are the thickness update hnew = hold - dh
+//   and, for fields stored in double, the difference and the final sum.
+// * C = double (FP64 form): GB300 issues an FP64 instruction at 1/64 of the
+//   float rate, so the number of FP64 instructions is the time of the pass.
+//   In increment form and with the division-free limiter on the integer pipe
+//   a cell takes 13 of them for the geometry and the thickness and 6 per
+//   field (superbee); the reference's order of evaluation took about 120 for
+//   one field, two thirds of them in its two divisions per field and in the
+//   extra face of each warp's first lane (or tile's first row).  Measured, us
+//   per pass: 120 x 100 x 30, one field, superbee, x 93.6 -> 27.5, y 97.2 ->
+//   28.5; 173 x 131 x 23, six fields, HSIMT and diffusion, x 446 -> 118, y 428
+//   -> 132 (FP64 pipe 77 % busy).  Against quad precision the five-pass split's
+//   error falls from 2.0e-16 to 1.3e-16 (a result is rounded once per pass,
+//   not three times).  Products and sums are rounded as written (intrinsics,
+//   no contraction): the separate passes and the one-launch substep share
+//   these functions and give the same bits.
 // ---------------------------------------------------------------------------
-// Storage type S of the advected field and of the velocities: float (the 3D
-// fields of the mixed form) or double (the 2D depth-averaged momentum of the
-// mixed form, whose state stays FP64 while its increments are evaluated in
-// float).  Differences of neighbouring values are formed in S and then
-// narrowed, so they keep their accuracy when the values are close.
+// Storage type S of the advected field and V of the velocities: float (the
+// 3D fields of the mixed form) or double (with C = float: the 2D
+// depth-averaged momentum and the tracers of the mixed form, whose state
+// stays FP64 while its increments are evaluated in float).  Differences of
+// neighbouring values are formed in S and then narrowed to C, so they keep
+// their accuracy when the values are close.
 
-// Limited face deviation from the upwind cell, given d = f[b] - f[a] across
-// the face and the differences on either side, dprev = f[a] - f[a-1] and
-// dnext = f[b+1] - f[b]; tf: the face's limiter constants.
-__device__ __forceinline__ float hx_dev(const TvdFaceF& tf, bool up, bool uu_ok, float dprev, float d, float dnext)
+// a value or a difference in S (or V) narrowed to the arithmetic type
+template <typename C, typename S>
+__device__ __forceinline__ C hx_c(S x)
 {
-    return up ? getm_tvd_dev_f(tf, d, uu_ok ? dprev : 0.f) : getm_tvd_dev_f(tf, -d, uu_ok ? -dnext : 0.f);
+    if constexpr (std::is_same<C, double>::value) return (double)x;
+    else return inc_f<S>(x);
+}
+
+// the metrics and the time step in the arithmetic type
+template <typename C, typename S, typename V>
+__device__ __forceinline__ const C* hx_dy(const HPassArgs<S, V>& a)
+{
+    if constexpr (std::is_same<C, double>::value) return a.dy;
+    else return a.dy_f;
+}
+
+template <typename C, typename S, typename V>
+__device__ __forceinline__ const C* hx_idx(const HPassArgs<S, V>& a)
+{
+    if constexpr (std::is_same<C, double>::value) return a.idx;
+    else return a.idx_f;
+}
+
+template <typename C, typename S, typename V>
+__device__ __forceinline__ const C* hx_iA(const HPassArgs<S, V>& a)
+{
+    if constexpr (std::is_same<C, double>::value) return a.iA;
+    else return a.iA_f;
+}
+
+template <typename C, typename S, typename V>
+__device__ __forceinline__ C hx_dt(const HPassArgs<S, V>& a)
+{
+    if constexpr (std::is_same<C, double>::value) return a.dt;
+    else return a.dtf;
+}
+
+__device__ __forceinline__ float hx_mul3(float x, float y, float z) { return x * y * z; }
+__device__ __forceinline__ double hx_mul3(double x, double y, double z) { return __dmul_rn(__dmul_rn(x, y), z); }
+__device__ __forceinline__ float hx_abs(float x) { return fabsf(x); }
+__device__ __forceinline__ double hx_abs(double x) { return fabs(x); }
+__device__ __forceinline__ bool hx_positive(float x) { return x > 0.f; }
+__device__ __forceinline__ bool hx_positive(double x) { return getm_positive_i(x); }
+__device__ __forceinline__ float hx_ahd(float ah, float hu, float idx, float dy) { return -ah * hu * idx * dy; }
+__device__ __forceinline__ double hx_ahd(double ah, double hu, double idx, double dy)
+{
+    return -__dmul_rn(hx_mul3(ah, hu, idx), dy);
+}
+
+// thickness of an updated cell and dt iA / hnew
+__device__ __forceinline__ void hx_cell(float dt, float QUe, float QUw, float iA, double hold, double& hnew,
+                                        float& coef)
+{
+    const float dh = dt * (QUe - QUw) * iA;
+    hnew = hold - getm_f2d(dh);
+    coef = dt * iA / (getm_d2f_approx(hold) - dh);
+}
+
+__device__ __forceinline__ void hx_cell(double dt, double QUe, double QUw, double iA, double hold, double& hnew,
+                                        double& coef)
+{
+    const double c = __dmul_rn(dt, iA);
+    hnew = __fma_rn(-c, __dadd_rn(QUe, -QUw), hold);
+    coef = __dmul_rn(c, getm_rcp(hnew));
+}
+
+// el and er of an active face, given d = f[b] - f[a] across the face and the
+// differences on either side, dprev = f[a] - f[a-1] and dnext = f[b+1] - f[b];
+// tf: the face's limiter constants; ahd = -Ah hu idx dy (diff: whether there
+// is horizontal diffusion).  The limiter is odd in its two differences, so the
+// side away from the flow is selected first and one evaluation serves both
+// flow directions.
+__device__ __forceinline__ void hx_face(const TvdFace<float>& tf, bool up, bool uu_ok, float QU, float dprev, float d,
+                                        float dnext, float ahd, bool, float& el, float& er)
+{
+    const float lim = getm_tvd_dev_c(tf, d, uu_ok ? (up ? dprev : dnext) : 0.f);
+    const float dev = up ? lim : -lim;
+    const float fd = ahd * d;
+    el = QU * (up ? dev : d + dev) + fd;
+    er = QU * (up ? dev - d : dev) + fd;
+}
+
+// FP64: with G = QU 0.5 (1 - cfl) phi(r) d and P = QU d, the upwind side's
+// value is +-G (+ the diffusive flux) and the other's differs from it by P:
+// four FP64 instructions with the product for G's first factor formed once
+// per face (tf.half1mc holds it).
+__device__ __forceinline__ void hx_face(const TvdFace<double>& tf, bool up, bool uu_ok, double QU, double dprev,
+                                        double d, double dnext, double ahd, bool diff, double& el, double& er)
+{
+    double G = getm_negate_if(__dmul_rn(tf.half1mc, getm_tvd_phi(tf, d, uu_ok ? (up ? dprev : dnext) : 0.0)), !up);
+    if (diff) G = __fma_rn(ahd, d, G);
+    const double other = __dadd_rn(G, getm_negate_if(__dmul_rn(QU, d), up));
+    el = up ? G : other;
+    er = up ? other : G;
+}
+
+// the face's limiter constants
+__device__ __forceinline__ TvdFace<float> hx_tvd(int scheme, float cfl, float) { return getm_tvd_face_c(scheme, cfl); }
+
+__device__ __forceinline__ TvdFace<double> hx_tvd(int scheme, double cfl, double QU)
+{
+    TvdFace<double> tf = getm_tvd_face_c(scheme, cfl);
+    tf.half1mc = __dmul_rn(QU, tf.half1mc);
+    return tf;
+}
+
+// the new value of a field in a cell: el_e of its east (north) face, er_w of
+// its west (south) face
+template <typename S>
+__device__ __forceinline__ S hx_new(S f, float coef, float el_e, float er_w)
+{
+    return inc_add<S>(f, -coef * (el_e - er_w));
+}
+
+__device__ __forceinline__ double hx_new(double f, double coef, double el_e, double er_w)
+{
+    return __fma_rn(-coef, __dadd_rn(el_e, -er_w), f);
 }
 
 // x-direction pass in increment form.  A warp owns one row segment: lane L
@@ -246,7 +222,7 @@ constexpr int HX_STRIDE = 31;
 // KB layers k0 .. k0+KB-1 (those below nk) of row j: the 2D fields (masks,
 // metrics) are loaded once for all of them, and every load of the KB layers
 // is issued before any value is used.
-template <typename S, int KB, typename Epi = NoEpi, typename V = S>
+template <typename S, int KB, typename Epi = NoEpi, typename V = S, typename C = float>
 __device__ __forceinline__ void hpass_x_inc_rows(const HPassArgs<S, V>& a, int bx, int j, int k0, int lane,
                                                  const Epi& epi = Epi())
 {
@@ -265,10 +241,10 @@ __device__ __forceinline__ void hpass_x_inc_rows(const HPassArgs<S, V>& a, int b
     const int iac = min(max(ia, 0), a.nx_ - 1), ixc = min(max(ix, 0), a.nx_ - 1), ibc = min(ib, a.nx_ - 1);
     const int um_raw = a.umask[r2 + iac];
     const int umx_raw = a.umask[r2 + ixc];
-    const float dyf = a.dy_f[r2 + iac], idxf = a.idx_f[r2 + iac];
-    const float ahraw = a.Ah ? getm_d2f_approx(a.Ah[r2 + iac]) : 0.f;
+    const C dyf = hx_dy<C>(a)[r2 + iac], idxf = hx_idx<C>(a)[r2 + iac];
+    const C ahraw = a.Ah ? hx_c<C>(a.Ah[r2 + iac]) : C(0);
     const int tm = a.tmask[r2 + ibc];
-    const float iaf = a.iA_f[r2 + ibc];
+    const C iaf = hx_iA<C>(a)[r2 + ibc];
     V uraw[KB];
     double huraw[KB], hold[KB];
 #pragma unroll
@@ -311,31 +287,27 @@ __device__ __forceinline__ void hpass_x_inc_rows(const HPassArgs<S, V>& a, int b
     for (int kk = 0; kk < KB; kk++) {
         if (k0 + kk >= a.nk) break;
         const long long r3 = (long long)(k0 + kk) * a.plane + r2;
-        float QU = 0.f, cfl = 0.f, ahd = 0.f;
+        C QU = C(0), cfl = C(0), ahd = C(0);
         bool up = false, uu_ok = false;
         if (act) {
-            const float uu = inc_f<V>(uraw[kk]);
-            const float huf = getm_d2f_approx(huraw[kk]);
-            QU = uu * huf * dyf;
-            cfl = fabsf(uu * a.dtf * idxf);
-            up = uu > 0.f;
+            const C uu = hx_c<C>(uraw[kk]);
+            const C huf = hx_c<C>(huraw[kk]);
+            QU = hx_mul3(uu, huf, dyf);
+            cfl = hx_abs(hx_mul3(uu, hx_dt<C>(a), idxf));
+            up = hx_positive(uu);
             uu_ok = getm_flux_point(up ? um_w : um_e);
-            if (a.Ah) ahd = -ahraw * huf * idxf * dyf;
+            if (a.Ah) ahd = hx_ahd(ahraw, huf, idxf, dyf);
         }
-        const float QUe = __shfl_down_sync(FULL, QU, 1);  // east face of cell ib
+        const C QUe = __shfl_down_sync(FULL, QU, 1);  // east face of cell ib
 
         // thickness update of cell ib
-        float coef = 0.f;  // dt iA / hnew
+        C coef = C(0);  // dt iA / hnew
         double hnew = hold[kk];
         if (bin) {
-            if (upd) {
-                const float dh = a.dtf * (QUe - QU) * iaf;
-                hnew = hold[kk] - getm_f2d(dh);
-                coef = a.dtf * iaf / (getm_d2f_approx(hold[kk]) - dh);
-            }
+            if (upd) hx_cell(hx_dt<C>(a), QUe, QU, iaf, hold[kk], hnew, coef);
             a.h_out[r3 + ib] = hnew;
         }
-        const TvdFaceF tf = getm_tvd_face_f(a.scheme, cfl);
+        const TvdFace<C> tf = hx_tvd(a.scheme, cfl, QU);
         // tracers two at a time (the first two preloaded with the layer)
         for (int t = 0; t < a.ntracer; t += 2) {
             const int nt = a.ntracer - t >= 2 ? 2 : 1;
@@ -359,23 +331,18 @@ __device__ __forceinline__ void hpass_x_inc_rows(const HPassArgs<S, V>& a, int b
                 S fb = __shfl_down_sync(FULL, fa, 1);  // f[ia+1]
                 const S x0 = __shfl_sync(FULL, fx, 0), x1 = __shfl_sync(FULL, fx, 1), x2 = __shfl_sync(FULL, fx, 2);
                 if (lane == 31) fb = x1;
-                const float d = inc_f<S>(fb - fa);
-                float dprev = __shfl_up_sync(FULL, d, 1), dnext = __shfl_down_sync(FULL, d, 1);
+                const C d = hx_c<C>(fb - fa);
+                C dprev = __shfl_up_sync(FULL, d, 1), dnext = __shfl_down_sync(FULL, d, 1);
                 // the two differences the shuffles cannot supply, in one operation
-                const float e = inc_f<S>(lane == 0 ? fa - x0 : x2 - x1);
+                const C e = hx_c<C>(lane == 0 ? fa - x0 : x2 - x1);
                 if (lane == 0) dprev = e;
                 if (lane == 31) dnext = e;
                 // el = QU (face - f[ia]) (east side of cell ia), er = QU (face - f[ib])
-                float el = 0.f, er = 0.f;
-                if (act) {
-                    const float dev = hx_dev(tf, up, uu_ok, dprev, d, dnext);
-                    const float fd = ahd * d;
-                    el = QU * (up ? dev : d + dev) + fd;
-                    er = QU * (up ? dev - d : dev) + fd;
-                }
-                const float el_e = __shfl_down_sync(FULL, el, 1);  // east face of cell ib, seen from ib
+                C el = C(0), er = C(0);
+                if (act) hx_face(tf, up, uu_ok, QU, dprev, d, dnext, ahd, a.Ah != nullptr, el, er);
+                const C el_e = __shfl_down_sync(FULL, el, 1);  // east face of cell ib, seen from ib
                 if (bin) {
-                    const S fn = upd ? inc_add<S>(fb, -coef * (el_e - er)) : fb;
+                    const S fn = upd ? hx_new(fb, coef, el_e, er) : fb;
                     a.fout[t + q][r3 + ib] = fn;
                     if (t + q == 0) epi(r3 + ib, j, (double)fn, hnew);
                 }
@@ -510,9 +477,7 @@ __device__ __forceinline__ void hpass_x_vec_row(const HPassArgs<S, V>& a, int j,
                 hnew[m] = hold[m];
                 if (upd[m]) {
                     const float QUw = m > 0 ? QU[m - 1] : QUw0;
-                    const float dh = a.dtf * (QU[m] - QUw) * iaf[m];
-                    hnew[m] = hold[m] - getm_f2d(dh);
-                    coef[m] = a.dtf * iaf[m] / (getm_d2f_approx(hold[m]) - dh);
+                    hx_cell(a.dtf, QU[m], QUw, iaf[m], hold[m], hnew[m], coef[m]);
                 }
             }
             if (g == 0 && lin) xv_store4(a.h_out + r3 + ib, hnew);
@@ -545,12 +510,9 @@ __device__ __forceinline__ void hpass_x_vec_row(const HPassArgs<S, V>& a, int j,
                 for (int m = 0; m < 4; m++) {
                     el[m] = 0.f; er[m] = 0.f;
                     if (act[m]) {
-                        const TvdFaceF tf = getm_tvd_face_f(a.scheme, cfl[m]);
+                        const TvdFace<float> tf = getm_tvd_face_c(a.scheme, cfl[m]);
                         const float dprev = m > 0 ? d[m - 1] : dW, dnext = m < 3 ? d[m + 1] : dE;
-                        const float dev = hx_dev(tf, up[m], uu_ok[m], dprev, d[m], dnext);
-                        const float fd = ahd[m] * d[m];
-                        el[m] = QU[m] * (up[m] ? dev : d[m] + dev) + fd;
-                        er[m] = QU[m] * (up[m] ? dev - d[m] : dev) + fd;
+                        hx_face(tf, up[m], uu_ok[m], QU[m], dprev, d[m], dnext, ahd[m], a.Ah != nullptr, el[m], er[m]);
                     }
                 }
                 float erW = __shfl_up_sync(FULL, er[3], 1);  // west face of the lane's first cell
@@ -559,7 +521,7 @@ __device__ __forceinline__ void hpass_x_vec_row(const HPassArgs<S, V>& a, int j,
 #pragma unroll
                 for (int m = 0; m < 4; m++) {
                     const float ew = m > 0 ? er[m - 1] : erW;
-                    out[m] = upd[m] ? inc_add<S>(fv[m], -coef[m] * (el[m] - ew)) : fv[m];
+                    out[m] = upd[m] ? hx_new(fv[m], coef[m], el[m], ew) : fv[m];
                 }
                 if (lin) xv_store4(a.fout[t0 + q] + r3 + ib, out);
                 cd[q] = __shfl_sync(FULL, d[3], 31);
@@ -572,14 +534,14 @@ __device__ __forceinline__ void hpass_x_vec_row(const HPassArgs<S, V>& a, int j,
 }
 
 // One row (layer k, row j) of the x pass: row = k ny_ + j.
-template <typename S, typename Epi = NoEpi, typename V = S>
+template <typename S, typename Epi = NoEpi, typename V = S, typename C = float>
 __device__ __forceinline__ void hpass_x_inc_body(const HPassArgs<S, V>& a, int bx, long long row, int lane,
                                                  const Epi& epi = Epi())
 {
     if (row >= (long long)a.ny_ * a.nk) return;  // whole warp shares one row
     const int k = (int)(row / a.ny_);
     const int j = (int)(row - (long long)k * a.ny_);
-    hpass_x_inc_rows<S, 1, Epi, V>(a, bx, j, k, lane, epi);
+    hpass_x_inc_rows<S, 1, Epi, V, C>(a, bx, j, k, lane, epi);
 }
 
 // y-direction pass in increment form: the transpose of hpass_x_inc_kernel.
@@ -592,16 +554,16 @@ __device__ __forceinline__ void hpass_x_inc_body(const HPassArgs<S, V>& a, int b
 constexpr int HY_BY = 16;
 constexpr int HY_STRIDE = HY_BY - 1;
 
-template <typename S>
+template <typename S, typename C = float>
 struct YIncSmem {
     S sf[HY_BY + 3][32];       // rows j0-2 .. j0+HY_BY
-    float sd[HY_BY + 2][32];   // differences f[j+1] - f[j], rows j0-2 .. j0+HY_BY-1
-    float sx[HY_BY][32];       // per-face exchange (QU, then el)
+    C sd[HY_BY + 2][32];      // differences f[j+1] - f[j], rows j0-2 .. j0+HY_BY-1
+    C sx[HY_BY][32];           // per-face exchange (QU, then el)
 };
 
-template <typename S, typename Epi = NoEpi, typename V = S>
+template <typename S, typename Epi = NoEpi, typename V = S, typename C = float>
 __device__ __forceinline__ void hpass_y_inc_body(const HPassArgs<S, V>& a, int bx, int by, int k, int tx, int ty,
-                                                 YIncSmem<S>& sm, const Epi& epi = Epi())
+                                                 YIncSmem<S, C>& sm, const Epi& epi = Epi())
 {
     auto& sf = sm.sf;
     auto& sd = sm.sd;
@@ -618,7 +580,7 @@ __device__ __forceinline__ void hpass_y_inc_body(const HPassArgs<S, V>& a, int b
 
     // face geometry
     const bool f_in = ain && iint && ja >= a.jlo - 1 && ja <= a.jhi;
-    float QU = 0.f, cfl = 0.f, ahd = 0.f;
+    C QU = C(0), cfl = C(0), ahd = C(0);
     bool up = false, uu_ok = false, act = false;
     if (f_in) {
         const long long q2 = (long long)ja * s + i;
@@ -626,33 +588,28 @@ __device__ __forceinline__ void hpass_y_inc_body(const HPassArgs<S, V>& a, int b
         if (act) {
             const int m_s = ja > 0 ? a.umask[q2 - s] : 0;
             const int m_n = ja + 1 < a.ny_ ? a.umask[q2 + s] : 0;
-            const float vv = inc_f<V>(a.u[base + ja * s]);
-            const float hvf = getm_d2f_approx(a.hu[base + ja * s]);
-            const float dxf = a.dy_f[q2], idyf = a.idx_f[q2];
-            QU = vv * hvf * dxf;
-            cfl = fabsf(vv * a.dtf * idyf);
-            up = vv > 0.f;
+            const C vv = hx_c<C>(a.u[base + ja * s]);
+            const C hvf = hx_c<C>(a.hu[base + ja * s]);
+            const C dxf = hx_dy<C>(a)[q2], idyf = hx_idx<C>(a)[q2];
+            QU = hx_mul3(vv, hvf, dxf);
+            cfl = hx_abs(hx_mul3(vv, hx_dt<C>(a), idyf));
+            up = hx_positive(vv);
             uu_ok = getm_flux_point(up ? m_s : m_n);
-            if (a.Ah) ahd = -getm_d2f_approx(a.Ah[q2]) * hvf * idyf * dxf;
+            if (a.Ah) ahd = hx_ahd(hx_c<C>(a.Ah[q2]), hvf, idyf, dxf);
         }
     }
     sx[ty][tx] = QU;
     __syncthreads();
-    const float QUn = ty + 1 < HY_BY ? sx[ty + 1][tx] : 0.f;  // north face of cell jb
+    const C QUn = ty + 1 < HY_BY ? sx[ty + 1][tx] : C(0);  // north face of cell jb
 
     const bool bin = ty < HY_STRIDE && icol && jb < a.ny_;
     const bool upd = bin && iint && jb >= a.jlo && jb <= a.jhi && a.tmask[(long long)jb * s + i] == 1;
-    float coef = 0.f;
+    C coef = C(0);
     double hnew = 0.0;
     if (bin) {
         const double hold = a.h_in[base + jb * s];
         hnew = hold;
-        if (upd) {
-            const float iaf = a.iA_f[(long long)jb * s + i];
-            const float dh = a.dtf * (QUn - QU) * iaf;
-            hnew = hold - getm_f2d(dh);
-            coef = a.dtf * iaf / (getm_d2f_approx(hold) - dh);
-        }
+        if (upd) hx_cell(hx_dt<C>(a), QUn, QU, hx_iA<C>(a)[(long long)jb * s + i], hold, hnew, coef);
         a.h_out[base + jb * s] = hnew;
     }
     // staging rows: thread row ty loads row ja (smem row ty + 1); rows 0-2
@@ -660,7 +617,7 @@ __device__ __forceinline__ void hpass_y_inc_body(const HPassArgs<S, V>& a, int b
     const int jx = ty == 0 ? j0 - 2 : j0 + HY_BY - 2 + ty;
     const int sxrow = ty == 0 ? 0 : HY_BY + ty;
     const bool xin = ty < 3 && icol && jx >= 0 && jx < a.ny_;
-    const TvdFaceF tf = getm_tvd_face_f(a.scheme, cfl);
+    const TvdFace<C> tf = hx_tvd(a.scheme, cfl, QU);
     for (int t = 0; t < a.ntracer; t++) {
         const S* __restrict__ f = a.fin[t] + base;
         __syncthreads();  // previous tracer's reads of sf, sd and sx are done
@@ -669,24 +626,19 @@ __device__ __forceinline__ void hpass_y_inc_body(const HPassArgs<S, V>& a, int b
         __syncthreads();
         // difference across this thread's face (smem row ty + 1 of sd); rows
         // 0 and 1 also form the differences below and above the block's faces
-        sd[ty + 1][tx] = inc_f<S>(sf[ty + 2][tx] - sf[ty + 1][tx]);
-        if (ty == 0) sd[0][tx] = inc_f<S>(sf[1][tx] - sf[0][tx]);
-        if (ty == 1) sd[HY_BY + 1][tx] = inc_f<S>(sf[HY_BY + 2][tx] - sf[HY_BY + 1][tx]);
+        sd[ty + 1][tx] = hx_c<C>(sf[ty + 2][tx] - sf[ty + 1][tx]);
+        if (ty == 0) sd[0][tx] = hx_c<C>(sf[1][tx] - sf[0][tx]);
+        if (ty == 1) sd[HY_BY + 1][tx] = hx_c<C>(sf[HY_BY + 2][tx] - sf[HY_BY + 1][tx]);
         __syncthreads();
-        const float dprev = sd[ty][tx], d = sd[ty + 1][tx], dnext = sd[ty + 2][tx];
+        const C dprev = sd[ty][tx], d = sd[ty + 1][tx], dnext = sd[ty + 2][tx];
         const S fb = sf[ty + 2][tx];
-        float el = 0.f, er = 0.f;
-        if (act) {
-            const float dev = hx_dev(tf, up, uu_ok, dprev, d, dnext);
-            const float fd = ahd * d;
-            el = QU * (up ? dev : d + dev) + fd;
-            er = QU * (up ? dev - d : dev) + fd;
-        }
+        C el = C(0), er = C(0);
+        if (act) hx_face(tf, up, uu_ok, QU, dprev, d, dnext, ahd, a.Ah != nullptr, el, er);
         sx[ty][tx] = el;
         __syncthreads();
-        const float el_n = ty + 1 < HY_BY ? sx[ty + 1][tx] : 0.f;
+        const C el_n = ty + 1 < HY_BY ? sx[ty + 1][tx] : C(0);
         if (bin) {
-            const S fn = upd ? inc_add<S>(fb, -coef * (el_n - er)) : fb;
+            const S fn = upd ? hx_new(fb, coef, el_n, er) : fb;
             a.fout[t][base + jb * s] = fn;
             if (t == 0) epi(base + jb * s, jb, (double)fn, hnew);
         }
@@ -705,7 +657,7 @@ __device__ __forceinline__ void hpass_y_inc_body(const HPassArgs<S, V>& a, int b
 // marched together, larger batches in groups of NT (the face geometry is
 // reloaded per group).
 
-template <typename S, int NT, typename V = S>
+template <typename S, int NT, typename V = S, typename C = float>
 __device__ __forceinline__ void hpass_y_march_body(const HPassArgs<S, V>& a, int bx, int chunk, int k, int lane,
                                                    int t0)
 {
@@ -734,25 +686,25 @@ __device__ __forceinline__ void hpass_y_march_body(const HPassArgs<S, V>& a, int
 
     // window at the first face j = jc0 - 1: rows j-1 .. j+1 and d(j-1), d(j)
     S fm1[NT], f0[NT], f1[NT];
-    float dm1[NT], d0[NT], er_s[NT];
+    C dm1[NT], d0[NT], er_s[NT];
 #pragma unroll
     for (int q = 0; q < NT; q++) {
         fm1[q] = rowv(f[q], jc0 - 2);
         f0[q] = rowv(f[q], jc0 - 1);
         f1[q] = rowv(f[q], jc0);
-        dm1[q] = inc_f<S>(f0[q] - fm1[q]);
-        d0[q] = inc_f<S>(f1[q] - f0[q]);
-        er_s[q] = 0.f;
+        dm1[q] = hx_c<C>(f0[q] - fm1[q]);
+        d0[q] = hx_c<C>(f1[q] - f0[q]);
+        er_s[q] = C(0);
     }
     int m_m = umask_at(jc0 - 2), m_0 = umask_at(jc0 - 1);
-    float QU_s = 0.f;
+    C QU_s = C(0);
     // every load of step j
     struct StepLoads {
         int m_1, tm;
         S f2[NT];
         V uraw;
         double huraw, hold;
-        float dxf, idyf, ahraw, iaf;
+        C dxf, idyf, ahraw, iaf;
     };
     auto load_step = [&](int j) -> StepLoads {
         StepLoads L;
@@ -762,12 +714,12 @@ __device__ __forceinline__ void hpass_y_march_body(const HPassArgs<S, V>& a, int
         const long long jr = (long long)((j >= 0 && j < a.ny_) ? j : 0) * s;
         L.uraw = a.u[base + jr];
         L.huraw = a.hu[base + jr];
-        L.dxf = a.dy_f[jr + ic];
-        L.idyf = a.idx_f[jr + ic];
-        L.ahraw = a.Ah ? getm_d2f_approx(a.Ah[jr + ic]) : 0.f;
+        L.dxf = hx_dy<C>(a)[jr + ic];
+        L.idyf = hx_idx<C>(a)[jr + ic];
+        L.ahraw = a.Ah ? hx_c<C>(a.Ah[jr + ic]) : C(0);
         L.hold = a.h_in[base + jr];
         L.tm = a.tmask[jr + ic];
-        L.iaf = a.iA_f[jr + ic];
+        L.iaf = hx_iA<C>(a)[jr + ic];
         return L;
     };
     // one tracer: prefetch a step ahead (more loads in flight per warp);
@@ -783,49 +735,41 @@ __device__ __forceinline__ void hpass_y_march_body(const HPassArgs<S, V>& a, int
         const long long jr = (long long)(jin ? j : 0) * s;
         const V uraw = cur.uraw;
         const double huraw = cur.huraw;
-        const float dxf = cur.dxf, idyf = cur.idyf, ahraw = cur.ahraw;
+        const C dxf = cur.dxf, idyf = cur.idyf, ahraw = cur.ahraw;
         const double hold = cur.hold;
         const int tm = cur.tm;
-        const float iaf = cur.iaf;
+        const C iaf = cur.iaf;
 
         // face j (between cells j and j+1)
         const bool f_in = jin && iint && j >= a.jlo - 1 && j <= a.jhi;
-        float QU = 0.f, cfl = 0.f, ahd = 0.f;
+        C QU = C(0), cfl = C(0), ahd = C(0);
         bool up = false, uu_ok = false, act = false;
         if (f_in) {
             act = getm_flux_point(m_0);
             if (act) {
-                const float vv = inc_f<V>(uraw);
-                const float hvf = getm_d2f_approx(huraw);
-                QU = vv * hvf * dxf;
-                cfl = fabsf(vv * a.dtf * idyf);
-                up = vv > 0.f;
+                const C vv = hx_c<C>(uraw);
+                const C hvf = hx_c<C>(huraw);
+                QU = hx_mul3(vv, hvf, dxf);
+                cfl = hx_abs(hx_mul3(vv, hx_dt<C>(a), idyf));
+                up = hx_positive(vv);
                 uu_ok = getm_flux_point(up ? m_m : m_1);
-                if (a.Ah) ahd = -ahraw * hvf * idyf * dxf;
+                if (a.Ah) ahd = hx_ahd(ahraw, hvf, idyf, dxf);
             }
         }
         // cell j: south face j-1 (previous step), north face j (this step)
         const bool upd_cell = j >= jc0 && iint && j >= a.jlo && j <= a.jhi && tm == 1;
-        float coef = 0.f;
+        C coef = C(0);
         double hnew = hold;
-        if (upd_cell) {
-            const float dh = a.dtf * (QU - QU_s) * iaf;
-            hnew = hold - getm_f2d(dh);
-            coef = a.dtf * iaf / (getm_d2f_approx(hold) - dh);
-        }
+        if (upd_cell) hx_cell(hx_dt<C>(a), QU, QU_s, iaf, hold, hnew, coef);
         if (j >= jc0 && icol && first_group) a.h_out[base + jr] = hnew;
-        const TvdFaceF tf = getm_tvd_face_f(a.scheme, cfl);
+        const TvdFace<C> tf = hx_tvd(a.scheme, cfl, QU);
 #pragma unroll
         for (int q = 0; q < NT; q++) {
-            const float d1 = inc_f<S>(f2[q] - f1[q]);
-            float el = 0.f, er = 0.f;
-            if (act) {
-                const float dev = hx_dev(tf, up, uu_ok, dm1[q], d0[q], d1);
-                const float fd = ahd * d0[q];
-                el = QU * (up ? dev : d0[q] + dev) + fd;
-                er = QU * (up ? dev - d0[q] : dev) + fd;
-            }
-            if (j >= jc0 && icol && q < nt) fo[q][jr] = upd_cell ? inc_add<S>(f0[q], -coef * (el - er_s[q])) : f0[q];
+            const C d1 = hx_c<C>(f2[q] - f1[q]);
+            C el = C(0), er = C(0);
+            if (act)
+                hx_face(tf, up, uu_ok, QU, dm1[q], d0[q], d1, ahd, a.Ah != nullptr, el, er);
+            if (j >= jc0 && icol && q < nt) fo[q][jr] = upd_cell ? hx_new(f0[q], coef, el, er_s[q]) : f0[q];
             er_s[q] = er;
             fm1[q] = f0[q]; f0[q] = f1[q]; f1[q] = f2[q];
             dm1[q] = d0[q]; d0[q] = d1;

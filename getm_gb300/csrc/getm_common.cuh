@@ -233,6 +233,56 @@ __device__ __forceinline__ double getm_div_refined(double num, double den)
     return fma(fma(-q0, den, num), r, q0);
 }
 
+// 1 / x in FP64 to within two units in the last place, from six instructions
+// of which three are FP64: a float reciprocal r (relative error e below 2^-21)
+// and one third-order Householder step, r (1 + e + e^2), whose own error is
+// e^3.  GB300 runs FP64 at 1/64 of its float rate and the correctly rounded
+// division takes about four times as many FP64 instructions, so this serves
+// where a quotient only scales an increment.  x zero, not finite or outside
+// the normal float range: the correctly rounded division, out of line.
+static __device__ __noinline__ double getm_rcp_hw(double x) { return 1.0 / x; }
+
+__device__ __forceinline__ double getm_rcp(double x)
+{
+    const float xf = getm_d2f_approx(x);
+    const float ax = fabsf(xf);
+    if (!(ax > 1e-30f && ax < 1e30f)) return getm_rcp_hw(x);
+    float rf;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rf) : "f"(xf));
+    const double r = getm_f2d(rf);
+    const double e = __fma_rn(-x, r, 1.0);
+    return __fma_rn(r, __fma_rn(e, e, e), r);
+}
+
+// 2 x on the integer pipe (exact; zeros, subnormals, infinities, NaNs and
+// overflow take the FP64 sum out of line)
+static __device__ __noinline__ double getm_twice_hw(double x) { return x + x; }
+
+__device__ __forceinline__ double getm_twice(double x)
+{
+    const long long b = __double_as_longlong(x);
+    const int e = (int)((b >> 52) & 0x7ff);
+    if (e > 0 && e < 0x7fe) return __longlong_as_double(b + (1ll << 52));
+    return (b << 1) == 0 ? x : getm_twice_hw(x);
+}
+
+// x, negated where neg is set, on the integer pipe
+__device__ __forceinline__ double getm_negate_if(double x, bool neg)
+{
+    return __longlong_as_double(__double_as_longlong(x) ^ ((long long)neg << 63));
+}
+
+// min and max of non-negative doubles (their bit patterns order as integers)
+__device__ __forceinline__ double getm_min_pos(double a, double b)
+{
+    return __double_as_longlong(a) < __double_as_longlong(b) ? a : b;
+}
+
+__device__ __forceinline__ double getm_max_pos(double a, double b)
+{
+    return __double_as_longlong(a) > __double_as_longlong(b) ? a : b;
+}
+
 // True for the mixed form's float bulk type.  Its update kernels use the
 // increment form x_new = x_old + dx, with dx formed from small differences,
 // so a field that does not change is reproduced exactly and float32 rounding
@@ -317,23 +367,25 @@ __device__ __forceinline__ T getm_tvd_dev(int scheme, T fuu, T fu, T fd, T cfl)
     return getm_tvd_dev_d<T>(scheme, fd - fu, fu - fuu, cfl);
 }
 
-// Float form of the limited deviation without a division per field.  For
-// deltaf and deltafu of the same sign s, phi(r) deltaf with r = deltafu /
-// deltaf equals s phi_a(a, b), a = |deltaf|, b = |deltafu|, where phi_a is
-// the limiter's expression with r replaced by b and every constant term
-// multiplied by a (all five limiters are piecewise linear in r).  The terms
-// that depend only on the Courant number are formed once per face
-// (getm_tvd_face_f) and shared by every field advected through the face.
-struct TvdFaceF {
+// The limited deviation without a division per field (C: float for the mixed
+// form, double for the FP64 form).  For deltaf and deltafu of the same sign s,
+// phi(r) deltaf with r = deltafu / deltaf equals s phi_a(a, b), a = |deltaf|,
+// b = |deltafu|, where phi_a is the limiter's expression with r replaced by b
+// and every constant term multiplied by a (all five limiters are piecewise
+// linear in r).  The terms that depend only on the Courant number are formed
+// once per face (getm_tvd_face_c) and shared by every field advected through
+// the face.
+template <typename C>
+struct TvdFace {
     int scheme;
-    float half1mc;     // 0.5 (1 - cfl)
-    float lin0, lin1;  // HSIMT, P2_PDM: phi = lin0 + lin1 r
-    float rcoef, cap;  // P2_PDM: 2 / (cfl + 1e-10), 2 / (1 - cfl)
+    C half1mc;     // 0.5 (1 - cfl)
+    C lin0, lin1;  // HSIMT, P2_PDM: phi = lin0 + lin1 r
+    C rcoef, cap;  // P2_PDM: 2 / (cfl + 1e-10), 2 / (1 - cfl)
 };
 
-__device__ __forceinline__ TvdFaceF getm_tvd_face_f(int scheme, float cfl)
+__device__ __forceinline__ TvdFace<float> getm_tvd_face_c(int scheme, float cfl)
 {
-    TvdFaceF f;
+    TvdFace<float> f;
     f.scheme = scheme;
     f.half1mc = 0.5f * (1.f - cfl);
     f.lin0 = f.lin1 = 0.f;
@@ -353,7 +405,31 @@ __device__ __forceinline__ TvdFaceF getm_tvd_face_f(int scheme, float cfl)
     return f;
 }
 
-__device__ __forceinline__ float getm_tvd_dev_f(const TvdFaceF& tf, float deltaf, float deltafu)
+// FP64: every product and sum rounded as written (no contraction), so that
+// all kernels that share these functions give the same bits.
+__device__ __forceinline__ TvdFace<double> getm_tvd_face_c(int scheme, double cfl)
+{
+    TvdFace<double> f;
+    f.scheme = scheme;
+    f.half1mc = __fma_rn(-0.5, cfl, 0.5);
+    f.lin0 = f.lin1 = 0.0;
+    f.rcoef = f.cap = 2.0;
+    if (scheme == GETM_SCHEME_HSIMT) {
+        const double kappa = __dadd_rn(1.0, -cfl);
+        const double x = __dmul_rn(0.25, __fma_rn(-1.0 / 3.0, getm_rcp(kappa), kappa));
+        f.lin0 = __dadd_rn(0.5, x);
+        f.lin1 = __dadd_rn(0.5, -x);
+    } else if (scheme == GETM_SCHEME_P2_PDM) {
+        const double x = __fma_rn(-1.0 / 3.0, cfl, 1.0 / 6.0);
+        f.lin0 = __dadd_rn(0.5, x);
+        f.lin1 = __dadd_rn(0.5, -x);
+        f.rcoef = __dmul_rn(2.0, getm_rcp(__dadd_rn(cfl, 1.e-10)));
+        f.cap = __dmul_rn(2.0, getm_rcp(__dadd_rn(1.0, -cfl)));
+    }
+    return f;
+}
+
+__device__ __forceinline__ float getm_tvd_dev_c(const TvdFace<float>& tf, float deltaf, float deltafu)
 {
     if (!(deltaf * deltafu > 0.f)) return 0.f;
     const float a = fabsf(deltaf), b = fabsf(deltafu);
@@ -367,6 +443,45 @@ __device__ __forceinline__ float getm_tvd_dev_f(const TvdFaceF& tf, float deltaf
     default: pa = 0.f; break;
     }
     return tf.half1mc * copysignf(pa, deltaf);
+}
+
+// FP64: the limited difference phi(r) deltaf itself, without the factor
+// half1mc; signs, doublings, minima and maxima on the integer pipe (superbee
+// needs no FP64 instruction at all).  The sign test is that of deltaf *
+// deltafu > 0 (false for NaN); where one of them is zero every limiter gives
+// zero.
+__device__ __forceinline__ double getm_tvd_phi(const TvdFace<double>& tf, double deltaf, double deltafu)
+{
+    const long long bd = __double_as_longlong(deltaf), bu = __double_as_longlong(deltafu);
+    const long long ia = bd & 0x7fffffffffffffffll, ib = bu & 0x7fffffffffffffffll;
+    if ((bd ^ bu) < 0 || ia > 0x7ff0000000000000ll || ib > 0x7ff0000000000000ll) return 0.0;
+    const double a = __longlong_as_double(ia), b = __longlong_as_double(ib);
+    double pa;
+    switch (tf.scheme) {
+    case GETM_SCHEME_HSIMT: {
+        const double lin = __fma_rn(tf.lin1, b, __dmul_rn(tf.lin0, a));
+        pa = getm_min_pos(getm_min_pos(getm_twice(b), getm_positive_i(lin) ? lin : 0.0), getm_twice(a));
+        break;
+    }
+    case GETM_SCHEME_MUSCL:
+        pa = getm_min_pos(getm_min_pos(getm_twice(b), getm_half(__dadd_rn(a, b))), getm_twice(a));
+        break;
+    case GETM_SCHEME_P2_PDM:
+        if (ia == 0 || ib == 0) return 0.0;  // its bounds may be negative beyond Courant numbers of 1
+        pa = getm_fmin_i(getm_fmin_i(__dmul_rn(tf.rcoef, b), __fma_rn(tf.lin1, b, __dmul_rn(tf.lin0, a))),
+                         __dmul_rn(tf.cap, a));
+        break;
+    case GETM_SCHEME_SPLMAX13:
+        pa = getm_min_pos(getm_min_pos(getm_twice(b),
+                                       __dmul_rn(1.0 / 3.0, __dadd_rn(__dadd_rn(a, b), getm_max_pos(a, b)))),
+                          getm_twice(a));
+        break;
+    case GETM_SCHEME_SUPERBEE:
+        pa = getm_max_pos(getm_min_pos(getm_twice(b), a), getm_min_pos(b, getm_twice(a)));
+        break;
+    default: return 0.0;
+    }
+    return __longlong_as_double(__double_as_longlong(pa) ^ (bd & (long long)0x8000000000000000ull));
 }
 
 __device__ __forceinline__ bool getm_flux_point(int m) { return m == 1 || m == 2; }

@@ -71,15 +71,12 @@ struct SubstepArgs {
     unsigned* sync;              // [0] barrier arrivals, [1] blocks done, [2] error
 };
 
-static_assert(SS_BY == GETM_V_BY && SS_BY == HY_BY, "the y passes run on the kernel's 32 x 16 blocks");
+static_assert(SS_BY == HY_BY, "the y passes run on the kernel's 32 x 16 blocks");
 
 union SubstepSmem {
     double szh[SS_BY + 2][UD_BX + 2];
-    struct {
-        double sQ[GETM_V_BY][32];
-        double sF[GETM_V_BY][32];
-    } y;
-    YIncSmem<double> yi;
+    YIncSmem<double, float> yf;   // mixed form
+    YIncSmem<double, double> yd;  // FP64 form
 };
 
 __device__ __forceinline__ unsigned ld_acquire(const unsigned* p)
@@ -159,8 +156,9 @@ template <bool MIXED, typename Epi = NoEpi>
 __device__ __forceinline__ void advection_pass(const HPassArgs<double>& pa, int dir, SubstepSmem& sm, int tx,
                                                int ty, const Epi& epi = Epi())
 {
+    using C = typename std::conditional<MIXED, float, double>::type;
     if (dir == 1) {
-        const int nbx = MIXED ? div_up(pa.nx_ + 1, HX_STRIDE) : div_up(pa.nx_, 32);
+        const int nbx = div_up(pa.nx_ + 1, HX_STRIDE);
         const long long items = (long long)nbx * pa.ny_;
         // equal contiguous runs of row segments per block (every SM busy)
         const long long per = (items + gridDim.x - 1) / gridDim.x;
@@ -168,15 +166,14 @@ __device__ __forceinline__ void advection_pass(const HPassArgs<double>& pa, int 
         for (long long w = wb + ty; w < we; w += SS_BY) {
             const int bx = (int)(w % nbx);
             const long long row = w / nbx;
-            if constexpr (MIXED) hpass_x_inc_body<double, Epi>(pa, bx, row, tx, epi);
-            else hpass_x_body<double, Epi>(pa, bx, row, tx, epi);
+            hpass_x_inc_body<double, Epi, double, C>(pa, bx, row, tx, epi);
         }
     } else {
         const int nbx = div_up(pa.nx_, 32);
-        const int nby = MIXED ? div_up(pa.ny_ + 1, HY_STRIDE) : div_up(pa.ny_, GETM_V_BY);
+        const int nby = div_up(pa.ny_ + 1, HY_STRIDE);
         for (int t = blockIdx.x; t < nbx * nby; t += gridDim.x) {
-            if constexpr (MIXED) hpass_y_inc_body<double, Epi>(pa, t % nbx, t / nbx, 0, tx, ty, sm.yi, epi);
-            else hpass_y_body<double, Epi>(pa, t % nbx, t / nbx, 0, tx, ty, sm.y.sQ, sm.y.sF, epi);
+            if constexpr (MIXED) hpass_y_inc_body<double, Epi, double, float>(pa, t % nbx, t / nbx, 0, tx, ty, sm.yf, epi);
+            else hpass_y_inc_body<double, Epi, double, double>(pa, t % nbx, t / nbx, 0, tx, ty, sm.yd, epi);
             __syncthreads();  // shared memory is reused by the next tile
         }
     }
@@ -470,11 +467,11 @@ template <bool MIXED>
 void pass_items(const HPassArgs<double>& pa, int dir, int& items, int& nbx)
 {
     if (dir == 1) {
-        nbx = MIXED ? sb_div_up(pa.nx_ + 1, HX_STRIDE) : sb_div_up(pa.nx_, 32);
+        nbx = sb_div_up(pa.nx_ + 1, HX_STRIDE);
         items = nbx * sb_div_up(pa.ny_, SS_BY);
     } else {
         nbx = sb_div_up(pa.nx_, 32);
-        const int nby = MIXED ? sb_div_up(pa.ny_ + 1, HY_STRIDE) : sb_div_up(pa.ny_, GETM_V_BY);
+        const int nby = sb_div_up(pa.ny_ + 1, HY_STRIDE);
         items = nbx * nby;
     }
 }
@@ -494,15 +491,13 @@ template <bool MIXED, typename Epi = NoEpi>
 __device__ __forceinline__ void batch_pass_item(const HPassArgs<double>& pa, int dir, int nbx, int q, SubstepSmem& sm,
                                                 int tx, int ty, const Epi& epi = Epi())
 {
+    using C = typename std::conditional<MIXED, float, double>::type;
     if (dir == 1) {
         const long long row = (long long)(q / nbx) * SS_BY + ty;
-        if (row < pa.ny_) {
-            if constexpr (MIXED) hpass_x_inc_body<double, Epi>(pa, q % nbx, row, tx, epi);
-            else hpass_x_body<double, Epi>(pa, q % nbx, row, tx, epi);
-        }
+        if (row < pa.ny_) hpass_x_inc_body<double, Epi, double, C>(pa, q % nbx, row, tx, epi);
     } else {
-        if constexpr (MIXED) hpass_y_inc_body<double, Epi>(pa, q % nbx, q / nbx, 0, tx, ty, sm.yi, epi);
-        else hpass_y_body<double, Epi>(pa, q % nbx, q / nbx, 0, tx, ty, sm.y.sQ, sm.y.sF, epi);
+        if constexpr (MIXED) hpass_y_inc_body<double, Epi, double, float>(pa, q % nbx, q / nbx, 0, tx, ty, sm.yf, epi);
+        else hpass_y_inc_body<double, Epi, double, double>(pa, q % nbx, q / nbx, 0, tx, ty, sm.yd, epi);
         __syncthreads();  // shared memory is reused by the block's next item
     }
 }

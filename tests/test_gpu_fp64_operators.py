@@ -1,0 +1,67 @@
+"""FP64 operators at the sizes where their kernels can go wrong: rows and
+columns around the 31-cell segments and 15-row tiles of the horizontal passes,
+batches around the field groups, land that holds NaN.
+
+Tolerance: a directional pass rounds at most about five times per cell in
+either order of evaluation (u = 1.1e-16 each, weights at most one, h/hnew
+below 1.2), five passes make some 30 u; 1e-14 is 90 u of the field's largest
+value."""
+
+import numpy as np
+import pytest
+
+from tests.gpu_helpers import host
+from tests.test_gpu_operators import close, setup, velocity, wrap
+
+pytestmark = pytest.mark.gpu
+RTOL = 1e-14
+
+
+@pytest.mark.parametrize("nx,ny,nz,nt,scheme", [(3, 3, 2, 1, 5), (26, 10, 3, 2, 1), (27, 11, 1, 3, 2), (28, 12, 4, 1, 3),
+                                                (58, 26, 5, 5, 4), (59, 27, 2, 33, 5), (89, 41, 3, 2, 6)])
+def test_split_at_tile_edges(nx, ny, nz, nt, scheme):
+    import oracle.oracle as O
+    from getm_gb300 import operators
+    from getm_gb300.core import CENTERS, INTERFACES
+
+    Th, To, Td, rng = setup(nz=nz, seed=nx, nx=nx, ny=ny)
+    u, v = velocity(Th.ugrid, rng, nz, 0.3), velocity(Th.vgrid, rng, nz, 0.3)
+    w = rng.uniform(-5e-4, 5e-4, (nz + 1, Th.ny_, Th.nx_))
+    w[0] = w[-1] = 0.0
+    tr = [rng.uniform(5.0, 10.0, (nz, Th.ny_, Th.nx_)) for _ in range(nt)]
+    ah = [rng.uniform(0, 50.0, (Th.ny_, Th.nx_)) for _ in range(2)] if nt > 1 else [None, None]
+    for t in tr:
+        t[:, Th.mask == 0] = np.nan
+    ao = O.Advection(To, scheme)
+    tro = [t.copy() for t in tr]
+    ao.apply_3d_batch(u, v, w, 600.0, tro, Ah_u=ah[0], Ah_v=ah[1])
+    ad = operators.Advection(Td, operators.AdvectionScheme(scheme))
+    trd = [wrap(Td, t, CENTERS) for t in tr]
+    ad.apply_3d_batch(wrap(Td.ugrid, u, CENTERS), wrap(Td.vgrid, v, CENTERS), wrap(Td, w, INTERFACES), 600.0, trd,
+                      Ah_u=None if ah[0] is None else wrap(Td.ugrid, ah[0], False),
+                      Ah_v=None if ah[1] is None else wrap(Td.vgrid, ah[1], False))
+    water = Th.mask != 0
+    for a, b in zip(trd, tro):
+        got = host(a.all_values)
+        assert np.isnan(got[:, ~water]).all()
+        close(got, b, rtol=RTOL, mask=water)
+    close(host(ad.h), ao.h, rtol=RTOL)
+
+
+@pytest.mark.parametrize("nx,ny", [(3, 3), (27, 11), (58, 26)])
+@pytest.mark.parametrize("split", [1, 2, 3])
+def test_plane_split_at_tile_edges(nx, ny, split):
+    import oracle.oracle as O
+    from getm_gb300 import operators
+
+    Th, To, Td, rng = setup(nz=1, seed=ny, nx=nx, ny=ny)
+    u, v = velocity(Th.ugrid, rng, 1, 0.3)[0], velocity(Th.vgrid, rng, 1, 0.3)[0]
+    t = rng.uniform(5.0, 10.0, (Th.ny_, Th.nx_))
+    ao = O.Advection(To, 5, O.AdvectionSplit(split))
+    to = t.copy()
+    ao(u, v, 600.0, to)
+    ad = operators.Advection(Td, operators.AdvectionScheme(5), operators.AdvectionSplit(split))
+    td = wrap(Td, t, False)
+    ad(wrap(Td.ugrid, u, False), wrap(Td.vgrid, v, False), 600.0, td)
+    close(host(td.all_values), to, rtol=RTOL)
+    close(host(ad.D), ao.D, rtol=RTOL)
