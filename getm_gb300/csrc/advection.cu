@@ -20,10 +20,11 @@
 // * y-direction: blocks of 32 x 16 threads cover 15 rows with the faces
 //   exchanged through shared memory, or (float arithmetic, several layers)
 //   warps march north with the rows in registers.
-// * Vertical pass: one thread per water column, sweeping k with a register
-//   window (the per-column update is in place, as in the reference).  The
-//   adaptive sub-stepping (itersmax = 200, restart semantics of
-//   template :286-368) runs through handle-owned column work arrays.
+// * Vertical pass: a warp's lanes are 32 water columns; each thread sweeps k
+//   with a register window, the whole column or (few columns) a segment of it.
+//   The per-column update is in place, as in the reference.  The adaptive
+//   sub-stepping (itersmax = 200, restart semantics of template :286-368) runs
+//   through handle-owned column work arrays.
 #include <stdlib.h>
 #include <string.h>
 
@@ -385,222 +386,295 @@ struct WPassArgs {
     T* f[GETM_MAX_BATCH];       // updated in place
 };
 
-// One sub-step over a column: reads (hs, fs) levels 0..nz-1 (C), writes
-// (hd, fdst).  hs == hd / fs == fdst (in place) is allowed: every level is
-// read into the register window before it is overwritten.  The Courant number
-// |w_var| dt / min(h) * itersm1 equals cfls(k)*itersm1 of the reference
-// (cfls = |w_var| dt / min(haux), haux = the sub-step's start thickness).
-template <typename T>
-__device__ void w_substep(const WPassArgs<T>& a, long long c, const T* wv, const double* hs, const T* fs,
-                          double* hd, T* fdst, double dtk, double itersm1)
-{
-    const long long P = a.plane;
-    const int nz = a.nz;
-    T fkm1 = T(0), fk = fs[c], fk1 = (nz > 1) ? fs[c + P] : T(0);
-    double hk = hs[c], hk1 = (nz > 1) ? hs[c + P] : 0.0;
-    T fluxm = T(0);  // flux(k-1), flux(0) = 0
-    T wkm1 = a.w[c];
-    for (int k = 0; k < nz; k++) {
-        // flux through the interface above C level k (Fortran interface k+1)
-        T flux = T(0);
-        T fk2 = T(0);
-        double hk2 = 0.0;
-        if (k + 2 < nz) { fk2 = fs[c + (k + 2) * P]; hk2 = hs[c + (k + 2) * P]; }
-        if (k < nz - 1) {
-            T wvk = wv[c + (k + 1) * P];
-            T cfl = fabs(wvk) * (T)a.dt / (T)fmin(hk, hk1) * (T)itersm1;
-            T fu, fuu, fdn;
-            if (wvk > T(0)) {
-                fu = fk;
-                fuu = (k > 0) ? fkm1 : fu;
-                fdn = fk1;
-            } else {
-                fu = fk1;
-                fuu = (k < nz - 2) ? fk2 : fu;
-                fdn = fk;
-            }
-            fu = getm_tvd_face<T>(a.scheme, fuu, fu, fdn, cfl);
-            flux = wvk * fu;
-        }
-        T wk = a.w[c + (k + 1) * P];
-        double dh = dtk * ((double)wk - (double)wkm1);
-        double hn = hk - dh;
-        T advn = flux - fluxm;
-        hd[c + k * P] = hn;
-        T hfo = (T)hk * fk;
-        fdst[c + k * P] = (hfo - (T)dtk * advn) / (T)hn;
-        // shift window
-        fluxm = flux; wkm1 = wk;
-        fkm1 = fk; fk = fk1; fk1 = fk2;
-        hk = hk1; hk1 = hk2;
-    }
-}
-
-// Mixed form of w_substep: the increment form of the horizontal passes in
-// the vertical (see hpass_x_inc_kernel).  With flux_k = W_k f + e_k at the
-// interface above level k (W_k = w_var there, 0 at the surface) and
-// dh = dtk (w_k - w_{k-1}), the reference update equals
+// The pass is explicit: every level's new value depends only on old values of
+// the levels around it.  So on domains with few columns (w_segments) a
+// column's levels are shared by several warps, each sweeping a segment k0 ..
+// k1-1 upwards; a segment's sweep runs in place: it reads its own levels before
+// it overwrites them, and the values of its neighbours' levels that it needs
+// (WHalo) are read before a block barrier, after which all segments write.
+//
+// One sub-step is in increment form (see hpass_x_inc_rows).  With flux_k =
+// W_k f + e_k at the interface above level k (W_k = w_var there, 0 at the
+// surface) and dh = dtk (w_k - w_{k-1}), the reference update equals
 //     f + dtk ((w_k - W_k - w_{k-1} + W_{k-1}) f - e_k + e'_{k-1}) / hn
 // with e_k = W_k (face_k - f_k) and e'_{k-1} = W_{k-1} (face_{k-1} - f_k).
-// NT fields advected with the same w_var share every thickness and velocity
-// load and the face constants; each field keeps its own window.
-// The operands of the levels a column sweep will need are staged W_STAGE
-// levels ahead into a per-thread ring in shared memory by asynchronous
-// copies (cp.async): the loads of W_STAGE levels are in flight without
-// holding registers, where register prefetch reached two levels.  Each
-// thread reads back only the slots it filled, so no block barrier is
-// involved; a slot is refilled only after its level was read.
+// The Courant number |w_var| dt / min(h) * itersm1 equals cfls(k)*itersm1 of
+// the reference (cfls = |w_var| dt / min(haux), haux = the sub-step's start
+// thickness).  NT fields advected with the same w_var share every thickness
+// and velocity load and the face constants; each field keeps its own window.
+// V: the velocities and the arithmetic, float (mixed form) or double.  The
+// FP64 form takes 13 FP64 instructions per level and 6 per field and level
+// (superbee, w_var = w) where the reference's order of evaluation, with its
+// five divisions, took about 140.  One thread per column in that order took
+// 134 us on 120 x 100 x 30 with one field and 672 us on 173 x 131 x 23 with six
+// (HSIMT); this form takes 41 us and 199 us.
+//
+// The operands of the levels a sweep will need are staged W_STAGE levels
+// ahead into a per-thread ring in shared memory by asynchronous copies
+// (cp.async): the loads of W_STAGE levels are in flight without holding
+// registers.  Each thread reads back only the slots it filled, so no block
+// barrier is involved; a slot is refilled only after its level was read.
 constexpr int W_STAGE = 6;
 constexpr int W_RING = W_STAGE + 1;
+constexpr int W_MAXSEG = 8;
 
-template <typename S>
+// With SEG the two slots after the ring hold the old values of the two levels
+// above the segment.
+template <bool SEG>
+constexpr int w_slots = SEG ? W_RING + 2 : W_RING;
+
+// A warp's ring in the block's dynamic shared memory: h, f, w_var and w of its
+// 32 columns, one behind the other at fixed offsets (widest types first, so
+// every slot is naturally aligned; one pointer for all four).
+extern __shared__ __align__(16) unsigned char w_smem[];
+
+template <bool SEG, typename S, typename V>
 struct WRing {
-    double* h;  // h of level L at h[(L % W_RING) * 32]
-    S* f;       // field q of level L at f[((L % W_RING) * 2 + q) * 32]
-    float* W;   // the field's vertical velocity (w_var) of level L
-    float* w;   // w of level L (nz + 1 interfaces)
+    static_assert(sizeof(S) == 8 || sizeof(S) == sizeof(V), "fields in double or in the velocities' type");
+    static constexpr size_t OFF_F = (size_t)w_slots<SEG> * 32 * sizeof(double);
+    static constexpr size_t OFF_W = OFF_F + (size_t)w_slots<SEG> * 64 * sizeof(S);
+    static constexpr size_t OFF_w = OFF_W + (size_t)W_RING * 32 * sizeof(V);
+    static constexpr size_t BYTES = OFF_w + (size_t)W_RING * 32 * sizeof(V);
+    int o8, oV;  // the lane's byte offsets of h and of w_var
+    __device__ __forceinline__ WRing(int warp, int lane)
+        : o8(warp * (int)BYTES + lane * 8), oV(warp * (int)BYTES + (int)OFF_W + lane * (int)sizeof(V))
+    {
+    }
+    __device__ __forceinline__ double& h(int slot) const { return *reinterpret_cast<double*>(w_smem + o8 + slot * 256); }
+    __device__ __forceinline__ S& f(int slot, int q) const
+    {
+        constexpr int n = sizeof(S);
+        const int o = n == 8 ? o8 : oV - (int)(OFF_W - OFF_F);  // (V is as wide as a narrow S)
+        return *reinterpret_cast<S*>(w_smem + o + (n == 8 ? (int)OFF_F : 0) + (slot * 2 + q) * 32 * n);
+    }
+    __device__ __forceinline__ V& W(int slot) const
+    {
+        return *reinterpret_cast<V*>(w_smem + oV + slot * 32 * (int)sizeof(V));
+    }
+    __device__ __forceinline__ V& w(int slot) const
+    {
+        return *reinterpret_cast<V*>(w_smem + oV + (int)(OFF_w - OFF_W) + slot * 32 * (int)sizeof(V));
+    }
 };
 
-template <typename S>
-constexpr size_t w_ring_bytes_per_thread()
-{
-    return (size_t)W_RING * (sizeof(double) + 2 * sizeof(S) + 2 * sizeof(float));
-}
-
-// the ring of thread (lane, warp) in the block's dynamic shared memory
-// (doubles first, so every slot is naturally aligned)
-template <typename S>
-__device__ __forceinline__ WRing<S> w_ring(unsigned char* smem, int nwarps, int warp, int lane)
-{
-    WRing<S> r;
-    double* hb = reinterpret_cast<double*>(smem);
-    S* fb = reinterpret_cast<S*>(hb + (size_t)nwarps * W_RING * 32);
-    float* Wb = reinterpret_cast<float*>(fb + (size_t)nwarps * W_RING * 64);
-    float* wb = Wb + (size_t)nwarps * W_RING * 32;
-    r.h = hb + (size_t)warp * W_RING * 32 + lane;
-    r.f = fb + (size_t)warp * W_RING * 64 + lane;
-    r.W = Wb + (size_t)warp * W_RING * 32 + lane;
-    r.w = wb + (size_t)warp * W_RING * 32 + lane;
-    return r;
-}
-
+// Old values beside a segment, zero where the column ends: levels k0-2 and
+// k0-1; those of levels k1 and k1+1 go to the thread's two slots after the ring.
 template <int NT, typename S>
-__device__ void w_substep_inc(const WPassArgs<S, float>& a, long long c, const float* wv, const double* hs,
-                              const S* const (&fs)[NT], double* hd, S* const (&fdst)[NT], double dtk,
-                              double itersm1, const WRing<S>& ring)
+struct WHalo {
+    S lo2[NT], lo1[NT];
+    double hlo;
+};
+
+template <int NT, typename S, typename V>
+__device__ __forceinline__ WHalo<NT, S> w_halo(long long c, long long P, int nz, int k0, int k1, const double* hs,
+                                               const S* const (&fs)[NT], const WRing<true, S, V>& ring)
+{
+    WHalo<NT, S> H;
+#pragma unroll
+    for (int q = 0; q < NT; q++) {
+        H.lo2[q] = k0 >= 2 ? fs[q][c + (k0 - 2) * P] : S(0);
+        H.lo1[q] = k0 >= 1 ? fs[q][c + (k0 - 1) * P] : S(0);
+        ring.f(W_RING, q) = k1 < nz ? fs[q][c + k1 * P] : S(0);
+        ring.f(W_RING + 1, q) = k1 + 1 < nz ? fs[q][c + (k1 + 1) * P] : S(0);
+    }
+    H.hlo = k0 >= 1 ? hs[c + (k0 - 1) * P] : 0.0;
+    ring.h(W_RING) = k1 < nz ? hs[c + k1 * P] : 0.0;
+    ring.h(W_RING + 1) = 0.0;  // (beyond the last interface: not used)
+    return H;
+}
+
+// e_k and e'_k of the interface between two levels of thickness h0 (below)
+// and h1, per field: tf and W are the interface's, d the difference across it,
+// dprev and dnext those below and above
+__device__ __forceinline__ void w_face(const TvdFace<float>& tf, float W, float dprev, float d, float dnext, float& el,
+                                       float& er)
+{
+    // the limiter is odd: one evaluation for both flow directions
+    const bool up = W > 0.f;
+    const float lim = getm_tvd_dev_c(tf, d, up ? dprev : dnext);
+    const float dev = up ? lim : -lim;
+    const float a = __fadd_rn(dev, up ? -d : d);
+    el = __fmul_rn(W, up ? dev : a);
+    er = __fmul_rn(W, up ? a : dev);
+}
+
+__device__ __forceinline__ void w_face(const TvdFace<double>& tf, double W, double dprev, double d, double dnext,
+                                       double& el, double& er)
+{
+    hx_face(tf, getm_positive_i(W), true, W, dprev, d, dnext, 0.0, false, el, er);
+}
+
+__device__ __forceinline__ TvdFace<float> w_tvd(int scheme, float W, float dt, float itersm1, float h0, float h1)
+{
+    const float cfl = fabsf(W) * dt / fminf(h0, h1) * itersm1;
+    return getm_tvd_face_c(scheme, cfl);
+}
+
+__device__ __forceinline__ TvdFace<double> w_tvd(int scheme, double W, double dt, double itersm1, double h0, double h1)
+{
+    const double cfl = __dmul_rn(__dmul_rn(fabs(W), __dmul_rn(dt, itersm1)), getm_rcp(getm_fmin_i(h0, h1)));
+    return hx_tvd(scheme, cfl, W);
+}
+
+// SEG: the column is split (else k0 = 0, k1 = nz, and nothing lies beside it).
+template <int NT, bool SEG, typename S, typename V>
+__device__ void w_substep(const WPassArgs<S, V>& a, long long c, int kbeg, int kend, const V* wv, const double* hs,
+                          const S* const (&fs)[NT], double* hd, S* const (&fdst)[NT], double dtk, double itersm1,
+                          const WHalo<NT, S>& H, const WRing<SEG, S, V>& ring)
 {
     const long long P = a.plane;
     const int nz = a.nz;
-    const float dtkf = (float)dtk, itf = (float)itersm1, dtf = (float)a.dt;
-    S fk[NT], fk1[NT];
-    float erm[NT];  // erm: e'_{k-1}, interface below, deviation from level k
+    const int k0 = SEG ? kbeg : 0, k1 = SEG ? kend : nz;
+    const V dtkf = (V)dtk, itf = (V)itersm1, dtf = (V)a.dt;
+    const bool own_w = wv == a.w;
     // the differences f[k+1] - f[k] (dk) and f[k] - f[k-1] (dkm1), narrowed:
     // each is formed once, as the level above's is needed next (the
     // downwind-side difference f[k+1] - f[k+2] is -(f[k+2] - f[k+1]), the
     // same bits up to the sign of a zero, which the limiter ignores)
-    float dk[NT], dkm1[NT];
+    S fk[NT], fk1[NT];
+    V dk[NT], dkm1[NT];
+    V erm[NT];  // e'_{k-1}, interface below, deviation from level k
+    const long long c0 = c + k0 * P;
+    double hk = hs[c0], hk1 = k0 + 1 < k1 ? hs[c0 + P] : (SEG ? ring.h(W_RING) : 0.0);
 #pragma unroll
     for (int q = 0; q < NT; q++) {
-        fk[q] = fs[q][c];
-        fk1[q] = (nz > 1) ? fs[q][c + P] : S(0);
-        dk[q] = (nz > 1) ? inc_f<S>(fk1[q] - fk[q]) : 0.f;
-        dkm1[q] = 0.f;
-        erm[q] = 0.f;
+        fk[q] = fs[q][c0];
+        fk1[q] = k0 + 1 < k1 ? fs[q][c0 + P] : (SEG ? ring.f(W_RING, q) : S(0));
+        dk[q] = k0 + 1 < nz ? hx_c<V>(fk1[q] - fk[q]) : V(0);
+        dkm1[q] = k0 > 0 ? hx_c<V>(fk[q] - H.lo1[q]) : V(0);
+        erm[q] = V(0);
     }
-    double hk = hs[c], hk1 = (nz > 1) ? hs[c + P] : 0.0;
-    float hkf = getm_d2f_approx(hk), hk1f = getm_d2f_approx(hk1);
-    float Wm = 0.f;    // W_{k-1} (0 below the bottom level)
-    float wkm1 = a.w[c];
+    V hkf = hx_c<V>(hk), hk1f = hx_c<V>(hk1);
+    V Wm = k0 > 0 ? wv[c0] : V(0);  // W_{k-1} (0 below the bottom level)
+    V wkm1 = a.w[c0];
     // the interface values above level k, one level ahead
-    float Wn = (nz > 1) ? wv[c + P] : 0.f;
-    float wkn = a.w[c + P];
-    // level L's operands into its slot (nothing past the column), one
-    // commit group per level
-    auto stage = [&](int L) {
-        const int s = L % W_RING;
-        if (L < nz) {
+    V Wn = k0 < nz - 1 ? wv[c0 + P] : V(0);
+    V wkn = a.w[c0 + P];
+    // level L's operands (at offset o) into a slot: those of the segment's own
+    // levels, and the velocities of the column; one commit group per level
+    auto stage = [&](int L, long long o, int slot) {
+        if (L < k1) {
 #pragma unroll
-            for (int q = 0; q < NT; q++)
-                __pipeline_memcpy_async(&ring.f[(s * 2 + q) * 32], &fs[q][c + (long long)L * P], sizeof(S));
-            __pipeline_memcpy_async(&ring.h[s * 32], &hs[c + (long long)L * P], sizeof(double));
-            __pipeline_memcpy_async(&ring.W[s * 32], &wv[c + (long long)L * P], sizeof(float));
+            for (int q = 0; q < NT; q++) __pipeline_memcpy_async(&ring.f(slot, q), &fs[q][o], sizeof(S));
+            __pipeline_memcpy_async(&ring.h(slot), &hs[o], sizeof(double));
         }
-        if (L <= nz) __pipeline_memcpy_async(&ring.w[s * 32], &a.w[c + (long long)L * P], sizeof(float));
+        if (L <= k1 && L < nz) __pipeline_memcpy_async(&ring.W(slot), &wv[o], sizeof(V));
+        if (L <= k1) __pipeline_memcpy_async(&ring.w(slot), &a.w[o], sizeof(V));
         __pipeline_commit();
     };
-    for (int L = 2; L < 2 + W_STAGE; L++) stage(L);
-    for (int k = 0; k < nz; k++) {
-        // level k + 2: its group is the oldest of the W_STAGE in flight
-        __pipeline_wait_prior(W_STAGE - 1);
-        const int s2 = (k + 2) % W_RING;
-        S fk2[NT];
-        double hk2 = 0.0;
-#pragma unroll
-        for (int q = 0; q < NT; q++) fk2[q] = (k + 2 < nz) ? ring.f[(s2 * 2 + q) * 32] : S(0);
-        if (k + 2 < nz) hk2 = ring.h[s2 * 32];
-        const float W = Wn;
-        const float wk = wkn;
-        Wn = (k + 1 < nz - 1) ? ring.W[s2 * 32] : 0.f;
-        wkn = (k + 1 < nz) ? ring.w[s2 * 32] : 0.f;
-        stage(k + 2 + W_STAGE);  // into the slot of level k + 1, read at k - 1
-        const float cfl = fabsf(W) * dtf / fminf(hkf, hk1f) * itf;
-        const TvdFace<float> tf = getm_tvd_face_c(a.scheme, cfl);
-        const float dh = dtkf * (wk - wkm1);
-        const double hn = hk - getm_f2d(dh);
-        hd[c + k * P] = hn;
+#pragma unroll 1
+    for (int n = 0; n < W_STAGE; n++) stage(k0 + 2 + n, c0 + (2 + n) * P, n);
+    if (k0 > 0) {  // the interface below the segment
+        const TvdFace<V> tf = w_tvd(a.scheme, Wm, dtf, itf, hx_c<V>(H.hlo), hkf);
 #pragma unroll
         for (int q = 0; q < NT; q++) {
-            // differences of neighbouring values in the storage type, then
-            // narrowed (exact for float storage)
-            const float dn = (k + 2 < nz) ? inc_f<S>(fk2[q] - fk1[q]) : 0.f;
-            float el = 0.f, er = 0.f;
-            if (k < nz - 1) {
-                const float d = dk[q];
-                float dev;
-                if (W > 0.f) dev = getm_tvd_dev_c(tf, d, dkm1[q]);
-                else dev = getm_tvd_dev_c(tf, -d, -dn);
-                el = W * (W > 0.f ? dev : d + dev);
-                er = W * (W > 0.f ? dev - d : dev);
+            V el;
+            w_face(tf, Wm, k0 > 1 ? hx_c<V>(H.lo1[q] - H.lo2[q]) : V(0), dkm1[q], dk[q], el, erm[q]);
+        }
+    }
+    int s2 = 0;          // slot of level k + 2
+    long long ck = c0;  // offset of level k
+    for (int k = k0; k < k1; k++, ck += P, s2 = s2 + 1 == W_RING ? 0 : s2 + 1) {
+        // level k + 2: its group is the oldest of the W_STAGE in flight
+        __pipeline_wait_prior(W_STAGE - 1);
+        const int sf = !SEG || k + 2 < k1 ? s2 : W_RING + (k + 2 - k1);
+        const bool in2 = SEG || k + 2 < nz;
+        S fk2[NT];
+        const double hk2 = in2 ? ring.h(sf) : 0.0;
+#pragma unroll
+        for (int q = 0; q < NT; q++) fk2[q] = in2 ? ring.f(sf, q) : S(0);
+        const V W = Wn;
+        const V wk = wkn;
+        Wn = (k + 1 < k1 && k + 1 < nz - 1) ? ring.W(s2) : V(0);
+        wkn = k + 1 < k1 ? ring.w(s2) : V(0);
+        // into the slot of level k + 1, read at k - 1
+        stage(k + 2 + W_STAGE, ck + (2 + W_STAGE) * P, s2 == 0 ? W_RING - 1 : s2 - 1);
+        const bool inner = k < nz - 1;  // no flux through the surface
+        if constexpr (std::is_same<V, double>::value) {
+            TvdFace<double> tf{};
+            if (inner) tf = w_tvd(a.scheme, W, dtf, itf, hk, hk1);
+            const double hn = __fma_rn(-dtkf, __dadd_rn(wk, -wkm1), hk);
+            hd[ck] = hn;
+            const double coef = __dmul_rn(dtkf, getm_rcp(hn));
+            // (w_k - W_k) - (w_{k-1} - W_{k-1}): zero inside a column moved by w itself
+            const bool slip = !own_w || k == 0 || !inner;
+            const double sl = slip ? __dadd_rn(__dadd_rn(wk, -W), -__dadd_rn(wkm1, -Wm)) : 0.0;
+#pragma unroll
+            for (int q = 0; q < NT; q++) {
+                const double dn = (k + 2 < nz) ? __dadd_rn(fk2[q], -fk1[q]) : 0.0;
+                double el = 0.0, er = 0.0;
+                if (inner) w_face(tf, W, dkm1[q], dk[q], dn, el, er);
+                double num = __dadd_rn(erm[q], -el);
+                if (slip) num = __fma_rn(sl, fk[q], num);
+                fdst[q][ck] = __fma_rn(coef, num, fk[q]);
+                erm[q] = er;
+                dkm1[q] = dk[q]; dk[q] = dn;
+                fk[q] = fk1[q]; fk1[q] = fk2[q];
             }
-            fdst[q][c + k * P] =
-                inc_add<S>(fk[q], dtkf * (((wk - W) - (wkm1 - Wm)) * inc_f<S>(fk[q]) - el + erm[q]) / (hkf - dh));
-            erm[q] = er;
-            dkm1[q] = dk[q]; dk[q] = dn;
-            fk[q] = fk1[q]; fk1[q] = fk2[q];
+        } else {
+            // (formed at the surface too, and not used there: no branch)
+            const TvdFace<float> tf = w_tvd(a.scheme, W, dtf, itf, hkf, hk1f);
+            // (products and sums rounded as written, so that all shapes of the
+            // kernel give the same bits)
+            const float dh = __fmul_rn(dtkf, wk - wkm1);
+            const float den = __fadd_rn(hkf, -dh), sl = (wk - W) - (wkm1 - Wm);
+            const double hn = hk - getm_f2d(dh);
+            hd[ck] = hn;
+#pragma unroll
+            for (int q = 0; q < NT; q++) {
+                // differences of neighbouring values in the storage type, then
+                // narrowed (exact for float storage)
+                const float dn = (k + 2 < nz) ? inc_f<S>(fk2[q] - fk1[q]) : 0.f;
+                float el = 0.f, er = 0.f;
+                if (inner) w_face(tf, W, dkm1[q], dk[q], dn, el, er);
+                const float num = __fadd_rn(__fmaf_rn(sl, inc_f<S>(fk[q]), -el), erm[q]);
+                fdst[q][ck] = inc_add<S>(fk[q], __fmul_rn(dtkf, num) / den);
+                erm[q] = er;
+                dkm1[q] = dk[q]; dk[q] = dn;
+                fk[q] = fk1[q]; fk1[q] = fk2[q];
+            }
         }
         Wm = W; wkm1 = wk;
         hk = hk1; hk1 = hk2;
-        hkf = hk1f; hk1f = getm_d2f_approx(hk2);
+        hkf = hk1f; hk1f = hx_c<V>(hk2);
     }
     __pipeline_wait_prior(0);  // the ring is free for the next sweep
 }
 
-// Largest Courant number over the interior interfaces of a column
-// (template :274, :294, :300).  Returns -1 when nz == 1 (no interfaces).
+// Largest Courant number over the interfaces above levels k0 .. k1-1 of a
+// column where it matters (template :274, :294, :300): -1 when there are none
+// or all are clearly below one, which is all the caller asks.  That first
+// sweep compares |w_var| dt with 0.999 of the thickness in float, without a
+// division; only segments that fail it (or hold a NaN) divide.  A NaN at the
+// column's first interface is the result, any other is passed over.
 template <typename T, typename V>
-__device__ double w_maxcfl(const WPassArgs<T, V>& a, long long c, const V* wv, const double* hs)
+__device__ V w_maxcfl(const WPassArgs<T, V>& a, long long c, int k0, int k1, const V* wv, const double* hs)
 {
     const long long P = a.plane;
-    V cmax = V(-1);
-    if constexpr (getm_increment_form<V>) {
-        const float dtf = (float)a.dt;
-        float hk = getm_d2f_approx(hs[c]);
-        for (int k = 1; k < a.nz; k++) {
-            const float hk1 = getm_d2f_approx(hs[c + k * P]);
-            const float cfl = fabsf(wv[c + k * P]) * dtf / fminf(hk, hk1);
-            if (k == 1 || cfl > cmax) cmax = cfl;
-            hk = hk1;
-        }
-        return (double)cmax;
-    }
-    double hk = hs[c];
-    for (int k = 1; k < a.nz; k++) {
-        double hk1 = hs[c + k * P];
-        V cfl = fabs(wv[c + k * P]) * (V)a.dt / (V)fmin(hk, hk1);
-        if (k == 1 || cfl > cmax) cmax = cfl;
+    const int ke = k1 < a.nz ? k1 + 1 : a.nz;  // levels k0 .. ke-1 bound the interfaces
+    const float dtf = (float)a.dt;
+    float hk = getm_d2f_approx(hs[c + k0 * P]);
+    bool low = true;
+#pragma unroll 4
+    for (int k = k0 + 1; k < ke; k++) {
+        const float hk1 = getm_d2f_approx(hs[c + k * P]);
+        low = low && fabsf(inc_f<V>(wv[c + k * P])) * dtf < 0.999f * fminf(hk, hk1);
         hk = hk1;
     }
-    return (double)cmax;
+    if (low) return V(-1);
+    V cmax = V(-1);
+    double hd = hs[c + k0 * P];
+    for (int k = k0 + 1; k < ke; k++) {
+        const double hd1 = hs[c + k * P];
+        V cfl;
+        if constexpr (getm_increment_form<V>)
+            cfl = fabsf(wv[c + k * P]) * dtf / fminf(getm_d2f_approx(hd), getm_d2f_approx(hd1));
+        else
+            cfl = fabs(wv[c + k * P]) * a.dt / fmin(hd, hd1);
+        if (k == 1 || cfl > cmax) cmax = cfl;
+        hd = hd1;
+    }
+    return cmax;
 }
 
 __device__ __forceinline__ int w_iters_from(double cfl)
@@ -610,83 +684,159 @@ __device__ __forceinline__ int w_iters_from(double cfl)
     return c > 1e9 ? 1000000000 : (int)c;
 }
 
-// Thread per column.
-// T: fields; V: velocities.  Blocks of 32 columns by GETM_TUNE_COLUMN_ROWS
-// rows (row lengths need not be multiples of 128 columns).
-template <typename T, typename V = T>
-__global__ void __launch_bounds__(128, getm_increment_form<V> ? 7 : 1) wpass_kernel(WPassArgs<T, V> a)
+// One group of NT fields through all sub-steps of the block's columns.  it,
+// iters and the rest of a column's state are the same in all its segments;
+// every thread of the block comes here and meets the barriers.
+template <int NT, bool SEG, typename T, typename V>
+__device__ void w_group(const WPassArgs<T, V>& a, long long c, bool touched, int k0, int k1, int t, bool last,
+                        const WRing<SEG, T, V>& ring, double* cm)
 {
-    extern __shared__ __align__(16) unsigned char w_smem[];
-    const int i = blockIdx.x * 32 + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= a.nx_ || j >= a.ny_) return;
-    const long long c = (long long)j * a.nx_ + i;
-    const bool touched = i >= a.ilo && i <= a.ihi && j >= a.jlo && j <= a.jhi && a.tmask[c] == 1 && a.ntracer > 0;
-    if (!touched) {
-        // a column the pass does not update keeps its thickness (h_out must
-        // be a complete field: it is a ping-pong buffer)
-        if (a.h_out != a.h_in)
-            for (int k = 0; k < a.nz; k++) a.h_out[c + k * a.plane] = a.h_in[c + k * a.plane];
-        return;
-    }
     const int itersmax = 200;
-    // mixed form: two consecutive fields with the same w_var are stepped
-    // together (the sub-step count depends only on w_var and h)
-    constexpr bool inc = getm_increment_form<V>;
-    // the second field's intermediate sub-steps use the upper half of the
-    // column work array colbuf[1] (2 n3 doubles)
-    constexpr bool pairs = inc;
-    for (int t = 0; t < a.ntracer;) {
-        const int nt = (pairs && t + 1 < a.ntracer && a.wvar[t + 1] == a.wvar[t]) ? 2 : 1;
-        const V* wv = a.wvar[t];
-        T* f = a.f[t];
-        int iters = 1;
-        double itersm1 = 1.0, dtk = a.dt;
-        int it = 1;
-        while (it <= iters) {
-            const double* hs = (it == 1) ? a.h_in : a.haux;
-            const T* fs = (it == 1) ? f : a.faux;
-            if (iters < itersmax) {
-                int iters_new = w_iters_from(w_maxcfl(a, c, wv, hs));
-                if (iters_new > iters) {
-                    if (iters_new > itersmax) {
-                        iters = itersmax;
-                        atomicOr(a.status, 1 << GETM_ERR_ITERS);
-                    } else {
-                        iters = iters_new;
-                    }
-                    itersm1 = 1.0 / iters;
-                    dtk = a.dt * itersm1;
-                    if (it > 1) { it = 1; continue; }
-                }
+    const V* wv = a.wvar[t];
+    int iters = 1, it = 1;
+    bool active = touched;
+    for (;;) {
+        const double* hs = it == 1 ? a.h_in : a.haux;
+        const bool ask = active && iters < itersmax;
+        double cmax = -1.0;
+        if (ask) cmax = (double)w_maxcfl(a, c, k0, k1, wv, hs);
+        if constexpr (SEG) {
+            cm[threadIdx.y * 32 + threadIdx.x] = cmax;
+            __syncthreads();
+            cmax = cm[threadIdx.x];
+            for (int s = 1; s < (int)blockDim.y; s++) {
+                const double m = cm[s * 32 + threadIdx.x];
+                if (m > cmax) cmax = m;
             }
-            // The last sub-step writes the tracer in place and the thickness
-            // into haux (the stage's h_in must survive for the next tracer);
-            // the last tracer's last sub-step writes the thickness straight
-            // into h_out, the pass's result.
-            T* fd = (it == iters) ? f : a.faux;
-            double* hd = (it == iters && t + nt == a.ntracer) ? a.h_out : a.haux;
-            if constexpr (inc) {
-                if (pairs && nt == 2) {
-                    T* f2 = a.f[t + 1];
-                    T* faux2 = a.faux + a.plane * a.nz;
-                    const T* const fs2[2] = {fs, (it == 1) ? f2 : faux2};
-                    T* const fd2[2] = {fd, (it == iters) ? f2 : faux2};
-                    w_substep_inc<2, T>(a, c, wv, hs, fs2, hd, fd2, dtk, itersm1,
-                                        w_ring<T>(w_smem, blockDim.y, threadIdx.y, threadIdx.x));
-                } else {
-                    const T* const fs1[1] = {fs};
-                    T* const fd1[1] = {fd};
-                    w_substep_inc<1, T>(a, c, wv, hs, fs1, hd, fd1, dtk, itersm1,
-                                        w_ring<T>(w_smem, blockDim.y, threadIdx.y, threadIdx.x));
-                }
-            } else {
-                w_substep(a, c, wv, hs, fs, hd, fd, dtk, itersm1);
-            }
-            it++;
         }
-        t += nt;
+        bool go = active;
+        if (ask) {
+            const int iters_new = w_iters_from(cmax);
+            if (iters_new > iters) {
+                if (iters_new > itersmax) {
+                    iters = itersmax;
+                    if (k0 == 0) atomicOr(a.status, 1 << GETM_ERR_ITERS);
+                } else {
+                    iters = iters_new;
+                }
+                if (it > 1) {  // start the column again
+                    it = 1;
+                    go = false;
+                }
+            }
+        }
+        // The last sub-step writes the tracer in place and the thickness
+        // into haux (the stage's h_in must survive for the next tracer);
+        // the last tracer's last sub-step writes the thickness straight
+        // into h_out, the pass's result.  The second field's intermediate
+        // sub-steps use the upper half of the column work array.
+        const T* fs[NT];
+        T* fd[NT];
+#pragma unroll
+        for (int q = 0; q < NT; q++) {
+            T* aux = a.faux + q * (a.plane * a.nz);
+            fs[q] = it == 1 ? a.f[t + q] : aux;
+            fd[q] = it == iters ? a.f[t + q] : aux;
+        }
+        hs = it == 1 ? a.h_in : a.haux;
+        double* hd = it == iters && last ? a.h_out : a.haux;
+        WHalo<NT, T> H;
+        if constexpr (SEG) {
+            if (go) H = w_halo<NT, T, V>(c, a.plane, a.nz, k0, k1, hs, fs, ring);
+            __syncthreads();  // every segment has read its neighbours' levels
+        }
+        if (go) {
+            // (not kept across the sweep: registers)
+            double itersm1 = 1.0, dtk = a.dt;
+            if (iters > 1) {
+                itersm1 = 1.0 / iters;
+                dtk = a.dt * itersm1;
+            }
+            w_substep<NT, SEG, T, V>(a, c, k0, k1, wv, hs, fs, hd, fd, dtk, itersm1, H, ring);
+            it++;
+            active = it <= iters;
+        }
+        if constexpr (SEG) {
+            if (!__syncthreads_or(active)) return;  // (and the writes are done)
+        } else {
+            if (!active) return;
+        }
     }
+}
+
+// T: fields; V: velocities.  SEG: a block is 32 columns of one row and
+// blockDim.y segments of their levels; else 32 columns of blockDim.y rows.
+template <bool SEG, typename T, typename V>
+__global__ void __launch_bounds__(SEG ? 32 * W_MAXSEG : 128, SEG ? 2 : (getm_increment_form<V> ? 7 : 4))
+    wpass_kernel(WPassArgs<T, V> a)
+{
+    const int i = blockIdx.x * 32 + threadIdx.x;
+    const int j = SEG ? blockIdx.y : blockIdx.y * blockDim.y + threadIdx.y;
+    const int k0 = SEG ? threadIdx.y * a.nz / blockDim.y : 0;
+    const int k1 = SEG ? (threadIdx.y + 1) * a.nz / blockDim.y : a.nz;
+    const bool in = i < a.nx_ && j < a.ny_;
+    const long long c = (long long)j * a.nx_ + i;
+    const bool touched =
+        in && i >= a.ilo && i <= a.ihi && j >= a.jlo && j <= a.jhi && a.tmask[c] == 1 && a.ntracer > 0;
+    // a column the pass does not update keeps its thickness (h_out must be a
+    // complete field: it is a ping-pong buffer)
+    if (in && !touched && a.h_out != a.h_in)
+        for (int k = k0; k < k1; k++) a.h_out[c + k * a.plane] = a.h_in[c + k * a.plane];
+    if constexpr (SEG) {
+        if (!__syncthreads_or(touched)) return;
+    } else {
+        if (!touched) return;
+    }
+    // the rings, then (SEG) the segments' largest Courant numbers
+    using Ring = WRing<SEG, T, V>;
+    const Ring ring(threadIdx.y, threadIdx.x);
+    double* cm = reinterpret_cast<double*>(w_smem + blockDim.y * Ring::BYTES);
+    // two consecutive fields with the same w_var are stepped together (the
+    // sub-step count depends only on w_var and h)
+    for (int t = 0; t < a.ntracer;) {
+        if (t + 1 < a.ntracer && a.wvar[t + 1] == a.wvar[t]) {
+            w_group<2, SEG, T, V>(a, c, touched, k0, k1, t, t + 2 == a.ntracer, ring, cm);
+            t += 2;
+        } else {
+            w_group<1, SEG, T, V>(a, c, touched, k0, k1, t, t + 1 == a.ntracer, ring, cm);
+            t++;
+        }
+    }
+}
+
+// Segments per column, of at least four levels each: one where the columns
+// alone give 20 warps per SM (FP64 form: 10, the FP64 pipe being busy with
+// fewer), more on smaller domains, whose time is the latency of a column's
+// sweep.  us with 1 / 2 / 4 segments: 96 x 96 x 20 mixed, two FP64-stored fields,
+// 58 / 29 / 18; 244 x 204 x 20 mixed, eight, 221 / 174 / 164; 404 x 304 x 40 mixed,
+// two, 133 / 175 / 180 (float fields 80 / 117 / 124); 124 x 104 x 30 FP64, one,
+// 83 / 52 / 41; 177 x 135 x 23 FP64, six, 267 / 199 / 272.
+static int w_segments(int nx_, int ny_, int nz, bool f64)
+{
+    const long long strips = (long long)getm_div_up(nx_, 32) * ny_;
+    int seg = 1;
+    while (seg < W_MAXSEG && strips * seg < (f64 ? 10 : 20) * GETM_SMS && nz / (2 * seg) >= 4) seg *= 2;
+    return seg;
+}
+
+template <bool SEG, typename T, typename V>
+static int launch_wpass(const WPassArgs<T, V>& a, dim3 grid, dim3 block, cudaStream_t stream)
+{
+    // the staging rings (w_substep); the largest carve-out of shared memory,
+    // so that they do not limit the resident warps
+    constexpr size_t per = WRing<SEG, T, V>::BYTES + (SEG ? 32 * sizeof(double) : 0);  // per warp
+    static bool attributes_set = false;  // per-function attributes: once per process
+    if (!attributes_set) {
+        if (cudaFuncSetAttribute(wpass_kernel<SEG, T, V>, cudaFuncAttributePreferredSharedMemoryCarveout, 100) !=
+                cudaSuccess ||
+            cudaFuncSetAttribute(wpass_kernel<SEG, T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(W_MAXSEG * per)) != cudaSuccess)
+            return GETM_ERR_CUDA;
+        attributes_set = true;
+    }
+    wpass_kernel<SEG, T, V><<<grid, block, block.y * per, stream>>>(a);
+    GETM_CHECK_LAUNCH();
+    return GETM_OK;
 }
 
 template <typename T, typename V = T>
@@ -702,22 +852,10 @@ static int run_wstage(getm_advection* adv, const getm_grid* tg, const V* w, cons
     a.tmask = tg->mask; a.w = w; a.dt = dt; a.scheme = adv->scheme; a.status = adv->status;
     a.haux = adv->colbuf[0]; a.faux = (T*)adv->colbuf[1];
     if (a.nz < 1) return GETM_ERR_ARG;
-    const int rows = getm_tune(GETM_TUNE_COLUMN_ROWS);
-    dim3 block(32, rows);
-    dim3 grid(getm_div_up(a.nx_, 32), getm_div_up(a.ny_, rows));
-    // the increment form's staging rings (w_substep_inc); the largest
-    // carve-out of shared memory, so seven blocks of four rows fit per SM
-    size_t smem = 0;
-    if constexpr (getm_increment_form<V>) {
-        smem = (size_t)32 * rows * w_ring_bytes_per_thread<T>();
-        static bool carveout_set = false;  // a per-function attribute: once per process
-        if (!carveout_set) {
-            if (cudaFuncSetAttribute(wpass_kernel<T, V>, cudaFuncAttributePreferredSharedMemoryCarveout, 100) !=
-                cudaSuccess)
-                return GETM_ERR_CUDA;
-            carveout_set = true;
-        }
-    }
+    const int seg = w_segments(a.nx_, a.ny_, a.nz, !getm_increment_form<V>);
+    const int rows = seg > 1 ? 1 : getm_tune(GETM_TUNE_COLUMN_ROWS);
+    const dim3 block(32, seg > 1 ? seg : rows);
+    const dim3 grid(getm_div_up(a.nx_, 32), getm_div_up(a.ny_, rows));
     // Chunks: every chunk starts from h_in; the final h is the last chunk's.
     int done = 0;
     do {
@@ -726,8 +864,9 @@ static int run_wstage(getm_advection* adv, const getm_grid* tg, const V* w, cons
         a.ntracer = n;
         a.h_in = h_in; a.h_out = h_out;
         for (int t = 0; t < n; t++) { a.wvar[t] = wvar[done + t]; a.f[t] = f[done + t]; }
-        wpass_kernel<T, V><<<grid, block, smem, stream>>>(a);
-        GETM_CHECK_LAUNCH();
+        const int rc = seg > 1 ? launch_wpass<true, T, V>(a, grid, block, stream)
+                               : launch_wpass<false, T, V>(a, grid, block, stream);
+        if (rc) return rc;
         done += n;
     } while (done < ntracer);
     return GETM_OK;

@@ -13,6 +13,9 @@
 #define GETM_KAPPA 0.4
 #define GETM_G 9.81
 
+// SMs of a GB300: the unit in which grids are made large enough
+#define GETM_SMS 152
+
 // Grid handle: index extent plus device pointers to the static metrics that
 // the reference reads from its type_getm_grid (src/domain/domain.F90:85-140)
 // inside advection_uv_calculate / c_momentum_diffusion.
@@ -233,23 +236,22 @@ __device__ __forceinline__ double getm_div_refined(double num, double den)
     return fma(fma(-q0, den, num), r, q0);
 }
 
-// 1 / x in FP64 to within two units in the last place, from six instructions
-// of which three are FP64: a float reciprocal r (relative error e below 2^-21)
-// and one third-order Householder step, r (1 + e + e^2), whose own error is
-// e^3.  GB300 runs FP64 at 1/64 of its float rate and the correctly rounded
-// division takes about four times as many FP64 instructions, so this serves
-// where a quotient only scales an increment.  x zero, not finite or outside
-// the normal float range: the correctly rounded division, out of line.
+// 1 / x in FP64 to within two units in the last place with three FP64
+// instructions: the approximate reciprocal r of PTX (rcp.approx.ftz.f64,
+// relative error e about 2^-20, not on the FP64 pipe) and one third-order
+// Householder step, r (1 + e + e^2) with e = 1 - x r, whose own error is e^3.
+// GB300 runs FP64 at 1/64 of its float rate and the correctly rounded
+// division takes several times as many FP64 instructions, so this serves
+// where a quotient only scales an increment.  Zero, subnormal, huge and
+// non-finite x: the correctly rounded division, out of line.
 static __device__ __noinline__ double getm_rcp_hw(double x) { return 1.0 / x; }
 
 __device__ __forceinline__ double getm_rcp(double x)
 {
-    const float xf = getm_d2f_approx(x);
-    const float ax = fabsf(xf);
-    if (!(ax > 1e-30f && ax < 1e30f)) return getm_rcp_hw(x);
-    float rf;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rf) : "f"(xf));
-    const double r = getm_f2d(rf);
+    const unsigned e11 = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
+    if (e11 - 2u > 2042u) return getm_rcp_hw(x);  // outside 2^-1021 .. 2^1022
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
     const double e = __fma_rn(-x, r, 1.0);
     return __fma_rn(r, __fma_rn(e, e, e), r);
 }
@@ -260,16 +262,15 @@ static __device__ __noinline__ double getm_twice_hw(double x) { return x + x; }
 
 __device__ __forceinline__ double getm_twice(double x)
 {
-    const long long b = __double_as_longlong(x);
-    const int e = (int)((b >> 52) & 0x7ff);
-    if (e > 0 && e < 0x7fe) return __longlong_as_double(b + (1ll << 52));
-    return (b << 1) == 0 ? x : getm_twice_hw(x);
+    const int hi = __double2hiint(x);
+    if ((((unsigned)hi >> 20) & 0x7ffu) - 1u < 0x7fdu) return __hiloint2double(hi + (1 << 20), __double2loint(x));
+    return getm_twice_hw(x);
 }
 
 // x, negated where neg is set, on the integer pipe
 __device__ __forceinline__ double getm_negate_if(double x, bool neg)
 {
-    return __longlong_as_double(__double_as_longlong(x) ^ ((long long)neg << 63));
+    return __hiloint2double(__double2hiint(x) ^ (neg ? (int)0x80000000 : 0), __double2loint(x));
 }
 
 // min and max of non-negative doubles (their bit patterns order as integers)
@@ -328,43 +329,6 @@ __device__ __forceinline__ T getm_limiter(int scheme, T ratio, T cfl)
         break;
     }
     return limiter;
-}
-
-// One TVD face value: given upstream-upstream, upstream and downstream values
-// and the face Courant number, return the limited face value
-// (advection.F90.template:82-88, 344-350).
-template <typename T>
-__device__ __forceinline__ T getm_tvd_face(int scheme, T fuu, T fu, T fd, T cfl)
-{
-    T deltaf = fd - fu;
-    T deltafu = fu - fuu;
-    if (deltaf * deltafu > T(0)) {
-        T ratio = deltafu / deltaf;
-        T limiter = getm_limiter<T>(scheme, ratio, cfl);
-        fu = fu + T(0.5) * limiter * (T(1) - cfl) * deltaf;
-    }
-    return fu;
-}
-
-// The limited part of the TVD face value, face - fu (0 where the limiter is
-// inactive), from the differences deltaf = fd - fu and deltafu = fu - fuu:
-// the same arithmetic as getm_tvd_face without the final sum, so the
-// increment form can work with deviations from cell values.
-template <typename T>
-__device__ __forceinline__ T getm_tvd_dev_d(int scheme, T deltaf, T deltafu, T cfl)
-{
-    if (deltaf * deltafu > T(0)) {
-        T ratio = deltafu / deltaf;
-        T limiter = getm_limiter<T>(scheme, ratio, cfl);
-        return T(0.5) * limiter * (T(1) - cfl) * deltaf;
-    }
-    return T(0);
-}
-
-template <typename T>
-__device__ __forceinline__ T getm_tvd_dev(int scheme, T fuu, T fu, T fd, T cfl)
-{
-    return getm_tvd_dev_d<T>(scheme, fd - fu, fu - fuu, cfl);
 }
 
 // The limited deviation without a division per field (C: float for the mixed
@@ -447,41 +411,44 @@ __device__ __forceinline__ float getm_tvd_dev_c(const TvdFace<float>& tf, float 
 
 // FP64: the limited difference phi(r) deltaf itself, without the factor
 // half1mc; signs, doublings, minima and maxima on the integer pipe (superbee
-// needs no FP64 instruction at all).  The sign test is that of deltaf *
-// deltafu > 0 (false for NaN); where one of them is zero every limiter gives
-// zero.
+// needs no FP64 instruction at all).  Differences of opposite signs give zero,
+// and where one of them is zero every limiter does.  Infinities and NaNs go
+// through the ratio, out of line.
+static __device__ __noinline__ double getm_tvd_phi_hw(int scheme, double half1mc, double deltaf, double deltafu)
+{
+    return deltaf * deltafu > 0.0 ? getm_limiter<double>(scheme, deltafu / deltaf, 1.0 - 2.0 * half1mc) * deltaf : 0.0;
+}
+
 __device__ __forceinline__ double getm_tvd_phi(const TvdFace<double>& tf, double deltaf, double deltafu)
 {
-    const long long bd = __double_as_longlong(deltaf), bu = __double_as_longlong(deltafu);
-    const long long ia = bd & 0x7fffffffffffffffll, ib = bu & 0x7fffffffffffffffll;
-    if ((bd ^ bu) < 0 || ia > 0x7ff0000000000000ll || ib > 0x7ff0000000000000ll) return 0.0;
-    const double a = __longlong_as_double(ia), b = __longlong_as_double(ib);
+    const int hd = __double2hiint(deltaf), hu = __double2hiint(deltafu);
+    const int ha = hd & 0x7fffffff, hb = hu & 0x7fffffff;
+    if (ha >= 0x7ff00000 || hb >= 0x7ff00000) return getm_tvd_phi_hw(tf.scheme, tf.half1mc, deltaf, deltafu);
+    if ((hd ^ hu) < 0) return 0.0;
+    const double a = __hiloint2double(ha, __double2loint(deltaf)), b = __hiloint2double(hb, __double2loint(deltafu));
     double pa;
     switch (tf.scheme) {
     case GETM_SCHEME_HSIMT: {
         const double lin = __fma_rn(tf.lin1, b, __dmul_rn(tf.lin0, a));
-        pa = getm_min_pos(getm_min_pos(getm_twice(b), getm_positive_i(lin) ? lin : 0.0), getm_twice(a));
+        pa = getm_min_pos(getm_twice(getm_min_pos(a, b)), getm_positive_i(lin) ? lin : 0.0);
         break;
     }
-    case GETM_SCHEME_MUSCL:
-        pa = getm_min_pos(getm_min_pos(getm_twice(b), getm_half(__dadd_rn(a, b))), getm_twice(a));
-        break;
+    case GETM_SCHEME_MUSCL: pa = getm_min_pos(getm_twice(getm_min_pos(a, b)), getm_half(__dadd_rn(a, b))); break;
     case GETM_SCHEME_P2_PDM:
-        if (ia == 0 || ib == 0) return 0.0;  // its bounds may be negative beyond Courant numbers of 1
+        if (a == 0.0 || b == 0.0) return 0.0;  // its bounds may be negative beyond Courant numbers of 1
         pa = getm_fmin_i(getm_fmin_i(__dmul_rn(tf.rcoef, b), __fma_rn(tf.lin1, b, __dmul_rn(tf.lin0, a))),
                          __dmul_rn(tf.cap, a));
         break;
     case GETM_SCHEME_SPLMAX13:
-        pa = getm_min_pos(getm_min_pos(getm_twice(b),
-                                       __dmul_rn(1.0 / 3.0, __dadd_rn(__dadd_rn(a, b), getm_max_pos(a, b)))),
-                          getm_twice(a));
+        pa = getm_min_pos(getm_twice(getm_min_pos(a, b)),
+                          __dmul_rn(1.0 / 3.0, __dadd_rn(__dadd_rn(a, b), getm_max_pos(a, b))));
         break;
-    case GETM_SCHEME_SUPERBEE:
-        pa = getm_max_pos(getm_min_pos(getm_twice(b), a), getm_min_pos(b, getm_twice(a)));
+    case GETM_SCHEME_SUPERBEE:  // max(min(2b, a), min(b, 2a))
+        pa = getm_min_pos(getm_twice(getm_min_pos(a, b)), getm_max_pos(a, b));
         break;
     default: return 0.0;
     }
-    return __longlong_as_double(__double_as_longlong(pa) ^ (bd & (long long)0x8000000000000000ull));
+    return getm_negate_if(pa, hd < 0);
 }
 
 __device__ __forceinline__ bool getm_flux_point(int m) { return m == 1 || m == 2; }

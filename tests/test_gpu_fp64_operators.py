@@ -65,3 +65,39 @@ def test_plane_split_at_tile_edges(nx, ny, split):
     ad(wrap(Td.ugrid, u, False), wrap(Td.vgrid, v, False), 600.0, td)
     close(host(td.all_values), to, rtol=RTOL)
     close(host(ad.D), ao.D, rtol=RTOL)
+
+
+@pytest.mark.parametrize("nx,ny,nz,scheme,wmax", [(3, 3, 1, 5, 5e-4), (30, 12, 2, 1, 5e-4), (31, 13, 3, 3, 5e-3),
+                                                  (60, 20, 9, 5, 2e-2), (29, 50, 40, 4, 2e-3)])
+def test_vertical_pass_columns(nx, ny, nz, scheme, wmax):
+    """Batches of one to three fields, the last with its own velocity, in
+    columns of one to forty levels with Courant numbers from below one to
+    several sub-steps.  A sub-step rounds some 15 u where the field's own
+    velocity moves up to four layers' worth of it; six of them stay below
+    1e-13."""
+    import oracle.oracle as O
+    from getm_gb300 import operators
+    from getm_gb300.core import CENTERS, INTERFACES
+
+    Th, To, Td, rng = setup(nz=nz, seed=nz, nx=nx, ny=ny)
+    zero3 = lambda g: np.zeros((nz, g.ny_, g.nx_))  # noqa: E731
+    w = rng.uniform(-2e-4, 2e-4, (nz + 1, Th.ny_, Th.nx_))
+    own = rng.uniform(-wmax, wmax, w.shape)
+    for a in (w, own):
+        a[0] = a[-1] = 0.0
+    for nt in (1, 2, 3):
+        tr = [rng.uniform(5.0, 10.0, (nz, Th.ny_, Th.nx_)) for _ in range(nt)]
+        ws = [own if q == 2 or nt == 1 else w for q in range(nt)]
+        ao = O.Advection(To, scheme)
+        tro = [t.copy() for t in tr]
+        it = iter(ws)
+        ao.apply_3d_batch(zero3(Th.ugrid), zero3(Th.vgrid), w, 300.0, tro, get_w=lambda _: next(it))
+        ad = operators.Advection(Td, operators.AdvectionScheme(scheme))
+        trd = [wrap(Td, t, CENTERS) for t in tr]
+        wd, od = wrap(Td, w, INTERFACES), wrap(Td, own, INTERFACES)
+        itd = iter([od if x is own else wd for x in ws])
+        ad.apply_3d_batch(wrap(Td.ugrid, zero3(Th.ugrid), CENTERS), wrap(Td.vgrid, zero3(Th.vgrid), CENTERS), wd, 300.0,
+                          trd, get_w=lambda _: next(itd))
+        for a, b in zip(trd, tro):
+            close(host(a.all_values), b, rtol=1e-13)
+        close(host(ad.h), ao.h, rtol=RTOL)
