@@ -10,9 +10,8 @@
 // tridiagonal matrix is never stored: its coefficients are formed on the fly
 // from nuh, ho, hn and var while sweeping down from the surface (the Thomas
 // forward elimination of diffusion.F90:285-292), keeping only the two
-// elimination coefficients per level for the back substitution (:304-307),
-// in shared memory or in a caller-provided global workspace.  prepare+apply
-// are fused (traffic per field: read nuh, ho, hn, var [+ea2, ea4], write
+// coefficients per level for the back substitution (:304-307), in shared
+// memory or in a caller-provided global workspace.  prepare+apply are fused (traffic per field: read nuh, ho, hn, var [+ea2, ea4], write
 // var).  The mixed form's solve (vd_inc_kernel) takes fields in pairs and
 // issues each level's loads one level ahead.  A warp-per-column PCR solve would
 // cost O(nz log nz) FP64 divides per column instead of O(nz); GB300's FP64
@@ -67,18 +66,13 @@ __device__ __forceinline__ T vd_h(double h)
 
 // Coupling coefficients of the interface above C level k (between levels k and
 // k+1): diffusion.F90:166-168 with Fortran k = C k + 1.
-template <typename T>
-__device__ __forceinline__ void vd_aux(const VDArgs<T>& a, long long c, int k, double mol, T& auxo, T& auxn)
+__device__ __forceinline__ void vd_aux(const VDArgs<float>& a, long long c, int k, double mol, float& auxo,
+                                       float& auxn)
 {
     const long long P = a.plane;
-    if (a.auxo) {
-        auxo = (T)a.auxo[c + k * P];
-        auxn = (T)a.auxn[c + k * P];
-        return;
-    }
-    T x = (T)(2.0 * a.dt) * (a.nuh[c + (k + 1) * P] + (T)mol);
-    auxo = (T)(1.0 - a.cnpar) * x / (vd_h<T>(a.ho[c + (k + 1) * P]) + vd_h<T>(a.ho[c + k * P]));
-    auxn = (T)a.cnpar * x / (vd_h<T>(a.hn[c + (k + 1) * P]) + vd_h<T>(a.hn[c + k * P]));
+    float x = (float)(2.0 * a.dt) * (a.nuh[c + (k + 1) * P] + (float)mol);
+    auxo = (float)(1.0 - a.cnpar) * x / (vd_h<float>(a.ho[c + (k + 1) * P]) + vd_h<float>(a.ho[c + k * P]));
+    auxn = (float)a.cnpar * x / (vd_h<float>(a.hn[c + (k + 1) * P]) + vd_h<float>(a.hn[c + k * P]));
 }
 
 // Increment form: (ho - hn) of one layer as float, exact-difference first;
@@ -88,28 +82,186 @@ __device__ __forceinline__ float vd_dh(const double* ho, const double* hn, long 
     return ho == hn ? 0.f : getm_d2f_approx(ho[q] - hn[q]);
 }
 
-// Thread per column; dynamic shared memory holds ru/qu (and, in the
-// increment form, the old values): vd_smem_arrays<T> * nz * blockDim values.
-//
-// Increment form (float): with x the old values and A x_new = a4 the
-// reference system, the kernel solves A dx = a4 - A x, whose right-hand side
-// reduces to differences that float32 holds exactly or nearly so:
+// A single layer (diffusion.F90:224-231): every point, mask not consulted.
+template <typename T, typename S>
+__device__ __forceinline__ void vd_single_layer(const VDArgs<T, S>& a, long long c)
+{
+    for (int t = 0; t < a.ntracer; t++) {
+        const S x = a.var[t][c];
+        T a2 = vd_h<T>(a.hn[c]);
+        if constexpr (getm_increment_form<T>) {
+            const float xf = inc_f<S>(x);
+            float r = xf * vd_dh(a.ho, a.hn, c);
+            if (a.ea2[t]) { a2 = a2 - a.ea2[t][c]; r = r + a.ea2[t][c] * xf; }
+            if (a.ea4[t]) r = r + a.ea4[t][c];
+            a.var[t][c] = inc_add<S>(x, r / a2);
+        } else {
+            if (a.ea2[t]) a2 = a2 - a.ea2[t][c];
+            T a4 = a.ho[c] * x;
+            if (a.ea4[t]) a4 = a4 + a.ea4[t][c];
+            a.var[t][c] = a4 / a2;
+        }
+    }
+}
+
+// The solves work in increments: with x the old values and A x_new = a4 the
+// reference system, they solve A dx = a4 - A x, whose right-hand side reduces
+// to differences of neighbouring values
 //   r_k = x_k (ho_k - hn_k) + (x_{k+1} - x_k)(auxo + auxn)_{k+1/2}
 //         + (x_{k-1} - x_k)(auxo + auxn)_{k-1/2} + ea4_k + ea2_k x_k
-// and writes x + dx.
-template <typename T>
-constexpr int vd_smem_arrays = getm_increment_form<T> ? 3 : 2;
+// and write x + dx, so rounding scales with the change of the field.
+//
+// FP64 form, thread per column.  GB300's FP64 rate bounds it, so it counts
+// FP64 instructions: one reciprocal per row and per interface (getm_rcp) in
+// place of the reference's four divisions and none for the explicit half of
+// the coupling when cnpar = 1: 20 per level, where the reference's order of
+// evaluation took about 130.  Eliminating downwards from the surface, with up
+// and lo the implicit couplings above and below a row, F = (auxo + auxn) (x_{k-1}
+// - x_k) the old field's flux term and src the remaining terms of r_k,
+//     t = hn - ea2 + up s',  den = t + lo,  r = lo / den,  s = t / den,
+//     y = s F + r (y' - src),
+// where ' marks the row above (zero at the surface), and upwards
+//     dx_k = r (x_{k-1} - x_k + dx_{k-1}) + (src + auxo (x_{k-1} - x_k) - y') / den.
+// Here t is the row's diagonal less lo (1 + the reference's r_k is s) and y the
+// flux left over from the rows above: no large terms are subtracted, so strong
+// mixing costs no digits (the reference's a2 - a3 r_k loses about lo / hn ulps).
+// As in vd_inc_sweep every operand of a level is loaded one level ahead.
+// Measured: 120 x 100 x 30, one field, 103 -> 41 us; 200 x 150 x 30, two fields with
+// sources and two thicknesses, 286 -> 130 us; error against quad precision
+// 1.3e-16 -> 0.5e-16.
+// r and the second term of dx are kept at stride rs per level, in shared
+// memory or the caller's workspace ([k][j][i]).  Prepared coupling
+// coefficients (a.auxo) replace those formed here.
+template <bool SRC>
+__device__ __forceinline__ void vd_f64_sweep(const VDArgs<double>& a, long long c, int t, double* ru, double* qu,
+                                             long long rs)
+{
+    const long long P = a.plane;
+    const int nz = a.nz;
+    const double* __restrict__ ho = a.ho + c;
+    const double* __restrict__ hn = a.hn + c;
+    const bool one_h = a.ho == a.hn, prep = a.auxo != nullptr;
+    const bool both = prep || a.cnpar != 1.0;  // an explicit half too
+    const bool use_ho = !one_h;
+    const double dt2 = 2.0 * a.dt, co = 1.0 - a.cnpar, mol = a.molecular[t];
+    double* v = a.var[t] + c;
+    const double* e2 = SRC && a.ea2[t] ? a.ea2[t] + c : nullptr;
+    const double* e4 = SRC && a.ea4[t] ? a.ea4[t] + c : nullptr;
+    // level k operands (current) and the raw loads of level k-1 (next)
+    int k = nz - 1;
+    double ho_c = use_ho ? ho[k * P] : 0.0, ho_n = use_ho ? ho[(k - 1) * P] : 0.0;
+    double hn_c = hn[k * P], hn_n = hn[(k - 1) * P];
+    double nuh_c = prep ? 0.0 : a.nuh[c + k * P];  // interface below level k
+    double vk = v[k * P], vn = v[(k - 1) * P];
+    double e2c = SRC && e2 ? e2[k * P] : 0.0, e4c = SRC && e4 ? e4[k * P] : 0.0;
+    double up = 0.0, sp = 0.0, yp = 0.0;  // of the row above
+    double dx = 0.0;
+    for (; k >= 0; k--) {
+        // the raw operands of level k-2 and of the interface below level k-1
+        double ho_nn = 0.0, hn_nn = 0.0, nuh_n = 0.0, vnn = 0.0, e2n = 0.0, e4n = 0.0;
+        if (k >= 2) {
+            if (use_ho) ho_nn = ho[(k - 2) * P];
+            hn_nn = hn[(k - 2) * P];
+            vnn = v[(k - 2) * P];
+        }
+        if (k >= 1) {
+            if (!prep) nuh_n = a.nuh[c + (k - 1) * P];
+            if (SRC && e2) e2n = e2[(k - 1) * P];
+            if (SRC && e4) e4n = e4[(k - 1) * P];
+        }
+        // y' - src of this row, and t
+        double hk = hn_c, ys = yp;
+        if (use_ho) ys = __fma_rn(-vk, __dadd_rn(ho_c, -hn_c), ys);
+        if (SRC && e2) {
+            hk = __dadd_rn(hk, -e2c);
+            ys = __fma_rn(-e2c, vk, ys);
+        }
+        if (SRC && e4) ys = __dadd_rn(ys, -e4c);
+        const double tk = __fma_rn(up, sp, hk);
+        if (k == 0) {  // no interface below
+            dx = -__dmul_rn(ys, getm_rcp(tk));
+            break;
+        }
+        // the interface below level k: lo implicit, eo explicit
+        double lo, eo = 0.0;
+        if (prep) {
+            lo = a.auxn[c + (k - 1) * P];
+            eo = a.auxo[c + (k - 1) * P];
+        } else {
+            const double x = __dmul_rn(dt2, __dadd_rn(nuh_c, mol));
+            const double rsn = getm_rcp(__dadd_rn(hn_c, hn_n));
+            if (both) {
+                lo = __dmul_rn(__dmul_rn(a.cnpar, x), rsn);
+                eo = __dmul_rn(__dmul_rn(co, x), one_h ? rsn : getm_rcp(__dadd_rn(ho_c, ho_n)));
+            } else {
+                lo = __dmul_rn(x, rsn);
+            }
+        }
+        const double dd = __dadd_rn(vn, -vk);
+        const double inv = getm_rcp(__dadd_rn(tk, lo));
+        const double r = __dmul_rn(lo, inv);
+        // s F = (t / den) lo dd = r t dd, and the explicit half's part
+        double q = ys;
+        sp = __dmul_rn(tk, inv);
+        yp = __dmul_rn(r, __fma_rn(tk, dd, ys));
+        if (both) {
+            const double fe = __dmul_rn(eo, dd);
+            yp = __fma_rn(sp, fe, yp);
+            q = __dadd_rn(q, -fe);
+        }
+        ru[k * rs] = r;
+        qu[k * rs] = -__dmul_rn(q, inv);
+        up = lo;
+        vk = vn; vn = vnn;
+        e2c = e2n; e4c = e4n;
+        hn_c = hn_n; hn_n = hn_nn;
+        ho_c = ho_n; ho_n = ho_nn;
+        nuh_c = nuh_n;
+    }
+    // back substitution (:304-307)
+    double xn = v[P], rn = ru[rs], qn = qu[rs];
+    double below = __dadd_rn(vk, dx);  // the new value of the level below
+    v[0] = below;
+    for (k = 1; k < nz; k++) {
+        const double x_old = xn, r = rn, q = qn;
+        if (k + 1 < nz) {
+            xn = v[(k + 1) * P];
+            rn = ru[(k + 1) * rs];
+            qn = qu[(k + 1) * rs];
+        }
+        below = __dadd_rn(x_old, __fma_rn(r, __dadd_rn(below, -x_old), q));
+        v[k * P] = below;
+    }
+}
 
-// GW: the elimination coefficients ru, qu live in a.work ([k][j][i], so every
-// level is again one coalesced access) instead of shared memory, which then
-// no longer limits the number of resident columns; the increment form
-// re-reads the old values from var during the back substitution (var[k] is
-// overwritten only after it is read).
-template <typename T, bool GW>
-__global__ void __launch_bounds__(128, getm_increment_form<T> ? 8 : 1) vd_column_kernel(VDArgs<T> a)
+// Blocks of 32 columns by blockDim.y rows, one field after the other (the
+// workspace a caller brings holds one field's coefficients: 2 nz planes, or NULL
+// for shared memory).
+template <bool SRC>
+__global__ void __launch_bounds__(128, 5) vd_f64_kernel(VDArgs<double> a)
 {
     extern __shared__ __align__(16) unsigned char vd_smem[];
-    constexpr bool inc = getm_increment_form<T>;
+    const int i = blockIdx.x * 32 + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    if (i >= a.nx_ || j >= a.ny_) return;
+    const long long c = (long long)j * a.nx_ + i;
+    if (a.nz == 1) {
+        vd_single_layer(a, c);
+        return;
+    }
+    if (a.mask[c] != 1) return;
+    double* const ru = a.work ? a.work + c : (double*)vd_smem + threadIdx.y * 32 + threadIdx.x;
+    const long long rs = a.work ? a.plane : 32 * (long long)blockDim.y;
+    for (int t = 0; t < a.ntracer; t++) vd_f64_sweep<SRC>(a, c, t, ru, ru + a.nz * rs, rs);
+}
+
+// Float solve without a workspace, thread per column; dynamic shared memory
+// holds ru, qu and the old values: 3 nz blockDim values.
+constexpr int VD_SMEM_ARRAYS = 3;
+
+__global__ void __launch_bounds__(128, 8) vd_column_kernel(VDArgs<float> a)
+{
+    extern __shared__ __align__(16) unsigned char vd_smem[];
     const int tid = threadIdx.x;
     const int nthreads = blockDim.x;
     const int i = blockIdx.x * blockDim.x + tid;
@@ -118,89 +270,53 @@ __global__ void __launch_bounds__(128, getm_increment_form<T> ? 8 : 1) vd_column
     const long long c = (long long)j * a.nx_ + i;
     const long long P = a.plane;
     const int nz = a.nz;
-    if (nz == 1) {  // diffusion.F90:224-231: every point, mask not consulted
-        for (int t = 0; t < a.ntracer; t++) {
-            T x = a.var[t][c];
-            T a2 = vd_h<T>(a.hn[c]);
-            if (a.ea2[t]) a2 = a2 - a.ea2[t][c];
-            if constexpr (inc) {
-                T r = x * vd_dh(a.ho, a.hn, c);
-                if (a.ea4[t]) r = r + a.ea4[t][c];
-                if (a.ea2[t]) r = r + a.ea2[t][c] * x;
-                a.var[t][c] = x + r / a2;
-            } else {
-                T a4 = vd_h<T>(a.ho[c]) * x;
-                if (a.ea4[t]) a4 = a4 + a.ea4[t][c];
-                a.var[t][c] = a4 / a2;
-            }
-        }
+    if (nz == 1) {
+        vd_single_layer(a, c);
         return;
     }
     if (a.mask[c] != 1) return;
-    // ru[k * rs], qu[k * rs] (and xo[k * rs], increment form in shared memory)
-    T* ru;
-    T* qu;
-    T* xo;
-    long long rs;
-    if constexpr (GW) {
-        ru = a.work + c;
-        qu = ru + P * nz;
-        xo = a.var[0] + c;  // not used: old values are re-read from var
-        rs = P;
-    } else {
-        ru = (T*)vd_smem + tid;
-        qu = ru + (size_t)nz * nthreads;
-        xo = qu + (size_t)nz * nthreads;
-        rs = nthreads;
-    }
+    float* ru = (float*)vd_smem + tid;
+    float* qu = ru + (size_t)nz * nthreads;
+    float* xo = qu + (size_t)nz * nthreads;
+    const int rs = nthreads;
     for (int t = 0; t < a.ntracer; t++) {
-        T* __restrict__ var = a.var[t];
-        const T* ea2 = a.ea2[t];
-        const T* ea4 = a.ea4[t];
+        float* __restrict__ var = a.var[t];
+        const float* ea2 = a.ea2[t];
+        const float* ea4 = a.ea4[t];
         const double mol = a.molecular[t];
         // surface layer (C level nz-1), diffusion.F90:238-245
         int k = nz - 1;
-        T aob, anb;                             // aux of the interface below level k
+        float aob, anb;                         // aux of the interface below level k
         vd_aux(a, c, k - 1, mol, aob, anb);
-        T vk = var[c + k * P];
-        T vkm1 = var[c + (k - 1) * P];
-        T a1 = -anb;
-        T a2 = vd_h<T>(a.hn[c + k * P]) + anb;
-        T a4;
-        if constexpr (inc) {
-            if constexpr (!GW) xo[k * rs] = vk;
-            a4 = vk * vd_dh(a.ho, a.hn, c + k * P) + (vkm1 - vk) * (aob + anb);
-            if (ea2) a4 = a4 + ea2[c + k * P] * vk;
-        } else {
-            a4 = vk * (T)a.ho[c + k * P] + (vkm1 - vk) * aob;
-        }
+        float vk = var[c + k * P];
+        float vkm1 = var[c + (k - 1) * P];
+        float a1 = -anb;
+        float a2 = vd_h<float>(a.hn[c + k * P]) + anb;
+        xo[k * rs] = vk;
+        float a4 = vk * vd_dh(a.ho, a.hn, c + k * P) + (vkm1 - vk) * (aob + anb);
+        if (ea2) a4 = a4 + ea2[c + k * P] * vk;
         if (ea2) a2 = a2 - ea2[c + k * P];
         if (ea4) a4 = a4 + ea4[c + k * P];
-        T rk = a1 / a2;
-        T qk = a4 / a2;
+        float rk = a1 / a2;
+        float qk = a4 / a2;
         ru[k * rs] = rk;
         qu[k * rs] = qk;
         // inner layers, diffusion.F90:247-258 and elimination :287-290
-        T aoa = aob, ana = anb;                 // interface above level k-1
-        T vkp1 = vk;
+        float aoa = aob, ana = anb;             // interface above level k-1
+        float vkp1 = vk;
         vk = vkm1;
         for (k = nz - 2; k >= 1; k--) {
             vd_aux(a, c, k - 1, mol, aob, anb);
             vkm1 = var[c + (k - 1) * P];
-            T a3 = -ana;
+            float a3 = -ana;
             a1 = -anb;
-            a2 = vd_h<T>(a.hn[c + k * P]) + ana + anb;
-            if constexpr (inc) {
-                if constexpr (!GW) xo[k * rs] = vk;
-                a4 = vk * vd_dh(a.ho, a.hn, c + k * P) + (vkp1 - vk) * (aoa + ana) +
-                     (vkm1 - vk) * (aob + anb);
-                if (ea2) a4 = a4 + ea2[c + k * P] * vk;
-            } else {
-                a4 = vk * (T)a.ho[c + k * P] + (vkp1 - vk) * aoa + (vkm1 - vk) * aob;
-            }
+            a2 = vd_h<float>(a.hn[c + k * P]) + ana + anb;
+            xo[k * rs] = vk;
+            a4 = vk * vd_dh(a.ho, a.hn, c + k * P) + (vkp1 - vk) * (aoa + ana) + (vkm1 - vk) * (aob + anb);
+            if (ea2) a4 = a4 + ea2[c + k * P] * vk;
             if (ea2) a2 = a2 - ea2[c + k * P];
             if (ea4) a4 = a4 + ea4[c + k * P];
-            T den = a2 - a3 * rk;
+            float den = a2 - a3 * rk;
             rk = a1 / den;
             qk = (a4 - a3 * qk) / den;
             ru[k * rs] = rk;
@@ -209,34 +325,18 @@ __global__ void __launch_bounds__(128, getm_increment_form<T> ? 8 : 1) vd_column
             vkp1 = vk; vk = vkm1;
         }
         // bottom layer, diffusion.F90:260-267 and :291-292
-        {
-            T a3 = -ana;
-            a2 = vd_h<T>(a.hn[c]) + ana;
-            if constexpr (inc) {
-                a4 = vk * vd_dh(a.ho, a.hn, c) + (vkp1 - vk) * (aoa + ana);
-                if (ea2) a4 = a4 + ea2[c] * vk;
-            } else {
-                a4 = vk * (T)a.ho[c] + (vkp1 - vk) * aoa;
-            }
-            if (ea2) a2 = a2 - ea2[c];
-            if (ea4) a4 = a4 + ea4[c];
-            T q0 = (a4 - a3 * qk) / (a2 - a3 * rk);
-            // back substitution :304-307
-            T vprev = q0;
-            if constexpr (inc) {
-                var[c] = vk + q0;
-                for (k = 1; k < nz; k++) {
-                    vprev = qu[k * rs] - ru[k * rs] * vprev;
-                    const T x_old = GW ? var[c + k * P] : xo[k * rs];
-                    var[c + k * P] = x_old + vprev;
-                }
-            } else {
-                var[c] = q0;
-                for (k = 1; k < nz; k++) {
-                    vprev = qu[k * rs] - ru[k * rs] * vprev;
-                    var[c + k * P] = vprev;
-                }
-            }
+        float a3 = -ana;
+        a2 = vd_h<float>(a.hn[c]) + ana;
+        a4 = vk * vd_dh(a.ho, a.hn, c) + (vkp1 - vk) * (aoa + ana);
+        if (ea2) a4 = a4 + ea2[c] * vk;
+        if (ea2) a2 = a2 - ea2[c];
+        if (ea4) a4 = a4 + ea4[c];
+        float vprev = (a4 - a3 * qk) / (a2 - a3 * rk);
+        // back substitution :304-307
+        var[c] = vk + vprev;
+        for (k = 1; k < nz; k++) {
+            vprev = qu[k * rs] - ru[k * rs] * vprev;
+            var[c + k * P] = xo[k * rs] + vprev;
         }
     }
 }
@@ -403,16 +503,8 @@ __global__ void __launch_bounds__(128, 7) vd_inc_kernel(VDArgs<float, S> a)
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     if (i >= a.nx_ || j >= a.ny_) return;
     const long long c = (long long)j * a.nx_ + i;
-    if (a.nz == 1) {  // diffusion.F90:224-231: every point, mask not consulted
-        for (int t = 0; t < a.ntracer; t++) {
-            const S x = a.var[t][c];
-            const float xf = inc_f<S>(x);
-            float a2 = vd_h<float>(a.hn[c]);
-            float r = xf * vd_dh(a.ho, a.hn, c);
-            if (a.ea2[t]) { a2 = a2 - a.ea2[t][c]; r = r + a.ea2[t][c] * xf; }
-            if (a.ea4[t]) r = r + a.ea4[t][c];
-            a.var[t][c] = inc_add<S>(x, r / a2);
-        }
+    if (a.nz == 1) {
+        vd_single_layer(a, c);
         return;
     }
     if (a.mask[c] != 1) return;
@@ -767,45 +859,71 @@ __global__ void vd_prepare_kernel(int nx_, int ny_, int nz, long long plane, dou
     auxn[p] = cnpar * x / (dzn[c + (k + 1) * plane] + dzn[c + k * plane]);
 }
 
-template <typename T>
-static int vd_launch(VDArgs<T>& a, cudaStream_t stream)
+static bool vd_sources(const VDArgs<float>& a)
 {
-    if (a.work) {
-        dim3 grid(getm_div_up(a.nx_, 128), a.ny_);
-        if constexpr (getm_increment_form<T>) {
-            if (a.nz > 1 && !a.auxo && vd_seg_applies(a.nz)) return vd_seg_launch(a, stream);
-            if (a.nz > 1 && !a.auxo) {
-                const int rows = getm_tune(GETM_TUNE_COLUMN_ROWS);
-                const dim3 grid(getm_div_up(a.nx_, 32), getm_div_up(a.ny_, rows)), block(32, rows);
-                bool src = false;
-                for (int t = 0; t < a.ntracer; t++) src = src || a.ea2[t] || a.ea4[t];
-                const bool pairs = a.ntracer > 1;
-                if (src && pairs) vd_inc_kernel<true, true><<<grid, block, 0, stream>>>(a);
-                else if (src) vd_inc_kernel<true, false><<<grid, block, 0, stream>>>(a);
-                else if (pairs) vd_inc_kernel<false, true><<<grid, block, 0, stream>>>(a);
-                else vd_inc_kernel<false, false><<<grid, block, 0, stream>>>(a);
-                GETM_CHECK_LAUNCH();
-                return GETM_OK;
-            }
-        }
-        vd_column_kernel<T, true><<<grid, 128, 0, stream>>>(a);
+    for (int t = 0; t < a.ntracer; t++)
+        if (a.ea2[t] || a.ea4[t]) return true;
+    return false;
+}
+
+static int vd_launch(VDArgs<float>& a, cudaStream_t stream)
+{
+    if (a.work && a.nz > 1) {
+        if (vd_seg_applies(a.nz)) return vd_seg_launch(a, stream);
+        const int rows = getm_tune(GETM_TUNE_COLUMN_ROWS);
+        const dim3 grid(getm_div_up(a.nx_, 32), getm_div_up(a.ny_, rows)), block(32, rows);
+        const bool src = vd_sources(a), pairs = a.ntracer > 1;
+        if (src && pairs) vd_inc_kernel<true, true><<<grid, block, 0, stream>>>(a);
+        else if (src) vd_inc_kernel<true, false><<<grid, block, 0, stream>>>(a);
+        else if (pairs) vd_inc_kernel<false, true><<<grid, block, 0, stream>>>(a);
+        else vd_inc_kernel<false, false><<<grid, block, 0, stream>>>(a);
         GETM_CHECK_LAUNCH();
         return GETM_OK;
     }
     int threads = 128;
-    const size_t per = (size_t)vd_smem_arrays<T> * a.nz * sizeof(T);
+    const size_t per = (size_t)VD_SMEM_ARRAYS * a.nz * sizeof(float);
     while (threads > 32 && per * threads > 160 * 1024) threads /= 2;
     size_t smem = per * threads;
     if (smem > 200 * 1024) return GETM_ERR_NZ;
     static bool attr_set = false;
     if (!attr_set) {
-        cudaFuncSetAttribute(vd_column_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        cudaFuncSetAttribute(vd_column_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         attr_set = true;
     }
     dim3 grid(getm_div_up(a.nx_, threads), a.ny_);
-    vd_column_kernel<T, false><<<grid, threads, smem, stream>>>(a);
+    vd_column_kernel<<<grid, threads, smem, stream>>>(a);
     GETM_CHECK_LAUNCH();
     return GETM_OK;
+}
+
+template <bool SRC>
+static int vd_f64_launch_one(VDArgs<double>& a, int rows, size_t smem, cudaStream_t stream)
+{
+    if (smem > 48 * 1024 && cudaFuncSetAttribute(vd_f64_kernel<SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 200 * 1024) != cudaSuccess)
+        return GETM_ERR_CUDA;
+    const dim3 grid(getm_div_up(a.nx_, 32), getm_div_up(a.ny_, rows)), block(32, rows);
+    vd_f64_kernel<SRC><<<grid, block, smem, stream>>>(a);
+    GETM_CHECK_LAUNCH();
+    return GETM_OK;
+}
+
+// FP64 form: blocks of fewer rows where four would leave SMs without work (an
+// SM's FP64 pipe is the bound, so the columns are spread over all).
+static int vd_launch(VDArgs<double>& a, cudaStream_t stream)
+{
+    bool src = false;
+    for (int t = 0; t < a.ntracer; t++) src = src || a.ea2[t] || a.ea4[t];
+    int rows = 4;
+    while (rows > 1 && (long long)getm_div_up(a.nx_, 32) * getm_div_up(a.ny_, rows) < 4 * GETM_SMS) rows /= 2;
+    size_t smem = 0;
+    if (!a.work && a.nz > 1) {
+        const size_t per = (size_t)2 * a.nz * 32 * sizeof(double);  // per row of 32 columns
+        while (rows > 1 && per * rows > 160 * 1024) rows /= 2;
+        smem = per * rows;
+        if (smem > 200 * 1024) return GETM_ERR_NZ;
+    }
+    return src ? vd_f64_launch_one<true>(a, rows, smem, stream) : vd_f64_launch_one<false>(a, rows, smem, stream);
 }
 
 extern "C" int getm_vertical_diffusion_create(getm_grid* tgrid, getm_vertical_diffusion** out)
@@ -894,7 +1012,7 @@ static int vd_batch_impl(int nx, int ny, int nz, const int* mask, const T* nuh, 
             a.ea4[t] = ea4 ? ea4[done + t] : NULL;
         }
         int rc;
-        if constexpr (std::is_same<T, S>::value) rc = vd_launch<T>(a, stream);
+        if constexpr (std::is_same<T, S>::value) rc = vd_launch(a, stream);
         else rc = vd_launch_f64s(a, stream);
         if (rc) return rc;
         done += n;

@@ -101,3 +101,62 @@ def test_vertical_pass_columns(nx, ny, nz, scheme, wmax):
         for a, b in zip(trd, tro):
             close(host(a.all_values), b, rtol=1e-13)
         close(host(ad.h), ao.h, rtol=RTOL)
+
+
+def _diffuse_extended(x, nuh, ho, hn, dt, mol, cnpar, ea2, ea4):
+    """diffusion.F90:135-314 of columns [k, n] in numpy's widest float."""
+    x, nuh, ho, hn = (np.asarray(a, dtype=np.longdouble) for a in (x, nuh, ho, hn))
+    nz, zero = x.shape[0], np.zeros_like(x[:1])
+    c = 2 * np.longdouble(dt) * (nuh[1:-1] + np.longdouble(mol))
+    ao, an = (1 - np.longdouble(cnpar)) * c / (ho[1:] + ho[:-1]), np.longdouble(cnpar) * c / (hn[1:] + hn[:-1])
+    up, lo = np.concatenate([an, zero]), np.concatenate([zero, an])
+    flux = ao * np.diff(x, axis=0)
+    diag = hn + up + lo - (0 if ea2 is None else ea2)
+    rhs = x * ho + np.concatenate([flux, zero]) - np.concatenate([zero, flux]) + (0 if ea4 is None else ea4)
+    r, q = np.zeros_like(x), np.zeros_like(x)
+    rk = qk = zero[0]
+    for k in range(nz - 1, -1, -1):
+        den = diag[k] - up[k] * rk
+        r[k], q[k] = rk, qk = lo[k] / den, (rhs[k] + up[k] * qk) / den
+    for k in range(1, nz):
+        q[k] += r[k] * q[k - 1]
+    return q.astype(np.float64)
+
+
+@pytest.mark.parametrize("nx,ny,nz,cnpar,sources", [(3, 3, 1, 1.0, True), (29, 9, 2, 1.0, False), (28, 8, 3, 0.6, True),
+                                                    (61, 20, 40, 1.0, True), (60, 5, 255, 0.6, False)])
+def test_column_solve_levels(nx, ny, nz, cnpar, sources):
+    """Fused, prepared and workspace-free solves of one to 255 levels, against
+    the same system solved in extended precision (the oracle's own sweep loses
+    digits to strong mixing).  A row of the elimination rounds about six times,
+    and strong mixing carries a level's error to all: 6 nz u, and ten for the
+    rest."""
+    from getm_gb300 import operators
+    from getm_gb300._lib import call
+    from getm_gb300.core import CENTERS, INTERFACES
+
+    Th, To, Td, rng = setup(nz=nz, seed=nz, nx=nx, ny=ny)
+    rtol = (10 + 6 * nz) * 1.2e-16
+    nuh = 10.0 ** rng.uniform(-6, -1, (nz + 1, Th.ny_, Th.nx_))
+    t = rng.uniform(5.0, 10.0, (nz, Th.ny_, Th.nx_))
+    t[:, Th.mask == 0] = np.nan
+    ea2 = -rng.uniform(0, 0.1, t.shape) if sources else None
+    ea4 = rng.uniform(0, 0.1, t.shape) if sources else None
+    water = Th.mask != 0
+    for use_ho in (False, True):
+        to = _diffuse_extended(t[:, water], nuh[:, water], (To.ho if use_ho else To.hn)[:, water], To.hn[:, water], 600.0,
+                               1e-6, cnpar, *[None if e is None else e[:, water] for e in (ea2, ea4)])
+        vd = operators.VerticalDiffusion(Td, cnpar)
+        nd = wrap(Td, nuh, INTERFACES)
+        e2, e4 = [None if e is None else wrap(Td, e, CENTERS) for e in (ea2, ea4)]
+        fused, other, prepared, bare = [wrap(Td, t, CENTERS) for _ in range(4)]
+        vd.batch(nd, 600.0, [fused, other], [1e-6, 1e-6], [e2, e2], [e4, e4], use_ho)
+        vd.prepare(nd, 600.0, 1e-6, use_ho)
+        vd.apply(prepared, e2, e4, use_ho)
+        arr = lambda *x: operators._lib.ptr_array([None if a is None else a.all_values.data_ptr() for a in x])  # noqa: E731
+        mol = (operators.ctypes.c_double * 1)(1e-6)
+        call("getm_vertical_diffusion_batch", Td.nx_, Td.ny_, nz, Td.mask.all_values.data_ptr(), nd.all_values.data_ptr(),
+             600.0, cnpar, (Td.ho if use_ho else Td.hn).all_values.data_ptr(), Td.hn.all_values.data_ptr(), 1, mol,
+             arr(bare), arr(e2), arr(e4), None, operators._s())
+        for got in (fused, other, prepared, bare):
+            close(host(got.all_values)[:, water], to, rtol=rtol)
