@@ -7,12 +7,11 @@
 //   1. thread per T column: vertical harmonic-mean slopes dR, dZ (kept in a
 //      register window, never stored) and the column pressure integral P,
 //      written to a caller-provided 3D work array;
-//   2. thread per (i, j, k) U/V point: horizontal harmonic-mean slopes from
-//      the three raw differences around the point, the density-Jacobian
-//      correction FC and the gradient.  The reference's per-level dZx/dRx
-//      work arrays are recomputed in registers (same operations, same values);
-//      the mixed form forms each raw difference once per 32 x 8 tile in
-//      shared memory.
+//   2. 32 x 8 tiles of one level: every raw horizontal difference (mixed form)
+//      and every harmonic-mean slope (FP64 form) is formed once into shared
+//      memory, then the density-Jacobian correction FC and the gradient.  (The
+//      all-float form recomputes the slopes per point in registers.)
+// The FP64 form is bound by GB300's FP64 rate; its slopes divide by getm_rcp.
 #include "getm_common.cuh"
 
 // ---------------------------------------------------------------------------
@@ -104,6 +103,20 @@ __device__ __forceinline__ T smcw_harm_cut(T a, T b)
     return (cff > T(SMCW_EPS)) ? cff / (a + b) : T(0);
 }
 
+// The same in FP64 without a division: 2 a b / (a + b) from one reciprocal.
+__device__ __forceinline__ double smcw_harm_d(double a, double b)
+{
+    return getm_twice(__dmul_rn(__dmul_rn(a, b), getm_rcp(__dadd_rn(a, b))));
+}
+
+__device__ __forceinline__ double smcw_harm_cut_d(double a, double b)
+{
+    const double p = __dmul_rn(a, b);
+    // 2 p > SMCW_EPS (false for NaN), on the integer pipe
+    if (!getm_positive_i(p) || __double_as_longlong(p) <= __double_as_longlong(0.5 * SMCW_EPS)) return 0.0;
+    return getm_twice(__dmul_rn(p, getm_rcp(__dadd_rn(a, b))));
+}
+
 // Phase 1 (internal_pressure.F90:80-118): column pressure integral P.
 // Columns with mask > 0 over C i in [ilo, ihi+1], j in [jlo, jhi+1].
 template <typename T>
@@ -111,9 +124,8 @@ __global__ void smcw_column_kernel(int nx, int ny, int nz, int ilo, int ihi, int
                                    const int* mask, const double* h, const double* zc,
                                    const T* buoy, double* Pw)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int j = blockIdx.y + jlo;
-    if (i < ilo || i > ihi + 1 || j > jhi + 1) return;
+    int i, j;
+    if (!getm_flat_column(nx, jlo, jhi - jlo + 2, i, j) || i < ilo || i > ihi + 1) return;
     const long long P = (long long)nx * ny;
     const long long p = (long long)j * nx + i;
     if (mask[p] <= 0) return;
@@ -128,28 +140,31 @@ __global__ void smcw_column_kernel(int nx, int ny, int nz, int ilo, int ihi, int
     Pw[p + (long long)(nz - 1) * P] = Pk;
     if (nz == 1) return;
     // window at level k+1 = nz: HR(nz) uses d(nz) = d(nz-1) and d(nz-1)
-    double bk1 = B(nz), zk1 = Z(nz);          // v(k+1)
+    double bk1 = B(nz);                       // v(k+1)
     double bk = B(nz - 1), zk = Z(nz - 1);    // v(k)
-    double dRk = bk1 - bk, dZk = zk1 - zk;    // d(k) with k = nz-1
-    double HR1 = smcw_harm_cut<double>(dRk, dRk);     // HR(nz): d(nz) = d(nz-1)
-    double HZ1 = 2.0 * dZk * dZk / (dZk + dZk);
+    double dRk = bk1 - bk, dZk = Z(nz) - zk;  // d(k) with k = nz-1
+    double HR1 = smcw_harm_cut_d(dRk, dRk);   // HR(nz): d(nz) = d(nz-1)
+    double HZ1 = smcw_harm_d(dZk, dZk);
+    // v(k-1), loaded one level ahead
+    double bn = nz > 2 ? B(nz - 2) : 0.0, zn = nz > 2 ? Z(nz - 2) : 0.0;
     for (int k = nz - 1; k >= 1; k--) {
         // d(k-1): for k == 1 it is d(0) = d(1)
-        double dRm, dZm, bkm1 = 0.0, zkm1 = 0.0;
+        double dRm, dZm;
+        const double bkm1 = bn, zkm1 = zn;
+        if (k > 2) { bn = B(k - 2); zn = Z(k - 2); }
         if (k > 1) {
-            bkm1 = B(k - 1); zkm1 = Z(k - 1);
             dRm = bk - bkm1; dZm = zk - zkm1;
         } else {
             dRm = dRk; dZm = dZk;
         }
-        double HR0 = smcw_harm_cut<double>(dRk, dRm);   // HR(k)
-        double HZ0 = 2.0 * dZk * dZm / (dZk + dZm);
-        Pk = Pk + 0.5 * ((bk1 + bk) * (zk1 - zk) - 0.2 * ((HR1 - HR0) * (zk1 - zk - x * (HZ1 + HZ0))
-                  - (HZ1 - HZ0) * (bk1 - bk - x * (HR1 + HR0))));
+        const double HR0 = smcw_harm_cut_d(dRk, dRm);   // HR(k)
+        const double HZ0 = smcw_harm_d(dZk, dZm);
+        const double corr = (HR1 - HR0) * (dZk - x * (HZ1 + HZ0)) - (HZ1 - HZ0) * (dRk - x * (HR1 + HR0));
+        Pk = Pk + 0.5 * ((bk1 + bk) * dZk - 0.2 * corr);
         Pw[p + (long long)(k - 1) * P] = Pk;
         // shift: level k becomes k+1
         HR1 = HR0; HZ1 = HZ0;
-        bk1 = bk; zk1 = zk; bk = bkm1; zk = zkm1;
+        bk1 = bk; bk = bkm1; zk = zkm1;
         dRk = dRm; dZk = dZm;
     }
 #undef B
@@ -195,6 +210,105 @@ __global__ void smcw_gradient_kernel(int nx, int ny, int nz, int ilo, int ihi, i
         T* out = dir ? idpdy : idpdx;
         out[q] = (T)(0.5 * (h[q] + h[q + s]) * id)
                  * ((T)(Pw[q + s] - Pw[q]) + FC - (T)(z[p + s] - z[p]) * T(0.5) * (buoy[qtop + s] + buoy[qtop]));
+    }
+}
+
+// Phase 2 in FP64, on 32 x SG_BY tiles of SG_KB levels.  Bound by FP64
+// instructions: the harmonic means (two per point and direction, shared by the
+// two faces beside the point) take six each instead of two divisions' worth
+// per face, and the raw differences are formed once; the surface term and the
+// metrics are loaded once for the tile's levels.  About 64 FP64 instructions per
+// point against some 250.  251 x 187 x 33: 438 -> 218 us here, 139 -> 100 us in the
+// column sweep; error against quad precision 6.1e-16 before and after.
+constexpr int SG_BX = 32, SG_BY = 8;
+constexpr int SG_KB = 4;
+
+__global__ void __launch_bounds__(SG_BX* SG_BY, 3) smcw_gradient_f64_kernel(
+    int nx, int ny, int nz, int ilo, int ihi, int jlo, int jhi, const int* __restrict__ umask,
+    const int* __restrict__ vmask, const double* __restrict__ idxu, const double* __restrict__ idyv,
+    const double* __restrict__ h, const double* __restrict__ z, const double* __restrict__ zc,
+    const double* __restrict__ buoy, const double* __restrict__ Pw, double* __restrict__ idpdx,
+    double* __restrict__ idpdy)
+{
+    // raw differences across the x faces of columns i0-1 .. i0+SG_BX and the y
+    // faces of rows j0-1 .. j0+SG_BY (zero where the mask is not positive);
+    // harmonic means at columns i0 .. i0+SG_BX and rows j0 .. j0+SG_BY
+    __shared__ double dZx[SG_BY][SG_BX + 2], dRx[SG_BY][SG_BX + 2], dZy[SG_BY + 2][SG_BX], dRy[SG_BY + 2][SG_BX];
+    __shared__ double hZx[SG_BY][SG_BX + 1], hRx[SG_BY][SG_BX + 1], hZy[SG_BY + 1][SG_BX], hRy[SG_BY + 1][SG_BX];
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const int i0 = blockIdx.x * SG_BX, j0 = jlo + blockIdx.y * SG_BY;
+    const int i = i0 + tx, j = j0 + ty;
+    const long long P = (long long)nx * ny;
+    const long long p = (long long)j * nx + i;
+    const bool rowin = j <= jhi, colin = i >= ilo && i <= ihi;
+    // this thread's own faces, and the extra ones: x faces at columns i0-1 and
+    // i0+SG_BX of every row by the last warp (lane 2r + side: row r), y faces at
+    // rows j0-1 (ty 0) and j0+SG_BY (ty 1)
+    const bool fx = rowin && i >= ilo - 1 && i <= ihi + 1 && umask[p] > 0;
+    const bool fy = colin && j <= jhi + 1 && vmask[p] > 0;
+    const int er = tx >> 1, eside = tx & 1;
+    const long long ep = (long long)(j0 + er) * nx + (eside == 0 ? i0 - 1 : i0 + SG_BX);
+    bool ex = false, ey = false;
+    if (ty == SG_BY - 1 && tx < 2 * SG_BY) {
+        const int ii = eside == 0 ? i0 - 1 : i0 + SG_BX;
+        ex = j0 + er <= jhi && ii >= ilo - 1 && ii <= ihi + 1 && umask[ep] > 0;
+    }
+    const int jj = ty == 0 ? j0 - 1 : j0 + SG_BY;
+    const long long yp = (long long)jj * nx + i;
+    if (ty < 2) ey = colin && jj <= jhi + 1 && vmask[yp] > 0;
+    const bool ux = rowin && colin && umask[p] == 1, vy = rowin && colin && vmask[p] == 1;
+    const long long qtop = p + (long long)(nz - 1) * P;
+    double surfx = 0.0, surfy = 0.0, ix = 0.0, iy = 0.0;
+    if (ux) {
+        surfx = (z[p + 1] - z[p]) * getm_half(buoy[qtop + 1] + buoy[qtop]);
+        ix = idxu[p];
+    }
+    if (vy) {
+        surfy = (z[p + nx] - z[p]) * getm_half(buoy[qtop + nx] + buoy[qtop]);
+        iy = idyv[p];
+    }
+    const int kend = min(nz, ((int)blockIdx.z + 1) * SG_KB);
+    for (int k = blockIdx.z * SG_KB; k < kend; k++) {
+        const long long kP = (long long)k * P, q = p + kP;
+        double rzx = 0.0, rrx = 0.0, rzy = 0.0, rry = 0.0;
+        if (fx) { rzx = zc[q + 1] - zc[q]; rrx = buoy[q + 1] - buoy[q]; }
+        if (fy) { rzy = zc[q + nx] - zc[q]; rry = buoy[q + nx] - buoy[q]; }
+        if (k > (int)blockIdx.z * SG_KB) __syncthreads();  // the previous level's reads are done
+        dZx[ty][tx + 1] = rzx; dRx[ty][tx + 1] = rrx;
+        dZy[ty + 1][tx] = rzy; dRy[ty + 1][tx] = rry;
+        if (ty == SG_BY - 1 && tx < 2 * SG_BY) {
+            const long long eq = ep + kP;
+            dZx[er][eside == 0 ? 0 : SG_BX + 1] = ex ? zc[eq + 1] - zc[eq] : 0.0;
+            dRx[er][eside == 0 ? 0 : SG_BX + 1] = ex ? buoy[eq + 1] - buoy[eq] : 0.0;
+        }
+        if (ty < 2) {
+            const long long yq = yp + kP;
+            dZy[ty == 0 ? 0 : SG_BY + 1][tx] = ey ? zc[yq + nx] - zc[yq] : 0.0;
+            dRy[ty == 0 ? 0 : SG_BY + 1][tx] = ey ? buoy[yq + nx] - buoy[yq] : 0.0;
+        }
+        __syncthreads();
+        hZx[ty][tx] = smcw_harm_cut_d(dZx[ty][tx], rzx);
+        hRx[ty][tx] = smcw_harm_cut_d(dRx[ty][tx], rrx);
+        hZy[ty][tx] = smcw_harm_cut_d(dZy[ty][tx], rzy);
+        hRy[ty][tx] = smcw_harm_cut_d(dRy[ty][tx], rry);
+        if (ty == 0) {  // the row north of the tile
+            hZy[SG_BY][tx] = smcw_harm_cut_d(dZy[SG_BY][tx], dZy[SG_BY + 1][tx]);
+            hRy[SG_BY][tx] = smcw_harm_cut_d(dRy[SG_BY][tx], dRy[SG_BY + 1][tx]);
+        }
+        if (ty == 1 && tx < 2 * SG_BY) {  // the column east of it: lane 2r + (0: heights, 1: buoyancy)
+            const double(*d)[SG_BX + 2] = eside == 0 ? dZx : dRx;
+            (eside == 0 ? hZx : hRx)[er][SG_BX] = smcw_harm_cut_d(d[er][SG_BX], d[er][SG_BX + 1]);
+        }
+        __syncthreads();
+        const double x = 1.0 / 12.0;
+        auto gradient = [&](double rz, double rr, double z0, double z1, double r0, double r1, long long s, double surf,
+                            double id) {
+            const double corr = (r1 - r0) * (rz - x * (z1 + z0)) - (z1 - z0) * (rr - x * (r1 + r0));
+            const double FC = getm_half((buoy[q + s] + buoy[q]) * rz - 0.2 * corr);
+            return getm_half(h[q] + h[q + s]) * id * ((Pw[q + s] - Pw[q]) + FC - surf);
+        };
+        if (ux) idpdx[q] = gradient(rzx, rrx, hZx[ty][tx], hZx[ty][tx + 1], hRx[ty][tx], hRx[ty][tx + 1], 1, surfx, ix);
+        if (vy) idpdy[q] = gradient(rzy, rry, hZy[ty][tx], hZy[ty + 1][tx], hRy[ty][tx], hRy[ty + 1][tx], nx, surfy, iy);
     }
 }
 
@@ -272,7 +386,6 @@ __global__ void smcw_column_mixed_kernel(int nx, int ny, int nz, int ilo, int ih
 // points that use them); a point keeps the FP64 differences of its own faces
 // for the density-Jacobian term.  The values are those of the per-point
 // form, operation for operation.
-constexpr int SG_BX = 32, SG_BY = 8;
 
 struct SgFace {
     float rz, rr;   // gated float differences (zero where the mask is not positive)
@@ -410,11 +523,18 @@ static int smcw_impl(int nx, int ny, int nz, int imin, int imax, int jmin, int j
     if (nx < 1 || ny < 1 || nz < 1 || imin < 2 || jmin < 2 || imax + 2 > nx || jmax + 2 > ny || jmax < jmin) return GETM_ERR_ARG;
     if (!mask || !umask || !vmask || !idxu || !idyv || !h || !z || !zc || !buoy || !idpdx || !idpdy || !P_work)
         return GETM_ERR_ARG;
-    dim3 g1(getm_div_up(nx, 128), jmax - jmin + 2);
+    const unsigned g1 = getm_div_up((long long)nx * (jmax - jmin + 2), 128);
     smcw_column_kernel<T><<<g1, 128, 0, stream>>>(nx, ny, nz, imin - 1, imax - 1, jmin - 1, jmax - 1, mask, h, zc, buoy, P_work);
     GETM_CHECK_LAUNCH();
-    dim3 g2(getm_div_up(nx, 128), jmax - jmin + 1, nz);
-    smcw_gradient_kernel<T><<<g2, 128, 0, stream>>>(nx, ny, nz, imin - 1, imax - 1, jmin - 1, jmax - 1, umask, vmask, idxu, idyv, h, z, zc, buoy, P_work, idpdx, idpdy);
+    if constexpr (std::is_same<T, double>::value) {
+        dim3 g2(getm_div_up(nx, SG_BX), getm_div_up(jmax - jmin + 1, SG_BY), getm_div_up(nz, SG_KB));
+        smcw_gradient_f64_kernel<<<g2, dim3(SG_BX, SG_BY), 0, stream>>>(nx, ny, nz, imin - 1, imax - 1, jmin - 1,
+                                                                        jmax - 1, umask, vmask, idxu, idyv, h, z, zc,
+                                                                        buoy, P_work, idpdx, idpdy);
+    } else {
+        dim3 g2(getm_div_up(nx, 128), jmax - jmin + 1, nz);
+        smcw_gradient_kernel<T><<<g2, 128, 0, stream>>>(nx, ny, nz, imin - 1, imax - 1, jmin - 1, jmax - 1, umask, vmask, idxu, idyv, h, z, zc, buoy, P_work, idpdx, idpdy);
+    }
     GETM_CHECK_LAUNCH();
     return GETM_OK;
 }

@@ -160,3 +160,36 @@ def test_column_solve_levels(nx, ny, nz, cnpar, sources):
              arr(bare), arr(e2), arr(e4), None, operators._s())
         for got in (fused, other, prepared, bare):
             close(host(got.all_values)[:, water], to, rtol=rtol)
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(3, 3, 1), (30, 8, 2), (31, 9, 4), (33, 16, 5), (64, 7, 13)])
+def test_internal_pressure_tiles(nx, ny, nz):
+    """Around the tiles of 32 columns, 8 rows and 4 levels.  The gradient is a
+    difference of column integrals P of nz terms, each rounded some ten times;
+    with the Jacobian's own ten that is 10 (nz + 2) u of the largest P, times the
+    thickness and the inverse spacing."""
+    import oracle.oracle as O
+    import torch
+    from getm_gb300 import _pygetm
+    from getm_gb300.core import CENTERS, Array
+
+    Th, To, Td, rng = setup(nz=nz, seed=nx + nz, nx=nx, ny=ny)
+    for g, d in ((To, Td),):
+        hn = np.where(Th.mask != 0, g.hn, 0.0)
+        zf = np.concatenate([0 * hn[:1], hn.cumsum(axis=0)]) - np.where(Th.mask != 0, g.D, 0.0)
+        g.zc[...] = 0.5 * (zf[1:] + zf[:-1])
+        d.zc.all_values.copy_(torch.from_numpy(g.zc))
+    z = rng.uniform(-0.3, 0.3, To.D.shape)
+    b = np.sort(rng.uniform(-0.05, 0.0, (nz,) + z.shape), axis=0)
+    b[:, Th.mask == 0] = np.nan
+    ox, oy = np.zeros_like(b), np.zeros_like(b)
+    O.shchepetkin_mcwilliams(To, b, ox, oy, z)
+    Td.zin = Array(Td, torch.from_numpy(z).cuda())
+    gx, gy = Td.ugrid.array(z=CENTERS, fill=0.0), Td.vgrid.array(z=CENTERS, fill=0.0)
+    _pygetm.shchepetkin_mcwilliams(wrap(Td, b, CENTERS), gx, gy)
+    hmax = hn.max()
+    scale = 0.05 * hn.sum(axis=0).max() * hmax / 1000.0
+    for got, want in ((gx, ox), (gy, oy)):
+        err = np.abs(host(got.all_values) - want)
+        assert np.isfinite(err).all()
+        assert err.max() <= 10 * (nz + 2) * 1.2e-16 * scale
