@@ -210,13 +210,13 @@ __global__ void __launch_bounds__(256) hpass_x_inc_kernel(HPassArgs<S, V> a)
     hpass_x_inc_rows<S, 1, NoEpi, V, C>(a, blockIdx.x, j, blockIdx.z, threadIdx.x);
 }
 
-// grid (1, ceil(ny_ / rows), nk): warp (ty) of block (0, y, k) sweeps row j = rows y + ty of layer k
+// grid (1, y, nk): each warp of block (0, y, k) sweeps nrow rows of layer k
 template <typename S, typename V = S>
-__global__ void __launch_bounds__(256) hpass_x_vec_kernel(HPassArgs<S, V> a)
+__global__ void __launch_bounds__(256) hpass_x_vec_kernel(HPassArgs<S, V> a, int nrow)
 {
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (j >= a.ny_) return;  // whole warp
-    hpass_x_vec_row<S, V>(a, j, blockIdx.z, threadIdx.x);
+    const int j0 = (blockIdx.y * blockDim.y + threadIdx.y) * nrow;
+    if (j0 >= a.ny_) return;  // whole warp
+    hpass_x_vec_rows<S, V>(a, j0, min(nrow, a.ny_ - j0), blockIdx.z, threadIdx.x);
 }
 
 // The four-cells-per-lane x pass applies: rows of whole 16-byte vectors and
@@ -266,8 +266,13 @@ static int launch_hpass_c(int direction, HPassArgs<S, V>& a, cudaStream_t stream
         // geometry once for all fields where the sweep repeats it per pair
         if constexpr (!f64) vec = getm_tune(GETM_TUNE_XPASS_VEC) && xpass_vec_ok(a);
         if (vec) {
-            dim3 grid(1, getm_div_up(a.ny_, rows), a.nk);
-            if constexpr (!f64) hpass_x_vec_kernel<S, V><<<grid, block, 0, stream>>>(a);
+            // rows per warp: as many (up to four) as leave 16 warps per SM; at
+            // most two warps per block, so that the last wave of blocks is short
+            int nrow = 4;
+            while (nrow > 1 && (long long)getm_div_up(a.ny_, nrow) * a.nk < 16 * GETM_SMS) nrow /= 2;
+            block.y = rows < 2 ? rows : 2;
+            dim3 grid(1, getm_div_up(getm_div_up(a.ny_, nrow), block.y), a.nk);
+            if constexpr (!f64) hpass_x_vec_kernel<S, V><<<grid, block, 0, stream>>>(a, nrow);
         } else {
             // lane 0 of the first segment handles the face west of cell 0
             dim3 grid(getm_div_up(a.nx_ + 1, HX_STRIDE), getm_div_up(a.ny_, rows), a.nk);

@@ -352,13 +352,17 @@ __device__ __forceinline__ void hpass_x_inc_rows(const HPassArgs<S, V>& a, int b
 }
 
 // x pass in increment form with four cells per lane, for the 3D passes.  A
-// warp sweeps one row (layer k, row j) from west to east in chunks of 128
-// cells; lane L of a chunk owns cells i0 + 4L .. i0 + 4L + 3 and their east
-// faces, so every load and store of the lane is one 16-byte vector (two for
-// doubles) at an aligned address (the caller checks nx_ % 4 == 0 and the
-// pointers' alignment).  A face needs the values of the lanes beside it
-// (shuffles), the chunk to the west hands its last face over in registers,
-// and the last lane reads the two cells east of the chunk.  Each difference
+// warp sweeps nrow rows of a layer from west to east, one behind the other, in
+// chunks of 128 cells; lane L of a chunk owns four cells and their east faces,
+// so every load and store of the lane is one 16-byte vector (two for doubles)
+// at an aligned address (the caller checks nx_ % 4 == 0 and the pointers'
+// alignment).  Rows are contiguous, so a chunk may end one row and begin the
+// next: with at least two halo cells no face or cell that is used looks across
+// that seam, and only a warp's last chunk has idle lanes (a 404-cell row by
+// itself fills 3.2 of its 4 chunks: 400 x 300 x 40, two FP64-stored tracers, 119 ->
+// 104 us, a float field 60 -> 55 us).  A face needs the values of the lanes
+// beside it (shuffles), the chunk to the west hands its last face over in
+// registers, and the last lane reads the two cells east of the chunk.  Each difference
 // of neighbouring values is formed once (it serves the face and, in the
 // limiter, both faces beside it: one FP64 subtraction per cell and field
 // instead of two for FP64 storage).  Every face and cell is evaluated with
@@ -392,29 +396,33 @@ __device__ __forceinline__ void xv_store4(T* p, const T (&v)[4])
     }
 }
 
-constexpr int XV_CHUNK = 128;
-
 template <typename S, typename V = S>
-__device__ __forceinline__ void hpass_x_vec_row(const HPassArgs<S, V>& a, int j, int k, int lane)
+__device__ __forceinline__ void hpass_x_vec_rows(const HPassArgs<S, V>& a, int j0, int nrow, int k, int lane)
 {
     constexpr unsigned FULL = 0xffffffffu;
     const int nx = a.nx_;
-    const long long r2 = (long long)j * nx;
+    const int nq = nx / 4;  // quads of cells per row
+    const int total = nq * nrow;
+    const long long r2 = (long long)j0 * nx;
     const long long r3 = (long long)k * a.plane + r2;
-    const bool jrow = j >= a.jlo && j <= a.jhi;
     const int ngroup = a.ntracer > 0 ? (a.ntracer + 1) / 2 : 1;
     for (int g = 0; g < ngroup; g++) {
         const int t0 = 2 * g;
         const int nt = a.ntracer - t0 >= 2 ? 2 : a.ntracer - t0;  // 0 with no fields
         // the west face of the chunk's first cell: the chunk to the west's
-        // last face (nothing west of the row: an inactive face)
+        // last face (nothing west of the rows: an inactive face)
         float cQU = 0.f;
         int cum = 0;
         float cd[2] = {0.f, 0.f}, cer[2] = {0.f, 0.f};
-        for (int i0 = 0; i0 < nx; i0 += XV_CHUNK) {
-            const int ib = i0 + 4 * lane;  // the lane's first cell and its east face
-            const bool lin = ib < nx;      // all four cells or none
-            const int ie = i0 + XV_CHUNK;  // the first cell east of the chunk
+        int row = lane / nq, iq = lane - row * nq;  // the lane's row and quad
+        for (int q0 = 0; q0 < total; q0 += 32) {
+            const int ib = 4 * (q0 + lane);  // the lane's first cell, from the first row's start
+            const int ic = 4 * iq;           // ... in its row
+            const bool lin = q0 + lane < total;  // all four cells or none
+            const int ie = 4 * (q0 + 32);        // the first cell east of the chunk
+            const bool ein = q0 + 32 < total;
+            const int j = j0 + row;
+            const bool jrow = j >= a.jlo && j <= a.jhi;
             int um[4] = {0, 0, 0, 0}, tm[4] = {0, 0, 0, 0};
             float dyf[4] = {0.f, 0.f, 0.f, 0.f}, idxf[4] = {0.f, 0.f, 0.f, 0.f}, iaf[4] = {0.f, 0.f, 0.f, 0.f};
             float ahraw[4] = {0.f, 0.f, 0.f, 0.f};
@@ -439,14 +447,14 @@ __device__ __forceinline__ void hpass_x_vec_row(const HPassArgs<S, V>& a, int j,
             // masks of the velocity points beside the lane's first and last faces
             int umW = __shfl_up_sync(FULL, um[3], 1), umE = __shfl_down_sync(FULL, um[0], 1);
             if (lane == 0) umW = cum;
-            if (lane == 31) umE = ie < nx ? a.umask[r2 + ie] : 0;
+            if (lane == 31) umE = ein ? a.umask[r2 + ie] : 0;
 
             // face geometry (the same expressions as hpass_x_inc_rows)
             float QU[4], cfl[4], ahd[4];
             bool up[4], uu_ok[4], act[4];
 #pragma unroll
             for (int m = 0; m < 4; m++) {
-                const int ia = ib + m;
+                const int ia = ic + m;
                 const bool f_in = lin && jrow && ia >= a.ilo - 1 && ia <= a.ihi;
                 act[m] = f_in && getm_flux_point(um[m]);
                 QU[m] = 0.f; cfl[m] = 0.f; ahd[m] = 0.f;
@@ -471,7 +479,7 @@ __device__ __forceinline__ void hpass_x_vec_row(const HPassArgs<S, V>& a, int j,
             double hnew[4];
 #pragma unroll
             for (int m = 0; m < 4; m++) {
-                const int c = ib + m;
+                const int c = ic + m;
                 upd[m] = lin && jrow && c >= a.ilo && c <= a.ihi && tm[m] == 1;
                 coef[m] = 0.f;
                 hnew[m] = hold[m];
@@ -490,8 +498,7 @@ __device__ __forceinline__ void hpass_x_vec_row(const HPassArgs<S, V>& a, int j,
                 if (lin) xv_load4(f + ib, fv);
                 S fE0 = S(0), fE1 = S(0);  // the two cells east of the chunk (last lane)
                 if (lane == 31) {
-                    if (ie < nx) fE0 = f[ie];
-                    if (ie + 1 < nx) fE1 = f[ie + 1];
+                    if (ein) { fE0 = f[ie]; fE1 = f[ie + 1]; }
                 }
                 S fn0 = __shfl_down_sync(FULL, fv[0], 1);
                 if (lane == 31) fn0 = fE0;
@@ -529,6 +536,7 @@ __device__ __forceinline__ void hpass_x_vec_row(const HPassArgs<S, V>& a, int j,
             }
             cQU = __shfl_sync(FULL, QU[3], 31);
             cum = __shfl_sync(FULL, um[3], 31);
+            for (iq += 32; iq >= nq; iq -= nq) row++;
         }
     }
 }
