@@ -42,7 +42,7 @@ constexpr int SS_BY = 16;
 constexpr int SS_THREADS = 32 * SS_BY;
 constexpr unsigned SS_SPIN_LIMIT = 1u << 22;
 
-__device__ __forceinline__ int div_up(int a, int b) { return (a + b - 1) / b; }
+__host__ __device__ inline int div_up(int a, int b) { return (a + b - 1) / b; }
 
 struct SubstepArgs {
     int nx, ny, halox, haloy;
@@ -197,10 +197,49 @@ __device__ __forceinline__ void coriolis_from(const SubstepArgs& a, int d, int i
                          j);
 }
 
+// The pointwise operations of phase ph + 1 (a constant where this is inlined)
+// at point p = (i, j); d1: the direction updated first.  Phase 4 has its
+// depth tiles besides, phase 6 its advection passes.
+template <bool MIXED>
+__device__ __forceinline__ void phase_point(const SubstepArgs& a, int ph, int d1, int i, int j, int p)
+{
+    using C = typename std::conditional<MIXED, float, double>::type;
+    const int nx = a.nx, ny = a.ny, d2 = 1 - d1;
+    const bool interior = i >= a.halox && i < nx - a.halox && j >= a.haloy && j < ny - a.haloy;
+    switch (ph) {
+    case 0:
+        if (interior) transport_update<MIXED>(a.tr[d1], a.dt, p);
+        break;
+    case 1:
+        coriolis_from<C>(a, d1, i, j);
+        if (interior) transport_update<MIXED>(a.tr[d2], a.dt, p);
+        break;
+    case 2:
+        coriolis_from<C>(a, d2, i, j);
+        if (a.accumulate) accumulate_2d_point(a.tr[0].U, a.tr[1].U, a.Ucum, a.Vcum, p);
+        surface_elevation_fused_point(nx, ny, a.halox, a.haloy, a.mT, a.dyU, a.dxV, a.iareaT, a.z, a.zo,
+                                      a.tr[0].U, a.tr[1].U, a.fwf, a.dt, i, j);
+        break;
+    case 3:
+        a.fwf[p] = a.pe[p];
+        if (i < nx - 1) interp_pair_point<double>(a.taux, a.tausx, p, 1, 0);
+        if (j < ny - 1) interp_pair_point<double>(a.tauy, a.tausy, p, nx, 0);
+        break;
+    case 4:
+        momentum_2d_velocities_point<C>(a.vel, i, j);
+        a.advD[0][p] = a.Dsrc[0][p];
+        a.advD[1][p] = a.Dsrc[1][p];
+        if (interior) spg_point<MIXED>(a.spg, p);
+        break;
+    default:
+        momentum_2d_friction_point<C>(a.fric, i, j);
+        break;
+    }
+}
+
 template <bool MIXED>
 __global__ void __launch_bounds__(SS_THREADS, MIXED ? 2 : 1) substep_2d_kernel(SubstepArgs a)
 {
-    using C = typename std::conditional<MIXED, float, double>::type;
     __shared__ SubstepSmem sm;
     __shared__ int s_ok;
     const int tx = threadIdx.x, ty = threadIdx.y;
@@ -215,35 +254,28 @@ __global__ void __launch_bounds__(SS_THREADS, MIXED ? 2 : 1) substep_2d_kernel(S
     const int n = nx * ny;  // < 2^30 (checked by the host)
     const int chunk = (n + (int)gridDim.x - 1) / (int)gridDim.x;
     const int pb = (int)blockIdx.x * chunk, pe = min(pb + chunk, n);
-    const int ilo = a.halox, ihi = nx - a.halox - 1, jlo = a.haloy, jhi = ny - a.haloy - 1;
+    const int jlo = a.haloy, jhi = ny - a.haloy - 1;
 
     unsigned target = 0;  // barrier count to wait for (thread 0)
     if (tx == 0 && ty == 0) s_ok = ld_acquire(&a.sync[2]) == 0;
     __syncthreads();
     if (!s_ok) return;
 
-    const int d1 = a.ufirst ? 0 : 1, d2 = 1 - d1;
+    const int d1 = a.ufirst ? 0 : 1;
+    auto points = [&](int ph) {
+        for (int p = pb + tid; p < pe; p += SS_THREADS) {
+            const int j = p / nx, i = p - j * nx;
+            phase_point<MIXED>(a, ph, d1, i, j, p);
+        }
+    };
     // 1: first transport update
-    for (int p = pb + tid; p < pe; p += SS_THREADS) {
-        const int j = p / nx, i = p - j * nx;
-        if (i >= ilo && i <= ihi && j >= jlo && j <= jhi) transport_update<MIXED>(a.tr[d1], a.dt, p);
-    }
+    points(0);
     if (!grid_barrier(a.sync, target, s_ok)) return grid_exit(a.sync);
     // 2: Coriolis from the first, second transport update
-    for (int p = pb + tid; p < pe; p += SS_THREADS) {
-        const int j = p / nx, i = p - j * nx;
-        coriolis_from<C>(a, d1, i, j);
-        if (i >= ilo && i <= ihi && j >= jlo && j <= jhi) transport_update<MIXED>(a.tr[d2], a.dt, p);
-    }
+    points(1);
     if (!grid_barrier(a.sync, target, s_ok)) return grid_exit(a.sync);
     // 3: Coriolis from the second, cumulative transports, surface elevation
-    for (int p = pb + tid; p < pe; p += SS_THREADS) {
-        const int j = p / nx, i = p - j * nx;
-        coriolis_from<C>(a, d2, i, j);
-        if (a.accumulate) accumulate_2d_point(a.tr[0].U, a.tr[1].U, a.Ucum, a.Vcum, p);
-        surface_elevation_fused_point(nx, ny, a.halox, a.haloy, a.mT, a.dyU, a.dxV, a.iareaT, a.z, a.zo,
-                                      a.tr[0].U, a.tr[1].U, a.fwf, a.dt, i, j);
-    }
+    points(2);
     if (!grid_barrier(a.sync, target, s_ok)) return grid_exit(a.sync);
     // 4: depths; fwf = pe; wind stress on U and V (interp_x/y, offset 0)
     {
@@ -253,29 +285,13 @@ __global__ void __launch_bounds__(SS_THREADS, MIXED ? 2 : 1) substep_2d_kernel(S
             __syncthreads();
         }
     }
-    for (int p = pb + tid; p < pe; p += SS_THREADS) {
-        const int j = p / nx, i = p - j * nx;
-        a.fwf[p] = a.pe[p];
-        if (i < nx - 1) interp_pair_point<double>(a.taux, a.tausx, p, 1, 0);
-        if (j < ny - 1) interp_pair_point<double>(a.tauy, a.tausy, p, nx, 0);
-    }
+    points(3);
     if (!grid_barrier(a.sync, target, s_ok)) return grid_exit(a.sync);
     // 5: velocities, advected thicknesses, surface pressure gradient
-    for (int p = pb + tid; p < pe; p += SS_THREADS) {
-        const int j = p / nx, i = p - j * nx;
-        momentum_2d_velocities_point<C>(a.vel, i, j);
-        a.advD[0][p] = a.Dsrc[0][p];
-        a.advD[1][p] = a.Dsrc[1][p];
-        if (i >= ilo && i <= ihi && j >= jlo && j <= jhi) spg_point<MIXED>(a.spg, p);
-    }
+    points(4);
     if (!grid_barrier(a.sync, target, s_ok)) return grid_exit(a.sync);
     // 6: bottom friction; first advection passes
-    if (a.friction) {
-        for (int p = pb + tid; p < pe; p += SS_THREADS) {
-            const int j = p / nx, i = p - j * nx;
-            momentum_2d_friction_point<C>(a.fric, i, j);
-        }
-    }
+    if (a.friction) points(5);
     advection_pass<MIXED>(a.adv[0].pass[0], a.adv[0].dir[0], sm, tx, ty);
     advection_pass<MIXED>(a.adv[1].pass[0], a.adv[1].dir[0], sm, tx, ty);
     if (!grid_barrier(a.sync, target, s_ok)) return grid_exit(a.sync);
@@ -368,7 +384,7 @@ int substep_args(SubstepArgs& a, const getm_split2d_fields* f, int nx, int ny, i
                           f->mask_v, f->H_v, f->dx_v, f->idy_v, f->cor_v, f->z0b_v, f->D_v, f->alpha_v, f->work_v,
                           f->V, f->dpdy, f->tausy, f->corV, f->advV, f->diffV, f->dampV, f->SyA, f->SyB, f->SyD,
                           f->SyF, f->rv, f->v1, f->Vcum, f->advD_v, f->vua, f->vva,
-                          f->mask_x, f->H_x, f->D_x, f->work_x, f->D_uu, f->D_uv, f->D_vu, f->D_vv, f->sync};
+                          f->mask_x, f->H_x, f->D_x, f->work_x, f->D_uu, f->D_uv, f->D_vu, f->D_vv};
     for (const void* q : ptrs)
         if (!q) return GETM_ERR_ARG;
     memset(&a, 0, sizeof(a));
@@ -422,10 +438,160 @@ extern "C" int getm_split2d_substep(const getm_split2d_fields* f, int nx, int ny
                                     getm_grid* vugrid, getm_grid* vvgrid, int vadv_ufirst, cudaStream_t stream)
 {
     SubstepArgs a;
+    if (!f || !f->sync) return GETM_ERR_ARG;
     int rc = substep_args(a, f, nx, ny, halox, haloy, mixed, ufirst, accumulate, friction, timestep, Dmin, Dcrit,
                           uadv, ugrid, uugrid, uvgrid, uadv_ufirst, vadv, vgrid, vugrid, vvgrid, vadv_ufirst);
     if (rc) return rc;
     return mixed ? launch_substep<true>(a, stream) : launch_substep<false>(a, stream);
+}
+
+// ---------------------------------------------------------------------------
+// One substep as seven ordinary launches
+// ---------------------------------------------------------------------------
+// For a domain that shares the GPU with others (ensemble members and served
+// requests replay on several streams): a cooperative launch would need every
+// SM at once, and the operations launched one by one are twenty kernels of a
+// few microseconds each on such planes, bound by their launches (a 92 x 92
+// member: 512 launches per 3D step of 24 substeps, 3.4 us each in a CUDA graph).
+// Here each phase above is one kernel over the whole plane, with the same
+// device functions per point, so the results are those of substep_2d_kernel.
+// Blocks are small (64 threads for the points) so that a small plane spreads
+// over as many SMs as it can; U's and V's advection passes and the friction
+// share a launch (grid z).  Each kernel is launched while the one before still
+// runs (programmatic dependent launch) and waits for its end before it
+// touches memory; the first is launched in the ordinary way, since what
+// precedes it on the stream may be anything.
+namespace {
+
+constexpr int PH_PY = 2;  // rows of a point block
+constexpr int PH_DY = 4;  // rows of a depth tile
+constexpr int PH_XY = 4;  // rows of an x pass block
+
+__device__ __forceinline__ void phase_begin()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <bool MIXED, int PH>
+__global__ void __launch_bounds__(32 * PH_PY) phase_points_kernel(const __grid_constant__ SubstepArgs a)
+{
+    phase_begin();
+    const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * PH_PY + threadIdx.y;
+    if (i < a.nx && j < a.ny) phase_point<MIXED>(a, PH, a.ufirst ? 0 : 1, i, j, j * a.nx + i);
+}
+
+template <bool MIXED>
+__global__ void __launch_bounds__(32 * PH_DY) phase_depth_kernel(const __grid_constant__ SubstepArgs a)
+{
+    __shared__ double szh[PH_DY + 2][UD_BX + 2];
+    phase_begin();
+    const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * PH_DY + threadIdx.y;
+    if (i < a.nx && j < a.ny) phase_point<MIXED>(a, 3, 0, i, j, j * a.nx + i);
+    update_depth_2d_tile<PH_DY, MIXED>(a.depth, blockIdx.x, blockIdx.y, threadIdx.x, threadIdx.y, szh);
+}
+
+// Advection pass PASS in direction DIR of U (block z 0; d0 = 0) and V; block z
+// ndir, where it is launched, holds the friction of phase 6.
+template <bool MIXED, int PASS, int DIR>
+__global__ void __launch_bounds__(DIR == 1 ? 32 * PH_XY : SS_THREADS)
+    phase_advection_kernel(const __grid_constant__ SubstepArgs a, int d0, int ndir)
+{
+    using C = typename std::conditional<MIXED, float, double>::type;
+    constexpr int BY = DIR == 1 ? PH_XY : SS_BY;
+    phase_begin();
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    if (blockIdx.z == ndir) {
+        const int n = a.nx * a.ny, step = 32 * BY * gridDim.x * gridDim.y;
+        for (int p = ((blockIdx.y * gridDim.x + blockIdx.x) * BY + ty) * 32 + tx; p < n; p += step)
+            phase_point<MIXED>(a, 5, 0, p % a.nx, p / a.nx, p);
+        return;
+    }
+    const int d = d0 + blockIdx.z;
+    const HPassArgs<double>& pa = a.adv[d].pass[PASS];
+    if (PASS == 1 && d == 0 && blockIdx.x == 0 && blockIdx.y == 0 && tx == 0 && ty == 0 && a.time)
+        *a.time = *a.time + a.dt;
+    auto pass = [&](const auto& epi) {
+        using E = typename std::decay<decltype(epi)>::type;
+        if constexpr (DIR == 1) {
+            const int row = blockIdx.y * BY + ty;
+            if (row < pa.ny_) hpass_x_inc_body<double, E, double, C>(pa, blockIdx.x, row, tx, epi);
+        } else {
+            __shared__ YIncSmem<double, C> sm;
+            hpass_y_inc_body<double, E, double, C>(pa, blockIdx.x, blockIdx.y, 0, tx, ty, sm, epi);
+        }
+    };
+    if constexpr (PASS == 1) pass(ReconstructEpi{a.advvar[d], a.Uo[d], a.idt, a.haloy, a.ny - a.haloy - 1});
+    else pass(NoEpi());
+}
+
+template <typename K, typename... A>
+int launch_phase(K kernel, dim3 grid, dim3 block, bool first, cudaStream_t stream, const A&... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = first ? 0 : 1;
+    if (cudaLaunchKernelEx(&cfg, kernel, args...) != cudaSuccess) return GETM_ERR_CUDA;
+    GETM_CHECK_LAUNCH();
+    return GETM_OK;
+}
+
+// One launch for both directions' pass where they share the axis (they do
+// unless the host gave the two advections different orders)
+template <bool MIXED, int PASS>
+int launch_phase_advection(const SubstepArgs& a, bool friction, cudaStream_t stream)
+{
+    const dim3 gx(div_up(a.nx + 1, HX_STRIDE), div_up(a.ny, PH_XY)), gy(div_up(a.nx, 32), div_up(a.ny + 1, HY_STRIDE));
+    const bool one = a.adv[0].dir[PASS] == a.adv[1].dir[PASS];
+    for (int d = 0; d < (one ? 1 : 2); d++) {
+        const int ndir = one ? 2 : 1;
+        dim3 g = a.adv[d].dir[PASS] == 1 ? gx : gy;
+        g.z = ndir + (friction && d == 0);
+        const int rc = a.adv[d].dir[PASS] == 1
+                           ? launch_phase(phase_advection_kernel<MIXED, PASS, 1>, g, dim3(32, PH_XY), false, stream, a,
+                                          d, ndir)
+                           : launch_phase(phase_advection_kernel<MIXED, PASS, 2>, g, dim3(32, SS_BY), false, stream, a,
+                                          d, ndir);
+        if (rc) return rc;
+    }
+    return GETM_OK;
+}
+
+template <bool MIXED>
+int launch_phases(const SubstepArgs& a, cudaStream_t stream)
+{
+    const dim3 pb(32, PH_PY), pg(div_up(a.nx, 32), div_up(a.ny, PH_PY));
+    const dim3 db(32, PH_DY), dg(div_up(a.nx + 1, UD_BX), div_up(a.ny + 1, PH_DY));
+    int rc = launch_phase(phase_points_kernel<MIXED, 0>, pg, pb, true, stream, a);
+    if (!rc) rc = launch_phase(phase_points_kernel<MIXED, 1>, pg, pb, false, stream, a);
+    if (!rc) rc = launch_phase(phase_points_kernel<MIXED, 2>, pg, pb, false, stream, a);
+    if (!rc) rc = launch_phase(phase_depth_kernel<MIXED>, dg, db, false, stream, a);
+    if (!rc) rc = launch_phase(phase_points_kernel<MIXED, 4>, pg, pb, false, stream, a);
+    if (!rc) rc = launch_phase_advection<MIXED, 0>(a, a.friction != 0, stream);
+    if (!rc) rc = launch_phase_advection<MIXED, 1>(a, false, stream);
+    return rc;
+}
+
+}  // namespace
+
+extern "C" int getm_split2d_substep_phases(const getm_split2d_fields* f, int nx, int ny, int halox, int haloy,
+                                           int mixed, int ufirst, int accumulate, int friction, double timestep,
+                                           double Dmin, double Dcrit, getm_advection* uadv, getm_grid* ugrid,
+                                           getm_grid* uugrid, getm_grid* uvgrid, int uadv_ufirst,
+                                           getm_advection* vadv, getm_grid* vgrid, getm_grid* vugrid,
+                                           getm_grid* vvgrid, int vadv_ufirst, cudaStream_t stream)
+{
+    SubstepArgs a;
+    int rc = substep_args(a, f, nx, ny, halox, haloy, mixed, ufirst, accumulate, friction, timestep, Dmin, Dcrit,
+                          uadv, ugrid, uugrid, uvgrid, uadv_ufirst, vadv, vgrid, vugrid, vvgrid, vadv_ufirst);
+    if (rc) return rc;
+    return mixed ? launch_phases<true>(a, stream) : launch_phases<false>(a, stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -460,18 +626,16 @@ struct BatchMember {
     int adv_nbx[2][2];     // [U/V][pass] row segments (x pass) or tile columns (y pass)
 };
 
-__host__ __device__ inline int sb_div_up(int a, int b) { return (a + b - 1) / b; }
-
 // Block items of one momentum advection pass over the plane.
 template <bool MIXED>
 void pass_items(const HPassArgs<double>& pa, int dir, int& items, int& nbx)
 {
     if (dir == 1) {
-        nbx = sb_div_up(pa.nx_ + 1, HX_STRIDE);
-        items = nbx * sb_div_up(pa.ny_, SS_BY);
+        nbx = div_up(pa.nx_ + 1, HX_STRIDE);
+        items = nbx * div_up(pa.ny_, SS_BY);
     } else {
-        nbx = sb_div_up(pa.nx_, 32);
-        const int nby = sb_div_up(pa.ny_ + 1, HY_STRIDE);
+        nbx = div_up(pa.nx_, 32);
+        const int nby = div_up(pa.ny_ + 1, HY_STRIDE);
         items = nbx * nby;
     }
 }
@@ -507,60 +671,40 @@ __device__ __forceinline__ void batch_pass_item(const HPassArgs<double>& pa, int
 template <bool MIXED>
 __device__ void batch_item(const BatchMember& m, int ph, int q, int ufirst, SubstepSmem& sm, int tx, int ty)
 {
-    using C = typename std::conditional<MIXED, float, double>::type;
     const SubstepArgs& a = m.a;
     const int nx = a.nx, ny = a.ny;
-    const int ilo = a.halox, ihi = nx - a.halox - 1, jlo = a.haloy, jhi = ny - a.haloy - 1;
-    const int d1 = ufirst ? 0 : 1, d2 = 1 - d1;
-    auto point = [&](int qq, int& p, int& i, int& j) {
-        p = qq * SS_THREADS + ty * 32 + tx;
-        j = p / nx;
-        i = p - j * nx;
-        return p < m.n;
+    const int jlo = a.haloy, jhi = ny - a.haloy - 1;
+    const int d1 = ufirst ? 0 : 1;
+    auto points = [&](int php, int qq) {
+        const int p = qq * SS_THREADS + ty * 32 + tx;
+        if (p < m.n) phase_point<MIXED>(a, php, d1, p % nx, p / nx, p);
     };
-    auto interior = [&](int i, int j) { return i >= ilo && i <= ihi && j >= jlo && j <= jhi; };
-    int p, i, j;
     switch (ph) {
     case 0:
-        if (point(q, p, i, j) && interior(i, j)) transport_update<MIXED>(a.tr[d1], a.dt, p);
+        points(0, q);
         break;
     case 1:
-        if (point(q, p, i, j)) {
-            coriolis_from<C>(a, d1, i, j);
-            if (interior(i, j)) transport_update<MIXED>(a.tr[d2], a.dt, p);
-        }
+        points(1, q);
         break;
     case 2:
-        if (point(q, p, i, j)) {
-            coriolis_from<C>(a, d2, i, j);
-            if (a.accumulate) accumulate_2d_point(a.tr[0].U, a.tr[1].U, a.Ucum, a.Vcum, p);
-            surface_elevation_fused_point(nx, ny, a.halox, a.haloy, a.mT, a.dyU, a.dxV, a.iareaT, a.z, a.zo,
-                                          a.tr[0].U, a.tr[1].U, a.fwf, a.dt, i, j);
-        }
+        points(2, q);
         break;
     case 3:
         if (q < m.dtiles) {
             update_depth_2d_tile<SS_BY, MIXED>(a.depth, q % m.dntx, q / m.dntx, tx, ty, sm.szh);
             __syncthreads();
-        } else if (point(q - m.dtiles, p, i, j)) {
-            a.fwf[p] = a.pe[p];
-            if (i < nx - 1) interp_pair_point<double>(a.taux, a.tausx, p, 1, 0);
-            if (j < ny - 1) interp_pair_point<double>(a.tauy, a.tausy, p, nx, 0);
+        } else {
+            points(3, q - m.dtiles);
         }
         break;
     case 4:
-        if (point(q, p, i, j)) {
-            momentum_2d_velocities_point<C>(a.vel, i, j);
-            a.advD[0][p] = a.Dsrc[0][p];
-            a.advD[1][p] = a.Dsrc[1][p];
-            if (interior(i, j)) spg_point<MIXED>(a.spg, p);
-        }
+        points(4, q);
         break;
     case 5: {
         int r = q;
         if (a.friction) {
             if (r < m.pts) {
-                if (point(r, p, i, j)) momentum_2d_friction_point<C>(a.fric, i, j);
+                points(5, r);
                 break;
             }
             r -= m.pts;
@@ -689,7 +833,8 @@ extern "C" int getm_substep_batch_set(getm_substep_batch* b, int member, int nsu
                                       int uadv_ufirst, getm_advection* vadv, getm_grid* vgrid, getm_grid* vugrid,
                                       getm_grid* vvgrid, int vadv_ufirst)
 {
-    if (!b || member < 0 || member >= b->nmember || nsub < 0 || split < nsub + 1 || b->dmem) return GETM_ERR_ARG;
+    if (!b || member < 0 || member >= b->nmember || nsub < 0 || split < nsub + 1 || b->dmem || !f || !f->sync)
+        return GETM_ERR_ARG;
     BatchMember& m = b->host[member];
     int rc = substep_args(m.a, f, nx, ny, halox, haloy, b->mixed, ufirst, accumulate, friction, timestep, Dmin,
                           Dcrit, uadv, ugrid, uugrid, uvgrid, uadv_ufirst, vadv, vgrid, vugrid, vvgrid, vadv_ufirst);
@@ -698,9 +843,9 @@ extern "C" int getm_substep_batch_set(getm_substep_batch* b, int member, int nsu
     m.nsub = nsub;
     m.split = split;
     m.n = nx * ny;
-    m.pts = sb_div_up(m.n, SS_THREADS);
-    m.dntx = sb_div_up(nx + 1, UD_BX);
-    m.dtiles = m.dntx * sb_div_up(ny + 1, SS_BY);
+    m.pts = div_up(m.n, SS_THREADS);
+    m.dntx = div_up(nx + 1, UD_BX);
+    m.dtiles = m.dntx * div_up(ny + 1, SS_BY);
     for (int d = 0; d < 2; d++)
         for (int s = 0; s < 2; s++) {
             if (b->mixed) pass_items<true>(m.a.adv[d].pass[s], m.a.adv[d].dir[s], m.adv_items[d][s], m.adv_nbx[d][s]);

@@ -87,8 +87,8 @@ class Fluxes:
 
 
 class _Split2DPlan:
-    """Arguments of the one-launch 2D substep: the fields struct and the
-    kernel's barrier words."""
+    """Arguments of the 2D substep kernels: the fields struct and, for the
+    one-launch kernel, its barrier words."""
 
     def __init__(self, fields, sync):
         self.fields = fields
@@ -122,7 +122,8 @@ class Simulation:
         ``substep_kernel``: in addition, a substep that is not followed by a
         3D step runs as one persistent kernel launch (closed domains with the
         default Coriolis scheme, FULL 2D advection split, no horizontal
-        momentum diffusion, 3D run types).  ``concurrent_3d``: in a 3D step,
+        momentum diffusion, 3D run types); without it, such a substep runs as
+        seven ordinary launches.  ``concurrent_3d``: in a 3D step,
         the shear frequency, the bottom stress, the advection of the 3D
         momentum and the slow terms it feeds run on a second stream,
         concurrently with the tracers, density and internal pressure
@@ -291,17 +292,20 @@ class Simulation:
         self.istep += 1
         macro_active = self.istep % self.split_factor == 0
         if self._split2d is not None and not macro_active:
-            self._split2d_substep()
+            self._split2d_substep(self._split2d)
+            return
+        if not macro_active and self.fused_2d and not self.substep_kernel and (plan := self._split2d_plan(sync=False)):
+            self._split2d_substep(plan, phases=True)
             return
         _lib.call("getm_advance_time", self._time.data_ptr(), float(self.timestep),
                   torch.cuda.current_stream(self._time.device).cuda_stream)
         self._advance_state(macro_active)
         self._update_forcing_and_diagnostics(macro_active)
 
-    def _split2d_plan(self):
-        """Fields of the one-launch 2D substep, or None where that kernel does
-        not cover the configuration (the substep then runs operation by
-        operation)."""
+    def _split2d_plan(self, sync: bool = True):
+        """Fields of the 2D substep kernels, or None where they do not cover
+        the configuration (the substep then runs operation by operation).
+        ``sync``: with the one-launch kernel's barrier words."""
         m = self.momentum
         if (self._ob is not None or self.runtype <= RunType.BAROTROPIC_2D or m.diffuse_momentum
                 or m.An_uu is not None or m.coriolis_scheme != CoriolisScheme.DEFAULT
@@ -309,7 +313,7 @@ class Simulation:
                 or self.T.device.type != "cuda"):
             return None
         T, U, V, X, a = self.T, self.U, self.V, self.X, self.airsea
-        sync = torch.zeros(4, dtype=torch.int32, device=T.device)  # barrier words, not model state
+        sync = torch.zeros(4, dtype=torch.int32, device=T.device) if sync else None  # barrier words, not model state
         fields = _pygetm.split2d_fields(
             mask_t=T.mask, H_t=T.H, iarea_t=T.iarea, z=T.z, zo=T.zo, D_t=T.D, Dclip_t=T.Dclip, work_t=T._work,
             fwf=self.fwf, pe=a.pe, sp=a.sp, taux=a.taux, tauy=a.tauy,
@@ -325,13 +329,15 @@ class Simulation:
             D_vv=V.vgrid.D, time=self._time, sync=sync)
         return _Split2DPlan(fields, sync)
 
-    def _split2d_substep(self):
-        """A substep without 3D step as one launch (the same operations as
-        _advance_state + _update_forcing_and_diagnostics with macro_active
-        false, in the same order, with bitwise the same results)."""
+    def _split2d_substep(self, plan, phases: bool = False):
+        """A substep without 3D step as one launch, or (``phases``) as one
+        launch per phase (the same operations as _advance_state +
+        _update_forcing_and_diagnostics with macro_active false, in the same
+        order, with bitwise the same results).  The launch per phase takes the
+        fields anew each time, as the operations one by one would."""
         m = self.momentum
-        _pygetm.split2d_substep(self._split2d.fields, self.T, self.dtype3d == torch.float32, m._ufirst, True,
-                                m.apply_bottom_friction, self.timestep, self.Dmin, self.Dcrit, m.uadv, m.vadv)
+        _pygetm.split2d_substep(plan.fields, self.T, self.dtype3d == torch.float32, m._ufirst, True,
+                                m.apply_bottom_friction, self.timestep, self.Dmin, self.Dcrit, m.uadv, m.vadv, phases)
         m._ufirst = not m._ufirst
 
     def split2d_status(self) -> int:

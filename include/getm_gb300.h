@@ -768,6 +768,13 @@ int getm_split2d_substep(const getm_split2d_fields* f, int nx, int ny, int halox
                          getm_advection* uadv, getm_grid* ugrid, getm_grid* uugrid, getm_grid* uvgrid,
                          int uadv_ufirst, getm_advection* vadv, getm_grid* vgrid, getm_grid* vugrid,
                          getm_grid* vvgrid, int vadv_ufirst, cudaStream_t stream);
+/* the same substep, with the same results, as seven ordinary launches: for
+ * domains that share the GPU with others.  f->sync may be NULL. */
+int getm_split2d_substep_phases(const getm_split2d_fields* f, int nx, int ny, int halox, int haloy, int mixed,
+                                int ufirst, int accumulate, int friction, double timestep, double Dmin,
+                                double Dcrit, getm_advection* uadv, getm_grid* ugrid, getm_grid* uugrid,
+                                getm_grid* uvgrid, int uadv_ufirst, getm_advection* vadv, getm_grid* vgrid,
+                                getm_grid* vugrid, getm_grid* vvgrid, int vadv_ufirst, cudaStream_t stream);
 
 /* ---- turbulence closure -----------------------------------------------
  * Replaces the GOTM call of python/pygetm/vertical_mixing.py:150-188
