@@ -330,11 +330,11 @@ class Runner:
             self.hook(self.sim)
 
     def check(self):
-        """Raise if a grid barrier of the one-launch substep gave up (its
+        """Raise if the 2D substep reported an error (its
         substeps would then have done no work)."""
         st = self.sim.split2d_status()
         if st != 0:
-            raise RuntimeError(f"one-launch substep reported status {st}: a grid barrier gave up")
+            raise RuntimeError(f"2D substep reported status {st}")
 
     def run_step(self):
         """One 3D step (graph replay of the step's parity)."""
@@ -377,7 +377,7 @@ class Runner:
 # cells per lane): profiles/hpass_x_f64s_seamount_400x300x40.md (184.0 +
 # 83.0 MB), and the float-storage one-cell pass of an earlier capture.
 TRAFFIC_X_PASS = {("_f32", 0): 152.51e6, ("_f64s", 1): 267.0e6, ("_f64s", 0): 263.9e6}
-# one one-launch substep, by form: profiles/substep_2d_seamount_400x300.md
+# one 2D substep, by form (one cooperative launch then): profiles/substep_2d_seamount_400x300.md
 # (60.8 + 5.3 MB; the plane's fields stay in L2)
 TRAFFIC_SUBSTEP = {"mixed": 66.1e6}
 
@@ -717,9 +717,9 @@ def _shelf_leg(args, device):
 
 
 def _substep_kernel_leg(runner, peak, peak_kind):
-    """Time the one-launch 2D substep (substep_2d_kernel) on the live state:
-    CUDA events around every substep of two 3D steps that is not followed
-    by a 3D step (one launch each), against the substep's algorithmic bytes
+    """Time the 2D substep (substep_transport, depth and two advection
+    kernels) on the live state: CUDA events around every substep of two 3D
+    steps that is not followed by a 3D step (four launches each), against the substep's algorithmic bytes
     (its 2D fields stay resident in L2, so the HBM figure is a reference
     point, not its bound)."""
     import torch
@@ -752,11 +752,11 @@ def _substep_kernel_leg(runner, peak, peak_kind):
     t = us[len(us) // 2] / 1e6
     T = sim.T
     b = roofline.substep_bytes(T.nx, T.ny)
-    return {"kernel": f"substep_2d_kernel<{'true' if sim.precision == 'mixed' else 'false'}>",
+    return {"kernel": f"substep_*_kernel<{'true' if sim.precision == 'mixed' else 'false'}>, four launches",
             "us_per_launch_median": us[len(us) // 2], "launches_timed": len(us),
             "bytes_per_launch": b, "achieved_gbs": b / t / 1e9, "peak": peak, "peak_kind": peak_kind,
             "frac_of_hbm": b / t / 1e9 / peak,
-            "note": "2D fields of one plane are L2-resident; bound by FP64 pipe, barriers and latency"}
+            "note": "2D fields of one plane are L2-resident; bound by instructions, FP64 pipe and latency"}
 
 
 def _tracer_transport_leg(args, device, threads):

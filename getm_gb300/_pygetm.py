@@ -393,7 +393,7 @@ def surface_elevation_fused(timestep, z, zo, U, V, fwf):
          _p(g.iarea), _p(z), _p(zo), _p(U), _p(V), _p(fwf), float(timestep), _s())
 
 
-# ---- one 2D substep as one launch -----------------------------------------
+# ---- one 2D substep as four launches --------------------------------------
 # field order of getm_split2d_fields (include/getm_gb300.h); every member is
 # a device pointer
 SPLIT2D_FIELDS = (
@@ -414,7 +414,7 @@ class Split2DFields(ctypes.Structure):
 
 def split2d_fields(**arrays) -> Split2DFields:
     """The fields struct from Arrays or tensors (every name of SPLIT2D_FIELDS;
-    ``time`` may be None, and ``sync`` where the phases are separate launches)."""
+    ``time`` may be None)."""
     missing = set(SPLIT2D_FIELDS) - set(arrays) - {"time"}
     if missing:
         raise ValueError(f"split2d_fields: missing {sorted(missing)}")
@@ -425,13 +425,11 @@ def split2d_fields(**arrays) -> Split2DFields:
     return f
 
 
-def split2d_substep(fields: Split2DFields, T, mixed, ufirst, accumulate, friction, timestep, Dmin, Dcrit, uadv, vadv,
-                    phases=False):
+def split2d_substep(fields: Split2DFields, T, mixed, ufirst, accumulate, friction, timestep, Dmin, Dcrit, uadv, vadv):
     """One non-macro 2D substep (simulation.py:1033-1304 with update_3d
-    false) as one cooperative launch, or (``phases``) as one ordinary launch
-    per phase; ``uadv``/``vadv``: the momentum Advection objects."""
+    false) as four launches; ``uadv``/``vadv``: the momentum Advection objects."""
     U, V = T.ugrid, T.vgrid
-    call("getm_split2d_substep_phases" if phases else "getm_split2d_substep", ctypes.byref(fields), T.nx_, T.ny_, T.halox, T.haloy, int(bool(mixed)),
+    call("getm_split2d_substep", ctypes.byref(fields), T.nx_, T.ny_, T.halox, T.haloy, int(bool(mixed)),
          int(bool(ufirst)), int(bool(accumulate)), int(bool(friction)), float(timestep), float(Dmin), float(Dcrit),
          uadv.p, U.handle, U.ugrid.handle, U.vgrid.handle, int(uadv.ufirst),
          vadv.p, V.handle, V.ugrid.handle, V.vgrid.handle, int(vadv.ufirst), _s())

@@ -3,8 +3,8 @@
 The library reads five launch-shape knobs at every launch (``getm_tune_set``,
 per host thread): the rows per block of the x advection pass, the rows a warp
 marches in the 3D y pass, the rows of 32 columns per block of the column
-kernels (w pass, float column solve), the blocks per SM of the one-launch
-2D substep and the form of the 3D x pass (four cells or one cell per lane).  The best shapes depend on the domain: a 64 x 64 x 20 member has
+kernels (w pass, float column solve), the blocks per SM of a former one-launch
+2D substep (accepted, without effect) and the form of the 3D x pass (four cells or one cell per lane).  The best shapes depend on the domain: a 64 x 64 x 20 member has
 too few columns to fill 152 SMs with 8-row blocks, a 400 x 300 x 40 box has
 plenty.
 
@@ -198,7 +198,7 @@ def step_timer(sim, replays: int = 4) -> Callable[[Dict[str, int]], float]:
         e1.record()
         torch.cuda.synchronize(dev)
         if sim.split2d_status() != 0:
-            raise RuntimeError("one-launch substep reported an error while tuning")
+            raise RuntimeError("the substep reported an error while tuning")
         del graphs
         return e0.elapsed_time(e1) / (2 * replays)
 
@@ -220,8 +220,7 @@ def tune(sim, rounds: int = 2, replays: int = 4, only: Optional[Iterable[str]] =
     torch.cuda.synchronize(sim.T.device)
     measure = step_timer(sim, replays)
     knobs = {k: v for k, v in KNOBS.items() if only is None or k in set(only)}
-    if sim._split2d is None:  # no one-launch substep in this configuration
-        knobs.pop("substep_blocks_per_sm", None)
+    knobs.pop("substep_blocks_per_sm", None)  # without effect
     if sim.precision != "mixed":
         for k in FLOAT_ONLY:
             knobs.pop(k, None)

@@ -48,7 +48,7 @@ struct HPassArgs {
 
 // Epilogue of a pass: called once per updated (or copied) cell with the
 // cell's flat index p3, its row j, the new value of the first field and the
-// new thickness.  The default does nothing; the one-launch 2D substep uses
+// new thickness.  The default does nothing; the 2D substep uses
 // it to form the momentum advection term as each cell is finished.
 struct NoEpi {
     __device__ __forceinline__ void operator()(long long, int, double, double) const {}
@@ -81,7 +81,7 @@ struct NoEpi {
 //   -> 132 (FP64 pipe 77 % busy).  Against quad precision the five-pass split's
 //   error falls from 2.0e-16 to 1.3e-16 (a result is rounded once per pass,
 //   not three times).  Products and sums are rounded as written (intrinsics,
-//   no contraction): the separate passes and the one-launch substep share
+//   no contraction): the separate passes and the 2D substep share
 //   these functions and give the same bits.
 // ---------------------------------------------------------------------------
 // Storage type S of the advected field and V of the velocities: float (the
@@ -562,24 +562,24 @@ __device__ __forceinline__ void hpass_x_inc_body(const HPassArgs<S, V>& a, int b
 constexpr int HY_BY = 16;
 constexpr int HY_STRIDE = HY_BY - 1;
 
-template <typename S, typename C = float>
+template <typename S, typename C = float, int BY = HY_BY>
 struct YIncSmem {
-    S sf[HY_BY + 3][32];       // rows j0-2 .. j0+HY_BY
-    C sd[HY_BY + 2][32];      // differences f[j+1] - f[j], rows j0-2 .. j0+HY_BY-1
-    C sx[HY_BY][32];           // per-face exchange (QU, then el)
+    S sf[BY + 3][32];       // rows j0-2 .. j0+BY
+    C sd[BY + 2][32];      // differences f[j+1] - f[j], rows j0-2 .. j0+BY-1
+    C sx[BY][32];           // per-face exchange (QU, then el)
 };
 
-template <typename S, typename Epi = NoEpi, typename V = S, typename C = float>
+template <typename S, typename Epi = NoEpi, typename V = S, typename C = float, int BY = HY_BY>
 __device__ __forceinline__ void hpass_y_inc_body(const HPassArgs<S, V>& a, int bx, int by, int k, int tx, int ty,
-                                                 YIncSmem<S, C>& sm, const Epi& epi = Epi())
+                                                 YIncSmem<S, C, BY>& sm, const Epi& epi = Epi())
 {
     auto& sf = sm.sf;
     auto& sd = sm.sd;
     auto& sx = sm.sx;
     const int i = bx * 32 + tx;
-    const int j0 = by * HY_STRIDE;
+    const int j0 = by * (BY - 1);
     const int ja = j0 - 1 + ty;  // this thread's face (V point) and its south cell
-    const int jb = ja + 1;       // the cell this thread updates (ty < HY_STRIDE)
+    const int jb = ja + 1;       // the cell this thread updates (ty < (BY - 1))
     const long long s = a.nx_;
     const long long base = (long long)k * a.plane + i;  // + j * s
     const bool icol = i < a.nx_;
@@ -608,9 +608,9 @@ __device__ __forceinline__ void hpass_y_inc_body(const HPassArgs<S, V>& a, int b
     }
     sx[ty][tx] = QU;
     __syncthreads();
-    const C QUn = ty + 1 < HY_BY ? sx[ty + 1][tx] : C(0);  // north face of cell jb
+    const C QUn = ty + 1 < BY ? sx[ty + 1][tx] : C(0);  // north face of cell jb
 
-    const bool bin = ty < HY_STRIDE && icol && jb < a.ny_;
+    const bool bin = ty < (BY - 1) && icol && jb < a.ny_;
     const bool upd = bin && iint && jb >= a.jlo && jb <= a.jhi && a.tmask[(long long)jb * s + i] == 1;
     C coef = C(0);
     double hnew = 0.0;
@@ -621,9 +621,9 @@ __device__ __forceinline__ void hpass_y_inc_body(const HPassArgs<S, V>& a, int b
         a.h_out[base + jb * s] = hnew;
     }
     // staging rows: thread row ty loads row ja (smem row ty + 1); rows 0-2
-    // also load rows j0-2, j0+HY_BY-1 and j0+HY_BY (smem rows 0, HY_BY+1, HY_BY+2)
-    const int jx = ty == 0 ? j0 - 2 : j0 + HY_BY - 2 + ty;
-    const int sxrow = ty == 0 ? 0 : HY_BY + ty;
+    // also load rows j0-2, j0+BY-1 and j0+BY (smem rows 0, BY+1, BY+2)
+    const int jx = ty == 0 ? j0 - 2 : j0 + BY - 2 + ty;
+    const int sxrow = ty == 0 ? 0 : BY + ty;
     const bool xin = ty < 3 && icol && jx >= 0 && jx < a.ny_;
     const TvdFace<C> tf = hx_tvd(a.scheme, cfl, QU);
     for (int t = 0; t < a.ntracer; t++) {
@@ -636,7 +636,7 @@ __device__ __forceinline__ void hpass_y_inc_body(const HPassArgs<S, V>& a, int b
         // 0 and 1 also form the differences below and above the block's faces
         sd[ty + 1][tx] = hx_c<C>(sf[ty + 2][tx] - sf[ty + 1][tx]);
         if (ty == 0) sd[0][tx] = hx_c<C>(sf[1][tx] - sf[0][tx]);
-        if (ty == 1) sd[HY_BY + 1][tx] = hx_c<C>(sf[HY_BY + 2][tx] - sf[HY_BY + 1][tx]);
+        if (ty == 1) sd[BY + 1][tx] = hx_c<C>(sf[BY + 2][tx] - sf[BY + 1][tx]);
         __syncthreads();
         const C dprev = sd[ty][tx], d = sd[ty + 1][tx], dnext = sd[ty + 2][tx];
         const S fb = sf[ty + 2][tx];
@@ -644,7 +644,7 @@ __device__ __forceinline__ void hpass_y_inc_body(const HPassArgs<S, V>& a, int b
         if (act) hx_face(tf, up, uu_ok, QU, dprev, d, dnext, ahd, a.Ah != nullptr, el, er);
         sx[ty][tx] = el;
         __syncthreads();
-        const C el_n = ty + 1 < HY_BY ? sx[ty + 1][tx] : C(0);
+        const C el_n = ty + 1 < BY ? sx[ty + 1][tx] : C(0);
         if (bin) {
             const S fn = upd ? hx_new(fb, coef, el_n, er) : fb;
             a.fout[t][base + jb * s] = fn;

@@ -252,6 +252,26 @@ __device__ __forceinline__ double getm_rcp(double x)
     return __fma_rn(r, __fma_rn(e, e, e), r);
 }
 
+// n / d in FP64 with six FP64 instructions: n getm_rcp(d) and one correction by
+// its own remainder, which leaves an error of half a unit in the last place
+// and less than 2^-6 of one beside it (the correctly rounded division takes
+// about twice as many).  Operands or quotients near the ends of the range,
+// infinities and NaNs: the division, out of line.
+static __device__ __noinline__ double getm_div_hw(double n, double d) { return n / d; }
+
+__device__ __forceinline__ double getm_div(double n, double d)
+{
+    const int en = (int)(((unsigned)__double2hiint(n) >> 20) & 0x7ffu);
+    const int ed = (int)(((unsigned)__double2hiint(d) >> 20) & 0x7ffu);
+    const bool zero = ((__double2hiint(n) & 0x7fffffff) | __double2loint(n)) == 0;
+    // both within 2^-959 .. 2^960, the quotient within 2^-900 .. 2^900
+    if ((unsigned)(ed - 64) > 1919u || (!zero && ((unsigned)(en - 64) > 1919u || (unsigned)(en - ed + 900) > 1800u)))
+        return getm_div_hw(n, d);
+    const double r = getm_rcp(d);
+    const double q = __dmul_rn(n, r);
+    return zero ? q : __fma_rn(__fma_rn(-q, d, n), r, q);  // (a signed zero keeps its sign)
+}
+
 // 2 x on the integer pipe (exact; zeros, subnormals, infinities, NaNs and
 // overflow take the FP64 sum out of line)
 static __device__ __noinline__ double getm_twice_hw(double x) { return x + x; }

@@ -178,7 +178,7 @@ __global__ void advance_2d_transport_kernel(int nx, int ny, int halox, int haloy
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     int j = blockIdx.y;
     if (i < halox || i >= nx - halox || j < haloy || j >= ny - haloy) return;
-    transport_2d_point(a, dt, (long long)j * nx + i);
+    transport_2d_point<false>(a, dt, (long long)j * nx + i);
 }
 
 extern "C" int getm_advance_2d_transport(int nx, int ny, int halox, int haloy, const int* mask,

@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(S2_THREADS) advance_2d_transport_mixed_kernel(
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y;
     if (i < halox || i >= nx - halox || j < haloy || j >= ny - haloy) return;
-    transport_2d_mixed_point(a, dt, (long long)j * nx + i);
+    transport_2d_point<true>(a, dt, (long long)j * nx + i);
 }
 
 __global__ void accumulate_2d_kernel(long long n, const double* U, const double* V, double* Uc, double* Vc)

@@ -14,30 +14,12 @@
 #include "getm_common.cuh"
 
 
-// torch.clamp(x, min=lo): NaN propagates
-__device__ __forceinline__ double clamp_min(double x, double lo) { return isnan(x) ? x : (x < lo ? lo : x); }
-
-// The same values with the comparisons on the integer pipe (I: the mixed
-// form) or on the FP64 pipe (the FP64 form, as written in the reference)
-template <bool I>
-__device__ __forceinline__ double dmax(double a, double b)
-{
-    if constexpr (I) return getm_fmax_i(a, b);
-    else return fmax(a, b);
-}
-
-template <bool I>
-__device__ __forceinline__ double dmin(double a, double b)
-{
-    if constexpr (I) return getm_fmin_i(a, b);
-    else return fmin(a, b);
-}
-
-template <bool I>
+// torch.clamp(x, min=lo) (NaN propagates), minima and maxima with the
+// comparisons on the integer pipe (the same values; an FP64 comparison costs
+// as much as a multiplication)
 __device__ __forceinline__ double dclamp_min(double x, double lo)
 {
-    if constexpr (I) return getm_isnan_i(x) ? x : (getm_dkey(x) < getm_dkey(lo) ? lo : x);
-    else return clamp_min(x, lo);
+    return getm_isnan_i(x) ? x : (getm_dkey(x) < getm_dkey(lo) ? lo : x);
 }
 
 struct DepthArgs {
@@ -58,7 +40,7 @@ constexpr int UD_BX = 32;  // tile width of update_depth_2d_tile
 // alpha (wrapper.F90:428-436) with the constant divisor as a reciprocal
 __device__ __forceinline__ double alpha_of(double d, double twoDmin, double ialpha)
 {
-    return fmax(0.0, fmin(1.0, (d - twoDmin) * ialpha));
+    return getm_fmax_i(0.0, getm_fmin_i(1.0, (d - twoDmin) * ialpha));
 }
 
 // ... in float, for the mixed form: alpha is a weight between 0 and 1 that
@@ -75,8 +57,7 @@ __device__ __forceinline__ double alpha_of_f(double d, float twoDmin, float ialp
 // shared memory.  Copies between grids are scattered by the point that
 // owns the source value (UU.D(j, i-1) = D_T_half(j, i), VV.D(j-1, i) =
 // D_T_half(j, i), UV.D(j-1, i-1) = VU.D(j-1, i-1) = X.D(j, i)).
-// MIXED: minima, maxima and clamps on the integer pipe (the same values) and
-// alpha in float (alpha_of_f); the sums stay FP64.
+// MIXED: alpha in float (alpha_of_f); the sums stay FP64.
 template <int BY, bool MIXED = false>
 __device__ __forceinline__ void update_depth_2d_tile(const DepthArgs& a, int bx, int by, int tx, int ty,
                                                      double (&szh)[BY + 2][UD_BX + 2])
@@ -125,7 +106,7 @@ __device__ __forceinline__ void update_depth_2d_tile(const DepthArgs& a, int bx,
         }
         double dx = DX0;
         if (mX != 0) {
-            dx = dmax<MIXED>(HX + zx, a.Dmin);
+            dx = getm_fmax_i(HX + zx, a.Dmin);
             a.DX[px] = dx;
         }
         if (j >= 1 && i >= 1 && j - 1 < ny && i - 1 < nx) {  // UV.D = X.D[1:, 1:]; VU.D = UV.D
@@ -138,10 +119,10 @@ __device__ __forceinline__ void update_depth_2d_tile(const DepthArgs& a, int bx,
     const double zh = szh[sj][si];
     // T: elevation2depth(z, H, -1000), Dclip = clamp(D, Dmin), D_T_half
     double DT = DT0;
-    if (mT != 0) DT = dmax<MIXED>(HT + zT, -1000.0);
+    if (mT != 0) DT = getm_fmax_i(HT + zT, -1000.0);
     a.DT[p] = DT;
-    a.DclipT[p] = dclamp_min<MIXED>(DT, a.Dmin);
-    const double dth = mT != 0 ? dmax<MIXED>(HT + zh, a.Dmin) : zh;
+    a.DclipT[p] = dclamp_min(DT, a.Dmin);
+    const double dth = mT != 0 ? getm_fmax_i(HT + zh, a.Dmin) : zh;
     a.workT[p] = dth;
     if (i >= 1) a.DUU[p - 1] = dth;   // UU.D[:, :-1] = D_T_half[:, 1:]
     if (j >= 1) a.DVV[p - nx] = dth;  // VV.D[:-1, :] = D_T_half[1:, :]
@@ -156,7 +137,7 @@ __device__ __forceinline__ void update_depth_2d_tile(const DepthArgs& a, int bx,
         zu = workU0;
     }
     if (mU != 0) {
-        const double d = dmax<MIXED>(HU + zu, a.Dmin);
+        const double d = getm_fmax_i(HU + zu, a.Dmin);
         a.DU[p] = d;
         a.alphaU[p] = MIXED ? alpha_of_f(d, twoDmin_f, ialpha_f) : alpha_of(d, twoDmin, a.ialpha);
     }
@@ -169,7 +150,7 @@ __device__ __forceinline__ void update_depth_2d_tile(const DepthArgs& a, int bx,
         zv = workV0;
     }
     if (mV != 0) {
-        const double d = dmax<MIXED>(HV + zv, a.Dmin);
+        const double d = getm_fmax_i(HV + zv, a.Dmin);
         a.DV[p] = d;
         a.alphaV[p] = MIXED ? alpha_of_f(d, twoDmin_f, ialpha_f) : alpha_of(d, twoDmin, a.ialpha);
     }
@@ -188,47 +169,59 @@ struct VelArgs {
 template <typename C>
 __device__ __forceinline__ double vel_div(double num, double den)
 {
-    if constexpr (std::is_same<C, double>::value) return num / den;
+    if constexpr (std::is_same<C, double>::value) return getm_div(num, den);
     else return getm_f2d(getm_d2f_approx(num) / getm_d2f_approx(den));
 }
 
 // Mixed form: u1 = U/D to ~2^-46 (getm_div_refined; u1 is advected and its
 // product with the new depth is differenced against U, so it stays FP64) and
 // the advection velocities entirely in float.
+// east, north: the neighbours (Ue, Ve at i + 1; Un, Vn at j + 1) exist
+template <typename C>
+__device__ __forceinline__ void momentum_2d_velocities_values(const VelArgs& a, long long p, bool east, bool north,
+                                                              double Up, double Ue, double Un, double Vp, double Ve,
+                                                              double Vn, double DU, double DV, double DUU, double DUV,
+                                                              double DVU, double DVV)
+{
+    // interp_x (ioffset 0) writes i < nx-1; elsewhere the old value is divided
+    if constexpr (std::is_same<C, double>::value) {
+        const double u1 = getm_div(Up, DU);
+        const double v1 = getm_div(Vp, DV);
+        a.u1[p] = u1; a.advU[p] = u1;
+        a.v1[p] = v1; a.advV[p] = v1;
+        const double uu = east ? getm_half(Up + Ue) : a.uua[p];
+        const double uv = east ? getm_half(Vp + Ve) : a.uva[p];
+        const double vu = north ? getm_half(Up + Un) : a.vua[p];
+        const double vv = north ? getm_half(Vp + Vn) : a.vva[p];
+        a.uua[p] = vel_div<C>(uu, DUU);
+        a.uva[p] = vel_div<C>(uv, DUV);
+        a.vua[p] = vel_div<C>(vu, DVU);
+        a.vva[p] = vel_div<C>(vv, DVV);
+    } else {
+        const double u1 = getm_div_refined(Up, DU);
+        const double v1 = getm_div_refined(Vp, DV);
+        a.u1[p] = u1; a.advU[p] = u1;
+        a.v1[p] = v1; a.advV[p] = v1;
+        const float Uf = getm_d2f_approx(Up), Vf = getm_d2f_approx(Vp);
+        const float uu = east ? 0.5f * (Uf + getm_d2f_approx(Ue)) : getm_d2f_approx(a.uua[p]);
+        const float uv = east ? 0.5f * (Vf + getm_d2f_approx(Ve)) : getm_d2f_approx(a.uva[p]);
+        const float vu = north ? 0.5f * (Uf + getm_d2f_approx(Un)) : getm_d2f_approx(a.vua[p]);
+        const float vv = north ? 0.5f * (Vf + getm_d2f_approx(Vn)) : getm_d2f_approx(a.vva[p]);
+        a.uua[p] = getm_f2d(uu / getm_d2f_approx(DUU));
+        a.uva[p] = getm_f2d(uv / getm_d2f_approx(DUV));
+        a.vua[p] = getm_f2d(vu / getm_d2f_approx(DVU));
+        a.vva[p] = getm_f2d(vv / getm_d2f_approx(DVV));
+    }
+}
+
 template <typename C>
 __device__ __forceinline__ void momentum_2d_velocities_point(const VelArgs& a, int i, int j)
 {
     const long long p = (long long)j * a.nx + i;
-    if constexpr (std::is_same<C, double>::value) {
-        const double u1 = a.U[p] / a.DU[p];
-        const double v1 = a.V[p] / a.DV[p];
-        a.u1[p] = u1; a.advU[p] = u1;
-        a.v1[p] = v1; a.advV[p] = v1;
-        // interp_x (ioffset 0) writes i < nx-1; elsewhere the old value is divided
-        const double uu = i < a.nx - 1 ? getm_half(a.U[p] + a.U[p + 1]) : a.uua[p];
-        const double uv = i < a.nx - 1 ? getm_half(a.V[p] + a.V[p + 1]) : a.uva[p];
-        const double vu = j < a.ny - 1 ? getm_half(a.U[p] + a.U[p + a.nx]) : a.vua[p];
-        const double vv = j < a.ny - 1 ? getm_half(a.V[p] + a.V[p + a.nx]) : a.vva[p];
-        a.uua[p] = vel_div<C>(uu, a.DUU[p]);
-        a.uva[p] = vel_div<C>(uv, a.DUV[p]);
-        a.vua[p] = vel_div<C>(vu, a.DVU[p]);
-        a.vva[p] = vel_div<C>(vv, a.DVV[p]);
-    } else {
-        const double Up = a.U[p], Vp = a.V[p];
-        const double u1 = getm_div_refined(Up, a.DU[p]);
-        const double v1 = getm_div_refined(Vp, a.DV[p]);
-        a.u1[p] = u1; a.advU[p] = u1;
-        a.v1[p] = v1; a.advV[p] = v1;
-        const float Uf = getm_d2f_approx(Up), Vf = getm_d2f_approx(Vp);
-        const float uu = i < a.nx - 1 ? 0.5f * (Uf + getm_d2f_approx(a.U[p + 1])) : getm_d2f_approx(a.uua[p]);
-        const float uv = i < a.nx - 1 ? 0.5f * (Vf + getm_d2f_approx(a.V[p + 1])) : getm_d2f_approx(a.uva[p]);
-        const float vu = j < a.ny - 1 ? 0.5f * (Uf + getm_d2f_approx(a.U[p + a.nx])) : getm_d2f_approx(a.vua[p]);
-        const float vv = j < a.ny - 1 ? 0.5f * (Vf + getm_d2f_approx(a.V[p + a.nx])) : getm_d2f_approx(a.vva[p]);
-        a.uua[p] = getm_f2d(uu / getm_d2f_approx(a.DUU[p]));
-        a.uva[p] = getm_f2d(uv / getm_d2f_approx(a.DUV[p]));
-        a.vua[p] = getm_f2d(vu / getm_d2f_approx(a.DVU[p]));
-        a.vva[p] = getm_f2d(vv / getm_d2f_approx(a.DVV[p]));
-    }
+    const bool east = i < a.nx - 1, north = j < a.ny - 1;
+    momentum_2d_velocities_values<C>(a, p, east, north, a.U[p], east ? a.U[p + 1] : 0.0, north ? a.U[p + a.nx] : 0.0,
+                                     a.V[p], east ? a.V[p + 1] : 0.0, north ? a.V[p + a.nx] : 0.0, a.DU[p], a.DV[p],
+                                     a.DUU[p], a.DUV[p], a.DVU[p], a.DVV[p]);
 }
 
 // Momentum.bottom_friction (momentum.py:1099-1125): u1 -> V grid and v1 -> U
@@ -256,42 +249,52 @@ __device__ __forceinline__ double from_c(C x)
 }
 
 template <typename C>
+__device__ __forceinline__ C quotient(C n, C d)
+{
+    if constexpr (std::is_same<C, double>::value) return getm_div(n, d);
+    else return n / d;
+}
+
+template <typename C>
 __device__ __forceinline__ double drag(C uu, C vv, double D, double z0)
 {
-    const C DD = to_c<C>(D);
-    const C sqrtcd = C(GETM_KAPPA) / log(C(1) + C(0.5) * DD / to_c<C>(z0));
+    const C x = C(0.5) * to_c<C>(D);
+    const C sqrtcd = quotient(C(GETM_KAPPA), log(C(1) + quotient(x, to_c<C>(z0))));
     return from_c<C>(sqrtcd * sqrtcd * sqrt(getm_speed2(uu, vv)));
+}
+
+// of the U equation (d 0) or the V equation (d 1)
+template <typename C>
+__device__ __forceinline__ void momentum_2d_friction_half(const FricArgs& a, int d, int i, int j)
+{
+    const int nx = a.nx, p = j * nx + i;
+    const bool u = d == 0;
+    // the point's own operands, loaded before any mask is tested
+    const int m = (u ? a.mU : a.mV)[p];
+    const double own = (u ? a.u1 : a.v1)[p], D = (u ? a.DU : a.DV)[p], z0 = (u ? a.z0bU : a.z0bV)[p];
+    const double* __restrict__ src = u ? a.v1 : a.u1;
+    double* work = u ? a.workU : a.workV;
+    // v_U = interp_xy(v1, ioffset 0, joffset 1): written at j >= 1, i <= nx-2;
+    // u_V = interp_xy(u1, ioffset 1, joffset 0): written at i >= 1, j <= ny-2
+    // (in arithmetic C: the drag coefficient is evaluated in C)
+    C other;
+    if (u ? j >= 1 && i <= nx - 2 : i >= 1 && j <= a.ny - 2) {
+        const int q = u ? p - nx : p - 1;
+        other = C(0.25) * (to_c<C>(src[q]) + to_c<C>(src[q + 1]) + to_c<C>(src[q + nx]) + to_c<C>(src[q + nx + 1]));
+        work[p] = from_c<C>(other);
+    } else {
+        other = to_c<C>(work[p]);
+    }
+    if (m != 1) return;
+    const C mine = to_c<C>(own);
+    (u ? a.ru : a.rv)[p] = drag<C>(u ? mine : other, u ? other : mine, D, z0);
 }
 
 template <typename C>
 __device__ __forceinline__ void momentum_2d_friction_point(const FricArgs& a, int i, int j)
 {
-    const long long p = (long long)j * a.nx + i;
-    const int nx = a.nx;
-    // the point's own operands, loaded before any mask is tested
-    const int mU = a.mU[p], mV = a.mV[p];
-    const double u1p = a.u1[p], v1p = a.v1[p], DUp = a.DU[p], DVp = a.DV[p], z0bUp = a.z0bU[p], z0bVp = a.z0bV[p];
-    // v_U = interp_xy(v1, ioffset 0, joffset 1): written at j >= 1, i <= nx-2
-    // (in arithmetic C: the drag coefficient is evaluated in C)
-    C vU;
-    if (j >= 1 && i <= nx - 2) {
-        const long long q = p - nx;
-        vU = C(0.25) * (to_c<C>(a.v1[q]) + to_c<C>(a.v1[q + 1]) + to_c<C>(a.v1[q + nx]) + to_c<C>(a.v1[q + nx + 1]));
-        a.workU[p] = from_c<C>(vU);
-    } else {
-        vU = to_c<C>(a.workU[p]);
-    }
-    // u_V = interp_xy(u1, ioffset 1, joffset 0): written at i >= 1, j <= ny-2
-    C uV;
-    if (i >= 1 && j <= a.ny - 2) {
-        const long long q = p - 1;
-        uV = C(0.25) * (to_c<C>(a.u1[q]) + to_c<C>(a.u1[q + 1]) + to_c<C>(a.u1[q + nx]) + to_c<C>(a.u1[q + nx + 1]));
-        a.workV[p] = from_c<C>(uV);
-    } else {
-        uV = to_c<C>(a.workV[p]);
-    }
-    if (mU == 1) a.ru[p] = drag<C>(to_c<C>(u1p), vU, DUp, z0bUp);
-    if (mV == 1) a.rv[p] = drag<C>(uV, to_c<C>(v1p), DVp, z0bVp);
+    momentum_2d_friction_half<C>(a, 0, i, j);
+    momentum_2d_friction_half<C>(a, 1, i, j);
 }
 
 // Momentum.coriolis, DEFAULT scheme (momentum.py:1127-1148): interp_xy of the
@@ -349,70 +352,58 @@ struct Transport2DArgs {
     double* U;
 };
 
-// The transport after the update at interior point p: the new value where
-// the mask is 1, else the old one (upd false).  cor: the Coriolis term at p.
-// Every operand is loaded before the mask is tested (one round of
-// independent loads per point).
-struct TransportNew {
-    double v;
-    bool upd;
+// The operands of one point but the Coriolis term, all loaded before the mask
+// is tested (one round of independent loads per point).
+struct TransportIn {
+    int m;
+    double U, SF, D, dp, alpha, taus, adv, diff, damp, SA, SB, SD, r;
 };
 
-__device__ __forceinline__ TransportNew transport_2d_value(const Transport2DArgs& a, double dt, long long p,
-                                                           double cor)
+__device__ __forceinline__ TransportIn transport_2d_load(const Transport2DArgs& a, long long p)
 {
-    const int m = a.mask[p];
-    const double Up = a.U[p], SF = a.SF[p], Dp = a.D[p], dp = a.dp[p], alpha = a.alpha[p], taus = a.taus[p];
-    const double adv = a.adv[p], diff = a.diff[p], damp = a.damp[p];
-    const double SA = a.SA[p], SB = a.SB[p], SD = a.SD[p], r = a.r[p];
-    if (m != 1) return TransportNew{Up, false};
-    const double rho0i = 1.0 / GETM_RHO0;
-    double Slr = (Up > 0.0) ? fmin(SF, 0.0) : fmax(SF, 0.0);
-    return TransportNew{(Up + dt * (-GETM_G * Dp * dp + alpha * (taus * rho0i + cor + adv + diff + damp + SA + SB + SD + Slr)))
-                            / (1.0 + dt * r / Dp),
-                        true};
+    return TransportIn{a.mask[p], a.U[p], a.SF[p], a.D[p], a.dp[p], a.alpha[p], a.taus[p],
+                       a.adv[p], a.diff[p], a.damp[p], a.SA[p], a.SB[p], a.SD[p], a.r[p]};
 }
 
+// The transport after the update: the new value where the mask is 1, else the
+// old one.  cor: the Coriolis term.  MIXED: the tendency is summed in float,
+// the transport is updated in double, and the implicit friction factor
+// 1/(1 + x), x = dt r / D, is applied as U - U x/(1 + x) with the small
+// correction in float (no FP64 division).
+template <bool MIXED>
+__device__ __forceinline__ double transport_2d_value(const TransportIn& a, double dt, double cor)
+{
+    if (a.m != 1) return a.U;
+    if constexpr (!MIXED) {
+        const double rho0i = 1.0 / GETM_RHO0;
+        const double Slr = getm_positive_i(a.U) ? getm_fmin_i(a.SF, 0.0) : getm_fmax_i(a.SF, 0.0);
+        // (contracted in one way in every kernel that forms it)
+        const double sum = __fma_rn(a.taus, rho0i, cor) + a.adv + a.diff + a.damp + a.SA + a.SB + a.SD + Slr;
+        const double tend = __fma_rn(a.alpha, sum, __dmul_rn(__dmul_rn(-GETM_G, a.D), a.dp));
+        return getm_div(__fma_rn(dt, tend, a.U), 1.0 + getm_div(__dmul_rn(dt, a.r), a.D));
+    } else {
+        const float rho0i = (float)(1.0 / GETM_RHO0);
+        const float sf = getm_d2f_approx(a.SF);
+        const float Slr = getm_positive_i(a.U) ? fminf(sf, 0.f) : fmaxf(sf, 0.f);
+        const float Dp = getm_d2f_approx(a.D);
+        const float dtf = (float)dt;
+        const float tend = -(float)GETM_G * Dp * getm_d2f_approx(a.dp) +
+                           getm_d2f_approx(a.alpha) *
+                               (getm_d2f_approx(a.taus) * rho0i + getm_d2f_approx(cor) + getm_d2f_approx(a.adv) +
+                                getm_d2f_approx(a.diff) + getm_d2f_approx(a.damp) + getm_d2f_approx(a.SA) +
+                                getm_d2f_approx(a.SB) + getm_d2f_approx(a.SD) + Slr);
+        const double num = a.U + getm_f2d(dtf * tend);
+        const float x = dtf * getm_d2f_approx(a.r) / Dp;
+        return num - getm_f2d(getm_d2f_approx(num) * (x / (1.f + x)));
+    }
+}
+
+template <bool MIXED>
 __device__ __forceinline__ void transport_2d_point(const Transport2DArgs& a, double dt, long long p)
 {
-    const TransportNew n = transport_2d_value(a, dt, p, a.cor[p]);
-    if (n.upd) a.U[p] = n.v;
-}
-
-// Momentum.advance_depth_integrated's transport update, mixed form
-// (momentum.F90:147-189): the tendency is summed in float, the transport is
-// updated in double, and the implicit friction factor 1/(1 + x), x =
-// dt r / D, is applied as U - U x/(1 + x) with the small correction in float
-// (no FP64 division).
-__device__ __forceinline__ TransportNew transport_2d_mixed_value(const Transport2DArgs& a, double dt, long long p,
-                                                                 double corp)
-{
-    const int* mask = a.mask;
-    const double *alpha = a.alpha, *D = a.D, *dp = a.dp, *taus = a.taus, *adv = a.adv;
-    const double *diff = a.diff, *damp = a.damp, *SA = a.SA, *SB = a.SB, *SD = a.SD, *SF = a.SF, *r = a.r;
-    const int m = mask[p];
-    const double Up = a.U[p], SFp = SF[p], Dd = D[p], dpp = dp[p], alp = alpha[p], tau = taus[p];
-    const double advp = adv[p], diffp = diff[p], dampp = damp[p], SAp = SA[p], SBp = SB[p], SDp = SD[p], rp = r[p];
-    if (m != 1) return TransportNew{Up, false};
-    const float rho0i = (float)(1.0 / GETM_RHO0);
-    const float sf = getm_d2f_approx(SFp);
-    const float Slr = getm_positive_i(Up) ? fminf(sf, 0.f) : fmaxf(sf, 0.f);
-    const float Dp = getm_d2f_approx(Dd);
-    const float dtf = (float)dt;
-    const float tend = -(float)GETM_G * Dp * getm_d2f_approx(dpp) +
-                       getm_d2f_approx(alp) *
-                           (getm_d2f_approx(tau) * rho0i + getm_d2f_approx(corp) + getm_d2f_approx(advp) +
-                            getm_d2f_approx(diffp) + getm_d2f_approx(dampp) + getm_d2f_approx(SAp) +
-                            getm_d2f_approx(SBp) + getm_d2f_approx(SDp) + Slr);
-    const double num = Up + getm_f2d(dtf * tend);
-    const float x = dtf * getm_d2f_approx(rp) / Dp;
-    return TransportNew{num - getm_f2d(getm_d2f_approx(num) * (x / (1.f + x))), true};
-}
-
-__device__ __forceinline__ void transport_2d_mixed_point(const Transport2DArgs& a, double dt, long long p)
-{
-    const TransportNew n = transport_2d_mixed_value(a, dt, p, a.cor[p]);
-    if (n.upd) a.U[p] = n.v;
+    const double cor = a.cor[p];
+    const TransportIn in = transport_2d_load(a, p);
+    if (in.m == 1) a.U[p] = transport_2d_value<MIXED>(in, dt, cor);
 }
 
 // _U_cum += U; _V_cum += V (momentum.py:716-718), every point
@@ -425,11 +416,13 @@ __device__ __forceinline__ void accumulate_2d_point(const double* U, const doubl
 
 // zo = z (every point), then the surface elevation update
 // (simulation.py:1468-1486 -> wrapper.F90:496-523)
-// the elevation update at an interior water point (wrapper.F90:496-523)
+// the elevation update at an interior water point (wrapper.F90:496-523),
+// contracted in one way in every kernel that forms it
 __device__ __forceinline__ double elevation_new(double zp, double dt, double Uw, double dyw, double Ue, double dye,
                                                 double Vs, double dxs, double Vn, double dxn, double ia, double fw)
 {
-    return zp + dt * ((Uw * dyw - Ue * dye + Vs * dxs - Vn * dxn) * ia + fw);
+    const double t = __fma_rn(-Vn, dxn, __fma_rn(Vs, dxs, __fma_rn(Uw, dyw, -__dmul_rn(Ue, dye))));
+    return __fma_rn(dt, __fma_rn(t, ia, fw), zp);
 }
 
 __device__ __forceinline__ void surface_elevation_fused_point(int nx, int ny, int halox, int haloy, const int* mask,
@@ -472,18 +465,12 @@ struct SpgArgs {
 // MIXED: the elevation bounds on the integer pipe, the two differences in
 // FP64 and the rest in float (the mixed transport update reads the gradient
 // as a float).
-template <bool MIXED = false>
-__device__ __forceinline__ void spg_point(const SpgArgs& a, long long p)
+// z, H, D, sp at the point (0) and its east (1) and north (n) neighbours
+template <bool MIXED>
+__device__ __forceinline__ void spg_values(const SpgArgs& a, long long p, int mu, int mv, double z0, double z1,
+                                           double zn, double H0, double H1, double Hn, double D0, double D1, double Dn,
+                                           double sp0, double sp1, double spn, double idx, double idy)
 {
-    const int nx = a.nx;
-    const double gammai = 1.0 / (GETM_G * GETM_RHO0);
-    // every operand is loaded before the masks are tested
-    const int mu = a.umask[p], mv = a.vmask[p];
-    const double z0 = a.z[p], z1 = a.z[p + 1], zn = a.z[p + nx];
-    const double H0 = a.H[p], H1 = a.H[p + 1], Hn = a.H[p + nx];
-    const double D0 = a.D[p], D1 = a.D[p + 1], Dn = a.D[p + nx];
-    const double sp0 = a.sp[p], sp1 = a.sp[p + 1], spn = a.sp[p + nx];
-    const double idx = a.idxu[p], idy = a.idyv[p];
     if constexpr (MIXED) {
         const float gi = (float)(1.0 / (GETM_G * GETM_RHO0));
         if (mu == 1) {
@@ -498,18 +485,28 @@ __device__ __forceinline__ void spg_point(const SpgArgs& a, long long p)
             const float g = getm_d2f_approx(zp - zm) + getm_d2f_approx(spn - sp0) * gi;
             a.dpdy[p] = getm_f2d(g * getm_d2f_approx(idy));
         }
-        return;
+    } else {
+        const double gammai = 1.0 / (GETM_G * GETM_RHO0);
+        if (mu == 1) {
+            const double zp = getm_fmax_i(z1, -H0 + getm_fmin_i(a.Dmin, D1));
+            const double zm = getm_fmax_i(z0, -H1 + getm_fmin_i(a.Dmin, D0));
+            a.dpdx[p] = (zp - zm + (sp1 - sp0) * gammai) * idx;
+        }
+        if (mv == 1) {
+            const double zp = getm_fmax_i(zn, -H0 + getm_fmin_i(a.Dmin, Dn));
+            const double zm = getm_fmax_i(z0, -Hn + getm_fmin_i(a.Dmin, D0));
+            a.dpdy[p] = (zp - zm + (spn - sp0) * gammai) * idy;
+        }
     }
-    if (mu == 1) {
-        double zp = fmax(z1, -H0 + fmin(a.Dmin, D1));
-        double zm = fmax(z0, -H1 + fmin(a.Dmin, D0));
-        a.dpdx[p] = (zp - zm + (sp1 - sp0) * gammai) * idx;
-    }
-    if (mv == 1) {
-        double zp = fmax(zn, -H0 + fmin(a.Dmin, Dn));
-        double zm = fmax(z0, -Hn + fmin(a.Dmin, D0));
-        a.dpdy[p] = (zp - zm + (spn - sp0) * gammai) * idy;
-    }
+}
+
+template <bool MIXED = false>
+__device__ __forceinline__ void spg_point(const SpgArgs& a, long long p)
+{
+    const long long n = p + a.nx;
+    // every operand is loaded before the masks are tested
+    spg_values<MIXED>(a, p, a.umask[p], a.vmask[p], a.z[p], a.z[p + 1], a.z[n], a.H[p], a.H[p + 1], a.H[n], a.D[p],
+                      a.D[p + 1], a.D[n], a.sp[p], a.sp[p + 1], a.sp[n], a.idxu[p], a.idyv[p]);
 }
 
 // interp_x / interp_y (interpolation.F90:9-40) of one point: t = mean of s

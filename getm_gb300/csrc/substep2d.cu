@@ -1,4 +1,4 @@
-// One split-explicit 2D substep as one persistent kernel for sm_103a.
+// One split-explicit 2D substep as four kernels for sm_103a.
 //
 // A 2D substep of pygetm's Simulation.advance that is not followed by a 3D
 // (macro) step (python/pygetm/simulation.py:1033-1304: advance_depth_integrated,
@@ -8,10 +8,8 @@
 // they leave GB300 idle between launches: each reads and writes ~10^5 points,
 // a microsecond of work behind several microseconds of launch and drain.
 //
-// Here one cooperative launch runs the whole substep.  Its blocks (one or
-// two per SM, 512 threads) walk through seven phases separated by grid-wide
-// barriers; a phase contains operations whose inputs at neighbouring points
-// were completed by an earlier phase:
+// The operations depend on one another through neighbouring points only, in
+// seven phases:
 //   1  transport update of the first direction (U or V, alternating)
 //   2  Coriolis term from it, then the second direction's update
 //   3  Coriolis term from the second, cumulative transports, zo = z and the
@@ -22,12 +20,19 @@
 //   6  bottom friction, first pass of the U and V momentum advection
 //   7  second pass of both, forming each cell's advection term from its
 //      transport change as the pass finishes the cell (reconstruct)
-// Every operation is the same device function the separate kernels run
-// (split2d_ops.cuh, advection_passes.cuh), so results are bitwise the same.
+// For one domain, a kernel forms what its tile needs of the phases before it
+// at the tile's edge once more (a row and a column), so that phases 1 and 2
+// are one launch and 3 to 5 another; the two advection passes are one launch
+// each (substep_* kernels below).  For many domains at once, one cooperative
+// launch walks through the seven phases with grid-wide barriers between them
+// (substep_batch_kernel at the end).  Every operation is the same device
+// function the separate kernels run (split2d_ops.cuh, advection_passes.cuh),
+// so results are bitwise the same.
 //
-// The barrier is a counter and a generation word in global memory.  Its wait
-// is bounded: after about a second it sets the error word, every block
-// returns, and later launches return at once until the host clears the word.
+// The batch kernel's barrier is a counter and a generation word in global
+// memory.  Its wait is bounded: after about a second it sets the error word,
+// every block returns, and later launches return at once until the host clears
+// the word.
 #include <string.h>
 
 #include <mutex>
@@ -135,8 +140,6 @@ __device__ __forceinline__ void grid_exit(unsigned* sync)
     }
 }
 
-// One advection pass over the whole plane, distributed over the grid: x
-// passes by warps (one row segment each), y passes by blocks (one tile each).
 // reconstruct_transport_change (momentum.F90:323-340) of a cell as soon as
 // the last advection pass has finished it: un = (un hn - Uo) / dt on rows
 // jlo..jhi (the same expression as reconstruct_point)
@@ -152,48 +155,14 @@ struct ReconstructEpi {
     }
 };
 
-template <bool MIXED, typename Epi = NoEpi>
-__device__ __forceinline__ void advection_pass(const HPassArgs<double>& pa, int dir, SubstepSmem& sm, int tx,
-                                               int ty, const Epi& epi = Epi())
-{
-    using C = typename std::conditional<MIXED, float, double>::type;
-    if (dir == 1) {
-        const int nbx = div_up(pa.nx_ + 1, HX_STRIDE);
-        const long long items = (long long)nbx * pa.ny_;
-        // equal contiguous runs of row segments per block (every SM busy)
-        const long long per = (items + gridDim.x - 1) / gridDim.x;
-        const long long wb = (long long)blockIdx.x * per, we = wb + per < items ? wb + per : items;
-        for (long long w = wb + ty; w < we; w += SS_BY) {
-            const int bx = (int)(w % nbx);
-            const long long row = w / nbx;
-            hpass_x_inc_body<double, Epi, double, C>(pa, bx, row, tx, epi);
-        }
-    } else {
-        const int nbx = div_up(pa.nx_, 32);
-        const int nby = div_up(pa.ny_ + 1, HY_STRIDE);
-        for (int t = blockIdx.x; t < nbx * nby; t += gridDim.x) {
-            if constexpr (MIXED) hpass_y_inc_body<double, Epi, double, float>(pa, t % nbx, t / nbx, 0, tx, ty, sm.yf, epi);
-            else hpass_y_inc_body<double, Epi, double, double>(pa, t % nbx, t / nbx, 0, tx, ty, sm.yd, epi);
-            __syncthreads();  // shared memory is reused by the next tile
-        }
-    }
-}
-
-template <bool MIXED>
-__device__ __forceinline__ void transport_update(const Transport2DArgs& t, double dt, long long p)
-{
-    if constexpr (MIXED) transport_2d_mixed_point(t, dt, p);
-    else transport_2d_point(t, dt, p);
-}
-
 // Coriolis term on the other velocity grid from the transport of direction
 // d (momentum.py:1127-1148): U -> V with offsets (1, 0), negated; V -> U
 // with offsets (0, 1).
 template <typename C>
-__device__ __forceinline__ void coriolis_from(const SubstepArgs& a, int d, int i, int j)
+__device__ __forceinline__ void coriolis_from(const SubstepArgs& a, int d, int i, int j, const double* src)
 {
     const int o = 1 - d;
-    coriolis_2d_point<C>(a.nx, a.ny, d == 0 ? 1 : 0, d == 0 ? 0 : 1, a.tr[d].U, a.corf[o], a.cor_out[o], d == 0, i,
+    coriolis_2d_point<C>(a.nx, a.ny, d == 0 ? 1 : 0, d == 0 ? 0 : 1, src, a.corf[o], a.cor_out[o], d == 0, i,
                          j);
 }
 
@@ -208,14 +177,14 @@ __device__ __forceinline__ void phase_point(const SubstepArgs& a, int ph, int d1
     const bool interior = i >= a.halox && i < nx - a.halox && j >= a.haloy && j < ny - a.haloy;
     switch (ph) {
     case 0:
-        if (interior) transport_update<MIXED>(a.tr[d1], a.dt, p);
+        if (interior) transport_2d_point<MIXED>(a.tr[d1], a.dt, p);
         break;
     case 1:
-        coriolis_from<C>(a, d1, i, j);
-        if (interior) transport_update<MIXED>(a.tr[d2], a.dt, p);
+        coriolis_from<C>(a, d1, i, j, a.tr[d1].U);
+        if (interior) transport_2d_point<MIXED>(a.tr[d2], a.dt, p);
         break;
     case 2:
-        coriolis_from<C>(a, d2, i, j);
+        coriolis_from<C>(a, d2, i, j, a.tr[d2].U);
         if (a.accumulate) accumulate_2d_point(a.tr[0].U, a.tr[1].U, a.Ucum, a.Vcum, p);
         surface_elevation_fused_point(nx, ny, a.halox, a.haloy, a.mT, a.dyU, a.dxV, a.iareaT, a.z, a.zo,
                                       a.tr[0].U, a.tr[1].U, a.fwf, a.dt, i, j);
@@ -237,137 +206,11 @@ __device__ __forceinline__ void phase_point(const SubstepArgs& a, int ph, int d1
     }
 }
 
-template <bool MIXED>
-__global__ void __launch_bounds__(SS_THREADS, MIXED ? 2 : 1) substep_2d_kernel(SubstepArgs a)
-{
-    __shared__ SubstepSmem sm;
-    __shared__ int s_ok;
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int gt = blockIdx.x * SS_THREADS + ty * 32 + tx;
-    // pointwise phases: the plane in equal contiguous chunks, one per block,
-    // so every SM gets the same number of points (a grid-stride loop over
-    // fewer points than threads would leave the last blocks idle and give
-    // the first SMs a third more work); consecutive threads take
-    // consecutive points
-    const int tid = ty * 32 + tx;
-    const int nx = a.nx, ny = a.ny;
-    const int n = nx * ny;  // < 2^30 (checked by the host)
-    const int chunk = (n + (int)gridDim.x - 1) / (int)gridDim.x;
-    const int pb = (int)blockIdx.x * chunk, pe = min(pb + chunk, n);
-    const int jlo = a.haloy, jhi = ny - a.haloy - 1;
-
-    unsigned target = 0;  // barrier count to wait for (thread 0)
-    if (tx == 0 && ty == 0) s_ok = ld_acquire(&a.sync[2]) == 0;
-    __syncthreads();
-    if (!s_ok) return;
-
-    const int d1 = a.ufirst ? 0 : 1;
-    auto points = [&](int ph) {
-        for (int p = pb + tid; p < pe; p += SS_THREADS) {
-            const int j = p / nx, i = p - j * nx;
-            phase_point<MIXED>(a, ph, d1, i, j, p);
-        }
-    };
-    // 1: first transport update
-    points(0);
-    if (!grid_barrier(a.sync, target, s_ok)) return grid_exit(a.sync);
-    // 2: Coriolis from the first, second transport update
-    points(1);
-    if (!grid_barrier(a.sync, target, s_ok)) return grid_exit(a.sync);
-    // 3: Coriolis from the second, cumulative transports, surface elevation
-    points(2);
-    if (!grid_barrier(a.sync, target, s_ok)) return grid_exit(a.sync);
-    // 4: depths; fwf = pe; wind stress on U and V (interp_x/y, offset 0)
-    {
-        const int ntx = div_up(nx + 1, UD_BX), nty = div_up(ny + 1, SS_BY);
-        for (int t = blockIdx.x; t < ntx * nty; t += gridDim.x) {
-            update_depth_2d_tile<SS_BY, MIXED>(a.depth, t % ntx, t / ntx, tx, ty, sm.szh);
-            __syncthreads();
-        }
-    }
-    points(3);
-    if (!grid_barrier(a.sync, target, s_ok)) return grid_exit(a.sync);
-    // 5: velocities, advected thicknesses, surface pressure gradient
-    points(4);
-    if (!grid_barrier(a.sync, target, s_ok)) return grid_exit(a.sync);
-    // 6: bottom friction; first advection passes
-    if (a.friction) points(5);
-    advection_pass<MIXED>(a.adv[0].pass[0], a.adv[0].dir[0], sm, tx, ty);
-    advection_pass<MIXED>(a.adv[1].pass[0], a.adv[1].dir[0], sm, tx, ty);
-    if (!grid_barrier(a.sync, target, s_ok)) return grid_exit(a.sync);
-    // 7: second advection passes, each cell's advection term formed as the
-    // pass finishes it (reconstruct_transport_change).  The model time moves
-    // on only here, after the last barrier: a substep abandoned at a barrier
-    // leaves it unchanged (no phase reads it).
-    if (gt == 0 && a.time) *a.time = *a.time + a.dt;
-    for (int d = 0; d < 2; d++) {
-        const ReconstructEpi epi{a.advvar[d], a.Uo[d], a.idt, jlo, jhi};
-        advection_pass<MIXED>(a.adv[d].pass[1], a.adv[d].dir[1], sm, tx, ty, epi);
-    }
-    grid_exit(a.sync);
-}
-
 static_assert(sizeof(SubstepArgs) <= 4096, "kernel parameter block");
 
 constexpr int SS_MAX_DEVICES = 64;
 
-// Co-resident blocks of substep_2d_kernel<MIXED> on device `dev` (SMs times
-// blocks per SM), queried once per device and kept under a mutex, so host
-// threads driving different GPUs each get their own device's count.
-template <bool MIXED>
-int substep_blocks(int dev, int* blocks)
-{
-    static int cache[SS_MAX_DEVICES];
-    static std::mutex mutex;
-    if (dev < 0 || dev >= SS_MAX_DEVICES) return GETM_ERR_ARG;
-    std::lock_guard<std::mutex> lock(mutex);
-    if (cache[dev] == 0) {
-        int sms = 0, coop = 0, per_sm = 0;
-        if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop)
-            return GETM_ERR_CUDA;
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return GETM_ERR_CUDA;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, substep_2d_kernel<MIXED>, SS_THREADS, 0) !=
-                cudaSuccess ||
-            per_sm < 1)
-            return GETM_ERR_CUDA;
-        cache[dev] = sms * per_sm;
-    }
-    *blocks = cache[dev];
-    return GETM_OK;
-}
-
-template <bool MIXED>
-int launch_substep(const SubstepArgs& a, cudaStream_t stream)
-{
-    int dev = 0, blocks = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return GETM_ERR_CUDA;
-    if (int rc = substep_blocks<MIXED>(dev, &blocks)) return rc;
-    // launch-shape knob: fewer blocks per SM than fit (never more)
-    const int per_sm = getm_tune(GETM_TUNE_SUBSTEP_BLOCKS);
-    if (per_sm > 0) {
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return GETM_ERR_CUDA;
-        if (per_sm * sms < blocks) blocks = per_sm * sms;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(32, SS_BY);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, substep_2d_kernel<MIXED>, a) != cudaSuccess) return GETM_ERR_CUDA;
-    GETM_CHECK_LAUNCH();
-    return GETM_OK;
-}
-
-}  // namespace
-
-namespace {
-
-// The kernel's arguments for one domain from its fields and handles; a
+// The kernels' arguments for one domain from its fields and handles; a
 // GETM_* status.
 int substep_args(SubstepArgs& a, const getm_split2d_fields* f, int nx, int ny, int halox, int haloy, int mixed,
                  int ufirst, int accumulate, int friction, double timestep, double Dmin, double Dcrit,
@@ -384,7 +227,7 @@ int substep_args(SubstepArgs& a, const getm_split2d_fields* f, int nx, int ny, i
                           f->mask_v, f->H_v, f->dx_v, f->idy_v, f->cor_v, f->z0b_v, f->D_v, f->alpha_v, f->work_v,
                           f->V, f->dpdy, f->tausy, f->corV, f->advV, f->diffV, f->dampV, f->SyA, f->SyB, f->SyD,
                           f->SyF, f->rv, f->v1, f->Vcum, f->advD_v, f->vua, f->vva,
-                          f->mask_x, f->H_x, f->D_x, f->work_x, f->D_uu, f->D_uv, f->D_vu, f->D_vv};
+                          f->mask_x, f->H_x, f->D_x, f->work_x, f->D_uu, f->D_uv, f->D_vu, f->D_vv, f->sync};
     for (const void* q : ptrs)
         if (!q) return GETM_ERR_ARG;
     memset(&a, 0, sizeof(a));
@@ -431,84 +274,269 @@ int substep_args(SubstepArgs& a, const getm_split2d_fields* f, int nx, int ny, i
 
 }  // namespace
 
-extern "C" int getm_split2d_substep(const getm_split2d_fields* f, int nx, int ny, int halox, int haloy, int mixed,
-                                    int ufirst, int accumulate, int friction, double timestep, double Dmin,
-                                    double Dcrit, getm_advection* uadv, getm_grid* ugrid, getm_grid* uugrid,
-                                    getm_grid* uvgrid, int uadv_ufirst, getm_advection* vadv, getm_grid* vgrid,
-                                    getm_grid* vugrid, getm_grid* vvgrid, int vadv_ufirst, cudaStream_t stream)
-{
-    SubstepArgs a;
-    if (!f || !f->sync) return GETM_ERR_ARG;
-    int rc = substep_args(a, f, nx, ny, halox, haloy, mixed, ufirst, accumulate, friction, timestep, Dmin, Dcrit,
-                          uadv, ugrid, uugrid, uvgrid, uadv_ufirst, vadv, vgrid, vugrid, vvgrid, vadv_ufirst);
-    if (rc) return rc;
-    return mixed ? launch_substep<true>(a, stream) : launch_substep<false>(a, stream);
-}
-
 // ---------------------------------------------------------------------------
-// One substep as seven ordinary launches
+// One substep of one domain: four launches
 // ---------------------------------------------------------------------------
-// For a domain that shares the GPU with others (ensemble members and served
-// requests replay on several streams): a cooperative launch would need every
-// SM at once, and the operations launched one by one are twenty kernels of a
-// few microseconds each on such planes, bound by their launches (a 92 x 92
-// member: 512 launches per 3D step of 24 substeps, 3.4 us each in a CUDA graph).
-// Here each phase above is one kernel over the whole plane, with the same
-// device functions per point, so the results are those of substep_2d_kernel.
-// Blocks are small (64 threads for the points) so that a small plane spreads
-// over as many SMs as it can; U's and V's advection passes and the friction
-// share a launch (grid z).  Each kernel is launched while the one before still
-// runs (programmatic dependent launch) and waits for its end before it
-// touches memory; the first is launched in the ordinary way, since what
-// precedes it on the stream may be anything.
+// What bounds these: on small planes the launches and one chain of latencies per
+// kernel; on large ones instructions, L2 traffic (about 75 fields of a plane)
+// and the FP64 pipe, which in the FP64 form is most of the time.  us per substep
+// in a CUDA graph, one cooperative launch with six grid barriers -> the seven
+// phases as seven launches -> these four:
+//   mixed  64 x 64  45 -> 27 -> 24    200 x 150  46 -> 30 -> 27    400 x 300  56 -> 51 -> 48
+//   FP64   64 x 64  56 -> 48 -> 32    150 x 120  58 -> 53 -> 42    220 x 160  68 -> 66 -> 57
+// A barrier cost about 1.3 us and left every SM to the slowest block, and one
+// register budget served all phases.  Each kernel but the first is launched
+// when the blocks of the one before are done (programmatic dependent launch
+// without an early trigger: blocks launched while the SMs are still busy land
+// on whichever has room, and the FP64 pipes of those SMs then set the pace:
+// FP64 220 x 160 57 -> 90 us) and waits for its end before it touches the
+// fields; what precedes the first on the stream may be anything.
 namespace {
 
-constexpr int PH_PY = 2;  // rows of a point block
-constexpr int PH_DY = 4;  // rows of a depth tile
 constexpr int PH_XY = 4;  // rows of an x pass block
 
-__device__ __forceinline__ void phase_begin()
+// Rows of a tile, chosen per plane (substep_rows): up to TR_MAX for the
+// transports ((by + 1) x 33 staged points, one per thread) and DV_MAX for the
+// depths ((by + 2) x 34).  Registers for two and three blocks of that size per SM.
+constexpr int TR_MAX = 14, TR_THREADS = 512, DV_MAX = 9, DV_THREADS = 384;
+static_assert((TR_MAX + 1) * 33 <= TR_THREADS && (DV_MAX + 2) * 34 <= DV_THREADS, "one staged point per thread");
+
+// Waits for the kernel before; true when the error word is set (the kernel then leaves every field as it is).  The word is
+// written only on the host's behalf, before the substep's first launch.
+__device__ __forceinline__ bool substep_begin(const SubstepArgs& a)
 {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    unsigned err;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(err) : "l"(a.sync + 2) : "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    return err != 0;
 }
 
-template <bool MIXED, int PH>
-__global__ void __launch_bounds__(32 * PH_PY) phase_points_kernel(const __grid_constant__ SubstepArgs a)
-{
-    phase_begin();
-    const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * PH_PY + threadIdx.y;
-    if (i < a.nx && j < a.ny) phase_point<MIXED>(a, PH, a.ufirst ? 0 : 1, i, j, j * a.nx + i);
-}
+// The updated transports between the first two kernels: the momentum
+// advections' scratch fields, free until the first advection pass.
+__device__ __forceinline__ double* new_transport(const SubstepArgs& a, int d) { return a.adv[d].pass[0].fout[0]; }
 
-template <bool MIXED>
-__global__ void __launch_bounds__(32 * PH_DY) phase_depth_kernel(const __grid_constant__ SubstepArgs a)
-{
-    __shared__ double szh[PH_DY + 2][UD_BX + 2];
-    phase_begin();
-    const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * PH_DY + threadIdx.y;
-    if (i < a.nx && j < a.ny) phase_point<MIXED>(a, 3, 0, i, j, j * a.nx + i);
-    update_depth_2d_tile<PH_DY, MIXED>(a.depth, blockIdx.x, blockIdx.y, threadIdx.x, threadIdx.y, szh);
-}
-
-// Advection pass PASS in direction DIR of U (block z 0; d0 = 0) and V; block z
-// ndir, where it is launched, holds the friction of phase 6.
-template <bool MIXED, int PASS, int DIR>
-__global__ void __launch_bounds__(DIR == 1 ? 32 * PH_XY : SS_THREADS)
-    phase_advection_kernel(const __grid_constant__ SubstepArgs a, int d0, int ndir)
+// Phases 1 and 2: both transports into scratch (a neighbouring tile may still
+// need the old ones), the Coriolis term of the second.  D1: the direction
+// updated first; a tile of 32 x by points needs it on one more row and
+// column, one point per thread; the second update's operands are loaded
+// before the exchange.
+template <bool MIXED, int D1>
+__global__ void __launch_bounds__(TR_THREADS, 2)
+    substep_transport_kernel(const __grid_constant__ SubstepArgs a, const int by)
 {
     using C = typename std::conditional<MIXED, float, double>::type;
-    constexpr int BY = DIR == 1 ? PH_XY : SS_BY;
-    phase_begin();
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    if (blockIdx.z == ndir) {
-        const int n = a.nx * a.ny, step = 32 * BY * gridDim.x * gridDim.y;
-        for (int p = ((blockIdx.y * gridDim.x + blockIdx.x) * BY + ty) * 32 + tx; p < n; p += step)
-            phase_point<MIXED>(a, 5, 0, p % a.nx, p / a.nx, p);
-        return;
+    constexpr int D2 = 1 - D1;
+    constexpr int OX = D1 == 0 ? 1 : 0, OY = 1 - OX;  // columns west and rows south of the tile
+    __shared__ double s1[TR_MAX + 1][33];
+    const bool err = substep_begin(a);
+    const int nx = a.nx, ny = a.ny, t = threadIdx.x;
+    const int i0 = blockIdx.x * 32, j0 = blockIdx.y * by;
+    auto interior = [&](int i, int j) {
+        return i >= a.halox && i < nx - a.halox && j >= a.haloy && j < ny - a.haloy;
+    };
+    // the second direction's operands of the thread's point
+    const int ty = t / 32, tx = t % 32, i = i0 + tx, j = j0 + ty;
+    const bool own = ty < by && i < nx && j < ny;
+    const int p = j * nx + i;
+    TransportIn in2 = {};
+    double cor2 = 0.0, f2 = 0.0, zp = 0.0;
+    if (own) {
+        in2 = transport_2d_load(a.tr[D2], p);
+        f2 = a.corf[D2][p];
+        zp = a.z[p];
     }
+    // the first direction's staged point
+    const int sj = t / 33, si = t - sj * 33, gi = i0 - OX + si, gj = j0 - OY + sj;
+    if (sj <= by && gi >= 0 && gi < nx && gj >= 0 && gj < ny) {
+        const int q = gj * nx + gi;
+        const double cor = a.tr[D1].cor[q];
+        const TransportIn in1 = transport_2d_load(a.tr[D1], q);
+        s1[sj][si] = interior(gi, gj) ? transport_2d_value<MIXED>(in1, a.dt, cor) : in1.U;
+    }
+    __syncthreads();
+    if (err || !own) return;
+    new_transport(a, D1)[p] = s1[ty + OY][tx + OX];
+    // U -> V with offsets (1, 0), negated; V -> U with offsets (0, 1)
+    constexpr int ioff = D1 == 0 ? 1 : 0, joff = 1 - ioff;
+    if (coriolis_2d_inside(nx, ny, ioff, joff, i, j)) {
+        auto at = [&](int ai, int aj) { return s1[aj - j0 + OY][ai - i0 + OX]; };
+        cor2 = coriolis_2d_value<C>(ioff, joff, i, j, at, f2, D1 == 0);
+    } else {
+        cor2 = coriolis_2d_outside<C>(a.cor_out[D2][p], f2, D1 == 0);
+    }
+    a.cor_out[D2][p] = cor2;
+    new_transport(a, D2)[p] = interior(i, j) ? transport_2d_value<MIXED>(in2, a.dt, cor2) : in2.U;
+    a.zo[p] = zp;
+}
+
+// Phases 3 to 5 on tiles of 32 x by points (T, U, V at (j, i) and X at
+// (j, i) and (j + 1, i + 1)): new elevations of the tile and a point around
+// it from the old ones (zo) and the new transports in scratch, the depths at
+// T, U, V and X, and from them the velocities and the surface pressure
+// gradient of the tile's points.  z, U and V are written, never read here.
+template <bool MIXED>
+__global__ void __launch_bounds__(DV_THREADS, 3)
+    substep_depth_kernel(const __grid_constant__ SubstepArgs a, const int by)
+{
+    using C = typename std::conditional<MIXED, float, double>::type;
+    __shared__ double sz[DV_MAX + 2][34], szh[DV_MAX + 2][34];  // elevation: new, and the mean with the old
+    __shared__ double sH[DV_MAX + 2][34], sD[DV_MAX + 2][34], sdh[DV_MAX + 2][34];  // T: H, D, D of the mean
+    __shared__ double sX[DV_MAX + 1][33];  // X depths
+    const bool err = substep_begin(a);
+    const DepthArgs& da = a.depth;
+    const int nx = a.nx, ny = a.ny, t = threadIdx.x;
+    const int i0 = blockIdx.x * 32, j0 = blockIdx.y * by;
+    const double* __restrict__ Us = new_transport(a, 0);
+    const double* __restrict__ Vs = new_transport(a, 1);
+    // operands of the thread's point and of its X point, loaded while the
+    // elevations are staged
+    const int ty = t / 32, tx = t % 32, i = i0 + tx, j = j0 + ty;
+    const bool own = ty < by && i < nx && j < ny;
+    const bool east = i < nx - 1, north = j < ny - 1;
+    const int p = j * nx + i;
+    int mU = 0, mV = 0;
+    double HU = 0.0, HV = 0.0, Up = 0.0, Ue = 0.0, Un = 0.0, Vp = 0.0, Ve = 0.0, Vn = 0.0;
+    if (own) {
+        mU = da.mU[p]; mV = da.mV[p]; HU = da.HU[p]; HV = da.HV[p];
+        Up = Us[p]; Vp = Vs[p];
+        if (east) { Ue = Us[p + 1]; Ve = Vs[p + 1]; }
+        if (north) { Un = Us[p + nx]; Vn = Vs[p + nx]; }
+    }
+    const int xj = t / 33, xi = t - xj * 33, Xj = j0 + xj, Xi = i0 + xi;
+    const bool xin = xj <= by && Xi <= nx && Xj <= ny;
+    const int px = Xj * (nx + 1) + Xi;
+    int mX = 0;
+    double HX = 0.0;
+    if (xin) { mX = da.mX[px]; HX = da.HX[px]; }
+
+    // elevation (simulation.py:1468-1486) and T depths of the staged point
+    const int sj = t / 34, si = t - sj * 34, gi = i0 - 1 + si, gj = j0 - 1 + sj;
+    if (sj < by + 2) {
+        double z = 0.0, zh = 0.0, D = 0.0, H = 0.0, dh = 0.0;
+        if (gi >= 0 && gi < nx && gj >= 0 && gj < ny) {
+            const int g = gj * nx + gi;
+            const int m = a.mT[g];
+            const double zo = a.zo[g];
+            H = da.HT[g];
+            z = zo;
+            if (gi >= a.halox && gi < nx - a.halox && gj >= a.haloy && gj < ny - a.haloy) {
+                const double Uw = Us[g - 1], dyw = a.dyU[g - 1], Uc = Us[g], dye = a.dyU[g];
+                const double Vs0 = Vs[g - nx], dxs = a.dxV[g - nx], Vc = Vs[g], dxn = a.dxV[g];
+                const double ia = a.iareaT[g], fw = a.fwf[g];
+                if (m == 1) z = elevation_new(zo, a.dt, Uw, dyw, Uc, dye, Vs0, dxs, Vc, dxn, ia, fw);
+            }
+            zh = getm_half(zo + z);
+            D = m != 0 ? getm_fmax_i(H + z, -1000.0) : da.DT[g];
+            dh = m != 0 ? getm_fmax_i(H + zh, da.Dmin) : zh;
+            if (!err && sj >= 1 && sj <= by && si >= 1 && si <= 32) {  // the tile's own point
+                if (m == 1) a.z[g] = z;
+                if (m != 0) da.DT[g] = D;
+                da.DclipT[g] = dclamp_min(D, da.Dmin);
+                da.workT[g] = dh;
+            }
+        }
+        sz[sj][si] = z; szh[sj][si] = zh; sH[sj][si] = H; sD[sj][si] = D; sdh[sj][si] = dh;
+    }
+    __syncthreads();
+    if (err) return;
+    // X depths: interp_xy T->X (offsets 1, 1) where it writes, else the
+    // previous X._work value
+    if (xin) {
+        const bool mine = xj < by && xi < 32;
+        double zx;
+        if (Xj >= 1 && Xj <= ny - 1 && Xi >= 1 && Xi <= nx - 1) {
+            zx = getm_quarter(szh[xj][xi] + szh[xj][xi + 1] + szh[xj + 1][xi] + szh[xj + 1][xi + 1]);
+            if (mine) da.workX[px] = zx;
+        } else {
+            zx = da.workX[px];
+        }
+        const double dx = mX != 0 ? getm_fmax_i(HX + zx, da.Dmin) : da.DX[px];
+        if (mine && mX != 0) da.DX[px] = dx;
+        sX[xj][xi] = dx;
+    }
+    double sp0 = 0.0, sp1 = 0.0, spn = 0.0, idx = 0.0, idy = 0.0;
+    const bool interior = own && i >= a.halox && i < nx - a.halox && j >= a.haloy && j < ny - a.haloy;
+    if (interior) {
+        sp0 = a.spg.sp[p]; sp1 = a.spg.sp[p + 1]; spn = a.spg.sp[p + nx];
+        idx = a.spg.idxu[p]; idy = a.spg.idyv[p];
+    }
+    __syncthreads();
+    if (!own) return;
+    const int y = ty + 1, x = tx + 1;  // the point in the staged tile
+    const double zh = szh[y][x];
+    const double twoDmin = 2 * da.Dmin;
+    const float twoDmin_f = 2.f * getm_d2f_approx(da.Dmin), ialpha_f = getm_d2f_approx(da.ialpha);
+    // U: z_U = interp_x(z_T_half, ioffset 0) for i < nx-1, else the old value
+    double zu, zv, DU, DV;
+    if (east) {
+        zu = getm_half(zh + szh[y][x + 1]);
+        da.workU[p] = zu;
+    } else {
+        zu = da.workU[p];
+    }
+    if (mU != 0) {
+        DU = getm_fmax_i(HU + zu, da.Dmin);
+        da.DU[p] = DU;
+        da.alphaU[p] = MIXED ? alpha_of_f(DU, twoDmin_f, ialpha_f) : alpha_of(DU, twoDmin, da.ialpha);
+    } else {
+        DU = da.DU[p];
+    }
+    // V: z_V = interp_y(z_T_half, joffset 0) for j < ny-1
+    if (north) {
+        zv = getm_half(zh + szh[y + 1][x]);
+        da.workV[p] = zv;
+    } else {
+        zv = da.workV[p];
+    }
+    if (mV != 0) {
+        DV = getm_fmax_i(HV + zv, da.Dmin);
+        da.DV[p] = DV;
+        da.alphaV[p] = MIXED ? alpha_of_f(DV, twoDmin_f, ialpha_f) : alpha_of(DV, twoDmin, da.ialpha);
+    } else {
+        DV = da.DV[p];
+    }
+    // UU.D[:, :-1] = D_T_half[:, 1:], VV.D[:-1, :] = D_T_half[1:, :], UV.D = VU.D = X.D[1:, 1:]
+    const double DUU = east ? sdh[y][x + 1] : da.DUU[p], DVV = north ? sdh[y + 1][x] : da.DVV[p];
+    const double DUV = sX[ty + 1][tx + 1];
+    if (east) da.DUU[p] = DUU;
+    if (north) da.DVV[p] = DVV;
+    da.DUV[p] = DUV;
+    da.DVU[p] = DUV;
+    a.advD[0][p] = DU;
+    a.advD[1][p] = DV;
+    momentum_2d_velocities_values<C>(a.vel, p, east, north, Up, Ue, Un, Vp, Ve, Vn, DU, DV, DUU, DUV, DUV, DVV);
+    // the transports' final values, and what only reads them
+    a.tr[0].U[p] = Up;
+    a.tr[1].U[p] = Vp;
+    if (a.accumulate) accumulate_2d_point(Us, Vs, a.Ucum, a.Vcum, p);
+    coriolis_from<C>(a, a.ufirst ? 1 : 0, i, j, a.ufirst ? Vs : Us);
+    if (east) interp_pair_point<double>(a.taux, a.tausx, p, 1, 0);
+    if (north) interp_pair_point<double>(a.tauy, a.tausy, p, nx, 0);
+    if (interior)
+        spg_values<MIXED>(a.spg, p, mU, mV, sz[y][x], sz[y][x + 1], sz[y + 1][x], sH[y][x], sH[y][x + 1], sH[y + 1][x],
+                          sD[y][x], sD[y][x + 1], sD[y + 1][x], sp0, sp1, spn, idx, idy);
+}
+
+// Phases 6 and 7: advection pass PASS in direction DIR of U (block z 0; d0 =
+// 0) and V.  With the first pass, the blocks share out the friction of their
+// direction's equation and fwf = pe (which phase 3 still needed): the FP64
+// form's friction takes as long as its pass, so every block gets its part.
+template <bool MIXED, int PASS, int DIR, int BY>
+__global__ void __launch_bounds__(32 * BY)
+    substep_advection_kernel(const __grid_constant__ SubstepArgs a, int d0)
+{
+    using C = typename std::conditional<MIXED, float, double>::type;
+    if (substep_begin(a)) return;
+    const int tx = threadIdx.x, ty = threadIdx.y;
     const int d = d0 + blockIdx.z;
     const HPassArgs<double>& pa = a.adv[d].pass[PASS];
+    if (PASS == 0) {
+        const int n = a.nx * a.ny, step = 32 * BY * gridDim.x * gridDim.y;
+        for (int p = ((blockIdx.y * gridDim.x + blockIdx.x) * BY + ty) * 32 + tx; p < n; p += step) {
+            if (d == 0) a.fwf[p] = a.pe[p];
+            if (a.friction) momentum_2d_friction_half<C>(a.fric, d, p % a.nx, p / a.nx);
+        }
+    }
     if (PASS == 1 && d == 0 && blockIdx.x == 0 && blockIdx.y == 0 && tx == 0 && ty == 0 && a.time)
         *a.time = *a.time + a.dt;
     auto pass = [&](const auto& epi) {
@@ -517,8 +545,8 @@ __global__ void __launch_bounds__(DIR == 1 ? 32 * PH_XY : SS_THREADS)
             const int row = blockIdx.y * BY + ty;
             if (row < pa.ny_) hpass_x_inc_body<double, E, double, C>(pa, blockIdx.x, row, tx, epi);
         } else {
-            __shared__ YIncSmem<double, C> sm;
-            hpass_y_inc_body<double, E, double, C>(pa, blockIdx.x, blockIdx.y, 0, tx, ty, sm, epi);
+            __shared__ YIncSmem<double, C, BY> sm;
+            hpass_y_inc_body<double, E, double, C, BY>(pa, blockIdx.x, blockIdx.y, 0, tx, ty, sm, epi);
         }
     };
     if constexpr (PASS == 1) pass(ReconstructEpi{a.advvar[d], a.Uo[d], a.idt, a.haloy, a.ny - a.haloy - 1});
@@ -526,7 +554,7 @@ __global__ void __launch_bounds__(DIR == 1 ? 32 * PH_XY : SS_THREADS)
 }
 
 template <typename K, typename... A>
-int launch_phase(K kernel, dim3 grid, dim3 block, bool first, cudaStream_t stream, const A&... args)
+int launch_substep(K kernel, dim3 grid, dim3 block, bool first, cudaStream_t stream, const A&... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -545,53 +573,73 @@ int launch_phase(K kernel, dim3 grid, dim3 block, bool first, cudaStream_t strea
 // One launch for both directions' pass where they share the axis (they do
 // unless the host gave the two advections different orders)
 template <bool MIXED, int PASS>
-int launch_phase_advection(const SubstepArgs& a, bool friction, cudaStream_t stream)
+int launch_substep_advection(const SubstepArgs& a, cudaStream_t stream)
 {
-    const dim3 gx(div_up(a.nx + 1, HX_STRIDE), div_up(a.ny, PH_XY)), gy(div_up(a.nx, 32), div_up(a.ny + 1, HY_STRIDE));
     const bool one = a.adv[0].dir[PASS] == a.adv[1].dir[PASS];
-    for (int d = 0; d < (one ? 1 : 2); d++) {
-        const int ndir = one ? 2 : 1;
-        dim3 g = a.adv[d].dir[PASS] == 1 ? gx : gy;
-        g.z = ndir + (friction && d == 0);
-        const int rc = a.adv[d].dir[PASS] == 1
-                           ? launch_phase(phase_advection_kernel<MIXED, PASS, 1>, g, dim3(32, PH_XY), false, stream, a,
-                                          d, ndir)
-                           : launch_phase(phase_advection_kernel<MIXED, PASS, 2>, g, dim3(32, SS_BY), false, stream, a,
-                                          d, ndir);
+    const int nd = one ? 2 : 1;
+    for (int d = 0; d < 3 - nd; d++) {
+        int rc;
+        if (a.adv[d].dir[PASS] == 1) {
+            const dim3 g(div_up(a.nx + 1, HX_STRIDE), div_up(a.ny, PH_XY), nd);
+            rc = launch_substep(substep_advection_kernel<MIXED, PASS, 1, PH_XY>, g, dim3(32, PH_XY), false, stream, a, d);
+        } else {
+            // tiles of 16 or 8 rows (one of them the edge), whichever loads
+            // the fullest SM less
+            const long long nbx = (long long)div_up(a.nx, 32) * nd;
+            const dim3 g16(div_up(a.nx, 32), div_up(a.ny + 1, 15), nd), g8(div_up(a.nx, 32), div_up(a.ny + 1, 7), nd);
+            if (2 * getm_div_up(nbx * g16.y, GETM_SMS) <= getm_div_up(nbx * g8.y, GETM_SMS))
+                rc = launch_substep(substep_advection_kernel<MIXED, PASS, 2, 16>, g16, dim3(32, 16), false, stream, a, d);
+            else
+                rc = launch_substep(substep_advection_kernel<MIXED, PASS, 2, 8>, g8, dim3(32, 8), false, stream, a, d);
+        }
         if (rc) return rc;
     }
     return GETM_OK;
 }
 
-template <bool MIXED>
-int launch_phases(const SubstepArgs& a, cudaStream_t stream)
+// Rows of a tile with `edge` more staged: the height up to `most` that leaves
+// the SM with most tiles the fewest staged rows.  A plane then goes in one
+// wave where it can (400 x 300: 442 depth tiles of 9 rows on 152 SMs of three),
+// and a small one spreads over as many SMs as it can, whose FP64 pipes it waits for.
+inline int substep_rows(int nx, int ny, int most, int edge)
 {
-    const dim3 pb(32, PH_PY), pg(div_up(a.nx, 32), div_up(a.ny, PH_PY));
-    const dim3 db(32, PH_DY), dg(div_up(a.nx + 1, UD_BX), div_up(a.ny + 1, PH_DY));
-    int rc = launch_phase(phase_points_kernel<MIXED, 0>, pg, pb, true, stream, a);
-    if (!rc) rc = launch_phase(phase_points_kernel<MIXED, 1>, pg, pb, false, stream, a);
-    if (!rc) rc = launch_phase(phase_points_kernel<MIXED, 2>, pg, pb, false, stream, a);
-    if (!rc) rc = launch_phase(phase_depth_kernel<MIXED>, dg, db, false, stream, a);
-    if (!rc) rc = launch_phase(phase_points_kernel<MIXED, 4>, pg, pb, false, stream, a);
-    if (!rc) rc = launch_phase_advection<MIXED, 0>(a, a.friction != 0, stream);
-    if (!rc) rc = launch_phase_advection<MIXED, 1>(a, false, stream);
+    int best = most;
+    long long least = 0;
+    for (int by = most; by >= 2; by--) {
+        const long long tiles = (long long)div_up(nx, 32) * div_up(ny, by);
+        const long long load = (tiles + GETM_SMS - 1) / GETM_SMS * (by + edge);
+        if (by == most || load < least) { least = load; best = by; }
+    }
+    return best;
+}
+
+template <bool MIXED>
+int launch_substep_kernels(const SubstepArgs& a, cudaStream_t stream)
+{
+    const int tr = substep_rows(a.nx, a.ny, TR_MAX, 1), dv = substep_rows(a.nx + 1, a.ny + 1, DV_MAX, 2);
+    const dim3 tg(div_up(a.nx, 32), div_up(a.ny, tr)), tb(div_up((tr + 1) * 33, 32) * 32);
+    const dim3 dg(div_up(a.nx + 1, 32), div_up(a.ny + 1, dv)), db(div_up((dv + 2) * 34, 32) * 32);
+    int rc = a.ufirst ? launch_substep(substep_transport_kernel<MIXED, 0>, tg, tb, true, stream, a, tr)
+                      : launch_substep(substep_transport_kernel<MIXED, 1>, tg, tb, true, stream, a, tr);
+    if (!rc) rc = launch_substep(substep_depth_kernel<MIXED>, dg, db, false, stream, a, dv);
+    if (!rc) rc = launch_substep_advection<MIXED, 0>(a, stream);
+    if (!rc) rc = launch_substep_advection<MIXED, 1>(a, stream);
     return rc;
 }
 
 }  // namespace
 
-extern "C" int getm_split2d_substep_phases(const getm_split2d_fields* f, int nx, int ny, int halox, int haloy,
-                                           int mixed, int ufirst, int accumulate, int friction, double timestep,
-                                           double Dmin, double Dcrit, getm_advection* uadv, getm_grid* ugrid,
-                                           getm_grid* uugrid, getm_grid* uvgrid, int uadv_ufirst,
-                                           getm_advection* vadv, getm_grid* vgrid, getm_grid* vugrid,
-                                           getm_grid* vvgrid, int vadv_ufirst, cudaStream_t stream)
+extern "C" int getm_split2d_substep(const getm_split2d_fields* f, int nx, int ny, int halox, int haloy, int mixed,
+                                    int ufirst, int accumulate, int friction, double timestep, double Dmin,
+                                    double Dcrit, getm_advection* uadv, getm_grid* ugrid, getm_grid* uugrid,
+                                    getm_grid* uvgrid, int uadv_ufirst, getm_advection* vadv, getm_grid* vgrid,
+                                    getm_grid* vugrid, getm_grid* vvgrid, int vadv_ufirst, cudaStream_t stream)
 {
     SubstepArgs a;
     int rc = substep_args(a, f, nx, ny, halox, haloy, mixed, ufirst, accumulate, friction, timestep, Dmin, Dcrit,
                           uadv, ugrid, uugrid, uvgrid, uadv_ufirst, vadv, vgrid, vugrid, vvgrid, vadv_ufirst);
     if (rc) return rc;
-    return mixed ? launch_phases<true>(a, stream) : launch_phases<false>(a, stream);
+    return mixed ? launch_substep_kernels<true>(a, stream) : launch_substep_kernels<false>(a, stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -602,7 +650,7 @@ extern "C" int getm_split2d_substep_phases(const getm_split2d_fields* f, int nx,
 // runs the member's 3D step.  The other substeps of every member run here as
 // one cooperative launch per substep index k: launch k advances every member
 // with more than k such substeps by one substep.  The seven phases and their
-// device functions are those of substep_2d_kernel; within a phase the blocks
+// device functions are those of the single substep; within a phase the blocks
 // walk one list of block-sized work items spanning all members (512-point
 // chunks, depth tiles, advection row groups or tiles), so the small planes
 // of many members fill the GPU together and one set of grid barriers serves
@@ -667,7 +715,7 @@ __device__ __forceinline__ void batch_pass_item(const HPassArgs<double>& pa, int
 }
 
 // Work item q of phase ph of one member: the same operations, in the same
-// order per point, as the phases of substep_2d_kernel.
+// order per point, as the phases listed at the top.
 template <bool MIXED>
 __device__ void batch_item(const BatchMember& m, int ph, int q, int ufirst, SubstepSmem& sm, int tx, int ty)
 {
@@ -833,8 +881,7 @@ extern "C" int getm_substep_batch_set(getm_substep_batch* b, int member, int nsu
                                       int uadv_ufirst, getm_advection* vadv, getm_grid* vgrid, getm_grid* vugrid,
                                       getm_grid* vvgrid, int vadv_ufirst)
 {
-    if (!b || member < 0 || member >= b->nmember || nsub < 0 || split < nsub + 1 || b->dmem || !f || !f->sync)
-        return GETM_ERR_ARG;
+    if (!b || member < 0 || member >= b->nmember || nsub < 0 || split < nsub + 1 || b->dmem) return GETM_ERR_ARG;
     BatchMember& m = b->host[member];
     int rc = substep_args(m.a, f, nx, ny, halox, haloy, b->mixed, ufirst, accumulate, friction, timestep, Dmin,
                           Dcrit, uadv, ugrid, uugrid, uvgrid, uadv_ufirst, vadv, vgrid, vugrid, vvgrid, vadv_ufirst);

@@ -27,9 +27,7 @@ def make_member(wl: Workload, precision: str = "mixed", device="cuda", substep_k
                 concurrent_3d: bool = True, tiles=None) -> Simulation:
     """Build and start a simulation for one ensemble member (rest state,
     linear temperature drop ``dT`` per 100 m from 20 degC at the surface).
-    Members replay concurrently on several streams, so by default their 2D
-    substeps run as separate kernels rather than as one cooperative launch
-    that needs every SM of the GPU at once.  ``tiles``: launch shapes
+    ``substep_kernel``: as ``Simulation``'s (a ``BatchedEnsemble`` needs it).  ``tiles``: launch shapes
     (``Simulation``), e.g. "auto" for the tuned shapes of the member's size."""
     p = wl.params
     sim = Simulation(wl.T, wl.dga, num=p["num"], nuh=p["nuh"], precision=precision, device=device,
@@ -188,7 +186,7 @@ class BatchedEnsemble:
     of the round, and one graph of each member's 3D substep per parity.
 
     Members must be built with ``substep_kernel=True`` (each then carries the
-    fields of the one-launch substep) and share one precision form; their
+    fields of the batched substep) and share one precision form; their
     results are bitwise those of advancing each alone."""
 
     def __init__(self, members: List[Simulation], lanes: int = 16, warmup_rounds: int = 2, device="cuda"):
@@ -205,7 +203,7 @@ class BatchedEnsemble:
             raise ValueError(f"members of one precision form only, not {sorted(forms)}")
         for m in self.members:
             if m._split2d is None:
-                raise ValueError("every member needs the one-launch substep (substep_kernel=True and a "
+                raise ValueError("every member needs the substep's fields (substep_kernel=True and a "
                                  "configuration it covers)")
         self.mixed = forms.pop() == "mixed"
         self.lanes = [torch.cuda.Stream(device=self.device) for _ in range(max(1, min(lanes, len(self.members))))]

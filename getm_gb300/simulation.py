@@ -87,8 +87,8 @@ class Fluxes:
 
 
 class _Split2DPlan:
-    """Arguments of the 2D substep kernels: the fields struct and, for the
-    one-launch kernel, its barrier words."""
+    """Arguments of the 2D substep kernels: the fields struct and its status
+    words."""
 
     def __init__(self, fields, sync):
         self.fields = fields
@@ -120,10 +120,10 @@ class Simulation:
         internal-pressure slope corrections are evaluated in float).
         ``fused_2d``: the 2D substep's operations run as fused kernels;
         ``substep_kernel``: in addition, a substep that is not followed by a
-        3D step runs as one persistent kernel launch (closed domains with the
-        default Coriolis scheme, FULL 2D advection split, no horizontal
-        momentum diffusion, 3D run types); without it, such a substep runs as
-        seven ordinary launches.  ``concurrent_3d``: in a 3D step,
+        3D step runs as four launches on fields fixed at ``start`` (closed
+        domains with the default Coriolis scheme, FULL 2D advection split, no
+        horizontal momentum diffusion, 3D run types); without it, as the same
+        launches on the fields of the moment.  ``concurrent_3d``: in a 3D step,
         the shear frequency, the bottom stress, the advection of the 3D
         momentum and the slow terms it feeds run on a second stream,
         concurrently with the tracers, density and internal pressure
@@ -281,7 +281,9 @@ class Simulation:
             self._ob.init_tracer_values(self.tracers._tracers)
         self._start()
         self._update_forcing_and_diagnostics(macro_active=True)
-        self._split2d = self._split2d_plan() if self.substep_kernel else None
+        words = torch.zeros(4, dtype=torch.int32, device=self.T.device)
+        self._split2d_words = (words,)  # (in a tuple: not model state)
+        self._split2d = self._split2d_plan(words) if self.substep_kernel else None
 
     def advance(self):
         """python/pygetm/simulation.py:291-325"""
@@ -294,18 +296,21 @@ class Simulation:
         if self._split2d is not None and not macro_active:
             self._split2d_substep(self._split2d)
             return
-        if not macro_active and self.fused_2d and not self.substep_kernel and (plan := self._split2d_plan(sync=False)):
-            self._split2d_substep(plan, phases=True)
-            return
+        if not macro_active and self.fused_2d and not self.substep_kernel:
+            # the fields taken anew each time, as the operations one by one would
+            plan = self._split2d_plan(self._split2d_words[0])
+            if plan is not None:
+                self._split2d_substep(plan)
+                return
         _lib.call("getm_advance_time", self._time.data_ptr(), float(self.timestep),
                   torch.cuda.current_stream(self._time.device).cuda_stream)
         self._advance_state(macro_active)
         self._update_forcing_and_diagnostics(macro_active)
 
-    def _split2d_plan(self, sync: bool = True):
+    def _split2d_plan(self, words):
         """Fields of the 2D substep kernels, or None where they do not cover
         the configuration (the substep then runs operation by operation).
-        ``sync``: with the one-launch kernel's barrier words."""
+        ``words``: the kernels' status words."""
         m = self.momentum
         if (self._ob is not None or self.runtype <= RunType.BAROTROPIC_2D or m.diffuse_momentum
                 or m.An_uu is not None or m.coriolis_scheme != CoriolisScheme.DEFAULT
@@ -313,7 +318,6 @@ class Simulation:
                 or self.T.device.type != "cuda"):
             return None
         T, U, V, X, a = self.T, self.U, self.V, self.X, self.airsea
-        sync = torch.zeros(4, dtype=torch.int32, device=T.device) if sync else None  # barrier words, not model state
         fields = _pygetm.split2d_fields(
             mask_t=T.mask, H_t=T.H, iarea_t=T.iarea, z=T.z, zo=T.zo, D_t=T.D, Dclip_t=T.Dclip, work_t=T._work,
             fwf=self.fwf, pe=a.pe, sp=a.sp, taux=a.taux, tauy=a.tauy,
@@ -326,30 +330,28 @@ class Simulation:
             dampV=m.dampV, SyA=m.SyA, SyB=m.SyB, SyD=m.SyD, SyF=m.SyF, rv=m.rv, v1=m.v1, Vcum=m._V_cum,
             advD_v=m.vadv.D, vua=m.vua, vva=m.vva,
             mask_x=X.mask, H_x=X.H, D_x=X.D, work_x=X._work, D_uu=U.ugrid.D, D_uv=U.vgrid.D, D_vu=V.ugrid.D,
-            D_vv=V.vgrid.D, time=self._time, sync=sync)
-        return _Split2DPlan(fields, sync)
+            D_vv=V.vgrid.D, time=self._time, sync=words)
+        return _Split2DPlan(fields, words)
 
-    def _split2d_substep(self, plan, phases: bool = False):
-        """A substep without 3D step as one launch, or (``phases``) as one
-        launch per phase (the same operations as _advance_state +
-        _update_forcing_and_diagnostics with macro_active false, in the same
-        order, with bitwise the same results).  The launch per phase takes the
-        fields anew each time, as the operations one by one would."""
+    def _split2d_substep(self, plan):
+        """A substep without 3D step as four launches (the same operations as
+        _advance_state + _update_forcing_and_diagnostics with macro_active
+        false, in the same order, with bitwise the same results)."""
         m = self.momentum
         _pygetm.split2d_substep(plan.fields, self.T, self.dtype3d == torch.float32, m._ufirst, True,
-                                m.apply_bottom_friction, self.timestep, self.Dmin, self.Dcrit, m.uadv, m.vadv, phases)
+                                m.apply_bottom_friction, self.timestep, self.Dmin, self.Dcrit, m.uadv, m.vadv)
         m._ufirst = not m._ufirst
 
     def split2d_status(self) -> int:
-        """Non-zero when a grid barrier of the one-launch substep gave up (the
-        substep did not complete; reads the device word)."""
+        """The substep kernels' error word (reads the device): non-zero, they
+        leave every field as it is."""
         return 0 if self._split2d is None else int(self._split2d.sync[2].item())
 
     def clear_split2d_status(self):
-        """Re-arm the one-launch substep after a barrier gave up: zero its
-        barrier words (stream-ordered, so call it with no substep in flight
-        on another stream).  Until then every substep launch returns at once
-        and leaves the fields and the model time unchanged."""
+        """Re-arm the substep kernels: zero their status words (stream-ordered,
+        so call it with no substep in flight on another stream).  Until then
+        every substep launch returns at once and leaves the fields and the
+        model time unchanged."""
         if self._split2d is not None:
             self._split2d.sync.zero_()
 

@@ -320,7 +320,7 @@ int getm_launch_count(unsigned long long* count);
  * requests keep being issued while a new request is recorded).            */
 int getm_graph_launch(void* graph_exec, cudaStream_t stream);
 
-/* The model time of a substep that is not the one-launch substep (which
+/* The model time of a substep that is not getm_split2d_substep's (which
  * advances it itself): *time += timestep on the device, so that a captured
  * step graph advances it too.  pygetm keeps its time on the host
  * (python/pygetm/simulation.py:291-325, self.time += self.timestep).      */
@@ -345,8 +345,8 @@ int getm_stream_destroy(cudaStream_t stream);
  *   GETM_TUNE_COLUMN_ROWS     rows of 32 columns per block of the w pass
  *                             (where it does not split the columns) and the
  *                             float column solve: 1, 2, 4 (default 4)
- *   GETM_TUNE_SUBSTEP_BLOCKS  blocks per SM of the one-launch 2D substep:
- *                             0 = as many as fit (default), 1, 2 (capped at what fits)
+ *   GETM_TUNE_SUBSTEP_BLOCKS  0 (default), 1, 2: kept so that stored shapes stay
+ *                             valid; the substep kernels choose their own blocks
  *   GETM_TUNE_XPASS_VEC       3D x pass in increment form: 1 = four cells per lane
  *                             where rows allow 16-byte vectors (default), 0 = one
  *                             cell per lane (both give the same bits)
@@ -719,7 +719,7 @@ typedef struct getm_depth3d_fields {
 
 int getm_update_depth_3d(const getm_depth3d_fields* f, int nx, int ny, int nz, cudaStream_t stream);
 
-/* ---- one 2D substep as one launch -----------------------------------------
+/* ---- one 2D substep as four launches --------------------------------------
  * Replaces, for a substep of python/pygetm/simulation.py:291-325
  * (Simulation.advance) that is not followed by a 3D step, the sequence
  * simulation.py:1033-1039 (momentum.advance_depth_integrated, momentum.py
@@ -735,9 +735,8 @@ int getm_update_depth_3d(const getm_depth3d_fields* f, int nx, int ny, int nz, c
  * ufirst: momentum order of this substep (U then V); accumulate: add U, V to
  * Ucum, Vcum (3D runs); friction: bottom friction (ru, rv).  uadv/vadv: the
  * momentum advection handles with their grids (T = U resp. V grid) and their
- * u-first flags.  sync: 4 words, zero before the first call; sync[2] != 0
- * after a call means a grid barrier gave up (the call did not complete and
- * every later call returns at once until the word is cleared).  All fields
+ * u-first flags.  sync: 4 words, zero before the first call; while
+ * sync[2] is not zero a call leaves every field as it is.  All fields
  * are [j][i] with the full extents nx, ny (X fields nx+1, ny+1).            */
 typedef struct getm_split2d_fields {
     /* T grid */
@@ -768,13 +767,6 @@ int getm_split2d_substep(const getm_split2d_fields* f, int nx, int ny, int halox
                          getm_advection* uadv, getm_grid* ugrid, getm_grid* uugrid, getm_grid* uvgrid,
                          int uadv_ufirst, getm_advection* vadv, getm_grid* vgrid, getm_grid* vugrid,
                          getm_grid* vvgrid, int vadv_ufirst, cudaStream_t stream);
-/* the same substep, with the same results, as seven ordinary launches: for
- * domains that share the GPU with others.  f->sync may be NULL. */
-int getm_split2d_substep_phases(const getm_split2d_fields* f, int nx, int ny, int halox, int haloy, int mixed,
-                                int ufirst, int accumulate, int friction, double timestep, double Dmin,
-                                double Dcrit, getm_advection* uadv, getm_grid* ugrid, getm_grid* uugrid,
-                                getm_grid* uvgrid, int uadv_ufirst, getm_advection* vadv, getm_grid* vgrid,
-                                getm_grid* vugrid, getm_grid* vvgrid, int vadv_ufirst, cudaStream_t stream);
 
 /* ---- turbulence closure -----------------------------------------------
  * Replaces the GOTM call of python/pygetm/vertical_mixing.py:150-188

@@ -1,5 +1,5 @@
-"""The 2D substep as one launch per phase (getm_split2d_substep_phases): the
-same state, bit for bit, as the operations launched one by one."""
+"""The 2D substep's four launches (getm_split2d_substep): the same state, bit
+for bit, as the operations launched one by one."""
 
 import numpy as np
 import pytest
@@ -9,7 +9,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("n,mixed_orders,friction", [(8, False, True), (31, True, True), (61, False, False)])
-def test_phases_match_single_operations(precision, n, mixed_orders, friction):
+def test_substep_matches_single_operations(precision, n, mixed_orders, friction):
     """Planes smaller than a block, one short of whole tiles and of several
     tiles; the two momentum advections in different orders; a wind field
     replaced after the start."""
@@ -19,13 +19,13 @@ def test_phases_match_single_operations(precision, n, mixed_orders, friction):
     from getm_gb300.core import Array
     from getm_gb300.ensemble import make_member
 
-    def member(phases):
+    def member(fused):
         wl = workloads.ensemble_member(np.random.default_rng(7), nmin=n, nmax=n, nzmin=4, nzmax=4)
         wl.params["split_factor"] = 5
         s = make_member(wl, precision)
         plans = []
         plan = s._split2d_plan
-        s._split2d_plan = (lambda **k: plans.append(1) or plan(**k)) if phases else (lambda **k: None)
+        s._split2d_plan = (lambda w: plans.append(1) or plan(w)) if fused else (lambda w: None)
         s.momentum.apply_bottom_friction = friction
         if mixed_orders:
             s.momentum.vadv.ufirst = not s.momentum.uadv.ufirst
@@ -35,7 +35,7 @@ def test_phases_match_single_operations(precision, n, mixed_orders, friction):
         for _ in range(6):
             s.advance()
         torch.cuda.synchronize()
-        assert len(plans) == (11 if phases else 0)
+        assert len(plans) == (11 if fused else 0)
         return s
 
     a, b = member(True), member(False)
