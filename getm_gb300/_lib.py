@@ -89,6 +89,7 @@ _SIGS = {
     "getm_accumulate_2d": "lpppps",
     "getm_surface_elevation_fused": "iiiipppppppppds",
     "getm_split2d_substep": "piiiiiiiidddppppippppis",
+    "getm_split2d_phases": "piiiiiiiidddppppippppiiiis",
     "getm_update_depth_3d": "piiis",
     "getm_transport_3d_finish": "iiipppppps",
     "getm_transport_3d_finish_f32": "iiipppppps",

@@ -425,14 +425,17 @@ def split2d_fields(**arrays) -> Split2DFields:
     return f
 
 
-def split2d_substep(fields: Split2DFields, T, mixed, ufirst, accumulate, friction, timestep, Dmin, Dcrit, uadv, vadv):
+def split2d_substep(fields: Split2DFields, T, mixed, ufirst, accumulate, friction, timestep, Dmin, Dcrit, uadv, vadv,
+                    phases=None):
     """One non-macro 2D substep (simulation.py:1033-1304 with update_3d
-    false) as four launches; ``uadv``/``vadv``: the momentum Advection objects."""
+    false) as four launches, or of any substep the ``phases`` (first, last,
+    with the surface pressure gradient), one launch each; ``uadv``/``vadv``:
+    the momentum Advection objects."""
     U, V = T.ugrid, T.vgrid
-    call("getm_split2d_substep", ctypes.byref(fields), T.nx_, T.ny_, T.halox, T.haloy, int(bool(mixed)),
+    call("getm_split2d_substep" if phases is None else "getm_split2d_phases", ctypes.byref(fields), T.nx_, T.ny_, T.halox, T.haloy, int(bool(mixed)),
          int(bool(ufirst)), int(bool(accumulate)), int(bool(friction)), float(timestep), float(Dmin), float(Dcrit),
          uadv.p, U.handle, U.ugrid.handle, U.vgrid.handle, int(uadv.ufirst),
-         vadv.p, V.handle, V.ugrid.handle, V.vgrid.handle, int(vadv.ufirst), _s())
+         vadv.p, V.handle, V.ugrid.handle, V.vgrid.handle, int(vadv.ufirst), *(int(q) for q in phases or ()), _s())
 
 
 def transport_3d_finish(vel3d, hn, tp2d, D, tp3d, dev):

@@ -170,7 +170,8 @@ __device__ __forceinline__ void coriolis_from(const SubstepArgs& a, int d, int i
 // at point p = (i, j); d1: the direction updated first.  Phase 4 has its
 // depth tiles besides, phase 6 its advection passes.
 template <bool MIXED>
-__device__ __forceinline__ void phase_point(const SubstepArgs& a, int ph, int d1, int i, int j, int p)
+__device__ __forceinline__ void phase_point(const SubstepArgs& a, int ph, int d1, int i, int j, int p,
+                                            bool spg = true)
 {
     using C = typename std::conditional<MIXED, float, double>::type;
     const int nx = a.nx, ny = a.ny, d2 = 1 - d1;
@@ -198,7 +199,7 @@ __device__ __forceinline__ void phase_point(const SubstepArgs& a, int ph, int d1
         momentum_2d_velocities_point<C>(a.vel, i, j);
         a.advD[0][p] = a.Dsrc[0][p];
         a.advD[1][p] = a.Dsrc[1][p];
-        if (interior) spg_point<MIXED>(a.spg, p);
+        if (spg && interior) spg_point<MIXED>(a.spg, p);
         break;
     default:
         momentum_2d_friction_point<C>(a.fric, i, j);
@@ -305,8 +306,8 @@ static_assert((TR_MAX + 1) * 33 <= TR_THREADS && (DV_MAX + 2) * 34 <= DV_THREADS
 // written only on the host's behalf, before the substep's first launch.
 __device__ __forceinline__ bool substep_begin(const SubstepArgs& a)
 {
-    unsigned err;
-    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(err) : "l"(a.sync + 2) : "memory");
+    unsigned err = 0;
+    if (a.sync) asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(err) : "l"(a.sync + 2) : "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     return err != 0;
 }
@@ -573,7 +574,7 @@ int launch_substep(K kernel, dim3 grid, dim3 block, bool first, cudaStream_t str
 // One launch for both directions' pass where they share the axis (they do
 // unless the host gave the two advections different orders)
 template <bool MIXED, int PASS>
-int launch_substep_advection(const SubstepArgs& a, cudaStream_t stream)
+int launch_substep_advection(const SubstepArgs& a, cudaStream_t stream, bool first = false)
 {
     const bool one = a.adv[0].dir[PASS] == a.adv[1].dir[PASS];
     const int nd = one ? 2 : 1;
@@ -581,16 +582,19 @@ int launch_substep_advection(const SubstepArgs& a, cudaStream_t stream)
         int rc;
         if (a.adv[d].dir[PASS] == 1) {
             const dim3 g(div_up(a.nx + 1, HX_STRIDE), div_up(a.ny, PH_XY), nd);
-            rc = launch_substep(substep_advection_kernel<MIXED, PASS, 1, PH_XY>, g, dim3(32, PH_XY), false, stream, a, d);
+            rc = launch_substep(substep_advection_kernel<MIXED, PASS, 1, PH_XY>, g, dim3(32, PH_XY), first && d == 0,
+                                stream, a, d);
         } else {
             // tiles of 16 or 8 rows (one of them the edge), whichever loads
             // the fullest SM less
             const long long nbx = (long long)div_up(a.nx, 32) * nd;
             const dim3 g16(div_up(a.nx, 32), div_up(a.ny + 1, 15), nd), g8(div_up(a.nx, 32), div_up(a.ny + 1, 7), nd);
             if (2 * getm_div_up(nbx * g16.y, GETM_SMS) <= getm_div_up(nbx * g8.y, GETM_SMS))
-                rc = launch_substep(substep_advection_kernel<MIXED, PASS, 2, 16>, g16, dim3(32, 16), false, stream, a, d);
+                rc = launch_substep(substep_advection_kernel<MIXED, PASS, 2, 16>, g16, dim3(32, 16), first && d == 0,
+                                    stream, a, d);
             else
-                rc = launch_substep(substep_advection_kernel<MIXED, PASS, 2, 8>, g8, dim3(32, 8), false, stream, a, d);
+                rc = launch_substep(substep_advection_kernel<MIXED, PASS, 2, 8>, g8, dim3(32, 8), first && d == 0,
+                                    stream, a, d);
         }
         if (rc) return rc;
     }
@@ -600,12 +604,14 @@ int launch_substep_advection(const SubstepArgs& a, cudaStream_t stream)
 // Rows of a tile with `edge` more staged: the height up to `most` that leaves
 // the SM with most tiles the fewest staged rows.  A plane then goes in one
 // wave where it can (400 x 300: 442 depth tiles of 9 rows on 152 SMs of three),
-// and a small one spreads over as many SMs as it can, whose FP64 pipes it waits for.
-inline int substep_rows(int nx, int ny, int most, int edge)
+// and a small one spreads over as many SMs as it can, whose FP64 pipes it waits
+// for (mixed form: four rows at least, as more blocks only add edges: a 92 x 92
+// member's step 948 us, with two rows 954).
+inline int substep_rows(int nx, int ny, int most, int edge, int least_rows)
 {
     int best = most;
     long long least = 0;
-    for (int by = most; by >= 2; by--) {
+    for (int by = most; by >= least_rows; by--) {
         const long long tiles = (long long)div_up(nx, 32) * div_up(ny, by);
         const long long load = (tiles + GETM_SMS - 1) / GETM_SMS * (by + edge);
         if (by == most || load < least) { least = load; best = by; }
@@ -616,7 +622,8 @@ inline int substep_rows(int nx, int ny, int most, int edge)
 template <bool MIXED>
 int launch_substep_kernels(const SubstepArgs& a, cudaStream_t stream)
 {
-    const int tr = substep_rows(a.nx, a.ny, TR_MAX, 1), dv = substep_rows(a.nx + 1, a.ny + 1, DV_MAX, 2);
+    const int tr = substep_rows(a.nx, a.ny, TR_MAX, 1, MIXED ? 4 : 2);
+    const int dv = substep_rows(a.nx + 1, a.ny + 1, DV_MAX, 2, MIXED ? 4 : 2);
     const dim3 tg(div_up(a.nx, 32), div_up(a.ny, tr)), tb(div_up((tr + 1) * 33, 32) * 32);
     const dim3 dg(div_up(a.nx + 1, 32), div_up(a.ny + 1, dv)), db(div_up((dv + 2) * 34, 32) * 32);
     int rc = a.ufirst ? launch_substep(substep_transport_kernel<MIXED, 0>, tg, tb, true, stream, a, tr)
@@ -640,6 +647,74 @@ extern "C" int getm_split2d_substep(const getm_split2d_fields* f, int nx, int ny
                           uadv, ugrid, uugrid, uvgrid, uadv_ufirst, vadv, vgrid, vugrid, vvgrid, vadv_ufirst);
     if (rc) return rc;
     return mixed ? launch_substep_kernels<true>(a, stream) : launch_substep_kernels<false>(a, stream);
+}
+
+// ---------------------------------------------------------------------------
+// Some phases of a substep, one launch each
+// ---------------------------------------------------------------------------
+// For a substep with work between its phases: the 3D step between the elevation
+// and the depths, the open boundaries' mirrored transports, depths and
+// elevations.  One by one its operations are nineteen launches.
+namespace {
+
+constexpr int PH_PY = 4;  // rows of a block
+
+template <bool MIXED, int PH>
+__global__ void __launch_bounds__(32 * PH_PY) phase_points_kernel(const __grid_constant__ SubstepArgs a, int spg)
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * PH_PY + threadIdx.y;
+    if (i < a.nx && j < a.ny) phase_point<MIXED>(a, PH, a.ufirst ? 0 : 1, i, j, j * a.nx + i, spg != 0);
+}
+
+template <bool MIXED>
+__global__ void __launch_bounds__(32 * PH_PY) phase_depth_kernel(const __grid_constant__ SubstepArgs a)
+{
+    __shared__ double szh[PH_PY + 2][UD_BX + 2];
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * PH_PY + threadIdx.y;
+    if (i < a.nx && j < a.ny) phase_point<MIXED>(a, 3, 0, i, j, j * a.nx + i);
+    update_depth_2d_tile<PH_PY, MIXED>(a.depth, blockIdx.x, blockIdx.y, threadIdx.x, threadIdx.y, szh);
+}
+
+template <bool MIXED>
+int launch_phases(const SubstepArgs& a, int first, int last, int spg, cudaStream_t stream)
+{
+    const dim3 b(32, PH_PY), g(div_up(a.nx, 32), div_up(a.ny, PH_PY));
+    const dim3 gd(div_up(a.nx + 1, UD_BX), div_up(a.ny + 1, PH_PY));
+    for (int ph = first; ph <= last; ph++) {
+        const bool f = ph == first;
+        int rc;
+        switch (ph) {
+        case 1: rc = launch_substep(phase_points_kernel<MIXED, 0>, g, b, f, stream, a, spg); break;
+        case 2: rc = launch_substep(phase_points_kernel<MIXED, 1>, g, b, f, stream, a, spg); break;
+        case 3: rc = launch_substep(phase_points_kernel<MIXED, 2>, g, b, f, stream, a, spg); break;
+        case 4: rc = launch_substep(phase_depth_kernel<MIXED>, gd, b, f, stream, a); break;
+        case 5: rc = launch_substep(phase_points_kernel<MIXED, 4>, g, b, f, stream, a, spg); break;
+        case 6: rc = launch_substep_advection<MIXED, 0>(a, stream, f); break;
+        default: rc = launch_substep_advection<MIXED, 1>(a, stream, f); break;
+        }
+        if (rc) return rc;
+    }
+    return GETM_OK;
+}
+
+}  // namespace
+
+extern "C" int getm_split2d_phases(const getm_split2d_fields* f, int nx, int ny, int halox, int haloy, int mixed,
+                                   int ufirst, int accumulate, int friction, double timestep, double Dmin,
+                                   double Dcrit, getm_advection* uadv, getm_grid* ugrid, getm_grid* uugrid,
+                                   getm_grid* uvgrid, int uadv_ufirst, getm_advection* vadv, getm_grid* vgrid,
+                                   getm_grid* vugrid, getm_grid* vvgrid, int vadv_ufirst, int first, int last,
+                                   int spg, cudaStream_t stream)
+{
+    if (first < 1 || last < first || last > 7) return GETM_ERR_ARG;
+    SubstepArgs a;
+    int rc = substep_args(a, f, nx, ny, halox, haloy, mixed, ufirst, accumulate, friction, timestep, Dmin, Dcrit,
+                          uadv, ugrid, uugrid, uvgrid, uadv_ufirst, vadv, vgrid, vugrid, vvgrid, vadv_ufirst);
+    if (rc) return rc;
+    a.sync = nullptr;  // (the error word concerns whole substeps)
+    return mixed ? launch_phases<true>(a, first, last, spg, stream) : launch_phases<false>(a, first, last, spg, stream);
 }
 
 // ---------------------------------------------------------------------------

@@ -304,15 +304,18 @@ class Simulation:
                 return
         _lib.call("getm_advance_time", self._time.data_ptr(), float(self.timestep),
                   torch.cuda.current_stream(self._time.device).cuda_stream)
-        self._advance_state(macro_active)
-        self._update_forcing_and_diagnostics(macro_active)
+        # the fields taken anew, as the operations one by one would
+        plan = self._split2d_plan(self._split2d_words[0], whole=False) if self.fused_2d else None
+        self._advance_state(macro_active, plan)
+        self._update_forcing_and_diagnostics(macro_active, plan)
 
-    def _split2d_plan(self, words):
+    def _split2d_plan(self, words, whole: bool = True):
         """Fields of the 2D substep kernels, or None where they do not cover
         the configuration (the substep then runs operation by operation).
-        ``words``: the kernels' status words."""
+        ``words``: the kernels' status words.  ``whole``: for a substep in one
+        call (no open boundaries; moves the model time on), else for its phases."""
         m = self.momentum
-        if (self._ob is not None or self.runtype <= RunType.BAROTROPIC_2D or m.diffuse_momentum
+        if ((whole and self._ob is not None) or self.runtype <= RunType.BAROTROPIC_2D or m.diffuse_momentum
                 or m.An_uu is not None or m.coriolis_scheme != CoriolisScheme.DEFAULT
                 or m.advection_split_2d != AdvectionSplit.FULL or not m.uadv.p.value or not m.vadv.p.value
                 or self.T.device.type != "cuda"):
@@ -330,17 +333,23 @@ class Simulation:
             dampV=m.dampV, SyA=m.SyA, SyB=m.SyB, SyD=m.SyD, SyF=m.SyF, rv=m.rv, v1=m.v1, Vcum=m._V_cum,
             advD_v=m.vadv.D, vua=m.vua, vva=m.vva,
             mask_x=X.mask, H_x=X.H, D_x=X.D, work_x=X._work, D_uu=U.ugrid.D, D_uv=U.vgrid.D, D_vu=V.ugrid.D,
-            D_vv=V.vgrid.D, time=self._time, sync=words)
+            D_vv=V.vgrid.D, time=self._time if whole else None, sync=words)
         return _Split2DPlan(fields, words)
 
     def _split2d_substep(self, plan):
         """A substep without 3D step as four launches (the same operations as
         _advance_state + _update_forcing_and_diagnostics with macro_active
         false, in the same order, with bitwise the same results)."""
+        self._split2d_run(plan)
+        self.momentum._ufirst = not self.momentum._ufirst
+
+    def _split2d_run(self, plan, *phases):
+        """The substep, or its phases first, last (with or without the
+        surface pressure gradient)."""
         m = self.momentum
         _pygetm.split2d_substep(plan.fields, self.T, self.dtype3d == torch.float32, m._ufirst, True,
-                                m.apply_bottom_friction, self.timestep, self.Dmin, self.Dcrit, m.uadv, m.vadv)
-        m._ufirst = not m._ufirst
+                                m.apply_bottom_friction, self.timestep, self.Dmin, self.Dcrit, m.uadv, m.vadv,
+                                phases or None)
 
     def split2d_status(self) -> int:
         """The substep kernels' error word (reads the device): non-zero, they
@@ -391,10 +400,23 @@ class Simulation:
             self.momentum.update_diagnostics(self.macrotimestep, self.num)
         T.z.all_values.copy_(z_backup)
 
-    def _advance_state(self, macro_active: bool):
-        """python/pygetm/simulation.py:1033-1136"""
-        self.momentum.advance_depth_integrated(self.timestep, self.tausx, self.tausy, self.dpdx, self.dpdy)
-        self.advance_surface_elevation(self.timestep, self.momentum.U, self.momentum.V, self.fwf)
+    def _advance_state(self, macro_active: bool, plan=None):
+        """python/pygetm/simulation.py:1033-1136 (``plan``: the 2D operations
+        as phases of the substep kernels)"""
+        m = self.momentum
+        if plan is None:
+            m.advance_depth_integrated(self.timestep, self.tausx, self.tausy, self.dpdx, self.dpdy)
+            self.advance_surface_elevation(self.timestep, m.U, m.V, self.fwf)
+        else:
+            if self._ob is None:
+                self._split2d_run(plan, 1, 3, False)
+            else:
+                order = (("U", m.U), ("V", m.V)) if m._ufirst else (("V", m.V), ("U", m.U))
+                for n, (name, field) in enumerate(order):
+                    self._split2d_run(plan, n + 1, n + 1, False)
+                    self._ob.mirror(name, field)
+                self._split2d_run(plan, 3, 3, False)
+            m._ufirst = not m._ufirst
         if self.runtype > RunType.BAROTROPIC_2D and macro_active:
             # add_freshwater_inputs (simulation.py:1335-1406) is an exact no-op
             # without rivers and with zero precipitation-evaporation.
@@ -415,8 +437,8 @@ class Simulation:
             if self.runtype == RunType.BAROCLINIC and self.delay_slow_ip:
                 _pygetm.column_sums([(self.idpdx, self.momentum.SxB), (self.idpdy, self.momentum.SyB)])
 
-    def _update_forcing_and_diagnostics(self, macro_active: bool):
-        """python/pygetm/simulation.py:1138-1304"""
+    def _update_forcing_and_diagnostics(self, macro_active: bool, plan=None):
+        """python/pygetm/simulation.py:1138-1304 (``plan``: as _advance_state)"""
         starting = self.istep == 0
         update_z0b = self.runtype == RunType.BAROTROPIC_2D and not starting
         update_3d = self.runtype > RunType.BAROTROPIC_2D and macro_active
@@ -432,18 +454,27 @@ class Simulation:
         if self._forked:  # the momentum advection and slow terms are done
             torch.cuda.current_stream(self.T.device).wait_stream(self._side_stream)
             self._forked = False
-        self.update_depth()
-        self.momentum.update_depth_integrated_diagnostics(self.timestep, skip_coriolis=not starting,
-                                                         update_z0b=update_z0b)
-        self.fwf.all_values.copy_(self.airsea.pe.all_values)
+        if plan is None:
+            self.update_depth()
+            self.momentum.update_depth_integrated_diagnostics(self.timestep, skip_coriolis=not starting,
+                                                             update_z0b=update_z0b)
+            self.fwf.all_values.copy_(self.airsea.pe.all_values)
+        elif self._ob is None:
+            self._split2d_run(plan, 4, 7, True)
+        else:
+            self._split2d_run(plan, 4, 4, False)
+            self._ob.update_depth(self, self.T.z, self.T.zo)
+            self._split2d_run(plan, 5, 7, False)
         if self._ob is not None:
             # elevation at the open boundaries, before the surface pressure
             # gradient (simulation.py:1252-1257)
             self._ob.prescribe(self._time)
             self._ob.update_elevation(self)
-        self.update_surface_pressure_gradient(self.T.z, self.airsea.sp)
-        self.airsea.taux.interp(self.tausx)
-        self.airsea.tauy.interp(self.tausy)
+        if plan is None or self._ob is not None:
+            self.update_surface_pressure_gradient(self.T.z, self.airsea.sp)
+        if plan is None:
+            self.airsea.taux.interp(self.tausx)
+            self.airsea.tauy.interp(self.tausy)
         if update_3d:
             self.tausxo.all_values.copy_(self.tausx.all_values)
             self.tausyo.all_values.copy_(self.tausy.all_values)

@@ -767,6 +767,20 @@ int getm_split2d_substep(const getm_split2d_fields* f, int nx, int ny, int halox
                          getm_advection* uadv, getm_grid* ugrid, getm_grid* uugrid, getm_grid* uvgrid,
                          int uadv_ufirst, getm_advection* vadv, getm_grid* vgrid, getm_grid* vugrid,
                          getm_grid* vvgrid, int vadv_ufirst, cudaStream_t stream);
+/* Phases first .. last of the substep, one launch each, for a substep with
+ * work between them (the 3D step after phase 3; open boundaries, whose
+ * points the host treats in between): 1 the transport update of the first
+ * direction; 2 its Coriolis term and the second direction's update; 3 the
+ * second's Coriolis term, cumulative transports, zo = z and the elevation; 4
+ * depths, fwf = pe, wind stress; 5 velocities, advected depths and (spg != 0)
+ * the surface pressure gradient; 6 friction and the first momentum advection
+ * passes, fwf = pe; 7 the second passes (and time += dt, where f->time is
+ * given).  f->sync is not looked at. */
+int getm_split2d_phases(const getm_split2d_fields* f, int nx, int ny, int halox, int haloy, int mixed, int ufirst,
+                        int accumulate, int friction, double timestep, double Dmin, double Dcrit,
+                        getm_advection* uadv, getm_grid* ugrid, getm_grid* uugrid, getm_grid* uvgrid,
+                        int uadv_ufirst, getm_advection* vadv, getm_grid* vgrid, getm_grid* vugrid,
+                        getm_grid* vvgrid, int vadv_ufirst, int first, int last, int spg, cudaStream_t stream);
 
 /* ---- turbulence closure -----------------------------------------------
  * Replaces the GOTM call of python/pygetm/vertical_mixing.py:150-188
