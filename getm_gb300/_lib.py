@@ -18,6 +18,7 @@ LIB_PATH = Path(os.environ.get("GETM_GB300_LIB", _HERE / "libgetm_gb300.so"))
 
 GETM_OK = 0
 GETM_MAX_TOTALS = 16      # include/getm_gb300.h
+GETM_MAX_BOUNDARIES = 64  # include/getm_gb300.h
 GETM_TOTALS_BLOCKS = 608  # include/getm_gb300.h
 ERRORS = {
     1: "invalid argument",
@@ -121,6 +122,10 @@ _SIGS = {
     "getm_column_sums_f32": "iiiipppppppps",
     "getm_velocities_3d_f32": "lpppppps",
     "getm_open_boundary_elevation": "iiipppppppppppppdps",
+    "getm_open_boundary_elevations": "ipiipppppppppppppdps",
+    "getm_open_boundary_tide": "iippppps",
+    "getm_open_boundaries_tracers": "ipiiiiippppppipps",
+    "getm_open_boundaries_tracers_f32": "ipiiiiippppppipps",
     "getm_open_boundary_tracers": "iiiiiiippppppipps",
     "getm_open_boundary_tracers_f32": "iiiiiiippppppipps",
     "getm_mirror": "ippilpps",

@@ -6,64 +6,79 @@
 // simulation.py:1160-1168 (tracers), :1252-1257 (elevation), :1545-1550
 // (depths) and momentum.py:679, :699, :1212 (transports).
 //
-// A boundary has a few hundred to a few thousand points, so one thread per
-// point (per level for 3D fields).  The reference updates its boundaries one
-// after the other; a zero-gradient point next to a corner reads a point of
-// another boundary, so the caller launches one boundary (a contiguous range
-// of the point tables) at a time, in the reference's order.
+// A boundary has a few hundred to a few thousand points, so these kernels are
+// bound by their launches and a few latencies.  The reference updates its
+// boundaries one after the other, and a zero-gradient point next to a corner
+// reads a point of another boundary; but no level or tracer looks at another,
+// so one block takes a plane (of one level and tracer) through all boundaries
+// in the reference's order, with a block barrier between them, and one launch
+// does them all (a shelf sea's six boundaries: elevation 6 x 4.7 -> 15 us, eight
+// tracers of 20 levels 6 x 20 -> 20 us).
 #include <math.h>
 
 #include "getm_common.cuh"
 
 #define OB_THREADS 128
+#define OB_BLOCK 256  // threads of a block that takes a plane through the boundaries
 
 namespace {
 
 __device__ __forceinline__ double np_maximum(double lo, double x) { return isnan(x) ? x : fmax(lo, x); }
 
-// elevation at boundary points start..stop-1 (open_boundaries.py:338-416),
-// clipped to its minimum Dmin - H (simulation.py:580-582)
-__global__ void ob_elevation_kernel(int start, int stop, int nx, const int* bi, const int* bj, const int* type,
-                                    const int* di, const int* dj, const int* side, const double* sign,
-                                    const double* H, const double* Dclip, const double* U, const double* V,
-                                    const double* z_ext, const double* flow_ext, double Dmin, double* z)
+// The boundaries of a launch, in order: ranges start, stop of the point tables.
+struct ObRanges {
+    int n;
+    int start[GETM_MAX_BOUNDARIES], stop[GETM_MAX_BOUNDARIES];
+};
+
+// elevation at the boundary points (open_boundaries.py:338-416), clipped to its
+// minimum Dmin - H (simulation.py:580-582); one block
+__global__ void __launch_bounds__(OB_BLOCK)
+    ob_elevation_kernel(ObRanges r, int nx, const int* bi, const int* bj, const int* type, const int* di,
+                        const int* dj, const int* side, const double* sign, const double* H, const double* Dclip,
+                        const double* U, const double* V, const double* z_ext, const double* flow_ext, double Dmin,
+                        double* z)
 {
-    const int p = start + blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= stop) return;
-    const long long q = (long long)bj[p] * nx + bi[p];
-    double v;
-    switch (type[p]) {
-    case 1:  // ZERO_GRADIENT
-        v = z[(long long)(bj[p] + dj[p]) * nx + (bi[p] + di[p])];
-        break;
-    case 3:  // CLAMPED
-        v = z_ext[p];
-        break;
-    default: {  // FLATHER_ELEV (4), FLATHER_TRANSPORT (-4)
-        // transport at the velocity point just inside (extract_uv_in, :149-152)
-        double tp;
-        switch (side[p]) {
-        case 1: tp = U[q]; break;       // WEST: U(j, l)
-        case 3: tp = U[q - 1]; break;   // EAST: U(j, l-1)
-        case 4: tp = V[q]; break;       // SOUTH: V(l, i)
-        default: tp = V[q - nx]; break; // NORTH: V(l-1, i)
+    for (int b = 0; b < r.n; b++) {
+        if (b > 0) __syncthreads();
+        for (int p = r.start[b] + threadIdx.x; p < r.stop[b]; p += OB_BLOCK) {
+            const long long q = (long long)bj[p] * nx + bi[p];
+            double v;
+            switch (type[p]) {
+            case 1:  // ZERO_GRADIENT
+                v = z[(long long)(bj[p] + dj[p]) * nx + (bi[p] + di[p])];
+                break;
+            case 3:  // CLAMPED
+                v = z_ext[p];
+                break;
+            default: {  // FLATHER_ELEV (4), FLATHER_TRANSPORT (-4)
+                // transport at the velocity point just inside (extract_uv_in, :149-152)
+                double tp;
+                switch (side[p]) {
+                case 1: tp = U[q]; break;       // WEST: U(j, l)
+                case 3: tp = U[q - 1]; break;   // EAST: U(j, l-1)
+                case 4: tp = V[q]; break;       // SOUTH: V(l, i)
+                default: tp = V[q - nx]; break; // NORTH: V(l-1, i)
+                }
+                const double D = Dclip[q];
+                const double ext = type[p] == 4 ? flow_ext[p] * D : flow_ext[p];
+                v = z_ext[p] - sign[p] * (tp - ext) / sqrt(D * GETM_G);
+                break;
+            }
+            }
+            z[q] = np_maximum(Dmin - H[q], v);
         }
-        const double D = Dclip[q];
-        const double ext = type[p] == 4 ? flow_ext[p] * D : flow_ext[p];
-        v = z_ext[p] - sign[p] * (tp - ext) / sqrt(D * GETM_G);
-        break;
     }
-    }
-    z[q] = np_maximum(Dmin - H[q], v);
 }
 
-// tracer values at boundary points start..stop-1 for every level and tracer
-// of the batch (ZeroGradient, Clamped; Sponge also relaxes the n points
+// tracer values at the boundary points for every level (grid x) and tracer (grid
+// y) of the batch (ZeroGradient, Clamped; Sponge also relaxes the n points
 // inward: v += sp_m (bdy - v), sp_m = ((n - m) / (n + 1))^2, only where the
 // mask is 1, open_boundaries.py:235-336 without flow-dependent relaxation)
 template <typename T>
 struct ObTracerArgs {
-    int start, stop, nx, nz, nsponge;
+    ObRanges r;
+    int nx, nz, nsponge;
     long long plane;
     const int *bi, *bj, *type, *di, *dj, *mask;
     int ntracer;
@@ -73,27 +88,28 @@ struct ObTracerArgs {
 };
 
 template <typename T>
-__global__ void ob_tracer_kernel(ObTracerArgs<T> a)
+__global__ void __launch_bounds__(OB_BLOCK) ob_tracer_kernel(const __grid_constant__ ObTracerArgs<T> a)
 {
-    const int p = a.start + blockIdx.x * blockDim.x + threadIdx.x;
-    const int k = blockIdx.y;
-    if (p >= a.stop || k >= a.nz) return;
-    const long long q = (long long)a.bj[p] * a.nx + a.bi[p] + k * a.plane;
-    for (int t = 0; t < a.ntracer; t++) {
-        T* f = a.var[t];
-        const int ty = a.type[p];
-        if (ty == 1) {
-            f[q] = f[q + (long long)a.dj[p] * a.nx + a.di[p]];
-        } else {
-            const T b = a.bdy[t][(long long)k * a.np + p];
-            f[q] = b;
-            if (ty == 5) {
-                for (int m = 0; m < a.nsponge; m++) {
-                    const long long o = (long long)(m + 1) * ((long long)a.dj[p] * a.nx + a.di[p]);
-                    const long long q2 = (long long)a.bj[p] * a.nx + a.bi[p] + o;  // 2D index of the sponge point
-                    if (a.mask[q2] != 1) continue;
-                    const T r = (T)(a.nsponge - m) / (T)(a.nsponge + 1);
-                    f[q + o] = f[q + o] + (r * r) * (b - f[q + o]);
+    const int k = blockIdx.x, t = blockIdx.y;
+    T* f = a.var[t];
+    for (int b = 0; b < a.r.n; b++) {
+        if (b > 0) __syncthreads();
+        for (int p = a.r.start[b] + threadIdx.x; p < a.r.stop[b]; p += OB_BLOCK) {
+            const long long q = (long long)a.bj[p] * a.nx + a.bi[p] + k * a.plane;
+            const int ty = a.type[p];
+            if (ty == 1) {
+                f[q] = f[q + (long long)a.dj[p] * a.nx + a.di[p]];
+            } else {
+                const T bv = a.bdy[t][(long long)k * a.np + p];
+                f[q] = bv;
+                if (ty == 5) {
+                    for (int m = 0; m < a.nsponge; m++) {
+                        const long long o = (long long)(m + 1) * ((long long)a.dj[p] * a.nx + a.di[p]);
+                        const long long q2 = (long long)a.bj[p] * a.nx + a.bi[p] + o;  // 2D index of the sponge point
+                        if (a.mask[q2] != 1) continue;
+                        const T r = (T)(a.nsponge - m) / (T)(a.nsponge + 1);
+                        f[q + o] = f[q + o] + (r * r) * (bv - f[q + o]);
+                    }
                 }
             }
         }
@@ -103,7 +119,29 @@ __global__ void ob_tracer_kernel(ObTracerArgs<T> a)
 // core.Array.mirror: field[tgt] = field[src] for n pairs of flat 2D indices
 // and nlev levels, with numpy's fancy-assignment semantics (every source is
 // read before any target is written: a point can be the target of one pair
-// and the source of another), hence a gather and a scatter launch.
+// and the source of another): one block per level holds the sources in
+// registers over a block barrier, or, with more than MR_BLOCK * MR_HOLD pairs, a
+// gather and a scatter launch.
+constexpr int MR_BLOCK = 512, MR_HOLD = 8;
+
+template <typename T>
+__global__ void __launch_bounds__(MR_BLOCK) mirror_kernel(int n, const int* src, const int* tgt, long long plane, T* field)
+{
+    T* f = field + blockIdx.x * plane;
+    T v[MR_HOLD];
+#pragma unroll
+    for (int m = 0; m < MR_HOLD; m++) {
+        const int p = m * MR_BLOCK + threadIdx.x;
+        if (p < n) v[m] = f[src[p]];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < MR_HOLD; m++) {
+        const int p = m * MR_BLOCK + threadIdx.x;
+        if (p < n) f[tgt[p]] = v[m];
+    }
+}
+
 template <typename T>
 __global__ void mirror_gather_kernel(int n, const int* src, int nlev, long long plane, const T* field, T* work)
 {
@@ -120,6 +158,27 @@ __global__ void mirror_scatter_kernel(int n, const int* tgt, int nlev, long long
     const int k = blockIdx.y;
     if (p >= n || k >= nlev) return;
     field[tgt[p] + k * plane] = work[(long long)k * n + p];
+}
+
+// Prescribed elevation from harmonic constituents at model time *time:
+// z_p = sum over c of amp_c(p) cos(*time om_c + ph_c(p)), every product and sum
+// rounded as written; start: the sum's first constituents (else added to z).
+struct ObTide {
+    int n;
+    double om[GETM_MAX_CONSTITUENTS];
+    const double *amp[GETM_MAX_CONSTITUENTS], *ph[GETM_MAX_CONSTITUENTS];
+};
+
+__global__ void __launch_bounds__(OB_THREADS) ob_tide_kernel(int np, const __grid_constant__ ObTide t,
+                                                             const double* time, double* z, int start)
+{
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= np) return;
+    const double now = *time;
+    double v = start ? 0.0 : z[p];
+    for (int c = 0; c < t.n; c++)
+        v = __dadd_rn(v, __dmul_rn(t.amp[c][p], cos(__dadd_rn(__dmul_rn(now, t.om[c]), t.ph[c][p]))));
+    z[p] = v;
 }
 
 // Depths at the velocity points just outside boundaries: z_T_half.mirror(z_U)
@@ -142,35 +201,82 @@ __global__ void ob_depth_kernel(int n, const int* srcT, const int* tgt, const do
 
 }  // namespace
 
+static int ob_ranges(ObRanges& r, int nrange, const int* ranges, int np)
+{
+    if (nrange < 0 || nrange > GETM_MAX_BOUNDARIES || (nrange && !ranges)) return GETM_ERR_ARG;
+    r.n = nrange;
+    for (int b = 0; b < nrange; b++) {
+        r.start[b] = ranges[2 * b];
+        r.stop[b] = ranges[2 * b + 1];
+        if (r.start[b] < 0 || r.stop[b] < r.start[b] || r.stop[b] > np) return GETM_ERR_ARG;
+    }
+    return GETM_OK;
+}
+
+extern "C" int getm_open_boundary_tide(int np, int nconstituent, const double* om, const double* const* amp,
+                                       const double* const* phase, const double* time, double* z, cudaStream_t stream)
+{
+    if (np < 0 || nconstituent < 0 || (nconstituent && (!om || !amp || !phase)) || !time || !z) return GETM_ERR_ARG;
+    if (np == 0) return GETM_OK;
+    for (int done = 0; done == 0 || done < nconstituent; done += GETM_MAX_CONSTITUENTS) {
+        ObTide t;
+        t.n = nconstituent - done < GETM_MAX_CONSTITUENTS ? nconstituent - done : GETM_MAX_CONSTITUENTS;
+        for (int c = 0; c < t.n; c++) {
+            if (!amp[done + c] || !phase[done + c]) return GETM_ERR_ARG;
+            t.om[c] = om[done + c];
+            t.amp[c] = amp[done + c];
+            t.ph[c] = phase[done + c];
+        }
+        ob_tide_kernel<<<getm_div_up(np, OB_THREADS), OB_THREADS, 0, stream>>>(np, t, time, z, done == 0);
+        GETM_CHECK_LAUNCH();
+    }
+    return GETM_OK;
+}
+
+extern "C" int getm_open_boundary_elevations(int nrange, const int* ranges, int np, int nx, const int* i, const int* j,
+                                            const int* type, const int* di, const int* dj, const int* side,
+                                            const double* inflow_sign, const double* H, const double* Dclip,
+                                            const double* U, const double* V, const double* z_ext,
+                                            const double* flow_ext, double Dmin, double* z, cudaStream_t stream)
+{
+    ObRanges r;
+    if (nx < 1 || ob_ranges(r, nrange, ranges, np)) return GETM_ERR_ARG;
+    if (nrange == 0) return GETM_OK;
+    const void* ptrs[] = {i, j, type, di, dj, side, inflow_sign, H, Dclip, U, V, z_ext, flow_ext, z};
+    for (const void* q : ptrs)
+        if (!q) return GETM_ERR_ARG;
+    ob_elevation_kernel<<<1, OB_BLOCK, 0, stream>>>(r, nx, i, j, type, di, dj, side, inflow_sign, H, Dclip, U, V,
+                                                    z_ext, flow_ext, Dmin, z);
+    GETM_CHECK_LAUNCH();
+    return GETM_OK;
+}
+
 extern "C" int getm_open_boundary_elevation(int start, int stop, int nx, const int* i, const int* j,
                                             const int* type, const int* di, const int* dj, const int* side,
                                             const double* inflow_sign, const double* H, const double* Dclip,
                                             const double* U, const double* V, const double* z_ext,
                                             const double* flow_ext, double Dmin, double* z, cudaStream_t stream)
 {
-    if (start < 0 || stop < start || nx < 1) return GETM_ERR_ARG;
-    if (stop == start) return GETM_OK;
-    const void* ptrs[] = {i, j, type, di, dj, side, inflow_sign, H, Dclip, U, V, z_ext, flow_ext, z};
-    for (const void* q : ptrs)
-        if (!q) return GETM_ERR_ARG;
-    ob_elevation_kernel<<<getm_div_up(stop - start, OB_THREADS), OB_THREADS, 0, stream>>>(
-        start, stop, nx, i, j, type, di, dj, side, inflow_sign, H, Dclip, U, V, z_ext, flow_ext, Dmin, z);
-    GETM_CHECK_LAUNCH();
-    return GETM_OK;
+    if (stop == start && start >= 0 && nx >= 1) return GETM_OK;
+    const int range[2] = {start, stop};
+    return getm_open_boundary_elevations(1, range, stop, nx, i, j, type, di, dj, side, inflow_sign, H, Dclip, U, V,
+                                         z_ext, flow_ext, Dmin, z, stream);
 }
 
 template <typename T>
-static int ob_tracer_impl(int start, int stop, int np, int nx, int ny, int nz, int nsponge, const int* i,
+static int ob_tracer_impl(int nrange, const int* ranges, int np, int nx, int ny, int nz, int nsponge, const int* i,
                           const int* j, const int* type, const int* di, const int* dj, const int* mask, int ntracer,
                           T* const* vars, const T* const* bdy, cudaStream_t stream)
 {
-    if (start < 0 || stop < start || stop > np || nx < 1 || ny < 1 || nz < 1 || nsponge < 0 || ntracer < 0 ||
+    ObTracerArgs<T> a;
+    if (ob_ranges(a.r, nrange, ranges, np) || nx < 1 || ny < 1 || nz < 1 || nsponge < 0 || ntracer < 0 ||
         ntracer > 16)
         return GETM_ERR_ARG;
-    if (stop == start || ntracer == 0) return GETM_OK;
+    int points = 0;
+    for (int b = 0; b < nrange; b++) points += a.r.stop[b] - a.r.start[b];
+    if (points == 0 || ntracer == 0) return GETM_OK;
     if (!i || !j || !type || !di || !dj || !mask || !vars || !bdy) return GETM_ERR_ARG;
-    ObTracerArgs<T> a;
-    a.start = start; a.stop = stop; a.nx = nx; a.nz = nz; a.nsponge = nsponge; a.np = np;
+    a.nx = nx; a.nz = nz; a.nsponge = nsponge; a.np = np;
     a.plane = (long long)nx * ny;
     a.bi = i; a.bj = j; a.type = type; a.di = di; a.dj = dj; a.mask = mask; a.ntracer = ntracer;
     for (int t = 0; t < ntracer; t++) {
@@ -178,8 +284,7 @@ static int ob_tracer_impl(int start, int stop, int np, int nx, int ny, int nz, i
         a.var[t] = vars[t];
         a.bdy[t] = bdy[t];
     }
-    dim3 grid(getm_div_up(stop - start, OB_THREADS), nz);
-    ob_tracer_kernel<T><<<grid, OB_THREADS, 0, stream>>>(a);
+    ob_tracer_kernel<T><<<dim3(nz, ntracer), OB_BLOCK, 0, stream>>>(a);
     GETM_CHECK_LAUNCH();
     return GETM_OK;
 }
@@ -189,7 +294,8 @@ extern "C" int getm_open_boundary_tracers(int start, int stop, int np, int nx, i
                                           const int* dj, const int* mask, int ntracer, double* const* vars,
                                           const double* const* bdy, cudaStream_t stream)
 {
-    return ob_tracer_impl<double>(start, stop, np, nx, ny, nz, nsponge, i, j, type, di, dj, mask, ntracer, vars, bdy,
+    const int range[2] = {start, stop};
+    return ob_tracer_impl<double>(1, range, np, nx, ny, nz, nsponge, i, j, type, di, dj, mask, ntracer, vars, bdy,
                                   stream);
 }
 
@@ -198,8 +304,28 @@ extern "C" int getm_open_boundary_tracers_f32(int start, int stop, int np, int n
                                               const int* dj, const int* mask, int ntracer, float* const* vars,
                                               const float* const* bdy, cudaStream_t stream)
 {
-    return ob_tracer_impl<float>(start, stop, np, nx, ny, nz, nsponge, i, j, type, di, dj, mask, ntracer, vars, bdy,
+    const int range[2] = {start, stop};
+    return ob_tracer_impl<float>(1, range, np, nx, ny, nz, nsponge, i, j, type, di, dj, mask, ntracer, vars, bdy,
                                  stream);
+}
+
+// every boundary in turn, one launch
+extern "C" int getm_open_boundaries_tracers(int nrange, const int* ranges, int np, int nx, int ny, int nz,
+                                            int nsponge, const int* i, const int* j, const int* type, const int* di,
+                                            const int* dj, const int* mask, int ntracer, double* const* vars,
+                                            const double* const* bdy, cudaStream_t stream)
+{
+    return ob_tracer_impl<double>(nrange, ranges, np, nx, ny, nz, nsponge, i, j, type, di, dj, mask, ntracer, vars,
+                                  bdy, stream);
+}
+
+extern "C" int getm_open_boundaries_tracers_f32(int nrange, const int* ranges, int np, int nx, int ny, int nz,
+                                                int nsponge, const int* i, const int* j, const int* type,
+                                                const int* di, const int* dj, const int* mask, int ntracer,
+                                                float* const* vars, const float* const* bdy, cudaStream_t stream)
+{
+    return ob_tracer_impl<float>(nrange, ranges, np, nx, ny, nz, nsponge, i, j, type, di, dj, mask, ntracer, vars,
+                                 bdy, stream);
 }
 
 template <typename T>
@@ -209,6 +335,11 @@ static int mirror_impl(int n, const int* src, const int* tgt, int nlev, long lon
     if (n < 0 || nlev < 1 || plane < 1) return GETM_ERR_ARG;
     if (n == 0) return GETM_OK;
     if (!src || !tgt || !field || !work) return GETM_ERR_ARG;
+    if (n <= MR_BLOCK * MR_HOLD) {
+        mirror_kernel<T><<<nlev, MR_BLOCK, 0, stream>>>(n, src, tgt, plane, field);
+        GETM_CHECK_LAUNCH();
+        return GETM_OK;
+    }
     dim3 grid(getm_div_up(n, OB_THREADS), nlev);
     mirror_gather_kernel<T><<<grid, OB_THREADS, 0, stream>>>(n, src, nlev, plane, field, work);
     GETM_CHECK_LAUNCH();

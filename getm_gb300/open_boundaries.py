@@ -270,11 +270,15 @@ class OpenBoundaries:
 
 class DeviceBoundaries:
     """Device copies of the point tables and the boundary operations of one
-    simulation (one launch per boundary where the reference updates the
-    boundaries in turn)."""
+    simulation (the reference updates the boundaries in turn, and so does the
+    launch that covers them)."""
 
     def __init__(self, ob: OpenBoundaries, T, dtype3d):
+        import ctypes
+
         import torch
+
+        from . import _lib
 
         dev = T.device
         self.T = T
@@ -290,6 +294,11 @@ class DeviceBoundaries:
         self.di, self.dj, self.side = it(ob.di), it(ob.dj), it(ob.side)
         self.sign = torch.from_numpy(ob.inflow_sign.astype(float)).to(dev)
         self.ranges = [(b.start, b.stop) for b in ob]
+        # the boundaries in launches of so many: (count, start and stop of each)
+        self._launches = []
+        for c in range(0, len(self.ranges), _lib.GETM_MAX_BOUNDARIES):
+            r = self.ranges[c:c + _lib.GETM_MAX_BOUNDARIES]
+            self._launches.append((len(r), (ctypes.c_int * (2 * len(r)))(*[q for se in r for q in se])))
         self.nsponge = ob.sponge_n
         # prescribed elevation, and velocity (FLATHER_ELEV) or transport
         # (FLATHER_TRANSPORT) normal to the boundary, per point
@@ -315,6 +324,23 @@ class DeviceBoundaries:
         ``time`` (0-d device tensor)."""
         if not self.constituents:
             return
+        import torch
+
+        given = [time, self.z] + [a for c in self.constituents for a in c[1:]]
+        if all(a.dtype == torch.float64 and a.is_cuda and a.is_contiguous() for a in given) and \
+                all(a.numel() == self.np for a in given[1:]) and time.numel() == 1:
+            import ctypes
+
+            from . import _lib
+            from ._pygetm import _s
+
+            n = len(self.constituents)
+            om = (ctypes.c_double * n)(*[float(c[0]) for c in self.constituents])
+            _lib.call("getm_open_boundary_tide", self.np, n, om,
+                      _lib.ptr_array([c[1].data_ptr() for c in self.constituents]),
+                      _lib.ptr_array([c[2].data_ptr() for c in self.constituents]), time.data_ptr(),
+                      self.z.data_ptr(), _s())
+            return
         self.z.zero_()
         for om, amp, ph in self.constituents:
             self.z.add_(amp * (time * om + ph).cos())
@@ -332,8 +358,8 @@ class DeviceBoundaries:
         from ._pygetm import _p, _s
 
         T = self.T
-        for s, e in self.ranges:
-            _lib.call("getm_open_boundary_elevation", s, e, T.nx_, self.i.data_ptr(), self.j.data_ptr(),
+        for n, ranges in self._launches:
+            _lib.call("getm_open_boundary_elevations", n, ranges, self.np, T.nx_, self.i.data_ptr(), self.j.data_ptr(),
                       self.type_2d.data_ptr(), self.di.data_ptr(), self.dj.data_ptr(), self.side.data_ptr(),
                       self.sign.data_ptr(), _p(T.H), _p(T.Dclip), _p(sim.momentum.U), _p(sim.momentum.V),
                       self.z.data_ptr(), self.flow.data_ptr(), float(sim.Dmin), _p(T.z), _s())
@@ -376,10 +402,10 @@ class DeviceBoundaries:
 
         T = self.T
         t = field.all_values
-        fn = "getm_open_boundary_tracers_f32" if t.dtype == torch.float32 else "getm_open_boundary_tracers"
+        fn = "getm_open_boundaries_tracers_f32" if t.dtype == torch.float32 else "getm_open_boundaries_tracers"
         ptr = _lib.ptr_array([t.data_ptr()])
-        for s, e in self.ranges:
-            _lib.call(fn, s, e, self.np, T.nx_, T.ny_, t.shape[0], 0, self.i.data_ptr(), self.j.data_ptr(),
+        for n, ranges in self._launches:
+            _lib.call(fn, n, ranges, self.np, T.nx_, T.ny_, t.shape[0], 0, self.i.data_ptr(), self.j.data_ptr(),
                       self.type_zero_gradient.data_ptr(), self.di.data_ptr(), self.dj.data_ptr(), _p(T.mask), 1,
                       ptr, ptr, _s())
 
@@ -393,12 +419,12 @@ class DeviceBoundaries:
             return
         T = self.T
         f32 = trs[0].all_values.dtype == torch.float32
-        fn = "getm_open_boundary_tracers_f32" if f32 else "getm_open_boundary_tracers"
+        fn = "getm_open_boundaries_tracers_f32" if f32 else "getm_open_boundaries_tracers"
         for c in range(0, len(trs), 16):
             chunk = trs[c:c + 16]
             vars_ = _lib.ptr_array([t.all_values.data_ptr() for t in chunk])
             bdy = _lib.ptr_array([self.tracer_values[t.name].data_ptr() for t in chunk])
-            for s, e in self.ranges:
-                _lib.call(fn, s, e, self.np, T.nx_, T.ny_, T.nz, self.nsponge, self.i.data_ptr(), self.j.data_ptr(),
+            for n, ranges in self._launches:
+                _lib.call(fn, n, ranges, self.np, T.nx_, T.ny_, T.nz, self.nsponge, self.i.data_ptr(), self.j.data_ptr(),
                           self.type_3d.data_ptr(), self.di.data_ptr(), self.dj.data_ptr(), _p(T.mask), len(chunk),
                           vars_, bdy, _s())

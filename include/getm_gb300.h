@@ -616,7 +616,16 @@ int getm_surface_elevation_fused(int nx, int ny, int halox, int haloy, const int
  * Point tables (halo-inclusive T indices i, j; condition type; inward
  * direction di, dj; side 1..4 = W, N, E, S; inflow sign) come from the host
  * collection.  The reference updates its boundaries one after another, so a
- * call covers the contiguous point range [start, stop) of one boundary.    */
+ * call covers the contiguous point range [start, stop) of one boundary, or
+ * (..._elevations, ..._boundaries_tracers) nrange <= GETM_MAX_BOUNDARIES
+ * boundaries in the order given: ranges is a HOST array of start, stop pairs. */
+#define GETM_MAX_BOUNDARIES 64
+/* prescribed elevation of np points from harmonic constituents (periods and
+ * device arrays of amplitude and phase per point; om, amp, phase: HOST
+ * arrays): z_p = sum_c amp_c(p) cos(*time om_c + phase_c(p))               */
+#define GETM_MAX_CONSTITUENTS 16
+int getm_open_boundary_tide(int np, int nconstituent, const double* om, const double* const* amp,
+                            const double* const* phase, const double* time, double* z, cudaStream_t stream);
 /* elevation: ZeroGradient (:338-356), Clamped (:358-375), Flather on
  * elevation or transport (:377-416); result clipped to Dmin - H
  * (simulation.py:580-582, :1252-1257).  z_ext, flow_ext: per point.        */
@@ -625,6 +634,11 @@ int getm_open_boundary_elevation(int start, int stop, int nx, const int* i, cons
                                  const double* inflow_sign, const double* H, const double* Dclip,
                                  const double* U, const double* V, const double* z_ext,
                                  const double* flow_ext, double Dmin, double* z, cudaStream_t stream);
+int getm_open_boundary_elevations(int nrange, const int* ranges, int np, int nx, const int* i, const int* j,
+                                  const int* type, const int* di, const int* dj, const int* side,
+                                  const double* inflow_sign, const double* H, const double* Dclip,
+                                  const double* U, const double* V, const double* z_ext,
+                                  const double* flow_ext, double Dmin, double* z, cudaStream_t stream);
 /* tracers (simulation.py:1160-1168): ZeroGradient, Clamped, Sponge with
  * nsponge points (:195-336, fixed relaxation).  vars, bdy: HOST arrays of
  * ntracer (<= 16) device pointers; bdy[t] holds nz x np prescribed values. */
@@ -636,6 +650,14 @@ int getm_open_boundary_tracers_f32(int start, int stop, int np, int nx, int ny, 
                                    const int* i, const int* j, const int* type, const int* di,
                                    const int* dj, const int* mask, int ntracer, float* const* vars,
                                    const float* const* bdy, cudaStream_t stream);
+int getm_open_boundaries_tracers(int nrange, const int* ranges, int np, int nx, int ny, int nz, int nsponge,
+                                 const int* i, const int* j, const int* type, const int* di,
+                                 const int* dj, const int* mask, int ntracer, double* const* vars,
+                                 const double* const* bdy, cudaStream_t stream);
+int getm_open_boundaries_tracers_f32(int nrange, const int* ranges, int np, int nx, int ny, int nz, int nsponge,
+                                     const int* i, const int* j, const int* type, const int* di,
+                                     const int* dj, const int* mask, int ntracer, float* const* vars,
+                                     const float* const* bdy, cudaStream_t stream);
 /* core.Array.mirror (python/pygetm/core.py:723-728): field[tgt] = field[src]
  * for n pairs of flat [j][i] indices, every one of nlev levels of size plane,
  * with every source read before any target is written (a point may be the
