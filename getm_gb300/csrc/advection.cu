@@ -247,9 +247,8 @@ __global__ void __launch_bounds__(256) hpass_y_march_kernel(HPassArgs<S, V> a, i
     const int w = blockIdx.y * blockDim.y + threadIdx.y;
     const int chunk = w % nchunk, k = w / nchunk;
     if (k >= a.nk) return;  // whole warp
-    // one sweep per group of NT tracers; with no tracers one sweep updates h
-    for (int t0 = 0; t0 == 0 || t0 < a.ntracer; t0 += NT)
-        hpass_y_march_body<S, NT, V>(a, blockIdx.x, chunk, k, threadIdx.x, t0);
+    // a group of NT tracers per block z; with no tracers one sweep updates h
+    hpass_y_march_body<S, NT, V>(a, blockIdx.x, chunk, k, threadIdx.x, NT * blockIdx.z);
 }
 
 // Launch one horizontal pass (storage type S, velocity type V, arithmetic C).
@@ -288,10 +287,20 @@ static int launch_hpass_c(int direction, HPassArgs<S, V>& a, cudaStream_t stream
         dim3 grid(getm_div_up(a.nx_, 32), getm_div_up(a.ny_ + 1, HY_STRIDE), a.nk);
         hpass_y_inc_kernel<S, V, C><<<grid, block, 0, stream>>>(a);
     } else {
+        // rows a warp marches: the knob's, halved (to four at least, which
+        // repeats one face in four) until there are 64 warps per SM: a warp's
+        // march is a chain of load latencies.  us per five-pass split with the
+        // knob's 32 -> this, groups of fields one after the other -> side by
+        // side: 92 x 92 x 20 two FP64-stored fields 140 -> 64, a float field 78 ->
+        // 45; 150 x 120 x 30 three 195 -> 151; 240 x 200 x 20 eight 860 -> 578, a float
+        // field 120 -> 102; 400 x 300 x 40 two 622 -> 582 (eight rows 594)
+        const int nt = a.ntracer >= 2 ? 2 : 1, ngroup = a.ntracer > nt ? getm_div_up(a.ntracer, nt) : 1;
+        const long long strips = (long long)getm_div_up(a.nx_, 32) * a.nk * ngroup;
         a.ych = getm_tune(GETM_TUNE_YMARCH_CHUNK);
+        while (a.ych > 4 && strips * getm_div_up(a.ny_, a.ych) < 64 * GETM_SMS) a.ych /= 2;
         const int nchunk = getm_div_up(a.ny_, a.ych);
         dim3 block(32, 8);
-        dim3 grid(getm_div_up(a.nx_, 32), getm_div_up((long long)nchunk * a.nk, 8));
+        dim3 grid(getm_div_up(a.nx_, 32), getm_div_up((long long)nchunk * a.nk, 8), ngroup);
         if constexpr (!f64) {
             if (a.ntracer >= 2) hpass_y_march_kernel<S, 2, V><<<grid, block, 0, stream>>>(a, nchunk);
             else hpass_y_march_kernel<S, 1, V><<<grid, block, 0, stream>>>(a, nchunk);

@@ -662,8 +662,8 @@ __device__ __forceinline__ void hpass_y_inc_body(const HPassArgs<S, V>& a, int b
 // (no shared memory, no block barriers) and updates cell j from its south
 // face (the previous step) and its north face (this step).  The arithmetic
 // is that of hpass_y_inc_body, operation for operation; NT tracers are
-// marched together, larger batches in groups of NT (the face geometry is
-// reloaded per group).
+// marched together, larger batches in groups of NT in warps of their own (the
+// face geometry is reloaded per group).
 
 template <typename S, int NT, typename V = S, typename C = float>
 __device__ __forceinline__ void hpass_y_march_body(const HPassArgs<S, V>& a, int bx, int chunk, int k, int lane,

@@ -341,7 +341,7 @@ int getm_stream_destroy(cudaStream_t stream);
  * it was captured with).  The table is per host thread and starts at the
  * defaults; a value outside the knob's set returns GETM_ERR_ARG.
  *   GETM_TUNE_XPASS_ROWS      rows (warps) per block of the x pass: 2, 4, 8 (default 8)
- *   GETM_TUNE_YMARCH_CHUNK    rows a warp marches in the 3D y pass: 16, 32, 64 (default 32)
+ *   GETM_TUNE_YMARCH_CHUNK    rows at most that a warp marches in the 3D y pass: 16, 32, 64 (default 32)
  *   GETM_TUNE_COLUMN_ROWS     rows of 32 columns per block of the w pass
  *                             (where it does not split the columns) and the
  *                             float column solve: 1, 2, 4 (default 4)
