@@ -210,13 +210,13 @@ __global__ void __launch_bounds__(256) hpass_x_inc_kernel(HPassArgs<S, V> a)
     hpass_x_inc_rows<S, 1, NoEpi, V, C>(a, blockIdx.x, j, blockIdx.z, threadIdx.x);
 }
 
-// grid (1, y, nk): each warp of block (0, y, k) sweeps nrow rows of layer k
+// grid (pairs of fields, y, nk): each warp of block (g, y, k) sweeps nrow rows of layer k
 template <typename S, typename V = S>
 __global__ void __launch_bounds__(256) hpass_x_vec_kernel(HPassArgs<S, V> a, int nrow)
 {
     const int j0 = (blockIdx.y * blockDim.y + threadIdx.y) * nrow;
     if (j0 >= a.ny_) return;  // whole warp
-    hpass_x_vec_rows<S, V>(a, j0, min(nrow, a.ny_ - j0), blockIdx.z, threadIdx.x);
+    hpass_x_vec_rows<S, V>(a, j0, min(nrow, a.ny_ - j0), blockIdx.z, threadIdx.x, 2 * blockIdx.x);
 }
 
 // The four-cells-per-lane x pass applies: rows of whole 16-byte vectors and
@@ -265,12 +265,20 @@ static int launch_hpass_c(int direction, HPassArgs<S, V>& a, cudaStream_t stream
         // geometry once for all fields where the sweep repeats it per pair
         if constexpr (!f64) vec = getm_tune(GETM_TUNE_XPASS_VEC) && xpass_vec_ok(a);
         if (vec) {
-            // rows per warp: as many (up to four) as leave 16 warps per SM; at
-            // most two warps per block, so that the last wave of blocks is short
+            // rows per warp: four where that fills the chunks better (a 404-cell
+            // row by itself fills 3.2 of its four, a 244-cell row 1.9 of two) and
+            // leaves 16 warps per SM; at most two warps per block, so that the
+            // last wave of blocks is short.  us per five-pass split of 240 x 200 x
+            // 20 with eight fields: pairs one after the other 578, side by side
+            // 566, and one row per warp 502
+            const int npair = a.ntracer > 0 ? (a.ntracer + 1) / 2 : 1, nq = a.nx_ / 4;
+            auto chunks = [&](int n) { return getm_div_up((long long)n * nq, 32) * (4 / n); };  // of four rows
             int nrow = 4;
-            while (nrow > 1 && (long long)getm_div_up(a.ny_, nrow) * a.nk < 16 * GETM_SMS) nrow /= 2;
+            while (nrow > 1 && (chunks(nrow / 2) * 97 <= chunks(4) * 100 ||
+                                (long long)getm_div_up(a.ny_, nrow) * a.nk * npair < 16 * GETM_SMS))
+                nrow /= 2;
             block.y = rows < 2 ? rows : 2;
-            dim3 grid(1, getm_div_up(getm_div_up(a.ny_, nrow), block.y), a.nk);
+            dim3 grid(npair, getm_div_up(getm_div_up(a.ny_, nrow), block.y), a.nk);
             if constexpr (!f64) hpass_x_vec_kernel<S, V><<<grid, block, 0, stream>>>(a, nrow);
         } else {
             // lane 0 of the first segment handles the face west of cell 0

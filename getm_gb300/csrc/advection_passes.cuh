@@ -367,8 +367,8 @@ __device__ __forceinline__ void hpass_x_inc_rows(const HPassArgs<S, V>& a, int b
 // limiter, both faces beside it: one FP64 subtraction per cell and field
 // instead of two for FP64 storage).  Every face and cell is evaluated with
 // the same expressions as hpass_x_inc_rows, so both give the same bits.
-// Fields are swept two at a time (the thickness is written by the first
-// sweep).
+// Fields t0 and t0 + 1 are swept together (the thickness is written with the
+// first), further pairs by warps of their own.
 template <typename T>
 __device__ __forceinline__ void xv_load4(const T* p, T (&o)[4])
 {
@@ -397,7 +397,7 @@ __device__ __forceinline__ void xv_store4(T* p, const T (&v)[4])
 }
 
 template <typename S, typename V = S>
-__device__ __forceinline__ void hpass_x_vec_rows(const HPassArgs<S, V>& a, int j0, int nrow, int k, int lane)
+__device__ __forceinline__ void hpass_x_vec_rows(const HPassArgs<S, V>& a, int j0, int nrow, int k, int lane, int t0)
 {
     constexpr unsigned FULL = 0xffffffffu;
     const int nx = a.nx_;
@@ -405,139 +405,135 @@ __device__ __forceinline__ void hpass_x_vec_rows(const HPassArgs<S, V>& a, int j
     const int total = nq * nrow;
     const long long r2 = (long long)j0 * nx;
     const long long r3 = (long long)k * a.plane + r2;
-    const int ngroup = a.ntracer > 0 ? (a.ntracer + 1) / 2 : 1;
-    for (int g = 0; g < ngroup; g++) {
-        const int t0 = 2 * g;
-        const int nt = a.ntracer - t0 >= 2 ? 2 : a.ntracer - t0;  // 0 with no fields
-        // the west face of the chunk's first cell: the chunk to the west's
-        // last face (nothing west of the rows: an inactive face)
-        float cQU = 0.f;
-        int cum = 0;
-        float cd[2] = {0.f, 0.f}, cer[2] = {0.f, 0.f};
-        int row = lane / nq, iq = lane - row * nq;  // the lane's row and quad
-        for (int q0 = 0; q0 < total; q0 += 32) {
-            const int ib = 4 * (q0 + lane);  // the lane's first cell, from the first row's start
-            const int ic = 4 * iq;           // ... in its row
-            const bool lin = q0 + lane < total;  // all four cells or none
-            const int ie = 4 * (q0 + 32);        // the first cell east of the chunk
-            const bool ein = q0 + 32 < total;
-            const int j = j0 + row;
-            const bool jrow = j >= a.jlo && j <= a.jhi;
-            int um[4] = {0, 0, 0, 0}, tm[4] = {0, 0, 0, 0};
-            float dyf[4] = {0.f, 0.f, 0.f, 0.f}, idxf[4] = {0.f, 0.f, 0.f, 0.f}, iaf[4] = {0.f, 0.f, 0.f, 0.f};
-            float ahraw[4] = {0.f, 0.f, 0.f, 0.f};
-            V uraw[4] = {V(0), V(0), V(0), V(0)};
-            double huraw[4] = {0.0, 0.0, 0.0, 0.0}, hold[4] = {0.0, 0.0, 0.0, 0.0};
-            if (lin) {
-                xv_load4(a.umask + r2 + ib, um);
-                xv_load4(a.tmask + r2 + ib, tm);
-                xv_load4(a.dy_f + r2 + ib, dyf);
-                xv_load4(a.idx_f + r2 + ib, idxf);
-                xv_load4(a.iA_f + r2 + ib, iaf);
-                xv_load4(a.u + r3 + ib, uraw);
-                xv_load4(a.hu + r3 + ib, huraw);
-                xv_load4(a.h_in + r3 + ib, hold);
-                if (a.Ah) {
-                    double ah[4];
-                    xv_load4(a.Ah + r2 + ib, ah);
+    const int nt = a.ntracer - t0 >= 2 ? 2 : a.ntracer - t0;  // 0 with no fields
+    // the west face of the chunk's first cell: the chunk to the west's
+    // last face (nothing west of the rows: an inactive face)
+    float cQU = 0.f;
+    int cum = 0;
+    float cd[2] = {0.f, 0.f}, cer[2] = {0.f, 0.f};
+    int row = lane / nq, iq = lane - row * nq;  // the lane's row and quad
+    for (int q0 = 0; q0 < total; q0 += 32) {
+        const int ib = 4 * (q0 + lane);  // the lane's first cell, from the first row's start
+        const int ic = 4 * iq;           // ... in its row
+        const bool lin = q0 + lane < total;  // all four cells or none
+        const int ie = 4 * (q0 + 32);        // the first cell east of the chunk
+        const bool ein = q0 + 32 < total;
+        const int j = j0 + row;
+        const bool jrow = j >= a.jlo && j <= a.jhi;
+        int um[4] = {0, 0, 0, 0}, tm[4] = {0, 0, 0, 0};
+        float dyf[4] = {0.f, 0.f, 0.f, 0.f}, idxf[4] = {0.f, 0.f, 0.f, 0.f}, iaf[4] = {0.f, 0.f, 0.f, 0.f};
+        float ahraw[4] = {0.f, 0.f, 0.f, 0.f};
+        V uraw[4] = {V(0), V(0), V(0), V(0)};
+        double huraw[4] = {0.0, 0.0, 0.0, 0.0}, hold[4] = {0.0, 0.0, 0.0, 0.0};
+        if (lin) {
+            xv_load4(a.umask + r2 + ib, um);
+            xv_load4(a.tmask + r2 + ib, tm);
+            xv_load4(a.dy_f + r2 + ib, dyf);
+            xv_load4(a.idx_f + r2 + ib, idxf);
+            xv_load4(a.iA_f + r2 + ib, iaf);
+            xv_load4(a.u + r3 + ib, uraw);
+            xv_load4(a.hu + r3 + ib, huraw);
+            xv_load4(a.h_in + r3 + ib, hold);
+            if (a.Ah) {
+                double ah[4];
+                xv_load4(a.Ah + r2 + ib, ah);
 #pragma unroll
-                    for (int m = 0; m < 4; m++) ahraw[m] = getm_d2f_approx(ah[m]);
-                }
+                for (int m = 0; m < 4; m++) ahraw[m] = getm_d2f_approx(ah[m]);
             }
-            // masks of the velocity points beside the lane's first and last faces
-            int umW = __shfl_up_sync(FULL, um[3], 1), umE = __shfl_down_sync(FULL, um[0], 1);
-            if (lane == 0) umW = cum;
-            if (lane == 31) umE = ein ? a.umask[r2 + ie] : 0;
-
-            // face geometry (the same expressions as hpass_x_inc_rows)
-            float QU[4], cfl[4], ahd[4];
-            bool up[4], uu_ok[4], act[4];
-#pragma unroll
-            for (int m = 0; m < 4; m++) {
-                const int ia = ic + m;
-                const bool f_in = lin && jrow && ia >= a.ilo - 1 && ia <= a.ihi;
-                act[m] = f_in && getm_flux_point(um[m]);
-                QU[m] = 0.f; cfl[m] = 0.f; ahd[m] = 0.f;
-                up[m] = false; uu_ok[m] = false;
-                if (act[m]) {
-                    const float uu = inc_f<V>(uraw[m]);
-                    const float huf = getm_d2f_approx(huraw[m]);
-                    QU[m] = uu * huf * dyf[m];
-                    cfl[m] = fabsf(uu * a.dtf * idxf[m]);
-                    up[m] = uu > 0.f;
-                    const int mw = m > 0 ? um[m - 1] : umW, me = m < 3 ? um[m + 1] : umE;
-                    uu_ok[m] = getm_flux_point(up[m] ? mw : me);
-                    if (a.Ah) ahd[m] = -ahraw[m] * huf * idxf[m] * dyf[m];
-                }
-            }
-            float QUw0 = __shfl_up_sync(FULL, QU[3], 1);  // west face of the lane's first cell
-            if (lane == 0) QUw0 = cQU;
-
-            // thickness update of the lane's cells
-            float coef[4];
-            bool upd[4];
-            double hnew[4];
-#pragma unroll
-            for (int m = 0; m < 4; m++) {
-                const int c = ic + m;
-                upd[m] = lin && jrow && c >= a.ilo && c <= a.ihi && tm[m] == 1;
-                coef[m] = 0.f;
-                hnew[m] = hold[m];
-                if (upd[m]) {
-                    const float QUw = m > 0 ? QU[m - 1] : QUw0;
-                    hx_cell(a.dtf, QU[m], QUw, iaf[m], hold[m], hnew[m], coef[m]);
-                }
-            }
-            if (g == 0 && lin) xv_store4(a.h_out + r3 + ib, hnew);
-
-#pragma unroll
-            for (int q = 0; q < 2; q++) {
-                if (q >= nt) break;
-                const S* __restrict__ f = a.fin[t0 + q] + r3;
-                S fv[4] = {S(0), S(0), S(0), S(0)};
-                if (lin) xv_load4(f + ib, fv);
-                S fE0 = S(0), fE1 = S(0);  // the two cells east of the chunk (last lane)
-                if (lane == 31) {
-                    if (ein) { fE0 = f[ie]; fE1 = f[ie + 1]; }
-                }
-                S fn0 = __shfl_down_sync(FULL, fv[0], 1);
-                if (lane == 31) fn0 = fE0;
-                // differences of neighbouring values in the storage type, then
-                // narrowed (d[m]: across face m)
-                float d[4];
-                d[0] = inc_f<S>(fv[1] - fv[0]);
-                d[1] = inc_f<S>(fv[2] - fv[1]);
-                d[2] = inc_f<S>(fv[3] - fv[2]);
-                d[3] = inc_f<S>(fn0 - fv[3]);
-                float dW = __shfl_up_sync(FULL, d[3], 1), dE = __shfl_down_sync(FULL, d[0], 1);
-                if (lane == 0) dW = cd[q];
-                if (lane == 31) dE = inc_f<S>(fE1 - fE0);
-                float el[4], er[4];
-#pragma unroll
-                for (int m = 0; m < 4; m++) {
-                    el[m] = 0.f; er[m] = 0.f;
-                    if (act[m]) {
-                        const TvdFace<float> tf = getm_tvd_face_c(a.scheme, cfl[m]);
-                        const float dprev = m > 0 ? d[m - 1] : dW, dnext = m < 3 ? d[m + 1] : dE;
-                        hx_face(tf, up[m], uu_ok[m], QU[m], dprev, d[m], dnext, ahd[m], a.Ah != nullptr, el[m], er[m]);
-                    }
-                }
-                float erW = __shfl_up_sync(FULL, er[3], 1);  // west face of the lane's first cell
-                if (lane == 0) erW = cer[q];
-                S out[4];
-#pragma unroll
-                for (int m = 0; m < 4; m++) {
-                    const float ew = m > 0 ? er[m - 1] : erW;
-                    out[m] = upd[m] ? hx_new(fv[m], coef[m], el[m], ew) : fv[m];
-                }
-                if (lin) xv_store4(a.fout[t0 + q] + r3 + ib, out);
-                cd[q] = __shfl_sync(FULL, d[3], 31);
-                cer[q] = __shfl_sync(FULL, er[3], 31);
-            }
-            cQU = __shfl_sync(FULL, QU[3], 31);
-            cum = __shfl_sync(FULL, um[3], 31);
-            for (iq += 32; iq >= nq; iq -= nq) row++;
         }
+        // masks of the velocity points beside the lane's first and last faces
+        int umW = __shfl_up_sync(FULL, um[3], 1), umE = __shfl_down_sync(FULL, um[0], 1);
+        if (lane == 0) umW = cum;
+        if (lane == 31) umE = ein ? a.umask[r2 + ie] : 0;
+
+        // face geometry (the same expressions as hpass_x_inc_rows)
+        float QU[4], cfl[4], ahd[4];
+        bool up[4], uu_ok[4], act[4];
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+            const int ia = ic + m;
+            const bool f_in = lin && jrow && ia >= a.ilo - 1 && ia <= a.ihi;
+            act[m] = f_in && getm_flux_point(um[m]);
+            QU[m] = 0.f; cfl[m] = 0.f; ahd[m] = 0.f;
+            up[m] = false; uu_ok[m] = false;
+            if (act[m]) {
+                const float uu = inc_f<V>(uraw[m]);
+                const float huf = getm_d2f_approx(huraw[m]);
+                QU[m] = uu * huf * dyf[m];
+                cfl[m] = fabsf(uu * a.dtf * idxf[m]);
+                up[m] = uu > 0.f;
+                const int mw = m > 0 ? um[m - 1] : umW, me = m < 3 ? um[m + 1] : umE;
+                uu_ok[m] = getm_flux_point(up[m] ? mw : me);
+                if (a.Ah) ahd[m] = -ahraw[m] * huf * idxf[m] * dyf[m];
+            }
+        }
+        float QUw0 = __shfl_up_sync(FULL, QU[3], 1);  // west face of the lane's first cell
+        if (lane == 0) QUw0 = cQU;
+
+        // thickness update of the lane's cells
+        float coef[4];
+        bool upd[4];
+        double hnew[4];
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+            const int c = ic + m;
+            upd[m] = lin && jrow && c >= a.ilo && c <= a.ihi && tm[m] == 1;
+            coef[m] = 0.f;
+            hnew[m] = hold[m];
+            if (upd[m]) {
+                const float QUw = m > 0 ? QU[m - 1] : QUw0;
+                hx_cell(a.dtf, QU[m], QUw, iaf[m], hold[m], hnew[m], coef[m]);
+            }
+        }
+        if (t0 == 0 && lin) xv_store4(a.h_out + r3 + ib, hnew);
+
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            if (q >= nt) break;
+            const S* __restrict__ f = a.fin[t0 + q] + r3;
+            S fv[4] = {S(0), S(0), S(0), S(0)};
+            if (lin) xv_load4(f + ib, fv);
+            S fE0 = S(0), fE1 = S(0);  // the two cells east of the chunk (last lane)
+            if (lane == 31) {
+                if (ein) { fE0 = f[ie]; fE1 = f[ie + 1]; }
+            }
+            S fn0 = __shfl_down_sync(FULL, fv[0], 1);
+            if (lane == 31) fn0 = fE0;
+            // differences of neighbouring values in the storage type, then
+            // narrowed (d[m]: across face m)
+            float d[4];
+            d[0] = inc_f<S>(fv[1] - fv[0]);
+            d[1] = inc_f<S>(fv[2] - fv[1]);
+            d[2] = inc_f<S>(fv[3] - fv[2]);
+            d[3] = inc_f<S>(fn0 - fv[3]);
+            float dW = __shfl_up_sync(FULL, d[3], 1), dE = __shfl_down_sync(FULL, d[0], 1);
+            if (lane == 0) dW = cd[q];
+            if (lane == 31) dE = inc_f<S>(fE1 - fE0);
+            float el[4], er[4];
+#pragma unroll
+            for (int m = 0; m < 4; m++) {
+                el[m] = 0.f; er[m] = 0.f;
+                if (act[m]) {
+                    const TvdFace<float> tf = getm_tvd_face_c(a.scheme, cfl[m]);
+                    const float dprev = m > 0 ? d[m - 1] : dW, dnext = m < 3 ? d[m + 1] : dE;
+                    hx_face(tf, up[m], uu_ok[m], QU[m], dprev, d[m], dnext, ahd[m], a.Ah != nullptr, el[m], er[m]);
+                }
+            }
+            float erW = __shfl_up_sync(FULL, er[3], 1);  // west face of the lane's first cell
+            if (lane == 0) erW = cer[q];
+            S out[4];
+#pragma unroll
+            for (int m = 0; m < 4; m++) {
+                const float ew = m > 0 ? er[m - 1] : erW;
+                out[m] = upd[m] ? hx_new(fv[m], coef[m], el[m], ew) : fv[m];
+            }
+            if (lin) xv_store4(a.fout[t0 + q] + r3 + ib, out);
+            cd[q] = __shfl_sync(FULL, d[3], 31);
+            cer[q] = __shfl_sync(FULL, er[3], 31);
+        }
+        cQU = __shfl_sync(FULL, QU[3], 31);
+        cum = __shfl_sync(FULL, um[3], 31);
+        for (iq += 32; iq >= nq; iq -= nq) row++;
     }
 }
 
