@@ -351,8 +351,9 @@ __global__ void __launch_bounds__(128, 8) vd_column_kernel(VDArgs<float> a)
 // sweep together (work: 2 nz planes per field of a group).  SRC: whether a
 // field of the group has ea2 or ea4 (without, no registers are spent on
 // them).
+// coef, rs: the thread's coefficients of the surface level and their stride.
 template <int NT, bool SRC, typename S>
-__device__ __forceinline__ void vd_inc_sweep(const VDArgs<float, S>& a, long long c, int t0)
+__device__ __forceinline__ void vd_inc_sweep(const VDArgs<float, S>& a, long long c, int t0, float* coef, long long rs)
 {
     const long long P = a.plane;
     const int nz = a.nz;
@@ -372,8 +373,8 @@ __device__ __forceinline__ void vd_inc_sweep(const VDArgs<float, S>& a, long lon
         v[t] = a.var[t0 + t] + c;
         e2[t] = SRC && a.ea2[t0 + t] ? a.ea2[t0 + t] + c : nullptr;
         e4[t] = SRC && a.ea4[t0 + t] ? a.ea4[t0 + t] + c : nullptr;
-        ru[t] = a.work + c + (long long)(2 * t) * nz * P;
-        qu[t] = ru[t] + (long long)nz * P;
+        ru[t] = coef + (long long)(2 * t) * nz * rs;
+        qu[t] = ru[t] + (long long)nz * rs;
         mol[t] = (float)a.molecular[t0 + t];
     }
     // level k operands (current) and the raw loads of level k-1 (next)
@@ -447,8 +448,8 @@ __device__ __forceinline__ void vd_inc_sweep(const VDArgs<float, S>& a, long lon
                 rk[t] = a1 / den;
                 qk[t] = (a4 - a3 * qk[t]) / den;
             }
-            ru[t][k * P] = rk[t];
-            qu[t][k * P] = qk[t];
+            ru[t][k * rs] = rk[t];
+            qu[t][k * rs] = qk[t];
             aoa[t] = aob; ana[t] = anb;
             vk[t] = vn[t]; vn[t] = vnn[t];
             e2c[t] = e2n[t]; e4c[t] = e4n[t];
@@ -473,8 +474,8 @@ __device__ __forceinline__ void vd_inc_sweep(const VDArgs<float, S>& a, long lon
         if (SRC && e4[t]) a4 = a4 + e4c[t];
         vprev[t] = (a4 - a3 * qk[t]) / (a2 - a3 * rk[t]);
         xn[t] = v[t][P];
-        rn[t] = ru[t][P];
-        qn[t] = qu[t][P];
+        rn[t] = ru[t][rs];
+        qn[t] = qu[t][rs];
         v[t][0] = inc_add<S>(vk[t], vprev[t]);
     }
     for (k = 1; k < nz; k++) {
@@ -484,8 +485,8 @@ __device__ __forceinline__ void vd_inc_sweep(const VDArgs<float, S>& a, long lon
             const float r = rn[t], q = qn[t];
             if (k + 1 < nz) {
                 xn[t] = v[t][(k + 1) * P];
-                rn[t] = ru[t][(k + 1) * P];
-                qn[t] = qu[t][(k + 1) * P];
+                rn[t] = ru[t][(k + 1) * rs];
+                qn[t] = qu[t][(k + 1) * rs];
             }
             vprev[t] = q - r * vprev[t];
             v[t][k * P] = inc_add<S>(x_old, vprev[t]);
@@ -495,23 +496,72 @@ __device__ __forceinline__ void vd_inc_sweep(const VDArgs<float, S>& a, long lon
 
 // PAIRS: fields in pairs (then an odd last one alone), else one at a time.
 // Blocks of 32 columns by GETM_TUNE_COLUMN_ROWS rows.  S: storage type of
-// the fields (float, or double for FP64 tracer storage).
-template <bool SRC, bool PAIRS, typename S = float>
+// the fields (float, or double for FP64 tracer storage).  SM (and not
+// PAIRS): the coefficients in shared memory and each field in blocks of its own
+// (grid z); else in the global workspace, fields or pairs one after the other.
+template <bool SRC, bool PAIRS, bool SM, typename S>
 __global__ void __launch_bounds__(128, 7) vd_inc_kernel(VDArgs<float, S> a)
 {
+    extern __shared__ __align__(16) unsigned char vd_smem[];
     const int i = blockIdx.x * 32 + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     if (i >= a.nx_ || j >= a.ny_) return;
     const long long c = (long long)j * a.nx_ + i;
     if (a.nz == 1) {
-        vd_single_layer(a, c);
+        if (blockIdx.z == 0) vd_single_layer(a, c);
         return;
     }
     if (a.mask[c] != 1) return;
-    int t0 = 0;
-    if constexpr (PAIRS)
-        for (; t0 + 2 <= a.ntracer; t0 += 2) vd_inc_sweep<2, SRC, S>(a, c, t0);
-    for (; t0 < a.ntracer; t0++) vd_inc_sweep<1, SRC, S>(a, c, t0);
+    if constexpr (SM) {
+        float* coef = reinterpret_cast<float*>(vd_smem) + threadIdx.y * 32 + threadIdx.x;
+        vd_inc_sweep<1, SRC, S>(a, c, blockIdx.z, coef, 32 * blockDim.y);
+    } else {
+        int t0 = 0;
+        if constexpr (PAIRS)
+            for (; t0 + 2 <= a.ntracer; t0 += 2) vd_inc_sweep<2, SRC, S>(a, c, t0, a.work + c, a.plane);
+        for (; t0 < a.ntracer; t0++) vd_inc_sweep<1, SRC, S>(a, c, t0, a.work + c, a.plane);
+    }
+}
+
+template <bool SRC, typename S>
+static int vd_inc_launch_src(VDArgs<float, S>& a, cudaStream_t stream)
+{
+    const int rows = getm_tune(GETM_TUNE_COLUMN_ROWS);
+    dim3 grid(getm_div_up(a.nx_, 32), getm_div_up(a.ny_, rows)), block(32, rows);
+    // Several fields on a domain with few columns (a sweep is then a chain of
+    // latencies): each field in blocks of its own, up to 20 warps of columns per
+    // SM, and up to the layers whose coefficients leave room for 20 warps per
+    // SM.  us, pairs in turn through the workspace -> fields side by side: 92 x 92
+    // x 20 two fields 31 -> 21; 150 x 120 x 30 three 80 -> 35; 240 x 200 x 20
+    // eight 155 -> 79 (pairs side by side 118); 300 x 250 x 25 two 60 -> 52; but
+    // 400 x 300 x 40 two (26 warps) 133 -> 164, and one field alone 75 -> 103.
+    const long long warps = (long long)grid.x * a.ny_;
+    if (a.ntracer > 1 && a.nz <= 45 && warps <= 20 * GETM_SMS) {
+        const size_t smem = (size_t)rows * 32 * a.nz * 2 * sizeof(float);  // at most 45 KB
+        static bool attr_set = false;
+        if (!attr_set) {
+            if (cudaFuncSetAttribute(vd_inc_kernel<SRC, false, true, S>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                     100) != cudaSuccess)
+                return GETM_ERR_CUDA;
+            attr_set = true;
+        }
+        grid.z = a.ntracer;
+        vd_inc_kernel<SRC, false, true, S><<<grid, block, smem, stream>>>(a);
+    } else if (a.ntracer > 1) {
+        vd_inc_kernel<SRC, true, false, S><<<grid, block, 0, stream>>>(a);
+    } else {
+        vd_inc_kernel<SRC, false, false, S><<<grid, block, 0, stream>>>(a);
+    }
+    GETM_CHECK_LAUNCH();
+    return GETM_OK;
+}
+
+template <typename S>
+static int vd_inc_launch(VDArgs<float, S>& a, cudaStream_t stream)
+{
+    bool src = false;
+    for (int t = 0; t < a.ntracer; t++) src = src || a.ea2[t] || a.ea4[t];
+    return src ? vd_inc_launch_src<true, S>(a, stream) : vd_inc_launch_src<false, S>(a, stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -830,17 +880,7 @@ static int vd_launch_f64s(VDArgs<float, double>& a, cudaStream_t stream)
 {
     if (a.nz > 1 && vd_seg_applies(a.nz)) return vd_seg_launch(a, stream);
     if (!a.work) return GETM_ERR_ARG;
-    const int rows = getm_tune(GETM_TUNE_COLUMN_ROWS);
-    const dim3 grid(getm_div_up(a.nx_, 32), getm_div_up(a.ny_, rows)), block(32, rows);
-    bool src = false;
-    for (int t = 0; t < a.ntracer; t++) src = src || a.ea2[t] || a.ea4[t];
-    const bool pairs = a.ntracer > 1;
-    if (src && pairs) vd_inc_kernel<true, true, double><<<grid, block, 0, stream>>>(a);
-    else if (src) vd_inc_kernel<true, false, double><<<grid, block, 0, stream>>>(a);
-    else if (pairs) vd_inc_kernel<false, true, double><<<grid, block, 0, stream>>>(a);
-    else vd_inc_kernel<false, false, double><<<grid, block, 0, stream>>>(a);
-    GETM_CHECK_LAUNCH();
-    return GETM_OK;
+    return vd_inc_launch(a, stream);
 }
 
 // prepare as a separate call (diffusion.F90:163-171): auxo/auxn at every
@@ -859,26 +899,11 @@ __global__ void vd_prepare_kernel(int nx_, int ny_, int nz, long long plane, dou
     auxn[p] = cnpar * x / (dzn[c + (k + 1) * plane] + dzn[c + k * plane]);
 }
 
-static bool vd_sources(const VDArgs<float>& a)
-{
-    for (int t = 0; t < a.ntracer; t++)
-        if (a.ea2[t] || a.ea4[t]) return true;
-    return false;
-}
-
 static int vd_launch(VDArgs<float>& a, cudaStream_t stream)
 {
     if (a.work && a.nz > 1) {
         if (vd_seg_applies(a.nz)) return vd_seg_launch(a, stream);
-        const int rows = getm_tune(GETM_TUNE_COLUMN_ROWS);
-        const dim3 grid(getm_div_up(a.nx_, 32), getm_div_up(a.ny_, rows)), block(32, rows);
-        const bool src = vd_sources(a), pairs = a.ntracer > 1;
-        if (src && pairs) vd_inc_kernel<true, true><<<grid, block, 0, stream>>>(a);
-        else if (src) vd_inc_kernel<true, false><<<grid, block, 0, stream>>>(a);
-        else if (pairs) vd_inc_kernel<false, true><<<grid, block, 0, stream>>>(a);
-        else vd_inc_kernel<false, false><<<grid, block, 0, stream>>>(a);
-        GETM_CHECK_LAUNCH();
-        return GETM_OK;
+        return vd_inc_launch(a, stream);
     }
     int threads = 128;
     const size_t per = (size_t)VD_SMEM_ARRAYS * a.nz * sizeof(float);
