@@ -244,7 +244,8 @@ __global__ void buoyancy_frequency_kernel(long long plane, int nz, const int* __
     const R drho = -R(SEOS_A0) * dT * (R(1) + R(0.5 * SEOS_LAMBDA1) * (Ta1 + Ta0) + R(SEOS_MU1) * zi)
                    + R(SEOS_B0) * dS * (R(1) - R(0.5 * SEOS_LAMBDA2) * (Sa1 + Sa0) - R(SEOS_MU2) * zi)
                    - R(SEOS_NU) * (dT * Sa1 + Ta0 * dS);
-    NN[q1] = R(-GETM_G / GETM_RHO0) * drho / dz;
+    if constexpr (std::is_same<R, double>::value) NN[q1] = getm_div((-GETM_G / GETM_RHO0) * drho, dz);
+    else NN[q1] = R(-GETM_G / GETM_RHO0) * drho / dz;
 }
 
 template <typename R>

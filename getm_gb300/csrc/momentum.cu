@@ -268,29 +268,42 @@ extern "C" int getm_w_momentum_3d_f32(int nx, int ny, int nz, int imin, int imax
     return w_momentum_impl<float>(nx, ny, nz, imin, imax, jmin, jmax, mask, dyu, dxv, iarea, ho, hn, pk, qk, dt, w, stream);
 }
 
-// momentum.F90:218-241 (T: type of uk, vk, SS and of the arithmetic)
+// momentum.F90:218-241 (T: type of uk, vk, SS and of the arithmetic).  The shear
+// across a face serves the points on both sides, so each is formed once: a
+// warp covers 31 columns and the face west of them (the west shear comes by
+// shuffle), and marches up to eight rows north, the north shear of one row
+// being the south shear of the next.  FP64 (the FP64 pipe is the time): 127 ->
+// 64 us on 200 x 150 x 30, its quotients by getm_div; float, bound by the
+// instructions that narrow the thicknesses: 70 -> 56 us on 400 x 300 x 40.
+
 template <typename T>
-__global__ void shear_frequency_kernel(int nx, int ny, int nz, int ilo, int ihi, int jlo, int jhi,
-                                       const int* __restrict__ mask, const double* __restrict__ hu, const double* __restrict__ hv,
-                                       const T* __restrict__ uk, const T* __restrict__ vk, T* __restrict__ SS)
+__global__ void __launch_bounds__(128)
+    shear_frequency_kernel(int nx, int ny, int nz, int ilo, int ihi, int jlo, int jhi, const int* __restrict__ mask,
+                           const double* __restrict__ hu, const double* __restrict__ hv, const T* __restrict__ uk,
+                           const T* __restrict__ vk, T* __restrict__ SS, int rows)
 {
-    int i, j;
-    const int k = blockIdx.y + 1;  // Fortran interface k = 1..nz-1
-    if (!getm_flat_column(nx, jlo, jhi - jlo + 1, i, j) || i < ilo || i > ihi) return;
-    long long p = (long long)j * nx + i;
-    if (mask[p] <= 0) return;
-    long long plane = (long long)nx * ny;
-    long long a = p + (k - 1) * plane, b = p + k * plane;
-    // thicknesses in T (float: narrowed on the integer pipe)
-    auto h = [](double x) -> T {
-        if constexpr (std::is_same<T, double>::value) return x;
-        else return getm_d2f_approx(x);
+    const int lane = threadIdx.x;
+    const int k = blockIdx.z + 1;  // Fortran interface k = 1..nz-1
+    const int i = ilo - 1 + blockIdx.x * 31 + lane;
+    const int j0 = jlo + (blockIdx.y * blockDim.y + threadIdx.y) * rows;
+    if (j0 > jhi) return;  // whole warp
+    const int j1 = min(j0 + rows - 1, jhi);
+    const int ic = i <= ihi ? i : ihi;  // (idle lanes repeat the last column)
+    const long long plane = (long long)nx * ny;
+    auto shear = [&](const T* __restrict__ v, const double* __restrict__ h, long long p) -> T {
+        const long long a = p + (k - 1) * plane, b = p + k * plane;
+        if constexpr (std::is_same<T, double>::value) return getm_div(v[b] - v[a], getm_half(h[b] + h[a]));
+        else return (v[b] - v[a]) / (T(0.5) * (getm_d2f_approx(h[b]) + getm_d2f_approx(h[a])));
     };
-    T t1 = (uk[b] - uk[a]) / (T(0.5) * (h(hu[b]) + h(hu[a])));
-    T t2 = (uk[b - 1] - uk[a - 1]) / (T(0.5) * (h(hu[b - 1]) + h(hu[a - 1])));
-    T t3 = (vk[b] - vk[a]) / (T(0.5) * (h(hv[b]) + h(hv[a])));
-    T t4 = (vk[b - nx] - vk[a - nx]) / (T(0.5) * (h(hv[b - nx]) + h(hv[a - nx])));
-    SS[b] = T(0.5) * (t1 * t1 + t2 * t2 + t3 * t3 + t4 * t4);
+    T t4 = shear(vk, hv, (long long)(j0 - 1) * nx + ic);
+#pragma unroll 2
+    for (int j = j0; j <= j1; j++) {
+        const long long p = (long long)j * nx + ic;
+        const T t1 = shear(uk, hu, p), t3 = shear(vk, hv, p);
+        const T t2 = __shfl_up_sync(0xffffffffu, t1, 1);
+        if (lane > 0 && i <= ihi && mask[p] > 0) SS[p + k * plane] = T(0.5) * (t1 * t1 + t2 * t2 + t3 * t3 + t4 * t4);
+        t4 = t3;
+    }
 }
 
 template <typename T>
@@ -300,8 +313,16 @@ static int shear_impl(int nx, int ny, int nz, int imin, int imax, int jmin, int 
     if (nx < 1 || ny < 1 || nz < 1 || imin < 2 || jmin < 2 || imax > nx || jmax > ny || jmax < jmin) return GETM_ERR_ARG;
     if (!mask || !hu || !hv || !uk || !vk || !SS) return GETM_ERR_ARG;
     if (nz < 2) return GETM_OK;
-    dim3 grid(getm_div_up((long long)nx * (jmax - jmin + 1), 128), nz - 1);
-    shear_frequency_kernel<T><<<grid, 128, 0, stream>>>(nx, ny, nz, imin - 1, imax - 1, jmin - 1, jmax - 1, mask, hu, hv, uk, vk, SS);
+    if (imax < imin) return GETM_OK;
+    // rows per warp: fewer where the warps would not hide a march's latencies
+    // (92 x 92 x 20 float with eight rows 25 us, with one 7 us; the FP64 pipe is
+    // busy with few)
+    const long long strips = (long long)getm_div_up(imax - imin + 1, 31) * (nz - 1);
+    int rows = 8;
+    while (rows > 1 && strips * getm_div_up(jmax - jmin + 1, rows) < (std::is_same<T, double>::value ? 16 : 64) * GETM_SMS)
+        rows /= 2;
+    const dim3 block(32, 4), grid(getm_div_up(imax - imin + 1, 31), getm_div_up(jmax - jmin + 1, 4 * rows), nz - 1);
+    shear_frequency_kernel<T><<<grid, block, 0, stream>>>(nx, ny, nz, imin - 1, imax - 1, jmin - 1, jmax - 1, mask, hu, hv, uk, vk, SS, rows);
     GETM_CHECK_LAUNCH();
     return GETM_OK;
 }
@@ -537,8 +558,8 @@ __global__ void velocities_3d_kernel(long long n, const T* pk, const double* hnu
     if (q >= n) return;
     T u, v;
     if constexpr (std::is_same<T, double>::value) {
-        u = pk[q] / hnu[q];
-        v = qk[q] / hnv[q];
+        u = getm_div(pk[q], hnu[q]);
+        v = getm_div(qk[q], hnv[q]);
     } else {
         u = pk[q] / getm_d2f_approx(hnu[q]);
         v = qk[q] / getm_d2f_approx(hnv[q]);

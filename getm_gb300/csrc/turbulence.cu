@@ -20,8 +20,20 @@
 //
 // One thread per water column (32 columns of a warp are adjacent at every
 // level, so each level's loads are coalesced); both equations are solved
-// implicitly in time over the interfaces 1..nz-1 with a Thomas sweep whose
-// elimination coefficients live in a [level][column] workspace.
+// implicitly in time over the interfaces 1..nz-1 with an elimination whose
+// coefficients live in a [level][column] workspace.  GB300's FP64 rate bounds
+// it (its FP64 instructions take 16 cycles of an SM each), so it counts those:
+// with U = dt K / h the coupling through a layer, which is the one above an
+// interface and then the one below the next, and s' of the interface below
+// (zero at the bottom, where c' = -1 would be the fixed value's),
+//     t = dz (1 - dt S) + U' s',  den = t + U,  c = U / den,  s = t / den,
+//     d = (dz (x + dt Q) + U' d') / den,   then downwards x = d + c x_above:
+// no large terms are subtracted (b - a c of the textbook form loses digits
+// where mixing is strong), one reciprocal per interface (getm_rcp) and one per
+// layer, and minima, maxima and comparisons on the integer pipe: about 85 per
+// level for both equations and the closure, where 18 divisions and square
+// roots alone took some 160.  The operands of a level are loaded a level
+// ahead.  200 x 150 x 30: 464 -> 215 us.
 #include "getm_common.cuh"
 
 namespace {
@@ -52,44 +64,70 @@ __device__ __forceinline__ void keps_wall(const getm_keps_params& p, double usta
     e = fmax(cm0 * cm0 * cm0 * k * sqrt(k) / (p.kappa * z0), p.eps_min);
 }
 
-// One implicit diffusion-source equation over interfaces 1..nz-1 of column
-// c: dz_i (x_i' - x_i) / dt = flux differences + dz_i (Q_i + S_i x_i'),
-// diffusivities K at the layers (between interfaces), Dirichlet values x0,
-// xn at interfaces 0 and nz.  Q and S come from src(i, Q, S).
-template <typename R, typename Src, typename Diff>
-__device__ __forceinline__ void keps_solve(const KepsArgs<R>& a, long long c, double* x, double x0, double xn,
-                                           Src src, Diff kdiff)
+// The operands of interface l (1..nz-1) and of the layer above it.
+struct KepsIn {
+    double h, num, nuh, SS, NN, k, e;
+};
+
+template <typename R>
+__device__ __forceinline__ KepsIn keps_load(const KepsArgs<R>& a, long long q)
+{
+    return KepsIn{a.h[q], getm_widen(a.num[q]), getm_widen(a.nuh[q]), getm_widen(a.SS[q]), getm_widen(a.NN[q]),
+                  a.tke[q], a.eps[q]};
+}
+
+// One implicit diffusion-source equation over interfaces 1..nz-1 of column c:
+// dz_i (x_i' - x_i) / dt = flux differences + dz_i (Q_i + S_i x_i'), S <= 0,
+// diffusivities at the layers (between interfaces) the mean of num over sigma,
+// Dirichlet values x0, xn at interfaces 0 and nz.  src(in, x, Q, S): the old
+// value and the sources; fin(x): the new value's bound.
+template <typename R, typename Src, typename Fin>
+__device__ __forceinline__ void keps_solve(const KepsArgs<R>& a, long long c, double* __restrict__ x, double sigma,
+                                           double x0, double xn, Src src, Fin fin)
 {
     const long long P = a.plane;
     const int nz = a.nz;
-    double* cp = a.work + c;
-    double* dp = a.work + (long long)(nz + 1) * P + c;
-    double cprev = 0.0, dprev = x0;  // interface 0 is fixed
-    double hb = a.h[c];              // layer below interface i
-    double Kb = kdiff(0);
+    double* __restrict__ cp = a.work + c;
+    double* __restrict__ dp = a.work + (long long)(nz + 1) * P + c;
+    const double dts = 0.5 * a.dt / sigma;  // coupling of a layer: dts (num below + num above) / h
+    const double numb = getm_widen(a.num[c]);
+    double hb = a.h[c];  // layer below interface i
+    KepsIn in = keps_load(a, c + P);
+    double U = dts * (numb + in.num) * getm_rcp(hb);
+    double s = 1.0, d = x0;  // (interface 0 is fixed: c = 0)
     for (int i = 1; i < nz; i++) {
-        const double ht = a.h[c + (long long)i * P];  // layer above interface i
-        const double Kt = kdiff(i);
-        const double dz = 0.5 * (hb + ht);
-        double Q, S;
-        src(i, Q, S);
-        const double lo = -a.dt * Kb / hb;
-        const double up = -a.dt * Kt / ht;
-        const double b = dz - lo - up - a.dt * dz * S;
-        double d = dz * (x[c + (long long)i * P] + a.dt * Q);
-        if (i == nz - 1) d -= up * xn;
-        const double den = b - lo * cprev;
-        cprev = up / den;
-        dprev = (d - lo * dprev) / den;
-        cp[(long long)i * P] = cprev;
-        dp[(long long)i * P] = dprev;
-        hb = ht;
-        Kb = Kt;
+        const long long q = c + (long long)i * P;
+        // interface i + 1 (its num and, but for the last, the rest)
+        KepsIn nx;
+        if (i + 1 < nz) nx = keps_load(a, q + P);
+        else nx.num = getm_widen(a.num[q + P]);
+        const double dz = getm_half(hb + in.h);
+        double xo, Q, S;
+        src(in, xo, Q, S);
+        const double Un = dts * (in.num + nx.num) * getm_rcp(in.h);
+        const double t = fma(U, s, dz * fma(-a.dt, S, 1.0));
+        const double r = getm_rcp(t + Un);
+        const double cc = Un * r;
+        s = t * r;
+        double rhs = fma(U, d, dz * fma(a.dt, Q, xo));
+        if (i == nz - 1) rhs = fma(Un, xn, rhs);  // (beside the substitution's own term, which starts from xn)
+        d = rhs * r;
+        cp[(long long)i * P] = cc;
+        dp[(long long)i * P] = d;
+        hb = in.h;
+        U = Un;
+        in = nx;
     }
     double xv = xn;
+    double cn = cp[(long long)(nz - 1) * P], dn = dp[(long long)(nz - 1) * P];
     for (int i = nz - 1; i >= 1; i--) {
-        xv = dp[(long long)i * P] - cp[(long long)i * P] * xv;
-        x[c + (long long)i * P] = xv;
+        const double cc = cn, dd = dn;
+        if (i > 1) {
+            cn = cp[(long long)(i - 1) * P];
+            dn = dp[(long long)(i - 1) * P];
+        }
+        xv = fma(cc, xv, dd);
+        x[c + (long long)i * P] = fin(xv);
     }
     x[c] = x0;
     x[c + (long long)nz * P] = xn;
@@ -113,53 +151,50 @@ __global__ void __launch_bounds__(128) keps_kernel(KepsArgs<R> a)
     keps_wall(p, a.ustar_s[c], a.z0s[c], ks, es);
 
     // turbulent kinetic energy (old epsilon and diffusivities in the sources)
-    auto kdiff_k = [&](int l) {
-        return 0.5 * ((double)a.num[c + (long long)l * P] + (double)a.num[c + (long long)(l + 1) * P]) / p.sig_k;
-    };
-    auto src_k = [&](int l, double& Q, double& S) {
-        const long long q = c + (long long)l * P;
-        const double prod = (double)a.num[q] * (double)a.SS[q], buoy = -(double)a.nuh[q] * (double)a.NN[q];
-        const double k = a.tke[q], e = a.eps[q];
-        if (prod + buoy > 0.0) { Q = prod + buoy; S = -e / k; }
-        else { Q = prod; S = -(e - buoy) / k; }
+    auto src_k = [&](const KepsIn& in, double& x, double& Q, double& S) {
+        const double prod = in.num * in.SS, buoy = -in.nuh * in.NN;
+        const double sum = prod + buoy;
+        const bool up = getm_positive_i(sum);
+        x = in.k;
+        Q = up ? sum : prod;
+        S = -getm_div(up ? in.e : in.e - buoy, in.k);
     };
     // (the forward sweep reads every old value before the back substitution
     // overwrites them, so the update is in place)
-    keps_solve(a, c, a.tke, kb, ks, src_k, kdiff_k);
-    for (int l = 1; l < nz; l++) {
-        const long long q = c + (long long)l * P;
-        a.tke[q] = fmax(a.tke[q], p.k_min);
-    }
+    keps_solve(a, c, a.tke, p.sig_k, kb, ks, src_k, [&](double x) { return getm_fmax_i(x, p.k_min); });
 
     // dissipation rate (sources from the new k and the old epsilon)
-    auto kdiff_e = [&](int l) {
-        return 0.5 * ((double)a.num[c + (long long)l * P] + (double)a.num[c + (long long)(l + 1) * P]) / p.sig_e;
-    };
-    auto src_e = [&](int l, double& Q, double& S) {
-        const long long q = c + (long long)l * P;
-        const double prod = (double)a.num[q] * (double)a.SS[q], buoy = -(double)a.nuh[q] * (double)a.NN[q];
-        const double r = a.eps[q] / a.tke[q];
-        const double c3 = buoy > 0.0 ? p.c3_plus : p.c3_minus;
-        Q = r * (p.c1 * prod + c3 * buoy);
+    auto src_e = [&](const KepsIn& in, double& x, double& Q, double& S) {
+        const double prod = in.num * in.SS, buoy = -in.nuh * in.NN;
+        const double r = getm_div(in.e, in.k);
+        const double c3 = getm_positive_i(buoy) ? p.c3_plus : p.c3_minus;
+        x = in.e;
+        Q = r * fma(p.c1, prod, c3 * buoy);
         S = -p.c2 * r;
     };
-    keps_solve(a, c, a.eps, eb, es, src_e, kdiff_e);
+    keps_solve(a, c, a.eps, p.sig_e, eb, es, src_e, [](double x) { return x; });
 
     // limits, length scale, viscosity and diffusivity at every interface
+    const double ilim = cde / p.galp, iprandtl = 1.0 / p.prandtl;
+    const bool one = p.prandtl == 1.0;
+    double kn = a.tke[c], en = a.eps[c], N2n = getm_widen(a.NN[c]);
     for (int l = 0; l <= nz; l++) {
         const long long q = c + (long long)l * P;
-        const double k = a.tke[q];
-        double e = fmax(a.eps[q], p.eps_min);
-        const double N2 = (double)a.NN[q];
-        if (l > 0 && l < nz && N2 > 0.0) {  // Galperin: L <= galp sqrt(2 k / N2)
-            const double lmax = p.galp * sqrt(2.0 * k / N2);
-            e = fmax(e, cde * k * sqrt(k) / lmax);
+        const double k = kn, N2 = N2n;
+        double e = getm_fmax_i(en, p.eps_min);
+        if (l < nz) {
+            kn = a.tke[q + P];
+            en = a.eps[q + P];
+            N2n = getm_widen(a.NN[q + P]);
         }
+        // Galperin: L = cde k^1.5 / eps <= galp sqrt(2 k / N2)
+        if (l > 0 && l < nz && getm_positive_i(N2)) e = getm_fmax_i(e, ilim * k * sqrt(getm_half(N2)));
         a.eps[q] = e;
-        a.L[q] = cde * k * sqrt(k) / e;
-        const double nu = cmu * k * k / e;
+        const double kr = k * getm_rcp(e);
+        a.L[q] = cde * kr * sqrt(k);
+        const double nu = cmu * k * kr;
         a.num[q] = (R)nu;
-        a.nuh[q] = (R)(nu / p.prandtl);
+        a.nuh[q] = (R)(one ? nu : nu * iprandtl);
     }
 }
 
