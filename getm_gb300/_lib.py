@@ -49,6 +49,7 @@ _SIGS = {
     "getm_advection_w_calculate": "ppppdpps",
     "getm_advection_apply_3d_batch": "ppppippppppdpppips",
     "getm_advection_2d": "ppppiippppdpppps",
+    "getm_advection_2d_from": "ppppiippppdpppppis",
     "getm_advection_2d_mixed": "ppppiippppdpppps",
     "getm_advection_get_status": "ps",
     "getm_advection_2d_noalloc": "ipppiippppdpppps",

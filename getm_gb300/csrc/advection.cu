@@ -234,11 +234,11 @@ static bool xpass_vec_ok(const HPassArgs<S, V>& a)
     return true;
 }
 
-template <typename S, typename V, typename C>
-__global__ void __launch_bounds__(32 * HY_BY) hpass_y_inc_kernel(HPassArgs<S, V> a)
+template <typename S, typename V, typename C, int BY>
+__global__ void __launch_bounds__(32 * BY) hpass_y_inc_kernel(HPassArgs<S, V> a)
 {
-    __shared__ YIncSmem<S, C> sm;
-    hpass_y_inc_body<S, NoEpi, V, C>(a, blockIdx.x, blockIdx.y, blockIdx.z, threadIdx.x, threadIdx.y, sm);
+    __shared__ YIncSmem<S, C, BY> sm;
+    hpass_y_inc_body<S, NoEpi, V, C, BY>(a, blockIdx.x, blockIdx.y, blockIdx.z, threadIdx.x, threadIdx.y, sm);
 }
 
 template <typename S, int NT, typename V = S>
@@ -287,13 +287,14 @@ static int launch_hpass_c(int direction, HPassArgs<S, V>& a, cudaStream_t stream
         }
     } else if (f64 || a.nk < 4) {
         // a single plane: too few columns x layers for marching warps to fill
-        // the GPU, so blocks of 32 x HY_BY threads cover tiles instead.  FP64
+        // the GPU, so blocks of 32 columns cover tiles instead.  FP64
         // form: the tile kernel forms a face's geometry once for all fields
-        // and has a block per 15 rows, where the marching kernel repeats the
+        // and has a block per 15 rows or less, where the marching kernel repeats the
         // geometry per pair and had blocks for 90 of 152 SMs on 173 x 131 x 23
-        dim3 block(32, HY_BY);
-        dim3 grid(getm_div_up(a.nx_, 32), getm_div_up(a.ny_ + 1, HY_STRIDE), a.nk);
-        hpass_y_inc_kernel<S, V, C><<<grid, block, 0, stream>>>(a);
+        const int by = hpass_y_rows((long long)getm_div_up(a.nx_, 32) * a.nk, a.ny_, f64);
+        const dim3 block(32, by), grid(getm_div_up(a.nx_, 32), getm_div_up(a.ny_ + 1, by - 1), a.nk);
+        if (by == 16) hpass_y_inc_kernel<S, V, C, 16><<<grid, block, 0, stream>>>(a);
+        else hpass_y_inc_kernel<S, V, C, 4><<<grid, block, 0, stream>>>(a);
     } else {
         // rows a warp marches: the knob's, halved (to four at least, which
         // repeats one face in four) until there are 64 warps per SM: a warp's
@@ -1067,28 +1068,30 @@ extern "C" int getm_advection_uv_pass_f64s(int direction, int nk, getm_advection
                                        var_in, var_out, stream);
 }
 
+// D0: the column heights before the first pass (D itself, or the caller's
+// field); D: those after the last.
 static int advection_2d_impl(getm_advection* adv, getm_grid* tgrid, getm_grid* ugrid, getm_grid* vgrid,
                              int ufirst, int split, const double* u, const double* v, const double* Ah_u,
-                             const double* Ah_v, double timestep, double* D, const double* DU,
+                             const double* Ah_v, double timestep, const double* D0, double* D, const double* DU,
                              const double* DV, double* var, int increment, cudaStream_t stream)
 {
     if (!adv) return GETM_OK;
-    if (!D || !var || split < 1 || split > 3) return GETM_ERR_ARG;
+    if (!D0 || !D || !var || split < 1 || split > 3) return GETM_ERR_ARG;
     HPassArgs<double> ax, ay;
     int rc = hpass_setup(ax, 1, adv, tgrid, ugrid, 1, u, Ah_u, timestep, DU, increment);
     if (rc) return rc;
     if ((rc = hpass_setup(ay, 2, adv, tgrid, vgrid, 1, v, Ah_v, timestep, DV, increment))) return rc;
     const size_t n2 = (size_t)ax.plane;
-    if ((rc = adv_reserve(adv, n2, 1))) return rc;
+    if ((rc = adv_reserve(adv, n2, 2))) return rc;
     HPassArgs<double>* p1 = ufirst ? &ax : &ay;
     HPassArgs<double>* p2 = ufirst ? &ay : &ax;
     const int d1 = ufirst ? 1 : 2, d2 = ufirst ? 2 : 1;
-    double* T = adv->tmp[0];
+    double* const* T = adv->tmp;
     double* A = adv->hbuf[0];
     double* B = adv->hbuf[1];
     const double* fin[1];
     double* fout[1];
-    // Sequence of (pass, dt factor); ping-pong var<->T and D->A->B->...
+    // Sequence of (pass, dt factor): var->T0->T1->...->var and D0->A->B->...->D
     int seq_n = 0;
     int seq_dir[4];
     double seq_dt[4];
@@ -1109,20 +1112,17 @@ static int advection_2d_impl(getm_advection* adv, getm_grid* tgrid, getm_grid* u
         seq_a[3] = p1; seq_dir[3] = d1; seq_dt[3] = 0.5 * timestep;
         seq_n = 4;
     }
-    const double* hsrc = D;
-    double* fsrc = var;
+    const double* hsrc = D0;
+    const double* fsrc = var;
     for (int s = 0; s < seq_n; s++) {
         double* hdst = (s == seq_n - 1) ? D : ((s % 2 == 0) ? A : B);
-        double* fdst = (fsrc == var) ? T : var;
+        double* fdst = (s == seq_n - 1) ? var : T[s % 2];
         seq_a[s]->dt = seq_dt[s];
         seq_a[s]->dtf = (float)seq_dt[s];
         fin[0] = fsrc; fout[0] = fdst;
         if ((rc = run_hstage(*seq_a[s], seq_dir[s], hsrc, hdst, 1, fin, fout, stream))) return rc;
         hsrc = hdst;
         fsrc = fdst;
-    }
-    if (fsrc != var) {
-        if (cudaMemcpyAsync(var, fsrc, n2 * sizeof(double), cudaMemcpyDeviceToDevice, stream) != cudaSuccess) return GETM_ERR_CUDA;
     }
     return GETM_OK;
 }
@@ -1156,7 +1156,7 @@ extern "C" int getm_advection_2d(getm_advection* adv, getm_grid* tgrid, getm_gri
                                  double timestep, double* D, const double* DU, const double* DV,
                                  double* var, cudaStream_t stream)
 {
-    return advection_2d_impl(adv, tgrid, ugrid, vgrid, ufirst, split, u, v, Ah_u, Ah_v, timestep, D, DU, DV, var,
+    return advection_2d_impl(adv, tgrid, ugrid, vgrid, ufirst, split, u, v, Ah_u, Ah_v, timestep, D, D, DU, DV, var,
                              0, stream);
 }
 
@@ -1166,8 +1166,18 @@ extern "C" int getm_advection_2d_mixed(getm_advection* adv, getm_grid* tgrid, ge
                                        double timestep, double* D, const double* DU, const double* DV,
                                        double* var, cudaStream_t stream)
 {
-    return advection_2d_impl(adv, tgrid, ugrid, vgrid, ufirst, split, u, v, Ah_u, Ah_v, timestep, D, DU, DV, var,
+    return advection_2d_impl(adv, tgrid, ugrid, vgrid, ufirst, split, u, v, Ah_u, Ah_v, timestep, D, D, DU, DV, var,
                              1, stream);
+}
+
+extern "C" int getm_advection_2d_from(getm_advection* adv, getm_grid* tgrid, getm_grid* ugrid, getm_grid* vgrid,
+                                      int ufirst, int split, const double* u, const double* v, const double* Ah_u,
+                                      const double* Ah_v, double timestep, const double* D0, double* D,
+                                      const double* DU, const double* DV, double* var, int mixed,
+                                      cudaStream_t stream)
+{
+    return advection_2d_impl(adv, tgrid, ugrid, vgrid, ufirst, split, u, v, Ah_u, Ah_v, timestep, D0, D, DU, DV, var,
+                             mixed != 0, stream);
 }
 
 // ---------------------------------------------------------------------------

@@ -558,6 +558,18 @@ __device__ __forceinline__ void hpass_x_inc_body(const HPassArgs<S, V>& a, int b
 constexpr int HY_BY = 16;
 constexpr int HY_STRIDE = HY_BY - 1;
 
+// Rows of a block (one of them the edge) for `tiles` columns of blocks of 32 cells
+// over ny rows: 4, so that a plane spreads evenly over the SMs (an FP64 pass
+// takes as long as its fullest SM), or 16 (FP64) where that leaves every SM a few
+// blocks all the same, for 16 rows repeat less at the edges.  us with 16 / 8 / 4
+// rows, FP64 2D advection 97 x 75 22.8 / 18.7 / 18.7, 400 x 300 37.2 / 37.6 / 37.6;
+// 2D substep FP64 64 x 64 38.6 / 33.0 / 30.6, 220 x 160 54.4 / 57.4 / 52.5, mixed
+// 400 x 300 48.6 / 47.6 / 47.0.
+inline int hpass_y_rows(long long tiles, int ny, bool f64)
+{
+    return f64 && tiles * ((ny + 15) / 15) > 2 * GETM_SMS ? 16 : 4;
+}
+
 template <typename S, typename C = float, int BY = HY_BY>
 struct YIncSmem {
     S sf[BY + 3][32];       // rows j0-2 .. j0+BY

@@ -283,8 +283,8 @@ int substep_args(SubstepArgs& a, const getm_split2d_fields* f, int nx, int ny, i
 // and the FP64 pipe, which in the FP64 form is most of the time.  us per substep
 // in a CUDA graph, one cooperative launch with six grid barriers -> the seven
 // phases as seven launches -> these four:
-//   mixed  64 x 64  45 -> 27 -> 24    200 x 150  46 -> 30 -> 27    400 x 300  56 -> 51 -> 48
-//   FP64   64 x 64  56 -> 48 -> 32    150 x 120  58 -> 53 -> 42    220 x 160  68 -> 66 -> 57
+//   mixed  64 x 64  45 -> 27 -> 24    200 x 150  46 -> 30 -> 27    400 x 300  56 -> 51 -> 47
+//   FP64   64 x 64  56 -> 48 -> 31    150 x 120  58 -> 53 -> 38    220 x 160  68 -> 66 -> 52
 // A barrier cost about 1.3 us and left every SM to the slowest block, and one
 // register budget served all phases.  Each kernel but the first is launched
 // when the blocks of the one before are done (programmatic dependent launch
@@ -294,7 +294,7 @@ int substep_args(SubstepArgs& a, const getm_split2d_fields* f, int nx, int ny, i
 // fields; what precedes the first on the stream may be anything.
 namespace {
 
-constexpr int PH_XY = 4;  // rows of an x pass block
+constexpr int PH_XY = 2;  // rows of an x pass block
 
 // Rows of a tile, chosen per plane (substep_rows): up to TR_MAX for the
 // transports ((by + 1) x 33 staged points, one per thread) and DV_MAX for the
@@ -585,16 +585,11 @@ int launch_substep_advection(const SubstepArgs& a, cudaStream_t stream, bool fir
             rc = launch_substep(substep_advection_kernel<MIXED, PASS, 1, PH_XY>, g, dim3(32, PH_XY), first && d == 0,
                                 stream, a, d);
         } else {
-            // tiles of 16 or 8 rows (one of them the edge), whichever loads
-            // the fullest SM less
-            const long long nbx = (long long)div_up(a.nx, 32) * nd;
-            const dim3 g16(div_up(a.nx, 32), div_up(a.ny + 1, 15), nd), g8(div_up(a.nx, 32), div_up(a.ny + 1, 7), nd);
-            if (2 * getm_div_up(nbx * g16.y, GETM_SMS) <= getm_div_up(nbx * g8.y, GETM_SMS))
-                rc = launch_substep(substep_advection_kernel<MIXED, PASS, 2, 16>, g16, dim3(32, 16), first && d == 0,
-                                    stream, a, d);
-            else
-                rc = launch_substep(substep_advection_kernel<MIXED, PASS, 2, 8>, g8, dim3(32, 8), first && d == 0,
-                                    stream, a, d);
+            const int by = hpass_y_rows((long long)div_up(a.nx, 32) * nd, a.ny, !MIXED);
+            const dim3 g(div_up(a.nx, 32), div_up(a.ny + 1, by - 1), nd), b(32, by);
+            const bool f = first && d == 0;
+            if (by == 16) rc = launch_substep(substep_advection_kernel<MIXED, PASS, 2, 16>, g, b, f, stream, a, d);
+            else rc = launch_substep(substep_advection_kernel<MIXED, PASS, 2, 4>, g, b, f, stream, a, d);
         }
         if (rc) return rc;
     }

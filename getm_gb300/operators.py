@@ -68,7 +68,7 @@ class Advection:
         the mixed form's increment form (float64 storage and updates)."""
         if increments_2d not in ("float64", "float32"):
             raise ValueError(f"increments_2d must be 'float64' or 'float32', not {increments_2d!r}")
-        self._call_2d = "getm_advection_2d" if increments_2d == "float64" else "getm_advection_2d_mixed"
+        self._mixed_2d = int(increments_2d == "float32")
         self.grid = grid
         self.ugrid = grid.ugrid
         self.vgrid = grid.vgrid
@@ -133,10 +133,9 @@ class Advection:
         assert var.grid is self.grid and not var.z
         assert Ah_u is None or (Ah_u.grid is self.ugrid and not Ah_u.z)
         assert Ah_v is None or (Ah_v.grid is self.vgrid and not Ah_v.z)
-        self.D.copy_(self.grid.D.all_values)
-        call(self._call_2d, self.p, self.grid.handle, self.ugrid.handle, self.vgrid.handle, int(self._ufirst),
-             self.split_2d.value, _p(u), _p(v), _p(Ah_u), _p(Ah_v), float(timestep), self.D.data_ptr(),
-             _p(self.ugrid.D), _p(self.vgrid.D), _p(var), _s())
+        call("getm_advection_2d_from", self.p, self.grid.handle, self.ugrid.handle, self.vgrid.handle, int(self._ufirst),
+             self.split_2d.value, _p(u), _p(v), _p(Ah_u), _p(Ah_v), float(timestep),
+             _p(self.grid.D), self.D.data_ptr(), _p(self.ugrid.D), _p(self.vgrid.D), _p(var), self._mixed_2d, _s())
 
     def apply_3d(self, u: Array, v: Array, w: Array, timestep: float, var: Array, Ah_u: Optional[Array] = None,
                  Ah_v: Optional[Array] = None, new_h: bool = False, skip_initial_halo_exchange: bool = False,

@@ -113,6 +113,12 @@ int getm_advection_2d(getm_advection* adv, getm_grid* tgrid, getm_grid* ugrid, g
                       int ufirst, int split, const double* u, const double* v,
                       const double* Ah_u, const double* Ah_v, double timestep, double* D,
                       const double* DU, const double* DV, double* var, cudaStream_t stream);
+/* the same from column heights D0, which stay (D0 may be D): D receives those
+ * after the last pass; mixed: as getm_advection_2d_mixed                    */
+int getm_advection_2d_from(getm_advection* adv, getm_grid* tgrid, getm_grid* ugrid, getm_grid* vgrid, int ufirst,
+                           int split, const double* u, const double* v, const double* Ah_u, const double* Ah_v,
+                           double timestep, const double* D0, double* D, const double* DU, const double* DV,
+                           double* var, int mixed, cudaStream_t stream);
 /* Allocation-free 2D split.  No counterpart in the reference: it is
  * getm_advection_2d for callers that cannot let the library call cudaMalloc
  * (a host model whose pool allocator owns all device memory, or a driver that
