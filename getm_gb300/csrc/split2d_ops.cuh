@@ -465,36 +465,49 @@ struct SpgArgs {
 // MIXED: the elevation bounds on the integer pipe, the two differences in
 // FP64 and the rest in float (the mixed transport update reads the gradient
 // as a float).
-// z, H, D, sp at the point (0) and its east (1) and north (n) neighbours
+// The bound -H + min(Dmin, D) of an elevation, H at one point and D at its
+// neighbour; dry = -H + Dmin, which it is wherever the neighbour is deeper
+// than Dmin (the sum is formed out of line elsewhere, so that it costs nothing).
+static __device__ __noinline__ double spg_shallow(double H, double m) { return -H + m; }
+
+__device__ __forceinline__ double spg_bound(double dry, double H, double Dmin, double D)
+{
+    const double m = getm_fmin_i(Dmin, D);
+    return __double_as_longlong(m) == __double_as_longlong(Dmin) ? dry : spg_shallow(H, m);
+}
+
+// z, H, D, sp and B = -H + Dmin at the point (0) and its east (1) and north (n)
+// neighbours
 template <bool MIXED>
 __device__ __forceinline__ void spg_values(const SpgArgs& a, long long p, int mu, int mv, double z0, double z1,
                                            double zn, double H0, double H1, double Hn, double D0, double D1, double Dn,
-                                           double sp0, double sp1, double spn, double idx, double idy)
+                                           double B0, double B1, double Bn, double sp0, double sp1, double spn,
+                                           double idx, double idy)
 {
     if constexpr (MIXED) {
         const float gi = (float)(1.0 / (GETM_G * GETM_RHO0));
         if (mu == 1) {
-            const double zp = getm_fmax_i(z1, -H0 + getm_fmin_i(a.Dmin, D1));
-            const double zm = getm_fmax_i(z0, -H1 + getm_fmin_i(a.Dmin, D0));
+            const double zp = getm_fmax_i(z1, spg_bound(B0, H0, a.Dmin, D1));
+            const double zm = getm_fmax_i(z0, spg_bound(B1, H1, a.Dmin, D0));
             const float g = getm_d2f_approx(zp - zm) + getm_d2f_approx(sp1 - sp0) * gi;
             a.dpdx[p] = getm_f2d(g * getm_d2f_approx(idx));
         }
         if (mv == 1) {
-            const double zp = getm_fmax_i(zn, -H0 + getm_fmin_i(a.Dmin, Dn));
-            const double zm = getm_fmax_i(z0, -Hn + getm_fmin_i(a.Dmin, D0));
+            const double zp = getm_fmax_i(zn, spg_bound(B0, H0, a.Dmin, Dn));
+            const double zm = getm_fmax_i(z0, spg_bound(Bn, Hn, a.Dmin, D0));
             const float g = getm_d2f_approx(zp - zm) + getm_d2f_approx(spn - sp0) * gi;
             a.dpdy[p] = getm_f2d(g * getm_d2f_approx(idy));
         }
     } else {
         const double gammai = 1.0 / (GETM_G * GETM_RHO0);
         if (mu == 1) {
-            const double zp = getm_fmax_i(z1, -H0 + getm_fmin_i(a.Dmin, D1));
-            const double zm = getm_fmax_i(z0, -H1 + getm_fmin_i(a.Dmin, D0));
+            const double zp = getm_fmax_i(z1, spg_bound(B0, H0, a.Dmin, D1));
+            const double zm = getm_fmax_i(z0, spg_bound(B1, H1, a.Dmin, D0));
             a.dpdx[p] = (zp - zm + (sp1 - sp0) * gammai) * idx;
         }
         if (mv == 1) {
-            const double zp = getm_fmax_i(zn, -H0 + getm_fmin_i(a.Dmin, Dn));
-            const double zm = getm_fmax_i(z0, -Hn + getm_fmin_i(a.Dmin, D0));
+            const double zp = getm_fmax_i(zn, spg_bound(B0, H0, a.Dmin, Dn));
+            const double zm = getm_fmax_i(z0, spg_bound(Bn, Hn, a.Dmin, D0));
             a.dpdy[p] = (zp - zm + (spn - sp0) * gammai) * idy;
         }
     }
@@ -505,8 +518,9 @@ __device__ __forceinline__ void spg_point(const SpgArgs& a, long long p)
 {
     const long long n = p + a.nx;
     // every operand is loaded before the masks are tested
-    spg_values<MIXED>(a, p, a.umask[p], a.vmask[p], a.z[p], a.z[p + 1], a.z[n], a.H[p], a.H[p + 1], a.H[n], a.D[p],
-                      a.D[p + 1], a.D[n], a.sp[p], a.sp[p + 1], a.sp[n], a.idxu[p], a.idyv[p]);
+    const double H0 = a.H[p], H1 = a.H[p + 1], Hn = a.H[n];
+    spg_values<MIXED>(a, p, a.umask[p], a.vmask[p], a.z[p], a.z[p + 1], a.z[n], H0, H1, Hn, a.D[p], a.D[p + 1],
+                      a.D[n], -H0 + a.Dmin, -H1 + a.Dmin, -Hn + a.Dmin, a.sp[p], a.sp[p + 1], a.sp[n], a.idxu[p], a.idyv[p]);
 }
 
 // interp_x / interp_y (interpolation.F90:9-40) of one point: t = mean of s
@@ -514,5 +528,6 @@ __device__ __forceinline__ void spg_point(const SpgArgs& a, long long p)
 template <typename T>
 __device__ __forceinline__ void interp_pair_point(const T* s, T* t, long long p, long long step, long long off)
 {
-    t[p + off] = T(0.5) * (s[p] + s[p + step]);
+    if constexpr (std::is_same<T, double>::value) t[p + off] = getm_half(s[p] + s[p + step]);
+    else t[p + off] = T(0.5) * (s[p] + s[p + step]);
 }

@@ -52,6 +52,7 @@ __host__ __device__ inline int div_up(int a, int b) { return (a + b - 1) / b; }
 struct SubstepArgs {
     int nx, ny, halox, haloy;
     int ufirst, accumulate, friction;
+    int early;                   // the next kernel is launched as each block begins
     double dt, idt;
     double* time;
     Transport2DArgs tr[2];       // [0]: U, [1]: V
@@ -290,8 +291,10 @@ int substep_args(SubstepArgs& a, const getm_split2d_fields* f, int nx, int ny, i
 // when the blocks of the one before are done (programmatic dependent launch
 // without an early trigger: blocks launched while the SMs are still busy land
 // on whichever has room, and the FP64 pipes of those SMs then set the pace:
-// FP64 220 x 160 57 -> 90 us) and waits for its end before it touches the
-// fields; what precedes the first on the stream may be anything.
+// FP64 220 x 160 57 -> 90 us; small planes of the mixed form, whose kernels
+// leave SMs idle and wait for latencies, trigger as they begin: a 92 x 92
+// member's step 948 -> 919 us, 184 x 184 1320 -> 1392) and waits for its end before
+// it touches the fields; what precedes the first on the stream may be anything.
 namespace {
 
 constexpr int PH_XY = 2;  // rows of an x pass block
@@ -308,6 +311,7 @@ __device__ __forceinline__ bool substep_begin(const SubstepArgs& a)
 {
     unsigned err = 0;
     if (a.sync) asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(err) : "l"(a.sync + 2) : "memory");
+    if (a.early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     return err != 0;
 }
@@ -382,7 +386,8 @@ __global__ void __launch_bounds__(DV_THREADS, 3)
     using C = typename std::conditional<MIXED, float, double>::type;
     __shared__ double sz[DV_MAX + 2][34], szh[DV_MAX + 2][34];  // elevation: new, and the mean with the old
     __shared__ double sH[DV_MAX + 2][34], sD[DV_MAX + 2][34], sdh[DV_MAX + 2][34];  // T: H, D, D of the mean
-    __shared__ double sX[DV_MAX + 1][33];  // X depths
+    __shared__ double sB[DV_MAX + 2][34];                        // -H + Dmin
+    __shared__ double sX[DV_MAX + 1][33], sU[DV_MAX + 1][33];    // X depths; sums of the means at i-1, i of row j-1
     const bool err = substep_begin(a);
     const DepthArgs& da = a.depth;
     const int nx = a.nx, ny = a.ny, t = threadIdx.x;
@@ -413,12 +418,13 @@ __global__ void __launch_bounds__(DV_THREADS, 3)
     // elevation (simulation.py:1468-1486) and T depths of the staged point
     const int sj = t / 34, si = t - sj * 34, gi = i0 - 1 + si, gj = j0 - 1 + sj;
     if (sj < by + 2) {
-        double z = 0.0, zh = 0.0, D = 0.0, H = 0.0, dh = 0.0;
+        double z = 0.0, zh = 0.0, D = 0.0, H = 0.0, dh = 0.0, B = 0.0;
         if (gi >= 0 && gi < nx && gj >= 0 && gj < ny) {
             const int g = gj * nx + gi;
             const int m = a.mT[g];
             const double zo = a.zo[g];
             H = da.HT[g];
+            B = -H + da.Dmin;
             z = zo;
             if (gi >= a.halox && gi < nx - a.halox && gj >= a.haloy && gj < ny - a.haloy) {
                 const double Uw = Us[g - 1], dyw = a.dyU[g - 1], Uc = Us[g], dye = a.dyU[g];
@@ -436,7 +442,7 @@ __global__ void __launch_bounds__(DV_THREADS, 3)
                 da.workT[g] = dh;
             }
         }
-        sz[sj][si] = z; szh[sj][si] = zh; sH[sj][si] = H; sD[sj][si] = D; sdh[sj][si] = dh;
+        sz[sj][si] = z; szh[sj][si] = zh; sH[sj][si] = H; sD[sj][si] = D; sdh[sj][si] = dh; sB[sj][si] = B;
     }
     __syncthreads();
     if (err) return;
@@ -444,9 +450,11 @@ __global__ void __launch_bounds__(DV_THREADS, 3)
     // previous X._work value
     if (xin) {
         const bool mine = xj < by && xi < 32;
+        const double south = szh[xj][xi] + szh[xj][xi + 1];  // (also z_U of the point south-west)
+        sU[xj][xi] = south;
         double zx;
         if (Xj >= 1 && Xj <= ny - 1 && Xi >= 1 && Xi <= nx - 1) {
-            zx = getm_quarter(szh[xj][xi] + szh[xj][xi + 1] + szh[xj + 1][xi] + szh[xj + 1][xi + 1]);
+            zx = getm_quarter(south + szh[xj + 1][xi] + szh[xj + 1][xi + 1]);
             if (mine) da.workX[px] = zx;
         } else {
             zx = da.workX[px];
@@ -470,7 +478,7 @@ __global__ void __launch_bounds__(DV_THREADS, 3)
     // U: z_U = interp_x(z_T_half, ioffset 0) for i < nx-1, else the old value
     double zu, zv, DU, DV;
     if (east) {
-        zu = getm_half(zh + szh[y][x + 1]);
+        zu = getm_half(sU[ty + 1][tx + 1]);
         da.workU[p] = zu;
     } else {
         zu = da.workU[p];
@@ -515,7 +523,8 @@ __global__ void __launch_bounds__(DV_THREADS, 3)
     if (north) interp_pair_point<double>(a.tauy, a.tausy, p, nx, 0);
     if (interior)
         spg_values<MIXED>(a.spg, p, mU, mV, sz[y][x], sz[y][x + 1], sz[y + 1][x], sH[y][x], sH[y][x + 1], sH[y + 1][x],
-                          sD[y][x], sD[y][x + 1], sD[y + 1][x], sp0, sp1, spn, idx, idy);
+                          sD[y][x], sD[y][x + 1], sD[y + 1][x], sB[y][x], sB[y][x + 1], sB[y + 1][x], sp0, sp1, spn,
+                          idx, idy);
 }
 
 // Phases 6 and 7: advection pass PASS in direction DIR of U (block z 0; d0 =
@@ -641,6 +650,8 @@ extern "C" int getm_split2d_substep(const getm_split2d_fields* f, int nx, int ny
     int rc = substep_args(a, f, nx, ny, halox, haloy, mixed, ufirst, accumulate, friction, timestep, Dmin, Dcrit,
                           uadv, ugrid, uugrid, uvgrid, uadv_ufirst, vadv, vgrid, vugrid, vvgrid, vadv_ufirst);
     if (rc) return rc;
+    // (see above: mixed form, depth tiles of four rows for at most every SM)
+    a.early = mixed && (long long)div_up(nx + 1, 32) * div_up(ny + 1, 4) <= GETM_SMS;
     return mixed ? launch_substep_kernels<true>(a, stream) : launch_substep_kernels<false>(a, stream);
 }
 
