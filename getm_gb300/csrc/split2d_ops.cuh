@@ -176,41 +176,30 @@ __device__ __forceinline__ double vel_div(double num, double den)
 // Mixed form: u1 = U/D to ~2^-46 (getm_div_refined; u1 is advected and its
 // product with the new depth is differenced against U, so it stays FP64) and
 // the advection velocities entirely in float.
-// east, north: the neighbours (Ue, Ve at i + 1; Un, Vn at j + 1) exist
+// One direction's: its transport T at the point and its neighbours (east at
+// i + 1, north at j + 1, where they exist) over the depth D of its grid and
+// those of the two advection velocity grids, De and Dn.
 template <typename C>
-__device__ __forceinline__ void momentum_2d_velocities_values(const VelArgs& a, long long p, bool east, bool north,
-                                                              double Up, double Ue, double Un, double Vp, double Ve,
-                                                              double Vn, double DU, double DV, double DUU, double DUV,
-                                                              double DVU, double DVV)
+__device__ __forceinline__ void momentum_2d_velocities_half(const VelArgs& a, int d, long long p, bool east, bool north,
+                                                            double T, double Te, double Tn, double D, double De,
+                                                            double Dn)
 {
+    double *vel = d == 0 ? a.u1 : a.v1, *adv = d == 0 ? a.advU : a.advV;
+    double *ve = d == 0 ? a.uua : a.uva, *vn = d == 0 ? a.vua : a.vva;
     // interp_x (ioffset 0) writes i < nx-1; elsewhere the old value is divided
     if constexpr (std::is_same<C, double>::value) {
-        const double u1 = getm_div(Up, DU);
-        const double v1 = getm_div(Vp, DV);
-        a.u1[p] = u1; a.advU[p] = u1;
-        a.v1[p] = v1; a.advV[p] = v1;
-        const double uu = east ? getm_half(Up + Ue) : a.uua[p];
-        const double uv = east ? getm_half(Vp + Ve) : a.uva[p];
-        const double vu = north ? getm_half(Up + Un) : a.vua[p];
-        const double vv = north ? getm_half(Vp + Vn) : a.vva[p];
-        a.uua[p] = vel_div<C>(uu, DUU);
-        a.uva[p] = vel_div<C>(uv, DUV);
-        a.vua[p] = vel_div<C>(vu, DVU);
-        a.vva[p] = vel_div<C>(vv, DVV);
+        const double v = getm_div(T, D);
+        vel[p] = v; adv[p] = v;
+        ve[p] = vel_div<C>(east ? getm_half(T + Te) : ve[p], De);
+        vn[p] = vel_div<C>(north ? getm_half(T + Tn) : vn[p], Dn);
     } else {
-        const double u1 = getm_div_refined(Up, DU);
-        const double v1 = getm_div_refined(Vp, DV);
-        a.u1[p] = u1; a.advU[p] = u1;
-        a.v1[p] = v1; a.advV[p] = v1;
-        const float Uf = getm_d2f_approx(Up), Vf = getm_d2f_approx(Vp);
-        const float uu = east ? 0.5f * (Uf + getm_d2f_approx(Ue)) : getm_d2f_approx(a.uua[p]);
-        const float uv = east ? 0.5f * (Vf + getm_d2f_approx(Ve)) : getm_d2f_approx(a.uva[p]);
-        const float vu = north ? 0.5f * (Uf + getm_d2f_approx(Un)) : getm_d2f_approx(a.vua[p]);
-        const float vv = north ? 0.5f * (Vf + getm_d2f_approx(Vn)) : getm_d2f_approx(a.vva[p]);
-        a.uua[p] = getm_f2d(uu / getm_d2f_approx(DUU));
-        a.uva[p] = getm_f2d(uv / getm_d2f_approx(DUV));
-        a.vua[p] = getm_f2d(vu / getm_d2f_approx(DVU));
-        a.vva[p] = getm_f2d(vv / getm_d2f_approx(DVV));
+        const double v = getm_div_refined(T, D);
+        vel[p] = v; adv[p] = v;
+        const float Tf = getm_d2f_approx(T);
+        const float te = east ? 0.5f * (Tf + getm_d2f_approx(Te)) : getm_d2f_approx(ve[p]);
+        const float tn = north ? 0.5f * (Tf + getm_d2f_approx(Tn)) : getm_d2f_approx(vn[p]);
+        ve[p] = getm_f2d(te / getm_d2f_approx(De));
+        vn[p] = getm_f2d(tn / getm_d2f_approx(Dn));
     }
 }
 
@@ -219,9 +208,10 @@ __device__ __forceinline__ void momentum_2d_velocities_point(const VelArgs& a, i
 {
     const long long p = (long long)j * a.nx + i;
     const bool east = i < a.nx - 1, north = j < a.ny - 1;
-    momentum_2d_velocities_values<C>(a, p, east, north, a.U[p], east ? a.U[p + 1] : 0.0, north ? a.U[p + a.nx] : 0.0,
-                                     a.V[p], east ? a.V[p + 1] : 0.0, north ? a.V[p + a.nx] : 0.0, a.DU[p], a.DV[p],
-                                     a.DUU[p], a.DUV[p], a.DVU[p], a.DVV[p]);
+    momentum_2d_velocities_half<C>(a, 0, p, east, north, a.U[p], east ? a.U[p + 1] : 0.0, north ? a.U[p + a.nx] : 0.0,
+                                   a.DU[p], a.DUU[p], a.DVU[p]);
+    momentum_2d_velocities_half<C>(a, 1, p, east, north, a.V[p], east ? a.V[p + 1] : 0.0, north ? a.V[p + a.nx] : 0.0,
+                                   a.DV[p], a.DUV[p], a.DVV[p]);
 }
 
 // Momentum.bottom_friction (momentum.py:1099-1125): u1 -> V grid and v1 -> U
@@ -476,40 +466,23 @@ __device__ __forceinline__ double spg_bound(double dry, double H, double Dmin, d
     return __double_as_longlong(m) == __double_as_longlong(Dmin) ? dry : spg_shallow(H, m);
 }
 
-// z, H, D, sp and B = -H + Dmin at the point (0) and its east (1) and north (n)
-// neighbours
+// One direction's gradient out (mask m): z, H, D, sp and B = -H + Dmin at the
+// point (0) and its neighbour (1)
 template <bool MIXED>
-__device__ __forceinline__ void spg_values(const SpgArgs& a, long long p, int mu, int mv, double z0, double z1,
-                                           double zn, double H0, double H1, double Hn, double D0, double D1, double Dn,
-                                           double B0, double B1, double Bn, double sp0, double sp1, double spn,
-                                           double idx, double idy)
+__device__ __forceinline__ void spg_half(double* out, double Dmin, long long p, int m, double z0, double z1, double H0,
+                                         double H1, double D0, double D1, double B0, double B1, double sp0, double sp1,
+                                         double id)
 {
+    if (m != 1) return;
+    const double zp = getm_fmax_i(z1, spg_bound(B0, H0, Dmin, D1));
+    const double zm = getm_fmax_i(z0, spg_bound(B1, H1, Dmin, D0));
     if constexpr (MIXED) {
         const float gi = (float)(1.0 / (GETM_G * GETM_RHO0));
-        if (mu == 1) {
-            const double zp = getm_fmax_i(z1, spg_bound(B0, H0, a.Dmin, D1));
-            const double zm = getm_fmax_i(z0, spg_bound(B1, H1, a.Dmin, D0));
-            const float g = getm_d2f_approx(zp - zm) + getm_d2f_approx(sp1 - sp0) * gi;
-            a.dpdx[p] = getm_f2d(g * getm_d2f_approx(idx));
-        }
-        if (mv == 1) {
-            const double zp = getm_fmax_i(zn, spg_bound(B0, H0, a.Dmin, Dn));
-            const double zm = getm_fmax_i(z0, spg_bound(Bn, Hn, a.Dmin, D0));
-            const float g = getm_d2f_approx(zp - zm) + getm_d2f_approx(spn - sp0) * gi;
-            a.dpdy[p] = getm_f2d(g * getm_d2f_approx(idy));
-        }
+        const float g = getm_d2f_approx(zp - zm) + getm_d2f_approx(sp1 - sp0) * gi;
+        out[p] = getm_f2d(g * getm_d2f_approx(id));
     } else {
         const double gammai = 1.0 / (GETM_G * GETM_RHO0);
-        if (mu == 1) {
-            const double zp = getm_fmax_i(z1, spg_bound(B0, H0, a.Dmin, D1));
-            const double zm = getm_fmax_i(z0, spg_bound(B1, H1, a.Dmin, D0));
-            a.dpdx[p] = (zp - zm + (sp1 - sp0) * gammai) * idx;
-        }
-        if (mv == 1) {
-            const double zp = getm_fmax_i(zn, spg_bound(B0, H0, a.Dmin, Dn));
-            const double zm = getm_fmax_i(z0, spg_bound(Bn, Hn, a.Dmin, D0));
-            a.dpdy[p] = (zp - zm + (spn - sp0) * gammai) * idy;
-        }
+        out[p] = (zp - zm + (sp1 - sp0) * gammai) * id;
     }
 }
 
@@ -518,9 +491,12 @@ __device__ __forceinline__ void spg_point(const SpgArgs& a, long long p)
 {
     const long long n = p + a.nx;
     // every operand is loaded before the masks are tested
-    const double H0 = a.H[p], H1 = a.H[p + 1], Hn = a.H[n];
-    spg_values<MIXED>(a, p, a.umask[p], a.vmask[p], a.z[p], a.z[p + 1], a.z[n], H0, H1, Hn, a.D[p], a.D[p + 1],
-                      a.D[n], -H0 + a.Dmin, -H1 + a.Dmin, -Hn + a.Dmin, a.sp[p], a.sp[p + 1], a.sp[n], a.idxu[p], a.idyv[p]);
+    const int mu = a.umask[p], mv = a.vmask[p];
+    const double z0 = a.z[p], z1 = a.z[p + 1], zn = a.z[n], H0 = a.H[p], H1 = a.H[p + 1], Hn = a.H[n];
+    const double D0 = a.D[p], D1 = a.D[p + 1], Dn = a.D[n], sp0 = a.sp[p], sp1 = a.sp[p + 1], spn = a.sp[n];
+    const double idx = a.idxu[p], idy = a.idyv[p], B0 = -H0 + a.Dmin;
+    spg_half<MIXED>(a.dpdx, a.Dmin, p, mu, z0, z1, H0, H1, D0, D1, B0, -H1 + a.Dmin, sp0, sp1, idx);
+    spg_half<MIXED>(a.dpdy, a.Dmin, p, mv, z0, zn, H0, Hn, D0, Dn, B0, -Hn + a.Dmin, sp0, spn, idy);
 }
 
 // interp_x / interp_y (interpolation.F90:9-40) of one point: t = mean of s

@@ -35,6 +35,7 @@
 // the word.
 #include <string.h>
 
+#include <algorithm>
 #include <mutex>
 #include <type_traits>
 
@@ -379,7 +380,7 @@ __global__ void __launch_bounds__(TR_THREADS, 2)
 // it from the old ones (zo) and the new transports in scratch, the depths at
 // T, U, V and X, and from them the velocities and the surface pressure
 // gradient of the tile's points.  z, U and V are written, never read here.
-template <bool MIXED>
+template <bool MIXED, bool SPLIT>
 __global__ void __launch_bounds__(DV_THREADS, 3)
     substep_depth_kernel(const __grid_constant__ SubstepArgs a, const int by)
 {
@@ -394,19 +395,37 @@ __global__ void __launch_bounds__(DV_THREADS, 3)
     const int i0 = blockIdx.x * 32, j0 = blockIdx.y * by;
     const double* __restrict__ Us = new_transport(a, 0);
     const double* __restrict__ Vs = new_transport(a, 1);
-    // operands of the thread's point and of its X point, loaded while the
-    // elevations are staged
-    const int ty = t / 32, tx = t % 32, i = i0 + tx, j = j0 + ty;
-    const bool own = ty < by && i < nx && j < ny;
+    // SPLIT: the first 32 by threads take the U halves of the points, the next the V
+    // halves (small planes, where one thread's chain of instructions is the
+    // time); else one thread takes both.  The operands of the thread's point and
+    // of its X point are loaded while the elevations are staged
+    const int npt = 32 * by, w = SPLIT && t >= npt ? t - npt : t;
+    const int ty = w / 32, tx = w % 32, i = i0 + tx, j = j0 + ty;
+    const bool own = w < npt && i < nx && j < ny;
     const bool east = i < nx - 1, north = j < ny - 1;
     const int p = j * nx + i;
-    int mU = 0, mV = 0;
-    double HU = 0.0, HV = 0.0, Up = 0.0, Ue = 0.0, Un = 0.0, Vp = 0.0, Ve = 0.0, Vn = 0.0;
-    if (own) {
-        mU = da.mU[p]; mV = da.mV[p]; HU = da.HU[p]; HV = da.HV[p];
-        Up = Us[p]; Vp = Vs[p];
-        if (east) { Ue = Us[p + 1]; Ve = Vs[p + 1]; }
-        if (north) { Un = Us[p + nx]; Vn = Vs[p + nx]; }
+    struct Half {
+        int m;
+        double H, T, Te, Tn;
+    };
+    auto load = [&](int h) {
+        Half o{0, 0.0, 0.0, 0.0, 0.0};
+        if (own) {
+            const double* __restrict__ Ts = h == 0 ? Us : Vs;
+            o.m = (h == 0 ? da.mU : da.mV)[p];
+            o.H = (h == 0 ? da.HU : da.HV)[p];
+            o.T = Ts[p];
+            if (east) o.Te = Ts[p + 1];
+            if (north) o.Tn = Ts[p + nx];
+        }
+        return o;
+    };
+    Half o0, o1;
+    if constexpr (SPLIT) {
+        o0 = load(t < npt ? 0 : 1);
+    } else {
+        o0 = load(0);
+        o1 = load(1);
     }
     const int xj = t / 33, xi = t - xj * 33, Xj = j0 + xj, Xi = i0 + xi;
     const bool xin = xj <= by && Xi <= nx && Xj <= ny;
@@ -463,90 +482,95 @@ __global__ void __launch_bounds__(DV_THREADS, 3)
         if (mine && mX != 0) da.DX[px] = dx;
         sX[xj][xi] = dx;
     }
-    double sp0 = 0.0, sp1 = 0.0, spn = 0.0, idx = 0.0, idy = 0.0;
-    const bool interior = own && i >= a.halox && i < nx - a.halox && j >= a.haloy && j < ny - a.haloy;
-    if (interior) {
-        sp0 = a.spg.sp[p]; sp1 = a.spg.sp[p + 1]; spn = a.spg.sp[p + nx];
-        idx = a.spg.idxu[p]; idy = a.spg.idyv[p];
-    }
     __syncthreads();
-    if (!own) return;
-    const int y = ty + 1, x = tx + 1;  // the point in the staged tile
-    const double zh = szh[y][x];
     const double twoDmin = 2 * da.Dmin;
     const float twoDmin_f = 2.f * getm_d2f_approx(da.Dmin), ialpha_f = getm_d2f_approx(da.ialpha);
-    // U: z_U = interp_x(z_T_half, ioffset 0) for i < nx-1, else the old value
-    double zu, zv, DU, DV;
-    if (east) {
-        zu = getm_half(sU[ty + 1][tx + 1]);
-        da.workU[p] = zu;
+    if (!own) return;
+    auto half = [&](int h, const Half& o) {
+        const int y = ty + 1, x = tx + 1;  // the point in the staged tile
+        // z_U = interp_x(z_T_half, ioffset 0) for i < nx-1, z_V = interp_y for
+        // j < ny-1, else the old value
+        double* work = h == 0 ? da.workU : da.workV;
+        double* Dp = h == 0 ? da.DU : da.DV;
+        double z, D;
+        if (h == 0 ? east : north) {
+            z = getm_half(h == 0 ? sU[y][x] : szh[y][x] + szh[y + 1][x]);
+            work[p] = z;
+        } else {
+            z = work[p];
+        }
+        if (o.m != 0) {
+            D = getm_fmax_i(o.H + z, da.Dmin);
+            Dp[p] = D;
+            (h == 0 ? da.alphaU : da.alphaV)[p] =
+                MIXED ? alpha_of_f(D, twoDmin_f, ialpha_f) : alpha_of(D, twoDmin, da.ialpha);
+        } else {
+            D = Dp[p];
+        }
+        a.advD[h][p] = D;
+        // UU.D[:, :-1] = D_T_half[:, 1:], VV.D[:-1, :] = D_T_half[1:, :], UV.D = VU.D = X.D[1:, 1:]
+        const double Dx = sX[ty + 1][tx + 1];
+        double Dt;
+        if (h == 0) {
+            Dt = east ? sdh[y][x + 1] : da.DUU[p];
+            if (east) da.DUU[p] = Dt;
+            da.DUV[p] = Dx;
+        } else {
+            Dt = north ? sdh[y + 1][x] : da.DVV[p];
+            if (north) da.DVV[p] = Dt;
+            da.DVU[p] = Dx;
+        }
+        momentum_2d_velocities_half<C>(a.vel, h, p, east, north, o.T, o.Te, o.Tn, D, h == 0 ? Dt : Dx, h == 0 ? Dx : Dt);
+        // the transport's final value, and what only reads it
+        a.tr[h].U[p] = o.T;
+        if (a.accumulate) {
+            double* cum = h == 0 ? a.Ucum : a.Vcum;
+            cum[p] = cum[p] + o.T;
+        }
+        if (h == 0) {
+            coriolis_from<C>(a, a.ufirst ? 1 : 0, i, j, a.ufirst ? Vs : Us);
+            if (east) interp_pair_point<double>(a.taux, a.tausx, p, 1, 0);
+        } else if (north) {
+            interp_pair_point<double>(a.tauy, a.tausy, p, nx, 0);
+        }
+        if (i >= a.halox && i < nx - a.halox && j >= a.haloy && j < ny - a.haloy) {
+            const int dx = h == 0 ? 1 : 0, dy = 1 - dx;
+            spg_half<MIXED>(h == 0 ? a.spg.dpdx : a.spg.dpdy, a.spg.Dmin, p, o.m, sz[y][x], sz[y + dy][x + dx], sH[y][x],
+                            sH[y + dy][x + dx], sD[y][x], sD[y + dy][x + dx], sB[y][x], sB[y + dy][x + dx], a.spg.sp[p],
+                            a.spg.sp[p + (h == 0 ? 1 : nx)], (h == 0 ? a.spg.idxu : a.spg.idyv)[p]);
+        }
+    };
+    if constexpr (SPLIT) {
+        half(t < npt ? 0 : 1, o0);
     } else {
-        zu = da.workU[p];
+        half(0, o0);
+        half(1, o1);
     }
-    if (mU != 0) {
-        DU = getm_fmax_i(HU + zu, da.Dmin);
-        da.DU[p] = DU;
-        da.alphaU[p] = MIXED ? alpha_of_f(DU, twoDmin_f, ialpha_f) : alpha_of(DU, twoDmin, da.ialpha);
-    } else {
-        DU = da.DU[p];
-    }
-    // V: z_V = interp_y(z_T_half, joffset 0) for j < ny-1
-    if (north) {
-        zv = getm_half(zh + szh[y + 1][x]);
-        da.workV[p] = zv;
-    } else {
-        zv = da.workV[p];
-    }
-    if (mV != 0) {
-        DV = getm_fmax_i(HV + zv, da.Dmin);
-        da.DV[p] = DV;
-        da.alphaV[p] = MIXED ? alpha_of_f(DV, twoDmin_f, ialpha_f) : alpha_of(DV, twoDmin, da.ialpha);
-    } else {
-        DV = da.DV[p];
-    }
-    // UU.D[:, :-1] = D_T_half[:, 1:], VV.D[:-1, :] = D_T_half[1:, :], UV.D = VU.D = X.D[1:, 1:]
-    const double DUU = east ? sdh[y][x + 1] : da.DUU[p], DVV = north ? sdh[y + 1][x] : da.DVV[p];
-    const double DUV = sX[ty + 1][tx + 1];
-    if (east) da.DUU[p] = DUU;
-    if (north) da.DVV[p] = DVV;
-    da.DUV[p] = DUV;
-    da.DVU[p] = DUV;
-    a.advD[0][p] = DU;
-    a.advD[1][p] = DV;
-    momentum_2d_velocities_values<C>(a.vel, p, east, north, Up, Ue, Un, Vp, Ve, Vn, DU, DV, DUU, DUV, DUV, DVV);
-    // the transports' final values, and what only reads them
-    a.tr[0].U[p] = Up;
-    a.tr[1].U[p] = Vp;
-    if (a.accumulate) accumulate_2d_point(Us, Vs, a.Ucum, a.Vcum, p);
-    coriolis_from<C>(a, a.ufirst ? 1 : 0, i, j, a.ufirst ? Vs : Us);
-    if (east) interp_pair_point<double>(a.taux, a.tausx, p, 1, 0);
-    if (north) interp_pair_point<double>(a.tauy, a.tausy, p, nx, 0);
-    if (interior)
-        spg_values<MIXED>(a.spg, p, mU, mV, sz[y][x], sz[y][x + 1], sz[y + 1][x], sH[y][x], sH[y][x + 1], sH[y + 1][x],
-                          sD[y][x], sD[y][x + 1], sD[y + 1][x], sB[y][x], sB[y][x + 1], sB[y + 1][x], sp0, sp1, spn,
-                          idx, idy);
 }
 
 // Phases 6 and 7: advection pass PASS in direction DIR of U (block z 0; d0 =
-// 0) and V.  With the first pass, the blocks share out the friction of their
-// direction's equation and fwf = pe (which phase 3 still needed): the FP64
-// form's friction takes as long as its pass, so every block gets its part.
+// 0) and V, nd of them.  With the first pass, the blocks share out the friction
+// of their direction's equation and fwf = pe (which phase 3 still needed): the
+// FP64 form's friction takes as long as its pass, so every block gets its part.
+// On small planes (early) blocks of their own, z >= nd, take it instead.
 template <bool MIXED, int PASS, int DIR, int BY>
 __global__ void __launch_bounds__(32 * BY)
-    substep_advection_kernel(const __grid_constant__ SubstepArgs a, int d0)
+    substep_advection_kernel(const __grid_constant__ SubstepArgs a, int d0, int nd)
 {
     using C = typename std::conditional<MIXED, float, double>::type;
     if (substep_begin(a)) return;
     const int tx = threadIdx.x, ty = threadIdx.y;
-    const int d = d0 + blockIdx.z;
+    const bool apart = blockIdx.z >= nd;
+    const int d = d0 + (apart ? blockIdx.z - nd : blockIdx.z);
     const HPassArgs<double>& pa = a.adv[d].pass[PASS];
-    if (PASS == 0) {
+    if (PASS == 0 && (apart || gridDim.z == nd)) {
         const int n = a.nx * a.ny, step = 32 * BY * gridDim.x * gridDim.y;
         for (int p = ((blockIdx.y * gridDim.x + blockIdx.x) * BY + ty) * 32 + tx; p < n; p += step) {
             if (d == 0) a.fwf[p] = a.pe[p];
             if (a.friction) momentum_2d_friction_half<C>(a.fric, d, p % a.nx, p / a.nx);
         }
     }
+    if (apart) return;
     if (PASS == 1 && d == 0 && blockIdx.x == 0 && blockIdx.y == 0 && tx == 0 && ty == 0 && a.time)
         *a.time = *a.time + a.dt;
     auto pass = [&](const auto& epi) {
@@ -586,19 +610,21 @@ template <bool MIXED, int PASS>
 int launch_substep_advection(const SubstepArgs& a, cudaStream_t stream, bool first = false)
 {
     const bool one = a.adv[0].dir[PASS] == a.adv[1].dir[PASS];
-    const int nd = one ? 2 : 1;
+    const int nd = one ? 2 : 1, nz = PASS == 0 && a.early ? 2 * nd : nd;
     for (int d = 0; d < 3 - nd; d++) {
         int rc;
         if (a.adv[d].dir[PASS] == 1) {
-            const dim3 g(div_up(a.nx + 1, HX_STRIDE), div_up(a.ny, PH_XY), nd);
+            const dim3 g(div_up(a.nx + 1, HX_STRIDE), div_up(a.ny, PH_XY), nz);
             rc = launch_substep(substep_advection_kernel<MIXED, PASS, 1, PH_XY>, g, dim3(32, PH_XY), first && d == 0,
-                                stream, a, d);
+                                stream, a, d, nd);
         } else {
             const int by = hpass_y_rows((long long)div_up(a.nx, 32) * nd, a.ny, !MIXED);
-            const dim3 g(div_up(a.nx, 32), div_up(a.ny + 1, by - 1), nd), b(32, by);
+            const dim3 g(div_up(a.nx, 32), div_up(a.ny + 1, by - 1), nz), b(32, by);
             const bool f = first && d == 0;
-            if (by == 16) rc = launch_substep(substep_advection_kernel<MIXED, PASS, 2, 16>, g, b, f, stream, a, d);
-            else rc = launch_substep(substep_advection_kernel<MIXED, PASS, 2, 4>, g, b, f, stream, a, d);
+            if (MIXED || by == 4)
+                rc = launch_substep(substep_advection_kernel<MIXED, PASS, 2, 4>, g, b, f, stream, a, d, nd);
+            else
+                rc = launch_substep(substep_advection_kernel<false, PASS, 2, 16>, g, b, f, stream, a, d, nd);
         }
         if (rc) return rc;
     }
@@ -629,10 +655,13 @@ int launch_substep_kernels(const SubstepArgs& a, cudaStream_t stream)
     const int tr = substep_rows(a.nx, a.ny, TR_MAX, 1, MIXED ? 4 : 2);
     const int dv = substep_rows(a.nx + 1, a.ny + 1, DV_MAX, 2, MIXED ? 4 : 2);
     const dim3 tg(div_up(a.nx, 32), div_up(a.ny, tr)), tb(div_up((tr + 1) * 33, 32) * 32);
-    const dim3 dg(div_up(a.nx + 1, 32), div_up(a.ny + 1, dv)), db(div_up((dv + 2) * 34, 32) * 32);
+    const bool split = 64 * dv <= DV_THREADS;
+    const int dt = div_up((dv + 2) * 34, 32) * 32;
+    const dim3 dg(div_up(a.nx + 1, 32), div_up(a.ny + 1, dv)), db(split ? std::max(dt, 64 * dv) : dt);
     int rc = a.ufirst ? launch_substep(substep_transport_kernel<MIXED, 0>, tg, tb, true, stream, a, tr)
                       : launch_substep(substep_transport_kernel<MIXED, 1>, tg, tb, true, stream, a, tr);
-    if (!rc) rc = launch_substep(substep_depth_kernel<MIXED>, dg, db, false, stream, a, dv);
+    if (!rc) rc = split ? launch_substep(substep_depth_kernel<MIXED, true>, dg, db, false, stream, a, dv)
+                        : launch_substep(substep_depth_kernel<MIXED, false>, dg, db, false, stream, a, dv);
     if (!rc) rc = launch_substep_advection<MIXED, 0>(a, stream);
     if (!rc) rc = launch_substep_advection<MIXED, 1>(a, stream);
     return rc;
