@@ -370,7 +370,8 @@ __device__ __forceinline__ double transport_2d_value(const TransportIn& a, doubl
         // (contracted in one way in every kernel that forms it)
         const double sum = __fma_rn(a.taus, rho0i, cor) + a.adv + a.diff + a.damp + a.SA + a.SB + a.SD + Slr;
         const double tend = __fma_rn(a.alpha, sum, __dmul_rn(__dmul_rn(-GETM_G, a.D), a.dp));
-        return getm_div(__fma_rn(dt, tend, a.U), 1.0 + getm_div(__dmul_rn(dt, a.r), a.D));
+        // (U + dt tend) / (1 + dt r / D) with one division
+        return getm_div(__dmul_rn(__fma_rn(dt, tend, a.U), a.D), __fma_rn(dt, a.r, a.D));
     } else {
         const float rho0i = (float)(1.0 / GETM_RHO0);
         const float sf = getm_d2f_approx(a.SF);
