@@ -197,6 +197,21 @@ extern "C" int getm_advance_2d_transport(int nx, int ny, int halox, int haloy, c
     return GETM_OK;
 }
 
+// A column's operands of so many levels k0, k0 + 1, ... below kend, loaded before
+// any of them is used: a thread per column is a chain of load latencies (the
+// stores between may alias as far as the compiler knows).  us level by level ->
+// in chunks, float: transport_3d_finish 40 -> 36 (400 x 300 x 40), 16 -> 10 (92 x 92 x
+// 20); w_momentum 75 -> 42, 22 -> 9; column sums of four fields 49 -> 45, 13 -> 6.
+constexpr int COL_CHUNK = 8;  // one or two operands per level
+constexpr int W_CHUNK = 4;    // six
+
+template <typename T, int N>
+__device__ __forceinline__ void col_load(T (&v)[N], const T* src, int k0, int kend, long long plane)
+{
+#pragma unroll
+    for (int u = 0; u < N; u++) v[u] = k0 + u < kend ? src[(k0 + u) * plane] : T(0);
+}
+
 // momentum.F90:191-216: thread per column; the recursion runs in FP64 for
 // both forms (T: type of pk, qk and w).
 template <typename T>
@@ -212,13 +227,25 @@ __global__ void w_momentum_3d_kernel(int nx, int ny, int nz, int ilo, int ihi, i
     long long plane = (long long)nx * ny;
     const double idt = 1.0 / dt;
     const double dyE = dyu[p], dyW = dyu[p - 1], dxN = dxv[p], dxS = dxv[p - nx], ia = iarea[p];
+    auto load = [&](int k0, auto& h1, auto& h0, auto& pe, auto& pw, auto& qn, auto& qs) {
+        col_load(h1, hn + p, k0, nz - 1, plane);
+        col_load(h0, ho + p, k0, nz - 1, plane);
+        col_load(pe, pk + p, k0, nz - 1, plane);
+        col_load(pw, pk + p - 1, k0, nz - 1, plane);
+        col_load(qn, qk + p, k0, nz - 1, plane);
+        col_load(qs, qk + p - nx, k0, nz - 1, plane);
+    };
     if constexpr (std::is_same<T, double>::value) {
         double wk = (double)w[p];
-        for (int k = 1; k <= nz - 1; k++) {
-            long long q = p + (k - 1) * plane;
-            wk = wk - (hn[q] - ho[q]) * idt
-                 - ((double)pk[q] * dyE - (double)pk[q - 1] * dyW + (double)qk[q] * dxN - (double)qk[q - nx] * dxS) * ia;
-            w[p + k * plane] = (T)wk;
+        for (int k0 = 0; k0 < nz - 1; k0 += W_CHUNK) {
+            T h1[W_CHUNK], h0[W_CHUNK], pe[W_CHUNK], pw[W_CHUNK], qn[W_CHUNK], qs[W_CHUNK];
+            load(k0, h1, h0, pe, pw, qn, qs);
+#pragma unroll
+            for (int u = 0; u < W_CHUNK; u++) {
+                if (k0 + u >= nz - 1) break;
+                wk = wk - (h1[u] - h0[u]) * idt - (pe[u] * dyE - pw[u] * dyW + qn[u] * dxN - qs[u] * dxS) * ia;
+                w[p + (k0 + u + 1) * plane] = (T)wk;
+            }
         }
     } else {
         // mixed form: the layer's increment in float (the thickness change
@@ -227,12 +254,18 @@ __global__ void w_momentum_3d_kernel(int nx, int ny, int nz, int ilo, int ihi, i
         const float dyEf = getm_d2f_approx(dyE), dyWf = getm_d2f_approx(dyW);
         const float dxNf = getm_d2f_approx(dxN), dxSf = getm_d2f_approx(dxS), iaf = getm_d2f_approx(ia);
         double wk = getm_f2d(w[p]);
-        for (int k = 1; k <= nz - 1; k++) {
-            long long q = p + (k - 1) * plane;
-            const float inc = getm_d2f_approx(hn[q] - ho[q]) * idtf +
-                              (pk[q] * dyEf - pk[q - 1] * dyWf + qk[q] * dxNf - qk[q - nx] * dxSf) * iaf;
-            wk = wk - getm_f2d(inc);
-            w[p + k * plane] = getm_d2f_approx(wk);
+        for (int k0 = 0; k0 < nz - 1; k0 += W_CHUNK) {
+            double h1[W_CHUNK], h0[W_CHUNK];
+            T pe[W_CHUNK], pw[W_CHUNK], qn[W_CHUNK], qs[W_CHUNK];
+            load(k0, h1, h0, pe, pw, qn, qs);
+#pragma unroll
+            for (int u = 0; u < W_CHUNK; u++) {
+                if (k0 + u >= nz - 1) break;
+                const float inc = getm_d2f_approx(h1[u] - h0[u]) * idtf +
+                                  (pe[u] * dyEf - pw[u] * dyWf + qn[u] * dxNf - qs[u] * dxSf) * iaf;
+                wk = wk - getm_f2d(inc);
+                w[p + (k0 + u + 1) * plane] = getm_d2f_approx(wk);
+            }
         }
     }
 }
@@ -482,20 +515,35 @@ __global__ void transport_3d_finish_kernel(long long plane, int nz, const T* __r
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= plane) return;
     double s = 0.0;
-    for (int k = 0; k < nz; k++) {
-        const long long q = p + k * plane;
-        T x;
-        if constexpr (std::is_same<T, double>::value) x = __dmul_rn(vel[q], hn[q]);
-        else x = vel[q] * getm_d2f_approx(hn[q]);
-        tp3d[q] = x;
-        s = s + getm_widen(x);
+    for (int k0 = 0; k0 < nz; k0 += COL_CHUNK) {
+        T v[COL_CHUNK];
+        double h[COL_CHUNK];
+        col_load(v, vel + p, k0, nz, plane);
+        col_load(h, hn + p, k0, nz, plane);
+#pragma unroll
+        for (int u = 0; u < COL_CHUNK; u++) {
+            if (k0 + u >= nz) break;
+            T x;
+            if constexpr (std::is_same<T, double>::value) x = __dmul_rn(v[u], h[u]);
+            else x = v[u] * getm_d2f_approx(h[u]);
+            tp3d[p + (k0 + u) * plane] = x;
+            s = s + getm_widen(x);
+        }
     }
     const double d = (s - tp2d[p]) / D[p];
     dev[p] = d;
-    for (int k = 0; k < nz; k++) {
-        const long long q = p + k * plane;
-        if constexpr (std::is_same<T, double>::value) tp3d[q] = __dsub_rn(tp3d[q], __dmul_rn(d, hn[q]));
-        else tp3d[q] = tp3d[q] - getm_d2f_approx(d) * getm_d2f_approx(hn[q]);
+    for (int k0 = 0; k0 < nz; k0 += COL_CHUNK) {
+        T v[COL_CHUNK];
+        double h[COL_CHUNK];
+        col_load(v, tp3d + p, k0, nz, plane);
+        col_load(h, hn + p, k0, nz, plane);
+#pragma unroll
+        for (int u = 0; u < COL_CHUNK; u++) {
+            if (k0 + u >= nz) break;
+            const long long q = p + (k0 + u) * plane;
+            if constexpr (std::is_same<T, double>::value) tp3d[q] = __dsub_rn(v[u], __dmul_rn(d, h[u]));
+            else tp3d[q] = v[u] - getm_d2f_approx(d) * getm_d2f_approx(h[u]);
+        }
     }
 }
 
@@ -516,7 +564,15 @@ __global__ void column_sums_kernel(long long plane, int nz, int subtract, const 
     double* dst = f == 0 ? a2 : f == 1 ? b2 : f == 2 ? c2 : d2;
     if (p >= plane || !src) return;
     double s = 0.0;
-    for (int k = 0; k < nz; k++) s = s + getm_widen(src[p + k * plane]);
+    for (int k0 = 0; k0 < nz; k0 += COL_CHUNK) {
+        T v[COL_CHUNK];
+        col_load(v, src + p, k0, nz, plane);
+#pragma unroll
+        for (int u = 0; u < COL_CHUNK; u++) {
+            if (k0 + u >= nz) break;
+            s = s + getm_widen(v[u]);
+        }
+    }
     dst[p] = subtract ? s - dst[p] : s;
 }
 

@@ -352,27 +352,33 @@ __global__ void smcw_column_mixed_kernel(int nx, int ny, int nz, int ilo, int ih
     double Pk = (B(nz) + cff) * 0.5 * h[p + (long long)(nz - 1) * P];
     Pw[p + (long long)(nz - 1) * P] = Pk;
     if (nz == 1) return;
-    double bk1 = B(nz), zk1 = Z(nz);
+    double bk1 = B(nz);
     double bk = B(nz - 1), zk = Z(nz - 1);
-    float dRk = getm_d2f_approx(bk1 - bk), dZk = getm_d2f_approx(zk1 - zk);
+    double dzk = Z(nz) - zk;  // between levels k and k + 1
+    float dRk = getm_d2f_approx(bk1 - bk), dZk = getm_d2f_approx(dzk);
     float HR1 = smcw_harm_f(dRk, dRk);
     float HZ1 = 2.f * dZk * dZk / (dZk + dZk);
+    // v(k-1), loaded one level ahead
+    double bn = nz > 2 ? B(nz - 2) : 0.0, zn = nz > 2 ? Z(nz - 2) : 0.0;
     for (int k = nz - 1; k >= 1; k--) {
         float dRm, dZm;
-        double bkm1 = 0.0, zkm1 = 0.0;
+        double dzm = 0.0;
+        const double bkm1 = bn, zkm1 = zn;
+        if (k > 2) { bn = B(k - 2); zn = Z(k - 2); }
         if (k > 1) {
-            bkm1 = B(k - 1); zkm1 = Z(k - 1);
-            dRm = getm_d2f_approx(bk - bkm1); dZm = getm_d2f_approx(zk - zkm1);
+            dzm = zk - zkm1;
+            dRm = getm_d2f_approx(bk - bkm1); dZm = getm_d2f_approx(dzm);
         } else {
             dRm = dRk; dZm = dZk;
         }
         const float HR0 = smcw_harm_f(dRk, dRm);
         const float HZ0 = 2.f * dZk * dZm / (dZk + dZm);
         const float corr = 0.2f * ((HR1 - HR0) * (dZk - x * (HZ1 + HZ0)) - (HZ1 - HZ0) * (dRk - x * (HR1 + HR0)));
-        Pk = Pk + 0.5 * ((bk1 + bk) * (zk1 - zk) - getm_f2d(corr));
+        Pk = Pk + 0.5 * ((bk1 + bk) * dzk - getm_f2d(corr));
         Pw[p + (long long)(k - 1) * P] = Pk;
         HR1 = HR0; HZ1 = HZ0;
-        bk1 = bk; zk1 = zk; bk = bkm1; zk = zkm1;
+        bk1 = bk; bk = bkm1; zk = zkm1;
+        dzk = dzm;
         dRk = dRm; dZk = dZm;
     }
 #undef B
