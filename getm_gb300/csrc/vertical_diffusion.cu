@@ -236,7 +236,7 @@ __device__ __forceinline__ void vd_f64_sweep(const VDArgs<double>& a, long long 
 
 // Blocks of 32 columns by blockDim.y rows, one field after the other (the
 // workspace a caller brings holds one field's coefficients: 2 nz planes, or NULL
-// for shared memory).
+// for shared memory), or side by side in blocks z.
 template <bool SRC>
 __global__ void __launch_bounds__(128, 5) vd_f64_kernel(VDArgs<double> a)
 {
@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(128, 5) vd_f64_kernel(VDArgs<double> a)
     if (a.mask[c] != 1) return;
     double* const ru = a.work ? a.work + c : (double*)vd_smem + threadIdx.y * 32 + threadIdx.x;
     const long long rs = a.work ? a.plane : 32 * (long long)blockDim.y;
-    for (int t = 0; t < a.ntracer; t++) vd_f64_sweep<SRC>(a, c, t, ru, ru + a.nz * rs, rs);
+    for (int t = blockIdx.z; t < a.ntracer; t += gridDim.z) vd_f64_sweep<SRC>(a, c, t, ru, ru + a.nz * rs, rs);
 }
 
 // Float solve without a workspace, thread per column; dynamic shared memory
@@ -922,12 +922,18 @@ static int vd_launch(VDArgs<float>& a, cudaStream_t stream)
 }
 
 template <bool SRC>
-static int vd_f64_launch_one(VDArgs<double>& a, int rows, size_t smem, cudaStream_t stream)
+static int vd_f64_launch_one(VDArgs<double>& a, int rows, int nz, size_t smem, cudaStream_t stream)
 {
-    if (smem > 48 * 1024 && cudaFuncSetAttribute(vd_f64_kernel<SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 200 * 1024) != cudaSuccess)
-        return GETM_ERR_CUDA;
-    const dim3 grid(getm_div_up(a.nx_, 32), getm_div_up(a.ny_, rows)), block(32, rows);
+    static bool attr_set = false;
+    if (smem > 0 && !attr_set) {
+        if (cudaFuncSetAttribute(vd_f64_kernel<SRC>, cudaFuncAttributePreferredSharedMemoryCarveout, 100) !=
+                cudaSuccess ||
+            cudaFuncSetAttribute(vd_f64_kernel<SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) !=
+                cudaSuccess)
+            return GETM_ERR_CUDA;
+        attr_set = true;
+    }
+    const dim3 grid(getm_div_up(a.nx_, 32), getm_div_up(a.ny_, rows), nz), block(32, rows);
     vd_f64_kernel<SRC><<<grid, block, smem, stream>>>(a);
     GETM_CHECK_LAUNCH();
     return GETM_OK;
@@ -939,8 +945,24 @@ static int vd_launch(VDArgs<double>& a, cudaStream_t stream)
 {
     bool src = false;
     for (int t = 0; t < a.ntracer; t++) src = src || a.ea2[t] || a.ea4[t];
+    // The fields of a batch side by side, their coefficients in shared memory
+    // instead of the workspace: where that keeps more warps on an SM than one
+    // field's columns alone (five blocks' worth, 20, at most), and where the
+    // columns do not fit at once (the last wave, of few warps, would take all
+    // fields again); up to the layers that leave room for ten warps.  us, fields in
+    // turn through the workspace -> side by side: 200 x 150 x 30 two 125 -> 119,
+    // 120 x 100 x 30 two 76 -> 53, 92 x 92 x 20 six 162 -> 68, 400 x 300 x 40 two 756
+    // -> 558, one 394 -> 319, 400 x 300 x 20 two 365 -> 267; but 300 x 200 x 30
+    // three (13 warps of columns, 14 in shared memory) 313 -> 343, 300 x 250 x 64
+    // one 342 -> 392.
+    const long long strips = getm_div_up(a.nx_, 32);
+    const double columns = (double)strips * a.ny_ / GETM_SMS;  // warps per SM
+    const double shared = fmin(224.0 * 1024 / (2.0 * a.nz * 32 * sizeof(double)), columns * a.ntracer);
+    const bool side = a.nz > 1 && a.nz <= 44 && a.ntracer > 0 && (columns > 20.0 || shared >= 1.25 * columns);
+    const int nz = side ? a.ntracer : 1;
+    if (side) a.work = nullptr;
     int rows = 4;
-    while (rows > 1 && (long long)getm_div_up(a.nx_, 32) * getm_div_up(a.ny_, rows) < 4 * GETM_SMS) rows /= 2;
+    while (rows > 1 && strips * getm_div_up(a.ny_, rows) * nz < 4 * GETM_SMS) rows /= 2;
     size_t smem = 0;
     if (!a.work && a.nz > 1) {
         const size_t per = (size_t)2 * a.nz * 32 * sizeof(double);  // per row of 32 columns
@@ -948,7 +970,7 @@ static int vd_launch(VDArgs<double>& a, cudaStream_t stream)
         smem = per * rows;
         if (smem > 200 * 1024) return GETM_ERR_NZ;
     }
-    return src ? vd_f64_launch_one<true>(a, rows, smem, stream) : vd_f64_launch_one<false>(a, rows, smem, stream);
+    return src ? vd_f64_launch_one<true>(a, rows, nz, smem, stream) : vd_f64_launch_one<false>(a, rows, nz, smem, stream);
 }
 
 extern "C" int getm_vertical_diffusion_create(getm_grid* tgrid, getm_vertical_diffusion** out)

@@ -45,6 +45,32 @@ def test_column_solve(nz, sources, storage):
     assert all(torch.equal(x.all_values, y.all_values) for x, y in zip(a, b))
 
 
+@pytest.mark.parametrize("sources", [False, True])
+@pytest.mark.parametrize("nx,ny,nz", [(40, 30, 1), (40, 30, 2), (40, 30, 44), (40, 30, 45), (700, 300, 3)])
+def test_column_solve_fp64(nx, ny, nz, sources):
+    """FP64: few columns on both sides of the layer count up to which the
+    coefficients stay in shared memory, and more columns than are resident."""
+    import torch
+
+    from getm_gb300.core import CENTERS, INTERFACES, Array
+    from getm_gb300.operators import VerticalDiffusion
+
+    _, _, Td, rng = setup(seed=nz, nx=nx, ny=ny, nz=nz)
+    n = 3
+    up = lambda lo, hi, k, z: Array(Td, torch.from_numpy(rng.uniform(lo, hi, (k, Td.ny_, Td.nx_))).cuda(), z=z)  # noqa: E731
+    nuh = up(1e-5, 1e-2, nz + 1, INTERFACES)
+    ea2 = [up(-1e-2, 0.0, nz, CENTERS) for _ in range(n)] if sources else None
+    ea4 = [up(0.0, 1e-2, nz, CENTERS) for _ in range(n)] if sources else None
+    mol = [1e-7 * (q + 1) for q in range(n)]
+    a = _fields(Td, rng, n, torch.float64)
+    b = [Array(Td, f.all_values.clone(), z=CENTERS) for f in a]
+    vd = VerticalDiffusion(Td, cnpar=0.8)
+    vd.batch(nuh, 300.0, a, mol, ea2, ea4)
+    for q in range(n):
+        vd.batch(nuh, 300.0, b[q:q + 1], mol[q:q + 1], ea2 and ea2[q:q + 1], ea4 and ea4[q:q + 1])
+    assert all(torch.equal(x.all_values, y.all_values) for x, y in zip(a, b))
+
+
 @pytest.mark.parametrize("nx,ny,nz,n", [(60, 9, 4, 3), (31, 70, 9, 5), (124, 33, 20, 2), (252, 40, 6, 9)])
 @pytest.mark.parametrize("form", ["mixed", "f32"])
 def test_advection(nx, ny, nz, n, form):
