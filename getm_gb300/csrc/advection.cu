@@ -850,15 +850,14 @@ static int launch_wpass(const WPassArgs<T, V>& a, dim3 grid, dim3 block, cudaStr
     // the staging rings (w_substep); the largest carve-out of shared memory,
     // so that they do not limit the resident warps
     constexpr size_t per = WRing<SEG, T, V>::BYTES + (SEG ? 32 * sizeof(double) : 0);  // per warp
-    static bool attributes_set = false;  // per-function attributes: once per process
-    if (!attributes_set) {
-        if (cudaFuncSetAttribute(wpass_kernel<SEG, T, V>, cudaFuncAttributePreferredSharedMemoryCarveout, 100) !=
-                cudaSuccess ||
-            cudaFuncSetAttribute(wpass_kernel<SEG, T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(W_MAXSEG * per)) != cudaSuccess)
-            return GETM_ERR_CUDA;
-        attributes_set = true;
-    }
+    static std::atomic<unsigned long long> done{0};
+    if (!getm_once_per_device(done, [] {
+            return cudaFuncSetAttribute(wpass_kernel<SEG, T, V>, cudaFuncAttributePreferredSharedMemoryCarveout, 100) ==
+                       cudaSuccess &&
+                   cudaFuncSetAttribute(wpass_kernel<SEG, T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)(W_MAXSEG * per)) == cudaSuccess;
+        }))
+        return GETM_ERR_CUDA;
     wpass_kernel<SEG, T, V><<<grid, block, block.y * per, stream>>>(a);
     GETM_CHECK_LAUNCH();
     return GETM_OK;

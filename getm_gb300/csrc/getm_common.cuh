@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include <type_traits>
 
 #include "getm_gb300.h"
@@ -59,6 +61,21 @@ extern "C" unsigned long long getm_launch_counter_add(void);
         cudaError_t e_ = cudaGetLastError();                    \
         if (e_ != cudaSuccess) return GETM_ERR_CUDA;            \
     } while (0)
+
+// Sets a kernel's attributes once per device (they belong to the device that is
+// current): done holds a bit per device, set(), which may run twice in two
+// threads, returns whether it succeeded.
+template <typename F>
+static inline bool getm_once_per_device(std::atomic<unsigned long long>& done, F set)
+{
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+    if (done.load() & bit) return true;
+    if (!set()) return false;
+    done.fetch_or(bit);
+    return true;
+}
 
 static inline unsigned int getm_div_up(long long a, long long b) { return (unsigned int)((a + b - 1) / b); }
 

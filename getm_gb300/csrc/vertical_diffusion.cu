@@ -538,13 +538,12 @@ static int vd_inc_launch_src(VDArgs<float, S>& a, cudaStream_t stream)
     const long long warps = (long long)grid.x * a.ny_;
     if (a.ntracer > 1 && a.nz <= 45 && warps <= 20 * GETM_SMS) {
         const size_t smem = (size_t)rows * 32 * a.nz * 2 * sizeof(float);  // at most 45 KB
-        static bool attr_set = false;
-        if (!attr_set) {
-            if (cudaFuncSetAttribute(vd_inc_kernel<SRC, false, true, S>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                     100) != cudaSuccess)
-                return GETM_ERR_CUDA;
-            attr_set = true;
-        }
+        static std::atomic<unsigned long long> done{0};
+        if (!getm_once_per_device(done, [] {
+                return cudaFuncSetAttribute(vd_inc_kernel<SRC, false, true, S>,
+                                            cudaFuncAttributePreferredSharedMemoryCarveout, 100) == cudaSuccess;
+            }))
+            return GETM_ERR_CUDA;
         grid.z = a.ntracer;
         vd_inc_kernel<SRC, false, true, S><<<grid, block, smem, stream>>>(a);
     } else if (a.ntracer > 1) {
@@ -924,15 +923,14 @@ static int vd_launch(VDArgs<float>& a, cudaStream_t stream)
 template <bool SRC>
 static int vd_f64_launch_one(VDArgs<double>& a, int rows, int nz, size_t smem, cudaStream_t stream)
 {
-    static bool attr_set = false;
-    if (smem > 0 && !attr_set) {
-        if (cudaFuncSetAttribute(vd_f64_kernel<SRC>, cudaFuncAttributePreferredSharedMemoryCarveout, 100) !=
-                cudaSuccess ||
-            cudaFuncSetAttribute(vd_f64_kernel<SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) !=
-                cudaSuccess)
-            return GETM_ERR_CUDA;
-        attr_set = true;
-    }
+    static std::atomic<unsigned long long> done{0};
+    if (smem > 0 && !getm_once_per_device(done, [] {
+            return cudaFuncSetAttribute(vd_f64_kernel<SRC>, cudaFuncAttributePreferredSharedMemoryCarveout, 100) ==
+                       cudaSuccess &&
+                   cudaFuncSetAttribute(vd_f64_kernel<SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        200 * 1024) == cudaSuccess;
+        }))
+        return GETM_ERR_CUDA;
     const dim3 grid(getm_div_up(a.nx_, 32), getm_div_up(a.ny_, rows), nz), block(32, rows);
     vd_f64_kernel<SRC><<<grid, block, smem, stream>>>(a);
     GETM_CHECK_LAUNCH();
