@@ -285,8 +285,8 @@ int substep_args(SubstepArgs& a, const getm_split2d_fields* f, int nx, int ny, i
 // and the FP64 pipe, which in the FP64 form is most of the time.  us per substep
 // in a CUDA graph, one cooperative launch with six grid barriers -> the seven
 // phases as seven launches -> these four:
-//   mixed  64 x 64  45 -> 27 -> 24    200 x 150  46 -> 30 -> 27    400 x 300  56 -> 51 -> 47
-//   FP64   64 x 64  56 -> 48 -> 31    150 x 120  58 -> 53 -> 38    220 x 160  68 -> 66 -> 52
+//   mixed  64 x 64  45 -> 27 -> 20    200 x 150  46 -> 30 -> 28    400 x 300  56 -> 51 -> 46
+//   FP64   64 x 64  56 -> 48 -> 26    150 x 120  58 -> 53 -> 36    220 x 160  68 -> 66 -> 52
 // A barrier cost about 1.3 us and left every SM to the slowest block, and one
 // register budget served all phases.  Each kernel but the first is launched
 // when the blocks of the one before are done (programmatic dependent launch
@@ -380,6 +380,9 @@ __global__ void __launch_bounds__(TR_THREADS, 2)
 // it from the old ones (zo) and the new transports in scratch, the depths at
 // T, U, V and X, and from them the velocities and the surface pressure
 // gradient of the tile's points.  z, U and V are written, never read here.
+// SPLIT where a block of DV_THREADS holds both halves (by <= 6): a 92 x 92 member's
+// step 904 -> 810 us with the friction in blocks of its own; on larger planes one
+// thread's two halves overlap better (mixed 400 x 300 47.9 us split, 46.5 not).
 template <bool MIXED, bool SPLIT>
 __global__ void __launch_bounds__(DV_THREADS, 3)
     substep_depth_kernel(const __grid_constant__ SubstepArgs a, const int by)
