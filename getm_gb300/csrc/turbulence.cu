@@ -108,7 +108,9 @@ __device__ __forceinline__ void keps_solve(const KepsArgs<R>& a, long long c, do
         const double t = fma(U, s, dz * fma(-a.dt, S, 1.0));
         const double r = getm_rcp(t + Un);
         const double cc = Un * r;
-        s = t * r;
+        // an infinite sink (S of a zero kinetic energy) fixes the value at zero, as
+        // a boundary would: c = 0, s = 1
+        s = ((__double2hiint(r) & 0x7fffffff) | __double2loint(r)) != 0 ? t * r : 1.0;
         double rhs = fma(U, d, dz * fma(a.dt, Q, xo));
         if (i == nz - 1) rhs = fma(Un, xn, rhs);  // (beside the substitution's own term, which starts from xn)
         d = rhs * r;
