@@ -317,7 +317,8 @@ class Simulation:
         m = self.momentum
         if ((whole and self._ob is not None) or self.runtype <= RunType.BAROTROPIC_2D or m.diffuse_momentum
                 or m.An_uu is not None or m.coriolis_scheme != CoriolisScheme.DEFAULT
-                or m.advection_split_2d != AdvectionSplit.FULL or not m.uadv.p.value or not m.vadv.p.value
+                or m.advection_split_2d != AdvectionSplit.FULL or m.uadv.split_2d != AdvectionSplit.FULL
+                or m.vadv.split_2d != AdvectionSplit.FULL or not m.uadv.p.value or not m.vadv.p.value
                 or self.T.device.type != "cuda"):
             return None
         T, U, V, X, a = self.T, self.U, self.V, self.X, self.airsea
