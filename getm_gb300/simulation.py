@@ -61,7 +61,7 @@ import enum  # noqa: E402
 from . import _lib, _pygetm  # noqa: E402
 from .domain import FILL_VALUE, GRAVITY, RHO0  # noqa: E402
 from .momentum import CoriolisScheme, Momentum  # noqa: E402
-from .operators import AdvectionSplit  # noqa: E402
+from .operators import Advection, AdvectionSplit  # noqa: E402
 
 
 class RunType(enum.IntEnum):
@@ -84,6 +84,12 @@ class Fluxes:
             a = grid.array(name=n)
             a.fill(v)
             setattr(self, n, a)
+
+
+# what the 2D substep kernels do in place of these methods
+_SUBSTEP_OPERATIONS = ("advance_surface_elevation", "update_depth", "update_surface_pressure_gradient")
+_MOMENTUM_OPERATIONS = ("advance_depth_integrated", "update_depth_integrated_diagnostics", "coriolis",
+                        "_transport_2d_momentum", "_transport_2d_momentum_fused")
 
 
 class _Split2DPlan:
@@ -296,7 +302,8 @@ class Simulation:
         if self._split2d is not None and not macro_active:
             self._split2d_substep(self._split2d)
             return
-        if not macro_active and self.fused_2d and not self.substep_kernel:
+        fused = self.fused_2d and self._stock_substep()
+        if not macro_active and fused and not self.substep_kernel:
             # the fields taken anew each time, as the operations one by one would
             plan = self._split2d_plan(self._split2d_words[0])
             if plan is not None:
@@ -305,9 +312,19 @@ class Simulation:
         _lib.call("getm_advance_time", self._time.data_ptr(), float(self.timestep),
                   torch.cuda.current_stream(self._time.device).cuda_stream)
         # the fields taken anew, as the operations one by one would
-        plan = self._split2d_plan(self._split2d_words[0], whole=False) if self.fused_2d else None
+        plan = self._split2d_plan(self._split2d_words[0], whole=False) if fused else None
         self._advance_state(macro_active, plan)
         self._update_forcing_and_diagnostics(macro_active, plan)
+
+    def _stock_substep(self) -> bool:
+        """Whether the operations that the substep kernels stand in for are this
+        package's own: one that a subclass or a host program has replaced is
+        called."""
+        m = self.momentum
+        return all(n not in vars(o) and getattr(type(o), n, None) is getattr(c, n)
+                   for o, c, names in ((self, Simulation, _SUBSTEP_OPERATIONS), (m, Momentum, _MOMENTUM_OPERATIONS),
+                                       (m.uadv, Advection, ("__call__",)), (m.vadv, Advection, ("__call__",)))
+                   for n in names)
 
     def _split2d_plan(self, words, whole: bool = True):
         """Fields of the 2D substep kernels, or None where they do not cover

@@ -1,5 +1,6 @@
 """Substeps that the fused 2D kernels must leave to the single operations: the
-momentum advections' own split."""
+momentum advections' own split, operations that a subclass or a host program has
+replaced."""
 
 import numpy as np
 import pytest
@@ -37,3 +38,32 @@ def test_split_of_the_advections(precision):
         a.advance()
         b.advance()
     _assert_same(a, b)
+
+
+@pytest.mark.parametrize("owner,name,per_substep", [
+    ("momentum", "advance_depth_integrated", 1), ("momentum", "update_depth_integrated_diagnostics", 1),
+    ("momentum", "_transport_2d_momentum_fused", 1), ("sim", "advance_surface_elevation", 1),
+    ("sim", "update_surface_pressure_gradient", 1)])
+@pytest.mark.parametrize("by", ["instance", "class"])
+def test_replaced_operations_run(owner, name, per_substep, by):
+    """An operation replaced on the object or by a subclass runs in every substep
+    of a simulation without the substep kernel, with and without a 3D step."""
+    calls = []
+
+    def replace(s):
+        o = s if owner == "sim" else s.momentum
+        own = getattr(type(o), name)
+
+        def counted(self, *a, **k):
+            calls.append(name)
+            return own(self, *a, **k)
+
+        if by == "instance":
+            setattr(o, name, counted.__get__(o))
+        else:
+            o.__class__ = type("Counting", (type(o),), {name: counted})
+
+    s = _member(prepare=replace)
+    for _ in range(6):  # the fourth with a 3D step
+        s.advance()
+    assert len(calls) >= 6 * per_substep
