@@ -180,7 +180,7 @@ __device__ __forceinline__ void hx_face(const TvdFace<float>& tf, bool up, bool 
 __device__ __forceinline__ void hx_face(const TvdFace<double>& tf, bool up, bool uu_ok, double QU, double dprev,
                                         double d, double dnext, double ahd, bool diff, double& el, double& er)
 {
-    double G = getm_negate_if(__dmul_rn(tf.half1mc, getm_tvd_phi(tf, d, uu_ok ? (up ? dprev : dnext) : 0.0)), !up);
+    double G = getm_negate_if(__dmul_rn(tf.half1mc, getm_tvd_phi(tf, QU, d, uu_ok ? (up ? dprev : dnext) : 0.0)), !up);
     if (diff) G = __fma_rn(ahd, d, G);
     const double other = __dadd_rn(G, getm_negate_if(__dmul_rn(QU, d), up));
     el = up ? G : other;

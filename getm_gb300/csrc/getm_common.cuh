@@ -446,17 +446,19 @@ __device__ __forceinline__ float getm_tvd_dev_c(const TvdFace<float>& tf, float 
 // half1mc; signs, doublings, minima and maxima on the integer pipe (superbee
 // needs no FP64 instruction at all).  Differences of opposite signs give zero,
 // and where one of them is zero every limiter does.  Infinities and NaNs go
-// through the ratio, out of line.
-static __device__ __noinline__ double getm_tvd_phi_hw(int scheme, double half1mc, double deltaf, double deltafu)
+// through the ratio, out of line, with the Courant number that half1mc holds
+// (times the face's transport QU, as hx_tvd leaves it).
+static __device__ __noinline__ double getm_tvd_phi_hw(int scheme, double half1mc, double QU, double deltaf, double deltafu)
 {
-    return deltaf * deltafu > 0.0 ? getm_limiter<double>(scheme, deltafu / deltaf, 1.0 - 2.0 * half1mc) * deltaf : 0.0;
+    const double cfl = QU != 0.0 ? 1.0 - 2.0 * half1mc / QU : 0.0;
+    return deltaf * deltafu > 0.0 ? getm_limiter<double>(scheme, deltafu / deltaf, cfl) * deltaf : 0.0;
 }
 
-__device__ __forceinline__ double getm_tvd_phi(const TvdFace<double>& tf, double deltaf, double deltafu)
+__device__ __forceinline__ double getm_tvd_phi(const TvdFace<double>& tf, double QU, double deltaf, double deltafu)
 {
     const int hd = __double2hiint(deltaf), hu = __double2hiint(deltafu);
     const int ha = hd & 0x7fffffff, hb = hu & 0x7fffffff;
-    if (ha >= 0x7ff00000 || hb >= 0x7ff00000) return getm_tvd_phi_hw(tf.scheme, tf.half1mc, deltaf, deltafu);
+    if (ha >= 0x7ff00000 || hb >= 0x7ff00000) return getm_tvd_phi_hw(tf.scheme, tf.half1mc, QU, deltaf, deltafu);
     if ((hd ^ hu) < 0) return 0.0;
     const double a = __hiloint2double(ha, __double2loint(deltaf)), b = __hiloint2double(hb, __double2loint(deltafu));
     double pa;
