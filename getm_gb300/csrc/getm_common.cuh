@@ -252,7 +252,8 @@ __device__ __forceinline__ double getm_div_refined(double num, double den)
 // 1 / x in FP64 to within two units in the last place with three FP64
 // instructions: the approximate reciprocal r of PTX (rcp.approx.ftz.f64,
 // relative error e about 2^-20, not on the FP64 pipe) and one third-order
-// Householder step, r (1 + e + e^2) with e = 1 - x r, whose own error is e^3.
+// Householder step (Householder 1970, The Numerical Treatment of a Single
+// Nonlinear Equation), r (1 + e + e^2) with e = 1 - x r, whose own error is e^3.
 // GB300 runs FP64 at 1/64 of its float rate and the correctly rounded
 // division takes several times as many FP64 instructions, so this serves
 // where a quotient only scales an increment.  Zero, subnormal, huge and
@@ -270,9 +271,10 @@ __device__ __forceinline__ double getm_rcp(double x)
 }
 
 // n / d in FP64 with six FP64 instructions: n getm_rcp(d) and one correction by
-// its own remainder, which leaves an error of half a unit in the last place
-// and less than 2^-6 of one beside it (the correctly rounded division takes
-// about twice as many).  Operands or quotients near the ends of the range,
+// its own remainder, formed exactly by a fused multiply-add (Markstein 1990, IBM
+// J. Res. Dev. 34, 111-119), which leaves an error of half a unit in the last
+// place and less than 2^-6 of one beside it (the correctly rounded division
+// takes about twice as many).  Operands or quotients near the ends of the range,
 // infinities and NaNs: the division, out of line.
 static __device__ __noinline__ double getm_div_hw(double n, double d) { return n / d; }
 
