@@ -1083,11 +1083,13 @@ static int advection_2d_impl(getm_advection* adv, getm_grid* tgrid, getm_grid* u
     if (rc) return rc;
     if ((rc = hpass_setup(ay, 2, adv, tgrid, vgrid, 1, v, Ah_v, timestep, DV, increment))) return rc;
     const size_t n2 = (size_t)ax.plane;
-    if ((rc = adv_reserve(adv, n2, 2))) return rc;
+    if ((rc = adv_reserve(adv, n2, 1))) return rc;
     HPassArgs<double>* p1 = ufirst ? &ax : &ay;
     HPassArgs<double>* p2 = ufirst ? &ay : &ax;
     const int d1 = ufirst ? 1 : 2, d2 = ufirst ? 2 : 1;
-    double* const* T = adv->tmp;
+    // (the vertical pass's work array, idle here, is the second buffer: a handle
+    // that a call with one field has sized allocates nothing more)
+    double* const T[2] = {adv->tmp[0], adv->colbuf[1]};
     double* A = adv->hbuf[0];
     double* B = adv->hbuf[1];
     const double* fin[1];
