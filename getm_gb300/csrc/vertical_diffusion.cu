@@ -549,6 +549,27 @@ __global__ void __launch_bounds__(128, 7) vd_inc_kernel(VDArgs<float, S> a)
     }
 }
 
+// Whether the fields of a batch may be swept side by side: none lies in memory
+// that the sweep of another one reads or writes (a field given twice, or as
+// another's source: those are swept in turn).
+template <typename T, typename S>
+static bool vd_fields_apart(const VDArgs<T, S>& a)
+{
+    const size_t n = (size_t)a.plane * a.nz;
+    for (int t = 0; t < a.ntracer; t++) {
+        const char* const f = (const char*)a.var[t];
+        auto apart = [&](const void* q, size_t bytes) {
+            return !q || f + n * sizeof(S) <= (const char*)q || (const char*)q + bytes <= f;
+        };
+        if (!apart(a.nuh, (n + a.plane) * sizeof(T)) || !apart(a.ho, n * sizeof(double)) || !apart(a.hn, n * sizeof(double)))
+            return false;
+        for (int s = 0; s < a.ntracer; s++)
+            if (s != t && !(apart(a.var[s], n * sizeof(S)) && apart(a.ea2[s], n * sizeof(T)) && apart(a.ea4[s], n * sizeof(T))))
+                return false;
+    }
+    return true;
+}
+
 template <bool SRC, typename S>
 static int vd_inc_launch_src(VDArgs<float, S>& a, cudaStream_t stream)
 {
@@ -562,7 +583,7 @@ static int vd_inc_launch_src(VDArgs<float, S>& a, cudaStream_t stream)
     // eight 155 -> 79 (pairs side by side 118); 300 x 250 x 25 two 60 -> 52; but
     // 400 x 300 x 40 two (26 warps) 133 -> 164, and one field alone 75 -> 103.
     const long long warps = (long long)grid.x * a.ny_;
-    if (a.ntracer > 1 && a.nz <= 45 && warps <= 20 * GETM_SMS) {
+    if (a.ntracer > 1 && a.nz <= 45 && warps <= 20 * GETM_SMS && vd_fields_apart(a)) {
         const size_t smem = (size_t)rows * 32 * a.nz * 2 * sizeof(float);  // at most 45 KB
         static std::atomic<unsigned long long> done{0};
         if (!getm_once_per_device(done, [] {
@@ -982,7 +1003,8 @@ static int vd_launch(VDArgs<double>& a, cudaStream_t stream)
     const long long strips = getm_div_up(a.nx_, 32);
     const double columns = (double)strips * a.ny_ / GETM_SMS;  // warps per SM
     const double shared = fmin(224.0 * 1024 / (2.0 * a.nz * 32 * sizeof(double)), columns * a.ntracer);
-    const bool side = a.nz > 1 && a.nz <= 44 && a.ntracer > 0 && (columns > 20.0 || shared >= 1.25 * columns);
+    const bool side = a.nz > 1 && a.nz <= 44 && a.ntracer > 0 && (columns > 20.0 || shared >= 1.25 * columns) &&
+                      (a.ntracer == 1 || vd_fields_apart(a));
     const int nz = side ? a.ntracer : 1;
     if (side) a.work = nullptr;
     int rows = 4;
