@@ -531,7 +531,7 @@ __device__ __forceinline__ void w_face(const TvdFace<double>& tf, double W, doub
 
 __device__ __forceinline__ TvdFace<float> w_tvd(int scheme, float W, float dt, float itersm1, float h0, float h1)
 {
-    const float cfl = fabsf(W) * dt / fminf(h0, h1) * itersm1;
+    const float cfl = __fmul_rn(fabsf(W) * dt / fminf(h0, h1), itersm1);
     return getm_tvd_face_c(scheme, cfl);
 }
 

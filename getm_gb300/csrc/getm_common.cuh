@@ -382,30 +382,31 @@ struct TvdFace {
     C rcoef, cap;  // P2_PDM: 2 / (cfl + 1e-10), 2 / (1 - cfl)
 };
 
+// Both forms: every product and sum rounded as written (intrinsics where the
+// compiler could contract), so that all kernels that share these functions, and
+// every shape of one kernel, give the same bits.
 __device__ __forceinline__ TvdFace<float> getm_tvd_face_c(int scheme, float cfl)
 {
     TvdFace<float> f;
     f.scheme = scheme;
-    f.half1mc = 0.5f * (1.f - cfl);
+    f.half1mc = 0.5f * __fadd_rn(1.f, -cfl);
     f.lin0 = f.lin1 = 0.f;
     f.rcoef = f.cap = 2.f;
     if (scheme == GETM_SCHEME_HSIMT) {
-        const float kappa = 1.f - cfl;
-        const float x = 0.25f * (kappa - 1.f / 3.f / kappa);
+        const float kappa = __fadd_rn(1.f, -cfl);
+        const float x = 0.25f * (kappa - 1.f / 3.f / kappa);  // (0.25 is exact)
         f.lin0 = 0.5f + x;
         f.lin1 = 0.5f - x;
     } else if (scheme == GETM_SCHEME_P2_PDM) {
-        const float x = 1.f / 6.f * (1.f - 2.f * cfl);
-        f.lin0 = 0.5f + x;
-        f.lin1 = 0.5f - x;
-        f.rcoef = 2.f / (cfl + 1.e-10f);
-        f.cap = 2.f / (1.f - cfl);
+        const float t = __fmaf_rn(-2.f, cfl, 1.f);
+        f.lin0 = __fmaf_rn(1.f / 6.f, t, 0.5f);
+        f.lin1 = __fmaf_rn(-1.f / 6.f, t, 0.5f);
+        f.rcoef = 2.f / __fadd_rn(cfl, 1.e-10f);
+        f.cap = 2.f / __fadd_rn(1.f, -cfl);
     }
     return f;
 }
 
-// FP64: every product and sum rounded as written (no contraction), so that
-// all kernels that share these functions give the same bits.
 __device__ __forceinline__ TvdFace<double> getm_tvd_face_c(int scheme, double cfl)
 {
     TvdFace<double> f;
@@ -434,9 +435,13 @@ __device__ __forceinline__ float getm_tvd_dev_c(const TvdFace<float>& tf, float 
     const float a = fabsf(deltaf), b = fabsf(deltafu);
     float pa;
     switch (tf.scheme) {
-    case GETM_SCHEME_HSIMT: pa = fminf(fminf(2.f * b, fmaxf(0.f, tf.lin0 * a + tf.lin1 * b)), 2.f * a); break;
+    case GETM_SCHEME_HSIMT:
+        pa = fminf(fminf(2.f * b, fmaxf(0.f, __fmaf_rn(tf.lin0, a, __fmul_rn(tf.lin1, b)))), 2.f * a);
+        break;
     case GETM_SCHEME_MUSCL: pa = fminf(fminf(2.f * b, 0.5f * (a + b)), 2.f * a); break;
-    case GETM_SCHEME_P2_PDM: pa = fminf(fminf(tf.rcoef * b, tf.lin0 * a + tf.lin1 * b), tf.cap * a); break;
+    case GETM_SCHEME_P2_PDM:
+        pa = fminf(fminf(tf.rcoef * b, __fmaf_rn(tf.lin0, a, __fmul_rn(tf.lin1, b))), tf.cap * a);
+        break;
     case GETM_SCHEME_SPLMAX13: pa = fminf(fminf(2.f * b, 1.f / 3.f * fmaxf(a + 2.f * b, 2.f * a + b)), 2.f * a); break;
     case GETM_SCHEME_SUPERBEE: pa = fmaxf(fminf(2.f * b, a), fminf(b, 2.f * a)); break;
     default: pa = 0.f; break;
