@@ -956,11 +956,12 @@ static int vd_launch(VDArgs<float>& a, cudaStream_t stream)
     while (threads > 32 && per * threads > 160 * 1024) threads /= 2;
     size_t smem = per * threads;
     if (smem > 200 * 1024) return GETM_ERR_NZ;
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaFuncSetAttribute(vd_column_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        attr_set = true;
-    }
+    static std::atomic<unsigned long long> done{0};
+    if (!getm_once_per_device(done, [] {
+            return cudaFuncSetAttribute(vd_column_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) ==
+                   cudaSuccess;
+        }))
+        return GETM_ERR_CUDA;
     dim3 grid(getm_div_up(a.nx_, threads), a.ny_);
     vd_column_kernel<<<grid, threads, smem, stream>>>(a);
     GETM_CHECK_LAUNCH();
