@@ -80,9 +80,10 @@ __device__ __forceinline__ KepsIn keps_load(const KepsArgs<R>& a, long long q)
 // dz_i (x_i' - x_i) / dt = flux differences + dz_i (Q_i + S_i x_i'), S <= 0,
 // diffusivities at the layers (between interfaces) the mean of num over sigma,
 // Dirichlet values x0, xn at interfaces 0 and nz.  src(in, x, Q, S): the old
-// value and the sources; fin(x): the new value's bound.
+// value and the sources; fin(x): the new value's bound.  (x is a.tke or a.eps,
+// which keps_load reads: not restrict)
 template <typename R, typename Src, typename Fin>
-__device__ __forceinline__ void keps_solve(const KepsArgs<R>& a, long long c, double* __restrict__ x, double sigma,
+__device__ __forceinline__ void keps_solve(const KepsArgs<R>& a, long long c, double* x, double sigma,
                                            double x0, double xn, Src src, Fin fin)
 {
     const long long P = a.plane;
