@@ -13,13 +13,27 @@
 // so one block takes a plane (of one level and tracer) through all boundaries
 // in the reference's order, with a block barrier between them, and one launch
 // does them all (a shelf sea's six boundaries: elevation 6 x 4.7 -> 15 us, eight
-// tracers of 20 levels 6 x 20 -> 20 us).
+// tracers of 20 levels 6 x 20 -> 20 us).  A boundary longer than a block's points
+// would go round the block's threads again and again on one SM: it gets a launch
+// of its own, its points spread over blocks (ob_launches).
 #include <math.h>
+
+#include <algorithm>
 
 #include "getm_common.cuh"
 
 #define OB_THREADS 128
-#define OB_BLOCK 256  // threads of a block that takes a plane through the boundaries
+// Most points of a boundary that one block takes with others, and its threads.
+// us for six boundaries, one launch each / all in one block per plane (elevation,
+// of 256 threads: Flather, clamped; tracers, a thread per point: two clamped,
+// two and eight with sponges, 20 levels):
+//   240 points   16.9, 10.2; 11.4, 37.9, 116  /  15.9, 5.3; 4.3, 24, 37
+//   400 points   16.9, 10.2; 11.6, 40, 127    /  26, 8.4; 4.6, 32, 52
+//   1000 points  16.9, 10.2; 11.9, 48, 152    /  56, 15; 6.0, 67, 133
+// The elevation is bound by one SM's FP64 pipe (square root and quotient), the
+// sponges by its loads and stores.
+#define OB_BLOCK 256
+#define OB_TRACER_BLOCK 512
 
 namespace {
 
@@ -32,7 +46,7 @@ struct ObRanges {
 };
 
 // elevation at the boundary points (open_boundaries.py:338-416), clipped to its
-// minimum Dmin - H (simulation.py:580-582); one block
+// minimum Dmin - H (simulation.py:580-582); one block for several boundaries
 __global__ void __launch_bounds__(OB_BLOCK)
     ob_elevation_kernel(ObRanges r, int nx, const int* bi, const int* bj, const int* type, const int* di,
                         const int* dj, const int* side, const double* sign, const double* H, const double* Dclip,
@@ -41,7 +55,7 @@ __global__ void __launch_bounds__(OB_BLOCK)
 {
     for (int b = 0; b < r.n; b++) {
         if (b > 0) __syncthreads();
-        for (int p = r.start[b] + threadIdx.x; p < r.stop[b]; p += OB_BLOCK) {
+        for (int p = r.start[b] + blockIdx.x * blockDim.x + threadIdx.x; p < r.stop[b]; p += gridDim.x * blockDim.x) {
             const long long q = (long long)bj[p] * nx + bi[p];
             double v;
             switch (type[p]) {
@@ -72,7 +86,7 @@ __global__ void __launch_bounds__(OB_BLOCK)
 }
 
 // tracer values at the boundary points for every level (grid x) and tracer (grid
-// y) of the batch (ZeroGradient, Clamped; Sponge also relaxes the n points
+// y; grid z: a single boundary's points) of the batch (ZeroGradient, Clamped; Sponge also relaxes the n points
 // inward: v += sp_m (bdy - v), sp_m = ((n - m) / (n + 1))^2, only where the
 // mask is 1, open_boundaries.py:235-336 without flow-dependent relaxation)
 template <typename T>
@@ -88,13 +102,13 @@ struct ObTracerArgs {
 };
 
 template <typename T>
-__global__ void __launch_bounds__(OB_BLOCK) ob_tracer_kernel(const __grid_constant__ ObTracerArgs<T> a)
+__global__ void __launch_bounds__(OB_TRACER_BLOCK) ob_tracer_kernel(const __grid_constant__ ObTracerArgs<T> a)
 {
     const int k = blockIdx.x, t = blockIdx.y;
     T* f = a.var[t];
     for (int b = 0; b < a.r.n; b++) {
         if (b > 0) __syncthreads();
-        for (int p = a.r.start[b] + threadIdx.x; p < a.r.stop[b]; p += OB_BLOCK) {
+        for (int p = a.r.start[b] + blockIdx.z * blockDim.x + threadIdx.x; p < a.r.stop[b]; p += gridDim.z * blockDim.x) {
             const long long q = (long long)a.bj[p] * a.nx + a.bi[p] + k * a.plane;
             const int ty = a.type[p];
             if (ty == 1) {
@@ -213,6 +227,28 @@ static int ob_ranges(ObRanges& r, int nrange, const int* ranges, int np)
     return GETM_OK;
 }
 
+// The boundaries in launches, in order: as many at a time as have up to `most`
+// points each, a longer one by itself; launch(ranges, points of the longest).
+template <typename F>
+static int ob_launches(const ObRanges& r, int most, F launch)
+{
+    auto points = [&](int b) { return r.stop[b] - r.start[b]; };
+    for (int b = 0; b < r.n;) {
+        ObRanges g;
+        g.n = 0;
+        int longest = 0;
+        do {
+            g.start[g.n] = r.start[b];
+            g.stop[g.n++] = r.stop[b];
+            longest = std::max(longest, points(b));
+        } while (++b < r.n && longest <= most && points(b) <= most);
+        if (longest == 0) continue;
+        const int rc = launch(g, longest);
+        if (rc) return rc;
+    }
+    return GETM_OK;
+}
+
 extern "C" int getm_open_boundary_tide(int np, int nconstituent, const double* om, const double* const* amp,
                                        const double* const* phase, const double* time, double* z, cudaStream_t stream)
 {
@@ -245,10 +281,13 @@ extern "C" int getm_open_boundary_elevations(int nrange, const int* ranges, int 
     const void* ptrs[] = {i, j, type, di, dj, side, inflow_sign, H, Dclip, U, V, z_ext, flow_ext, z};
     for (const void* q : ptrs)
         if (!q) return GETM_ERR_ARG;
-    ob_elevation_kernel<<<1, OB_BLOCK, 0, stream>>>(r, nx, i, j, type, di, dj, side, inflow_sign, H, Dclip, U, V,
-                                                    z_ext, flow_ext, Dmin, z);
-    GETM_CHECK_LAUNCH();
-    return GETM_OK;
+    return ob_launches(r, OB_BLOCK, [&](const ObRanges& g, int longest) {
+        const bool alone = longest > OB_BLOCK;
+        ob_elevation_kernel<<<alone ? getm_div_up(longest, OB_THREADS) : 1, alone ? OB_THREADS : OB_BLOCK, 0, stream>>>(
+            g, nx, i, j, type, di, dj, side, inflow_sign, H, Dclip, U, V, z_ext, flow_ext, Dmin, z);
+        GETM_CHECK_LAUNCH();
+        return GETM_OK;
+    });
 }
 
 extern "C" int getm_open_boundary_elevation(int start, int stop, int nx, const int* i, const int* j,
@@ -284,9 +323,14 @@ static int ob_tracer_impl(int nrange, const int* ranges, int np, int nx, int ny,
         a.var[t] = vars[t];
         a.bdy[t] = bdy[t];
     }
-    ob_tracer_kernel<T><<<dim3(nz, ntracer), OB_BLOCK, 0, stream>>>(a);
-    GETM_CHECK_LAUNCH();
-    return GETM_OK;
+    return ob_launches(ObRanges(a.r), OB_TRACER_BLOCK, [&](const ObRanges& g, int longest) {
+        a.r = g;
+        const bool alone = longest > OB_TRACER_BLOCK;
+        const int threads = alone ? OB_BLOCK : std::max(OB_BLOCK, (longest + 31) / 32 * 32);
+        ob_tracer_kernel<T><<<dim3(nz, ntracer, alone ? getm_div_up(longest, OB_BLOCK) : 1), threads, 0, stream>>>(a);
+        GETM_CHECK_LAUNCH();
+        return GETM_OK;
+    });
 }
 
 extern "C" int getm_open_boundary_tracers(int start, int stop, int np, int nx, int ny, int nz, int nsponge,
