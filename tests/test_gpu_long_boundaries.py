@@ -96,3 +96,22 @@ def test_elevations(lengths):
     _lib.call("getm_open_boundary_elevations", nb, (ctypes.c_int * (2 * nb))(*ranges), n, nx, *[t.data_ptr() for t in up], 0.02,
               zd.data_ptr(), _s())
     assert np.abs(zd.cpu().numpy() - want).max() <= 6 * 1.2e-16 * 2.0
+
+
+@pytest.mark.parametrize("n", [1536, 1537, 2500])
+def test_mirror(n):
+    """Pairs on both sides of the number that one block holds."""
+    import torch
+
+    from getm_gb300 import _lib
+    from getm_gb300._pygetm import _s
+
+    rng = np.random.default_rng(n)
+    f = torch.from_numpy(rng.standard_normal((2, 6000))).cuda()
+    src = rng.permutation(6000)[:n].astype(np.int32)
+    tgt = np.roll(src, 1)
+    want = f.clone()
+    want[:, torch.from_numpy(tgt).long()] = f[:, torch.from_numpy(src).long()]
+    ds, dt, work = torch.from_numpy(src).cuda(), torch.from_numpy(tgt).cuda(), torch.empty(2 * n, dtype=f.dtype, device="cuda")
+    _lib.call("getm_mirror", n, ds.data_ptr(), dt.data_ptr(), 2, 6000, f.data_ptr(), work.data_ptr(), _s())
+    assert torch.equal(f, want)
