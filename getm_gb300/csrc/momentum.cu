@@ -200,10 +200,10 @@ extern "C" int getm_advance_2d_transport(int nx, int ny, int halox, int haloy, c
 // A column's operands of so many levels k0, k0 + 1, ... below kend, loaded before
 // any of them is used: a thread per column is a chain of load latencies (the
 // stores between may alias as far as the compiler knows).  us level by level ->
-// in chunks, float: transport_3d_finish 40 -> 36 (400 x 300 x 40), 16 -> 10 (92 x 92 x
-// 20); w_momentum 75 -> 42, 22 -> 9; column sums of four fields 49 -> 45, 13 -> 6.
-constexpr int COL_CHUNK = 8;  // one or two operands per level
-constexpr int W_CHUNK = 4;    // six
+// in chunks of four, float: transport_3d_finish 25.4 -> 21.7 (400 x 300 x 40), 9.2 ->
+// 6.7 (150 x 120 x 20); w_momentum 27.6 -> 11.1 (64 x 64 x 40), 15.6 -> 8.4 (240 x
+// 200 x 20).
+constexpr int COL_CHUNK = 4;
 
 template <typename T, int N>
 __device__ __forceinline__ void col_load(T (&v)[N], const T* src, int k0, int kend, long long plane)
@@ -214,7 +214,7 @@ __device__ __forceinline__ void col_load(T (&v)[N], const T* src, int k0, int ke
 
 // momentum.F90:191-216: thread per column; the recursion runs in FP64 for
 // both forms (T: type of pk, qk and w).
-template <typename T>
+template <typename T, int N>
 __global__ void w_momentum_3d_kernel(int nx, int ny, int nz, int ilo, int ihi, int jlo, int jhi,
                                      const int* __restrict__ mask, const double* __restrict__ dyu, const double* __restrict__ dxv,
                                      const double* __restrict__ iarea, const double* __restrict__ ho, const double* __restrict__ hn,
@@ -237,11 +237,11 @@ __global__ void w_momentum_3d_kernel(int nx, int ny, int nz, int ilo, int ihi, i
     };
     if constexpr (std::is_same<T, double>::value) {
         double wk = (double)w[p];
-        for (int k0 = 0; k0 < nz - 1; k0 += W_CHUNK) {
-            T h1[W_CHUNK], h0[W_CHUNK], pe[W_CHUNK], pw[W_CHUNK], qn[W_CHUNK], qs[W_CHUNK];
+        for (int k0 = 0; k0 < nz - 1; k0 += N) {
+            T h1[N], h0[N], pe[N], pw[N], qn[N], qs[N];
             load(k0, h1, h0, pe, pw, qn, qs);
 #pragma unroll
-            for (int u = 0; u < W_CHUNK; u++) {
+            for (int u = 0; u < N; u++) {
                 if (k0 + u >= nz - 1) break;
                 wk = wk - (h1[u] - h0[u]) * idt - (pe[u] * dyE - pw[u] * dyW + qn[u] * dxN - qs[u] * dxS) * ia;
                 w[p + (k0 + u + 1) * plane] = (T)wk;
@@ -254,12 +254,12 @@ __global__ void w_momentum_3d_kernel(int nx, int ny, int nz, int ilo, int ihi, i
         const float dyEf = getm_d2f_approx(dyE), dyWf = getm_d2f_approx(dyW);
         const float dxNf = getm_d2f_approx(dxN), dxSf = getm_d2f_approx(dxS), iaf = getm_d2f_approx(ia);
         double wk = getm_f2d(w[p]);
-        for (int k0 = 0; k0 < nz - 1; k0 += W_CHUNK) {
-            double h1[W_CHUNK], h0[W_CHUNK];
-            T pe[W_CHUNK], pw[W_CHUNK], qn[W_CHUNK], qs[W_CHUNK];
+        for (int k0 = 0; k0 < nz - 1; k0 += N) {
+            double h1[N], h0[N];
+            T pe[N], pw[N], qn[N], qs[N];
             load(k0, h1, h0, pe, pw, qn, qs);
 #pragma unroll
-            for (int u = 0; u < W_CHUNK; u++) {
+            for (int u = 0; u < N; u++) {
                 if (k0 + u >= nz - 1) break;
                 const float inc = getm_d2f_approx(h1[u] - h0[u]) * idtf +
                                   (pe[u] * dyEf - pw[u] * dyWf + qn[u] * dxNf - qs[u] * dxSf) * iaf;
@@ -278,7 +278,17 @@ static int w_momentum_impl(int nx, int ny, int nz, int imin, int imax, int jmin,
     if (nx < 1 || ny < 1 || nz < 1 || imin < 2 || jmin < 2 || imax > nx || jmax > ny || jmax < jmin) return GETM_ERR_ARG;
     if (!mask || !dyu || !dxv || !iarea || !ho || !hn || !pk || !qk || !w) return GETM_ERR_ARG;
     const unsigned grid = getm_div_up((long long)nx * (jmax - jmin + 1), 128);
-    w_momentum_3d_kernel<T><<<grid, 128, 0, stream>>>(nx, ny, nz, imin - 1, imax - 1, jmin - 1, jmax - 1, mask, dyu, dxv, iarea, ho, hn, pk, qk, dt, w);
+    auto run = [&](auto kernel) {
+        kernel<<<grid, 128, 0, stream>>>(nx, ny, nz, imin - 1, imax - 1, jmin - 1, jmax - 1, mask, dyu, dxv, iarea, ho, hn, pk, qk, dt, w);
+    };
+    // six operands a level: four levels at once where few columns leave registers to
+    // spare, else one at a time (its operands still before its store).  us, one /
+    // four: 64 x 64 x 40 FP64 18.8 / 13.7, float 14.6 / 11.1; 240 x 200 x 20 16.1 /
+    // 16.0, 9.2 / 8.4; 400 x 300 x 20 38.1 / 39.8, 13.4 / 17.0; 1000 x 800 x 5
+    // 50 / 62, 27 / 47
+    const bool few = (long long)nx * ny <= 16 * 32 * GETM_SMS && nz > COL_CHUNK;
+    if (few) run(w_momentum_3d_kernel<T, COL_CHUNK>);
+    else run(w_momentum_3d_kernel<T, 1>);
     GETM_CHECK_LAUNCH();
     return GETM_OK;
 }
@@ -508,20 +518,20 @@ extern "C" int getm_bottom_shear_velocity(int nx, int ny, int imin, int imax, in
 // array operations (products and differences not contracted); the sum runs
 // bottom to top.  Mixed form (T float): the products in float from the
 // thickness narrowed on the integer pipe.
-template <typename T>
+template <typename T, int N>
 __global__ void transport_3d_finish_kernel(long long plane, int nz, const T* __restrict__ vel, const double* __restrict__ hn,
                                            const double* __restrict__ tp2d, const double* __restrict__ D, T* __restrict__ tp3d, double* __restrict__ dev)
 {
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= plane) return;
     double s = 0.0;
-    for (int k0 = 0; k0 < nz; k0 += COL_CHUNK) {
-        T v[COL_CHUNK];
-        double h[COL_CHUNK];
+    for (int k0 = 0; k0 < nz; k0 += N) {
+        T v[N];
+        double h[N];
         col_load(v, vel + p, k0, nz, plane);
         col_load(h, hn + p, k0, nz, plane);
 #pragma unroll
-        for (int u = 0; u < COL_CHUNK; u++) {
+        for (int u = 0; u < N; u++) {
             if (k0 + u >= nz) break;
             T x;
             if constexpr (std::is_same<T, double>::value) x = __dmul_rn(v[u], h[u]);
@@ -532,13 +542,13 @@ __global__ void transport_3d_finish_kernel(long long plane, int nz, const T* __r
     }
     const double d = (s - tp2d[p]) / D[p];
     dev[p] = d;
-    for (int k0 = 0; k0 < nz; k0 += COL_CHUNK) {
-        T v[COL_CHUNK];
-        double h[COL_CHUNK];
+    for (int k0 = 0; k0 < nz; k0 += N) {
+        T v[N];
+        double h[N];
         col_load(v, tp3d + p, k0, nz, plane);
         col_load(h, hn + p, k0, nz, plane);
 #pragma unroll
-        for (int u = 0; u < COL_CHUNK; u++) {
+        for (int u = 0; u < N; u++) {
             if (k0 + u >= nz) break;
             const long long q = p + (k0 + u) * plane;
             if constexpr (std::is_same<T, double>::value) tp3d[q] = __dsub_rn(v[u], __dmul_rn(d, h[u]));
@@ -550,8 +560,9 @@ __global__ void transport_3d_finish_kernel(long long plane, int nz, const T* __r
 // Column sums of up to four 3D fields into 2D FP64 fields (the slow terms of
 // momentum.py:989-1012 and simulation.py:1186-1192): dst = sum_k src
 // (- dst when subtract is set), summed bottom to top in FP64; NULL pairs are
-// skipped.
-template <typename T>
+// skipped.  N: levels loaded at once (the FP64 form needs no more than the
+// compiler's own unrolling).
+template <typename T, int N>
 __global__ void column_sums_kernel(long long plane, int nz, int subtract, const T* __restrict__ a3,
                                    double* __restrict__ a2, const T* __restrict__ b3, double* __restrict__ b2,
                                    const T* __restrict__ c3, double* __restrict__ c2, const T* __restrict__ d3,
@@ -564,13 +575,17 @@ __global__ void column_sums_kernel(long long plane, int nz, int subtract, const 
     double* dst = f == 0 ? a2 : f == 1 ? b2 : f == 2 ? c2 : d2;
     if (p >= plane || !src) return;
     double s = 0.0;
-    for (int k0 = 0; k0 < nz; k0 += COL_CHUNK) {
-        T v[COL_CHUNK];
-        col_load(v, src + p, k0, nz, plane);
+    if constexpr (N == 1) {
+        for (int k = 0; k < nz; k++) s = s + getm_widen(src[p + k * plane]);
+    } else {
+        for (int k0 = 0; k0 < nz; k0 += N) {
+            T v[N];
+            col_load(v, src + p, k0, nz, plane);
 #pragma unroll
-        for (int u = 0; u < COL_CHUNK; u++) {
-            if (k0 + u >= nz) break;
-            s = s + getm_widen(v[u]);
+            for (int u = 0; u < N; u++) {
+                if (k0 + u >= nz) break;
+                s = s + getm_widen(v[u]);
+            }
         }
     }
     dst[p] = subtract ? s - dst[p] : s;
@@ -583,8 +598,13 @@ static int column_sums_impl(int nx, int ny, int nz, int subtract, const T* a3, d
     if (nx < 1 || ny < 1 || nz < 1) return GETM_ERR_ARG;
     if (!a3 != !a2 || !b3 != !b2 || !c3 != !c2 || !d3 != !d2) return GETM_ERR_ARG;
     const long long plane = (long long)nx * ny;
-    column_sums_kernel<T><<<dim3(getm_div_up(plane, 128), 4), 128, 0, stream>>>(plane, nz, subtract, a3, a2, b3, b2,
-                                                                                 c3, c2, d3, d2);
+    auto run = [&](auto kernel) {
+        kernel<<<dim3(getm_div_up(plane, 128), 4), 128, 0, stream>>>(plane, nz, subtract, a3, a2, b3, b2, c3, c2, d3, d2);
+    };
+    // us level by level / eight at once, float: 64 x 64 x 20 5.5 / 3.0, 240 x 200 x 40
+    // 20.3 / 16.7; 1000 x 800 x 2 14.4 / 17.3; FP64 64 x 64 x 20 2.7 / 2.9
+    if (std::is_same<T, float>::value && nz > 2) run(column_sums_kernel<T, 8>);
+    else run(column_sums_kernel<T, 1>);
     GETM_CHECK_LAUNCH();
     return GETM_OK;
 }
@@ -634,7 +654,12 @@ static int transport_3d_finish_impl(int nx, int ny, int nz, const T* vel, const 
 {
     if (nx < 1 || ny < 1 || nz < 1 || !vel || !hn || !tp2d || !D || !tp3d || !dev) return GETM_ERR_ARG;
     const long long plane = (long long)nx * ny;
-    transport_3d_finish_kernel<T><<<getm_div_up(plane, 128), 128, 0, stream>>>(plane, nz, vel, hn, tp2d, D, tp3d, dev);
+    auto run = [&](auto kernel) {
+        kernel<<<getm_div_up(plane, 128), 128, 0, stream>>>(plane, nz, vel, hn, tp2d, D, tp3d, dev);
+    };
+    // (three levels: 1000 x 800 FP64 33.6 us one at a time, 39.4 as a part of a chunk)
+    if (nz >= COL_CHUNK) run(transport_3d_finish_kernel<T, COL_CHUNK>);
+    else run(transport_3d_finish_kernel<T, 1>);
     GETM_CHECK_LAUNCH();
     return GETM_OK;
 }
