@@ -312,40 +312,53 @@ extern "C" int getm_w_momentum_3d_f32(int nx, int ny, int nz, int imin, int imax
 }
 
 // momentum.F90:218-241 (T: type of uk, vk, SS and of the arithmetic).  The shear
-// across a face serves the points on both sides, so each is formed once: a
-// warp covers 31 columns and the face west of them (the west shear comes by
-// shuffle), and marches up to eight rows north, the north shear of one row
-// being the south shear of the next.  FP64 (the FP64 pipe is the time): 127 ->
-// 64 us on 200 x 150 x 30, its quotients by getm_div; float, bound by the
-// instructions that narrow the thicknesses: 70 -> 56 us on 400 x 300 x 40.
-
-template <typename T>
+// across a face serves the points on both sides, so each is formed once: SEG
+// lanes cover SEG - 1 columns and the face west of them (the west shear comes by
+// shuffle), and march up to eight rows north, the north shear of one row being
+// the south shear of the next.  A point's own four shears -> this, us: FP64 (the
+// FP64 pipe is the time; quotients by getm_div) 200 x 150 x 30 85 -> 49, 4 x 2000 x 10
+// 19 -> 11 (32 lanes a group 40); float (bound by the instructions that narrow
+// the thicknesses) 400 x 300 x 40 71 -> 51.  Faces that no point asks for are not
+// divided: on land without thickness the division is the slow one, and with a
+// fifth of 200 x 150 x 30 such land all faces took 112 us, these 83 (95 before).
+template <typename T, int SEG>
 __global__ void __launch_bounds__(128)
     shear_frequency_kernel(int nx, int ny, int nz, int ilo, int ihi, int jlo, int jhi, const int* __restrict__ mask,
                            const double* __restrict__ hu, const double* __restrict__ hv, const T* __restrict__ uk,
                            const T* __restrict__ vk, T* __restrict__ SS, int rows)
 {
-    const int lane = threadIdx.x;
+    constexpr int groups = 32 / SEG;
+    const int c = threadIdx.x % SEG, g = threadIdx.x / SEG;
     const int k = blockIdx.z + 1;  // Fortran interface k = 1..nz-1
-    const int i = ilo - 1 + blockIdx.x * 31 + lane;
-    const int j0 = jlo + (blockIdx.y * blockDim.y + threadIdx.y) * rows;
-    if (j0 > jhi) return;  // whole warp
-    const int j1 = min(j0 + rows - 1, jhi);
-    const int ic = i <= ihi ? i : ihi;  // (idle lanes repeat the last column)
+    const int i = ilo - 1 + blockIdx.x * (SEG - 1) + c;
+    const int jw = jlo + (blockIdx.y * blockDim.y + threadIdx.y) * groups * rows, j0 = jw + g * rows;
+    if (jw > jhi) return;  // whole warp
+    const bool column = c > 0 && i <= ihi;
+    const int ic = i <= ihi ? i : ihi;  // (idle lanes repeat the last column, idle groups the last row)
     const long long plane = (long long)nx * ny;
-    auto shear = [&](const T* __restrict__ v, const double* __restrict__ h, long long p) -> T {
+    auto asked = [&](int j, int r) { return column && r < rows && j <= jhi && mask[(long long)j * nx + ic] > 0; };
+    auto shear = [&](const T* __restrict__ v, const double* __restrict__ h, long long p, bool any) -> T {
         const long long a = p + (k - 1) * plane, b = p + k * plane;
-        if constexpr (std::is_same<T, double>::value) return getm_div(v[b] - v[a], getm_half(h[b] + h[a]));
-        else return (v[b] - v[a]) / (T(0.5) * (getm_d2f_approx(h[b]) + getm_d2f_approx(h[a])));
+        const T dv = v[b] - v[a];
+        if constexpr (std::is_same<T, double>::value) {
+            const double hm = getm_half(h[b] + h[a]);
+            return any ? getm_div(dv, hm) : 0.0;
+        } else {
+            return dv / (T(0.5) * (getm_d2f_approx(h[b]) + getm_d2f_approx(h[a])));
+        }
     };
-    T t4 = shear(vk, hv, (long long)(j0 - 1) * nx + ic);
+    bool own = asked(j0, 0);
+    T t4 = shear(vk, hv, (long long)(min(j0, jhi) - 1) * nx + ic, own);
 #pragma unroll 2
-    for (int j = j0; j <= j1; j++) {
-        const long long p = (long long)j * nx + ic;
-        const T t1 = shear(uk, hu, p), t3 = shear(vk, hv, p);
-        const T t2 = __shfl_up_sync(0xffffffffu, t1, 1);
-        if (lane > 0 && i <= ihi && mask[p] > 0) SS[p + k * plane] = T(0.5) * (t1 * t1 + t2 * t2 + t3 * t3 + t4 * t4);
+    for (int r = 0; r < rows; r++) {
+        const long long p = (long long)min(j0 + r, jhi) * nx + ic;
+        const bool next = asked(j0 + r + 1, r + 1);
+        const bool east = __shfl_down_sync(0xffffffffu, own, 1, SEG);
+        const T t1 = shear(uk, hu, p, own || east), t3 = shear(vk, hv, p, own || next);
+        const T t2 = __shfl_up_sync(0xffffffffu, t1, 1, SEG);
+        if (own) SS[p + k * plane] = T(0.5) * (t1 * t1 + t2 * t2 + t3 * t3 + t4 * t4);
         t4 = t3;
+        own = next;
     }
 }
 
@@ -357,15 +370,28 @@ static int shear_impl(int nx, int ny, int nz, int imin, int imax, int jmin, int 
     if (!mask || !hu || !hv || !uk || !vk || !SS) return GETM_ERR_ARG;
     if (nz < 2) return GETM_OK;
     if (imax < imin) return GETM_OK;
-    // rows per warp: fewer where the warps would not hide a march's latencies
+    const int width = imax - imin + 1, height = jmax - jmin + 1;
+    // lanes per group of columns: fewer where that leaves a tenth fewer of them
+    // idle (33 columns: 64 lanes in two groups of 32, 40 in five of eight)
+    auto lanes = [&](int n) { return getm_div_up(width, n - 1) * n; };
+    int seg = 32;
+    for (int n = 16; n >= 4; n /= 2)
+        if (10 * lanes(n) < 9 * lanes(seg)) seg = n;
+    // rows per group: fewer where the warps would not hide a march's latencies
     // (92 x 92 x 20 float with eight rows 25 us, with one 7 us; the FP64 pipe is
     // busy with few)
-    const long long strips = (long long)getm_div_up(imax - imin + 1, 31) * (nz - 1);
+    const long long strips = (long long)lanes(seg) * (nz - 1);
     int rows = 8;
-    while (rows > 1 && strips * getm_div_up(jmax - jmin + 1, rows) < (std::is_same<T, double>::value ? 16 : 64) * GETM_SMS)
+    while (rows > 1 && strips * getm_div_up(height, rows) < (std::is_same<T, double>::value ? 16 : 64) * 32 * GETM_SMS)
         rows /= 2;
-    const dim3 block(32, 4), grid(getm_div_up(imax - imin + 1, 31), getm_div_up(jmax - jmin + 1, 4 * rows), nz - 1);
-    shear_frequency_kernel<T><<<grid, block, 0, stream>>>(nx, ny, nz, imin - 1, imax - 1, jmin - 1, jmax - 1, mask, hu, hv, uk, vk, SS, rows);
+    const dim3 block(32, 4), grid(getm_div_up(width, seg - 1), getm_div_up(height, 4 * (32 / seg) * rows), nz - 1);
+    auto run = [&](auto kernel) {
+        kernel<<<grid, block, 0, stream>>>(nx, ny, nz, imin - 1, imax - 1, jmin - 1, jmax - 1, mask, hu, hv, uk, vk, SS, rows);
+    };
+    if (seg == 32) run(shear_frequency_kernel<T, 32>);
+    else if (seg == 16) run(shear_frequency_kernel<T, 16>);
+    else if (seg == 8) run(shear_frequency_kernel<T, 8>);
+    else run(shear_frequency_kernel<T, 4>);
     GETM_CHECK_LAUNCH();
     return GETM_OK;
 }
