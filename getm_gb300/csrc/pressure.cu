@@ -213,7 +213,7 @@ __global__ void smcw_gradient_kernel(int nx, int ny, int nz, int ilo, int ihi, i
     }
 }
 
-// Phase 2 in FP64, on 32 x SG_BY tiles of SG_KB levels.  Bound by FP64
+// Phase 2 in FP64, on 32 x BY tiles of kb levels.  Bound by FP64
 // instructions: the harmonic means (two per point and direction, shared by the
 // two faces beside the point) take six each instead of two divisions' worth
 // per face, and the raw differences are formed once; the surface term and the
@@ -223,37 +223,38 @@ __global__ void smcw_gradient_kernel(int nx, int ny, int nz, int ilo, int ihi, i
 constexpr int SG_BX = 32, SG_BY = 8;
 constexpr int SG_KB = 4;
 
-__global__ void __launch_bounds__(SG_BX* SG_BY, 3) smcw_gradient_f64_kernel(
+template <int BY>
+__global__ void __launch_bounds__(SG_BX* BY, 24 / BY) smcw_gradient_f64_kernel(
     int nx, int ny, int nz, int ilo, int ihi, int jlo, int jhi, const int* __restrict__ umask,
     const int* __restrict__ vmask, const double* __restrict__ idxu, const double* __restrict__ idyv,
     const double* __restrict__ h, const double* __restrict__ z, const double* __restrict__ zc,
     const double* __restrict__ buoy, const double* __restrict__ Pw, double* __restrict__ idpdx,
-    double* __restrict__ idpdy)
+    double* __restrict__ idpdy, int kb)
 {
     // raw differences across the x faces of columns i0-1 .. i0+SG_BX and the y
-    // faces of rows j0-1 .. j0+SG_BY (zero where the mask is not positive);
-    // harmonic means at columns i0 .. i0+SG_BX and rows j0 .. j0+SG_BY
-    __shared__ double dZx[SG_BY][SG_BX + 2], dRx[SG_BY][SG_BX + 2], dZy[SG_BY + 2][SG_BX], dRy[SG_BY + 2][SG_BX];
-    __shared__ double hZx[SG_BY][SG_BX + 1], hRx[SG_BY][SG_BX + 1], hZy[SG_BY + 1][SG_BX], hRy[SG_BY + 1][SG_BX];
+    // faces of rows j0-1 .. j0+BY (zero where the mask is not positive);
+    // harmonic means at columns i0 .. i0+SG_BX and rows j0 .. j0+BY
+    __shared__ double dZx[BY][SG_BX + 2], dRx[BY][SG_BX + 2], dZy[BY + 2][SG_BX], dRy[BY + 2][SG_BX];
+    __shared__ double hZx[BY][SG_BX + 1], hRx[BY][SG_BX + 1], hZy[BY + 1][SG_BX], hRy[BY + 1][SG_BX];
     const int tx = threadIdx.x, ty = threadIdx.y;
-    const int i0 = blockIdx.x * SG_BX, j0 = jlo + blockIdx.y * SG_BY;
+    const int i0 = blockIdx.x * SG_BX, j0 = jlo + blockIdx.y * BY;
     const int i = i0 + tx, j = j0 + ty;
     const long long P = (long long)nx * ny;
     const long long p = (long long)j * nx + i;
     const bool rowin = j <= jhi, colin = i >= ilo && i <= ihi;
     // this thread's own faces, and the extra ones: x faces at columns i0-1 and
     // i0+SG_BX of every row by the last warp (lane 2r + side: row r), y faces at
-    // rows j0-1 (ty 0) and j0+SG_BY (ty 1)
+    // rows j0-1 (ty 0) and j0+BY (ty 1)
     const bool fx = rowin && i >= ilo - 1 && i <= ihi + 1 && umask[p] > 0;
     const bool fy = colin && j <= jhi + 1 && vmask[p] > 0;
     const int er = tx >> 1, eside = tx & 1;
     const long long ep = (long long)(j0 + er) * nx + (eside == 0 ? i0 - 1 : i0 + SG_BX);
     bool ex = false, ey = false;
-    if (ty == SG_BY - 1 && tx < 2 * SG_BY) {
+    if (ty == BY - 1 && tx < 2 * BY) {
         const int ii = eside == 0 ? i0 - 1 : i0 + SG_BX;
         ex = j0 + er <= jhi && ii >= ilo - 1 && ii <= ihi + 1 && umask[ep] > 0;
     }
-    const int jj = ty == 0 ? j0 - 1 : j0 + SG_BY;
+    const int jj = ty == 0 ? j0 - 1 : j0 + BY;
     const long long yp = (long long)jj * nx + i;
     if (ty < 2) ey = colin && jj <= jhi + 1 && vmask[yp] > 0;
     const bool ux = rowin && colin && umask[p] == 1, vy = rowin && colin && vmask[p] == 1;
@@ -267,24 +268,24 @@ __global__ void __launch_bounds__(SG_BX* SG_BY, 3) smcw_gradient_f64_kernel(
         surfy = (z[p + nx] - z[p]) * getm_half(buoy[qtop + nx] + buoy[qtop]);
         iy = idyv[p];
     }
-    const int kend = min(nz, ((int)blockIdx.z + 1) * SG_KB);
-    for (int k = blockIdx.z * SG_KB; k < kend; k++) {
+    const int kend = min(nz, ((int)blockIdx.z + 1) * kb);
+    for (int k = blockIdx.z * kb; k < kend; k++) {
         const long long kP = (long long)k * P, q = p + kP;
         double rzx = 0.0, rrx = 0.0, rzy = 0.0, rry = 0.0;
         if (fx) { rzx = zc[q + 1] - zc[q]; rrx = buoy[q + 1] - buoy[q]; }
         if (fy) { rzy = zc[q + nx] - zc[q]; rry = buoy[q + nx] - buoy[q]; }
-        if (k > (int)blockIdx.z * SG_KB) __syncthreads();  // the previous level's reads are done
+        if (k > (int)blockIdx.z * kb) __syncthreads();  // the previous level's reads are done
         dZx[ty][tx + 1] = rzx; dRx[ty][tx + 1] = rrx;
         dZy[ty + 1][tx] = rzy; dRy[ty + 1][tx] = rry;
-        if (ty == SG_BY - 1 && tx < 2 * SG_BY) {
+        if (ty == BY - 1 && tx < 2 * BY) {
             const long long eq = ep + kP;
             dZx[er][eside == 0 ? 0 : SG_BX + 1] = ex ? zc[eq + 1] - zc[eq] : 0.0;
             dRx[er][eside == 0 ? 0 : SG_BX + 1] = ex ? buoy[eq + 1] - buoy[eq] : 0.0;
         }
         if (ty < 2) {
             const long long yq = yp + kP;
-            dZy[ty == 0 ? 0 : SG_BY + 1][tx] = ey ? zc[yq + nx] - zc[yq] : 0.0;
-            dRy[ty == 0 ? 0 : SG_BY + 1][tx] = ey ? buoy[yq + nx] - buoy[yq] : 0.0;
+            dZy[ty == 0 ? 0 : BY + 1][tx] = ey ? zc[yq + nx] - zc[yq] : 0.0;
+            dRy[ty == 0 ? 0 : BY + 1][tx] = ey ? buoy[yq + nx] - buoy[yq] : 0.0;
         }
         __syncthreads();
         hZx[ty][tx] = smcw_harm_cut_d(dZx[ty][tx], rzx);
@@ -292,10 +293,10 @@ __global__ void __launch_bounds__(SG_BX* SG_BY, 3) smcw_gradient_f64_kernel(
         hZy[ty][tx] = smcw_harm_cut_d(dZy[ty][tx], rzy);
         hRy[ty][tx] = smcw_harm_cut_d(dRy[ty][tx], rry);
         if (ty == 0) {  // the row north of the tile
-            hZy[SG_BY][tx] = smcw_harm_cut_d(dZy[SG_BY][tx], dZy[SG_BY + 1][tx]);
-            hRy[SG_BY][tx] = smcw_harm_cut_d(dRy[SG_BY][tx], dRy[SG_BY + 1][tx]);
+            hZy[BY][tx] = smcw_harm_cut_d(dZy[BY][tx], dZy[BY + 1][tx]);
+            hRy[BY][tx] = smcw_harm_cut_d(dRy[BY][tx], dRy[BY + 1][tx]);
         }
-        if (ty == 1 && tx < 2 * SG_BY) {  // the column east of it: lane 2r + (0: heights, 1: buoyancy)
+        if (ty == 1 && tx < 2 * BY) {  // the column east of it: lane 2r + (0: heights, 1: buoyancy)
             const double(*d)[SG_BX + 2] = eside == 0 ? dZx : dRx;
             (eside == 0 ? hZx : hRx)[er][SG_BX] = smcw_harm_cut_d(d[er][SG_BX], d[er][SG_BX + 1]);
         }
@@ -533,10 +534,18 @@ static int smcw_impl(int nx, int ny, int nz, int imin, int imax, int jmin, int j
     smcw_column_kernel<T><<<g1, 128, 0, stream>>>(nx, ny, nz, imin - 1, imax - 1, jmin - 1, jmax - 1, mask, h, zc, buoy, P_work);
     GETM_CHECK_LAUNCH();
     if constexpr (std::is_same<T, double>::value) {
-        dim3 g2(getm_div_up(nx, SG_BX), getm_div_up(jmax - jmin + 1, SG_BY), getm_div_up(nz, SG_KB));
-        smcw_gradient_f64_kernel<<<g2, dim3(SG_BX, SG_BY), 0, stream>>>(nx, ny, nz, imin - 1, imax - 1, jmin - 1,
-                                                                        jmax - 1, umask, vmask, idxu, idyv, h, z, zc,
-                                                                        buoy, P_work, idpdx, idpdy);
+        // half the rows and one level per block where whole tiles would leave the FP64
+        // pipes to a few blocks' levels in turn.  us of both launches, whole tiles / these:
+        // 10 x 10 x 5 31.3 / 13.8, 64 x 64 x 2 18.4 / 10.6, 400 x 300 x 4 113 / 102; but
+        // 251 x 187 x 33 308 / 317
+        auto run = [&](auto kernel, int by, int kb) {
+            const dim3 g2(getm_div_up(nx, SG_BX), getm_div_up(jmax - jmin + 1, by), getm_div_up(nz, kb));
+            kernel<<<g2, dim3(SG_BX, by), 0, stream>>>(nx, ny, nz, imin - 1, imax - 1, jmin - 1, jmax - 1, umask, vmask, idxu,
+                                                       idyv, h, z, zc, buoy, P_work, idpdx, idpdy, kb);
+        };
+        const long long tiles = (long long)getm_div_up(nx, SG_BX) * getm_div_up(jmax - jmin + 1, SG_BY) * getm_div_up(nz, SG_KB);
+        if (tiles < 6 * GETM_SMS) run(smcw_gradient_f64_kernel<SG_BY / 2>, SG_BY / 2, 1);
+        else run(smcw_gradient_f64_kernel<SG_BY>, SG_BY, SG_KB);
     } else {
         dim3 g2(getm_div_up(nx, 128), jmax - jmin + 1, nz);
         smcw_gradient_kernel<T><<<g2, 128, 0, stream>>>(nx, ny, nz, imin - 1, imax - 1, jmin - 1, jmax - 1, umask, vmask, idxu, idyv, h, z, zc, buoy, P_work, idpdx, idpdy);
