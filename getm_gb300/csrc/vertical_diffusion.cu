@@ -352,11 +352,11 @@ __global__ void __launch_bounds__(128, 8) vd_column_kernel(VDArgs<float> a)
 // field of the group has ea2 or ea4 (without, no registers are spent on
 // them).
 // coef, rs: the thread's coefficients of the surface level and their stride.
-// Pairs, which run on domains of many columns only, also ask for the operands of
+// Pairs (domains of many columns) also ask for the operands of
 // the level VD_AHEAD levels further into the cache: their streams come from
 // DRAM, and one level ahead does not cover that (400 x 300 x 40, two FP64-stored
 // fields, 134 -> 118 us; where one field sweeps alone the extra instructions
-// cost 5 %).
+// cost 5 %, and two float fields with sources gain nothing).
 constexpr int VD_AHEAD = 3;
 
 template <typename T>
@@ -524,7 +524,8 @@ __device__ __forceinline__ void vd_inc_sweep(const VDArgs<float, S>& a, long lon
 // Blocks of 32 columns by GETM_TUNE_COLUMN_ROWS rows.  S: storage type of
 // the fields (float, or double for FP64 tracer storage).  SM (and not
 // PAIRS): the coefficients in shared memory and each field in blocks of its own
-// (grid z); else in the global workspace, fields or pairs one after the other.
+// (grid z); else in the global workspace, pairs one after the other, or single
+// fields in as many blocks (grid z) as the workspace holds fields.
 template <bool SRC, bool PAIRS, bool SM, typename S>
 __global__ void __launch_bounds__(128, 7) vd_inc_kernel(VDArgs<float, S> a)
 {
@@ -542,10 +543,11 @@ __global__ void __launch_bounds__(128, 7) vd_inc_kernel(VDArgs<float, S> a)
         float* coef = reinterpret_cast<float*>(vd_smem) + threadIdx.y * 32 + threadIdx.x;
         vd_inc_sweep<1, SRC, S>(a, c, blockIdx.z, coef, 32 * blockDim.y);
     } else {
-        int t0 = 0;
+        int t0 = blockIdx.z;
         if constexpr (PAIRS)
             for (; t0 + 2 <= a.ntracer; t0 += 2) vd_inc_sweep<2, SRC, S>(a, c, t0, a.work + c, a.plane);
-        for (; t0 < a.ntracer; t0++) vd_inc_sweep<1, SRC, S>(a, c, t0, a.work + c, a.plane);
+        float* coef = a.work + c + (long long)blockIdx.z * 2 * a.nz * a.plane;
+        for (; t0 < a.ntracer; t0 += gridDim.z) vd_inc_sweep<1, SRC, S>(a, c, t0, coef, a.plane);
     }
 }
 
@@ -583,7 +585,8 @@ static int vd_inc_launch_src(VDArgs<float, S>& a, cudaStream_t stream)
     // eight 155 -> 79 (pairs side by side 118); 300 x 250 x 25 two 60 -> 52; but
     // 400 x 300 x 40 two (26 warps) 133 -> 164, and one field alone 75 -> 103.
     const long long warps = (long long)grid.x * a.ny_;
-    if (a.ntracer > 1 && a.nz <= 45 && warps <= 20 * GETM_SMS && vd_fields_apart(a)) {
+    const bool side = a.ntracer > 1 && warps <= 20 * GETM_SMS && vd_fields_apart(a);
+    if (side && a.nz <= 45) {
         const size_t smem = (size_t)rows * 32 * a.nz * 2 * sizeof(float);  // at most 45 KB
         static std::atomic<unsigned long long> done{0};
         if (!getm_once_per_device(done, [] {
@@ -593,6 +596,13 @@ static int vd_inc_launch_src(VDArgs<float, S>& a, cudaStream_t stream)
             return GETM_ERR_CUDA;
         grid.z = a.ntracer;
         vd_inc_kernel<SRC, false, true, S><<<grid, block, smem, stream>>>(a);
+    } else if (side && warps <= 10 * GETM_SMS) {
+        // more layers, up to ten warps per SM: through the workspace, which holds two
+        // fields' coefficients.  us, pairs in turn -> these: 64 x 48 x 60 two
+        // float fields 81 -> 50, with sources 105 -> 52, FP64-stored 96 -> 57; 200 x
+        // 150 x 60 FP64-stored 108 -> 80
+        grid.z = 2;
+        vd_inc_kernel<SRC, false, false, S><<<grid, block, 0, stream>>>(a);
     } else if (a.ntracer > 1) {
         vd_inc_kernel<SRC, true, false, S><<<grid, block, 0, stream>>>(a);
     } else {
