@@ -997,7 +997,7 @@ static int vd_f64_launch_one(VDArgs<double>& a, int rows, int nz, size_t smem, c
 
 // FP64 form: blocks of fewer rows where four would leave SMs without work (an
 // SM's FP64 pipe is the bound, so the columns are spread over all).
-static int vd_launch(VDArgs<double>& a, cudaStream_t stream)
+static int vd_launch(VDArgs<double> a, cudaStream_t stream)
 {
     bool src = false;
     for (int t = 0; t < a.ntracer; t++) src = src || a.ea2[t] || a.ea4[t];
