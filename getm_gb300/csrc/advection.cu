@@ -277,7 +277,7 @@ static int launch_hpass_c(int direction, HPassArgs<S, V>& a, cudaStream_t stream
             while (nrow > 1 && (chunks(nrow / 2) * 97 <= chunks(4) * 100 ||
                                 (long long)getm_div_up(a.ny_, nrow) * a.nk * npair < 16 * GETM_SMS))
                 nrow /= 2;
-            block.y = rows < 2 ? rows : 2;
+            block.y = rows < 2 || getm_div_up(a.ny_, 2 * nrow) > 65535 ? rows : 2;  // (a grid's most blocks)
             dim3 grid(npair, getm_div_up(getm_div_up(a.ny_, nrow), block.y), a.nk);
             if constexpr (!f64) hpass_x_vec_kernel<S, V><<<grid, block, 0, stream>>>(a, nrow);
         } else {
@@ -293,10 +293,8 @@ static int launch_hpass_c(int direction, HPassArgs<S, V>& a, cudaStream_t stream
         // geometry per pair and had blocks for 90 of 152 SMs on 173 x 131 x 23
         const int by = hpass_y_rows((long long)getm_div_up(a.nx_, 32) * a.nk, a.ny_, f64);
         const dim3 block(32, by), grid(getm_div_up(a.nx_, 32), getm_div_up(a.ny_ + 1, by - 1), a.nk);
-        if constexpr (f64) {
-            if (by == 16) hpass_y_inc_kernel<S, V, C, 16><<<grid, block, 0, stream>>>(a);
-        }
-        if (by == 4) hpass_y_inc_kernel<S, V, C, 4><<<grid, block, 0, stream>>>(a);
+        if (by == 16) hpass_y_inc_kernel<S, V, C, 16><<<grid, block, 0, stream>>>(a);
+        else hpass_y_inc_kernel<S, V, C, 4><<<grid, block, 0, stream>>>(a);
     } else {
         // rows a warp marches: the knob's, halved (to four at least, which
         // repeats one face in four) until there are 64 warps per SM: a warp's

@@ -564,10 +564,11 @@ constexpr int HY_STRIDE = HY_BY - 1;
 // blocks all the same, for 16 rows repeat less at the edges.  us with 16 / 8 / 4
 // rows, FP64 2D advection 97 x 75 22.8 / 18.7 / 18.7, 400 x 300 37.2 / 37.6 / 37.6;
 // 2D substep FP64 64 x 64 38.6 / 33.0 / 30.6, 220 x 160 54.4 / 57.4 / 52.5, mixed
-// 400 x 300 48.6 / 47.6 / 47.0.
+// 400 x 300 48.6 / 47.6 / 47.0.  16 also where a grid's 65535 blocks of 4 rows do
+// not reach.
 inline int hpass_y_rows(long long tiles, int ny, bool f64)
 {
-    return f64 && tiles * ((ny + 15) / 15) > 2 * GETM_SMS ? 16 : 4;
+    return (f64 && tiles * ((ny + 15) / 15) > 2 * GETM_SMS) || ny >= 3 * 65535 ? 16 : 4;
 }
 
 template <typename S, typename C = float, int BY = HY_BY>

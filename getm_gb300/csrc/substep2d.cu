@@ -621,10 +621,10 @@ int launch_substep_advection(const SubstepArgs& a, cudaStream_t stream, bool fir
             rc = launch_substep(substep_advection_kernel<MIXED, PASS, 1, PH_XY>, g, dim3(32, PH_XY), first && d == 0,
                                 stream, a, d, nd);
         } else {
-            const int by = hpass_y_rows((long long)div_up(a.nx, 32) * nd, a.ny, !MIXED);
+            const int by = MIXED ? 4 : hpass_y_rows((long long)div_up(a.nx, 32) * nd, a.ny, true);
             const dim3 g(div_up(a.nx, 32), div_up(a.ny + 1, by - 1), nz), b(32, by);
             const bool f = first && d == 0;
-            if (MIXED || by == 4)
+            if (by == 4)
                 rc = launch_substep(substep_advection_kernel<MIXED, PASS, 2, 4>, g, b, f, stream, a, d, nd);
             else
                 rc = launch_substep(substep_advection_kernel<false, PASS, 2, 16>, g, b, f, stream, a, d, nd);
