@@ -213,7 +213,8 @@ __device__ __forceinline__ void col_load(T (&v)[N], const T* src, int k0, int ke
 }
 
 // momentum.F90:191-216: thread per column; the recursion runs in FP64 for
-// both forms (T: type of pk, qk and w).
+// both forms (T: type of pk, qk and w).  N: levels loaded at once; multiply-adds
+// contracted in one way for every N.
 template <typename T, int N>
 __global__ void w_momentum_3d_kernel(int nx, int ny, int nz, int ilo, int ihi, int jlo, int jhi,
                                      const int* __restrict__ mask, const double* __restrict__ dyu, const double* __restrict__ dxv,
@@ -243,7 +244,9 @@ __global__ void w_momentum_3d_kernel(int nx, int ny, int nz, int ilo, int ihi, i
 #pragma unroll
             for (int u = 0; u < N; u++) {
                 if (k0 + u >= nz - 1) break;
-                wk = wk - (h1[u] - h0[u]) * idt - (pe[u] * dyE - pw[u] * dyW + qn[u] * dxN - qs[u] * dxS) * ia;
+                double s = __fma_rn(pe[u], dyE, -__dmul_rn(pw[u], dyW));
+                s = __fma_rn(-qs[u], dxS, __fma_rn(qn[u], dxN, s));
+                wk = __fma_rn(-s, ia, __fma_rn(-(h1[u] - h0[u]), idt, wk));
                 w[p + (k0 + u + 1) * plane] = (T)wk;
             }
         }
@@ -261,8 +264,9 @@ __global__ void w_momentum_3d_kernel(int nx, int ny, int nz, int ilo, int ihi, i
 #pragma unroll
             for (int u = 0; u < N; u++) {
                 if (k0 + u >= nz - 1) break;
-                const float inc = getm_d2f_approx(h1[u] - h0[u]) * idtf +
-                                  (pe[u] * dyEf - pw[u] * dyWf + qn[u] * dxNf - qs[u] * dxSf) * iaf;
+                float s = __fmaf_rn(pe[u], dyEf, -__fmul_rn(pw[u], dyWf));
+                s = __fmaf_rn(-qs[u], dxSf, __fmaf_rn(qn[u], dxNf, s));
+                const float inc = __fmaf_rn(getm_d2f_approx(h1[u] - h0[u]), idtf, __fmul_rn(s, iaf));
                 wk = wk - getm_f2d(inc);
                 w[p + (k0 + u + 1) * plane] = getm_d2f_approx(wk);
             }

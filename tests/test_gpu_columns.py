@@ -89,3 +89,28 @@ def test_transports_and_sums(nx, ny, nz, form):
             for a in src.double().cpu().numpy():
                 ref = ref + a
             assert np.array_equal(got.cpu().numpy(), ref if subtract == 0 else ref - ref)
+
+
+@pytest.mark.parametrize("form", ["fp64", "f32"])
+def test_vertical_velocity_of_any_domain(form):
+    """Columns of a small domain, and the same columns repeated over one beyond the
+    size up to which four levels are loaded at once: the same bits."""
+    import torch
+
+    from getm_gb300 import _lib
+    from getm_gb300._pygetm import _s
+
+    rng = np.random.default_rng(1)
+    dt = torch.float64 if form == "fp64" else torch.float32
+    nx, ny, nz, outs = 40, 30, 11, []
+    r = lambda lo, hi, *k: rng.uniform(lo, hi, (*k, ny, nx))  # noqa: E731
+    fields = [np.ones((ny, nx), np.int32), r(1990, 2010), r(1990, 2010), r(2.4e-7, 2.6e-7), r(90, 110, nz), r(90, 110, nz),
+              r(-10, 10, nz), r(-10, 10, nz), 0 * r(0, 1, nz + 1)]
+    for reps in ((1, 1), (9, 8)):
+        up = [_up(np.tile(a, (1,) * (a.ndim - 2) + reps)) for a in fields]
+        up[6:] = [t.to(dt) for t in up[6:]]
+        ny_, nx_ = up[0].shape
+        _lib.call("getm_w_momentum_3d" + ("" if form == "fp64" else "_f32"), nx_, ny_, nz, 3, nx_ - 2, 3, ny_ - 2,
+                  *[t.data_ptr() for t in up[:8]], 120.0, up[8].data_ptr(), _s())
+        outs.append(up[8][:, 2:ny - 2, 2:nx - 2])
+    assert torch.equal(*outs) and float(outs[0].abs().max()) > 0.0
