@@ -377,14 +377,14 @@ class Runner:
 # cells per lane): profiles/hpass_x_f64s_seamount_400x300x40.md (184.0 +
 # 83.0 MB), and the float-storage one-cell pass of an earlier capture.
 TRAFFIC_X_PASS = {("_f32", 0): 152.51e6, ("_f64s", 1): 267.0e6, ("_f64s", 0): 263.9e6}
-# one 2D substep, by form (one cooperative launch then): profiles/substep_2d_seamount_400x300.md
-# (60.8 + 5.3 MB; the plane's fields stay in L2)
-TRAFFIC_SUBSTEP = {"mixed": 66.1e6}
+# one 2D substep (four launches, each from a cold L2), by form: profiles/substep_kernels.md
+# (84.6 + 0.3 MB; in a step the plane's fields stay in L2)
+TRAFFIC_SUBSTEP = {"mixed": 84.9e6}
 
 
 def _roofline(sim, peak, peak_kind):
     """Time the dominant kernel alone on the live state: one x-direction
-    advection pass of both tracers (hpass_x_kernel, one launch)."""
+    advection pass of both tracers (one launch)."""
     import torch
 
     from getm_gb300 import _lib
@@ -434,7 +434,7 @@ def _roofline(sim, peak, peak_kind):
     vec = int(sfx != "" and autotune.current()["xpass_vec"] == 1 and T.nx_ % 4 == 0)
     kernel = {("_f32", 0): "hpass_x_inc_kernel<float, float>", ("_f32", 1): "hpass_x_vec_kernel<float, float>",
               ("_f64s", 0): "hpass_x_inc_kernel<double, float>", ("_f64s", 1): "hpass_x_vec_kernel<double, float>",
-              ("", 0): "hpass_x_kernel<double>"}[(sfx, vec)]
+              ("", 0): "hpass_x_inc_kernel<double, double, double>"}[(sfx, vec)]
     # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one launch
     # of this kernel on this workload, from an ncu capture of this bench
     traffic = TRAFFIC_X_PASS.get((sfx, vec))
@@ -904,7 +904,7 @@ def run_ours(args):
                          "kernel": substep["kernel"], "bytes_per_launch": substep["bytes_per_launch"],
                          "us_per_launch": substep["us_per_launch_median"], "peak_kind": peak_kind,
                          "note": "one 2D substep; its fields stay resident in L2, so HBM is a reference point "
-                                 "(bound: FP64 pipe and grid barriers)"}
+                                 "(bound: instructions, FP64 pipe and latency)"}
     else:
         roofline_main = roofline_kernel
     r = runners[primary]

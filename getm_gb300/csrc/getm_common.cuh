@@ -322,8 +322,8 @@ __device__ __forceinline__ double getm_max_pos(double a, double b)
 // True for the mixed form's float bulk type.  Its update kernels use the
 // increment form x_new = x_old + dx, with dx formed from small differences,
 // so a field that does not change is reproduced exactly and float32 rounding
-// scales with the change rather than with the field; the FP64 form keeps the
-// reference's evaluation order operation by operation.
+// scales with the change rather than with the field.  (The FP64 form's advection
+// and column solves work in increments too, in FP64 throughout.)
 template <typename T>
 constexpr bool getm_increment_form = std::is_same<T, float>::value;
 

@@ -1,7 +1,8 @@
 // Point and tile functions of the split-explicit 2D substep, shared by the
-// one-operation kernels (split2d.cu, momentum.cu, grid_ops.cu) and the
-// persistent substep kernel (substep2d.cu), so that every operation has a
-// single definition and both paths give the same results bit for bit.
+// one-operation kernels (split2d.cu, momentum.cu, grid_ops.cu) and the substep's
+// kernels (substep2d.cu: one domain's four, its phases, many domains' batch), so
+// that every operation has a single definition and all give the same results
+// bit for bit.
 //
 // Layout: every field is [j][i] with the full halo-inclusive extents of its
 // grid (nx_, ny_ for T, U, V and their velocity grids, nx_+1, ny_+1 for X).

@@ -880,7 +880,7 @@ __device__ void batch_item(const BatchMember& m, int ph, int q, int ufirst, Subs
     }
     default: {
         // the model time moves on once per member, in its first item of the
-        // last phase (after the last barrier, as in substep_2d_kernel)
+        // last phase (after the last barrier)
         if (q == 0 && tx == 0 && ty == 0 && a.time) *a.time = *a.time + a.dt;
         const int d = q < m.adv_items[0][1] ? 0 : 1;
         const int r = d == 0 ? q : q - m.adv_items[0][1];

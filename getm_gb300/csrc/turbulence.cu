@@ -22,10 +22,9 @@
 // level, so each level's loads are coalesced); both equations are solved
 // implicitly in time over the interfaces 1..nz-1 with an elimination whose
 // coefficients live in a [level][column] workspace.  GB300's FP64 rate bounds
-// it (its FP64 instructions take 16 cycles of an SM each), so it counts those:
-// with U = dt K / h the coupling through a layer, which is the one above an
-// interface and then the one below the next, and s' of the interface below
-// (zero at the bottom, where c' = -1 would be the fixed value's),
+// it, so it counts FP64 instructions: with U = dt K / h the coupling through a
+// layer, which is the one above an interface and then the one below the next,
+// and s' = 1 - c' of the interface below (the fixed bottom value: c' = 0, s' = 1),
 //     t = dz (1 - dt S) + U' s',  den = t + U,  c = U / den,  s = t / den,
 //     d = (dz (x + dt Q) + U' d') / den,   then downwards x = d + c x_above:
 // no large terms are subtracted (b - a c of the textbook form loses digits
@@ -113,7 +112,9 @@ __device__ __forceinline__ void keps_solve(const KepsArgs<R>& a, long long c, do
         // a boundary would: c = 0, s = 1
         s = ((__double2hiint(r) & 0x7fffffff) | __double2loint(r)) != 0 ? t * r : 1.0;
         double rhs = fma(U, d, dz * fma(a.dt, Q, xo));
-        if (i == nz - 1) rhs = fma(Un, xn, rhs);  // (beside the substitution's own term, which starts from xn)
+        // the surface value's coupling enters here and once more in the substitution,
+        // which starts from xn with c as it is: it counts twice, as in the oracle
+        if (i == nz - 1) rhs = fma(Un, xn, rhs);
         d = rhs * r;
         cp[(long long)i * P] = cc;
         dp[(long long)i * P] = d;

@@ -341,9 +341,9 @@ __global__ void __launch_bounds__(128, 8) vd_column_kernel(VDArgs<float> a)
     }
 }
 
-// Increment form with the elimination coefficients in global memory (the
-// mixed form's column solve): the same arithmetic as vd_column_kernel<float,
-// true>, restructured for memory-level parallelism.  The loads of the
+// Increment form of the float solve with the elimination coefficients in global
+// or shared memory: the arithmetic of vd_column_kernel, restructured for
+// memory-level parallelism.  The loads of the
 // forward elimination do not depend on the elimination itself, so the
 // operands of the next level (thicknesses, nuh, field values, sources) are
 // issued one level ahead of the arithmetic, and those of the back

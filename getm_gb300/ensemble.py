@@ -177,7 +177,7 @@ class Ensemble:
 
 class BatchedEnsemble:
     """Advance many members together with the 2D substeps of all members in
-    one persistent kernel: per 3D step (a "round"), one cooperative launch
+    one persistent kernel each: per 3D step (a "round"), one cooperative launch
     per substep index k advances every member with more than k substeps left
     before its 3D step (``getm_substep_batch_launch``), then every member's
     last substep and its 3D step run on one of ``lanes`` streams.  Members

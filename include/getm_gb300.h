@@ -159,7 +159,7 @@ int getm_vertical_diffusion_apply(getm_vertical_diffusion* diff, int nx, int ny,
  * NULL; the arrays themselves may be NULL).  work: NULL (elimination
  * coefficients in shared memory) or a device buffer of 2*nx*ny*nz elements
  * of the field type (more columns resident per SM); the _f32 form solves
- * its fields in pairs and needs 4*nx*ny*nz elements when ntracer > 1.       */
+ * two fields at a time and needs 4*nx*ny*nz elements when ntracer > 1.      */
 int getm_vertical_diffusion_batch(int nx, int ny, int nz, const int* mask, const double* nuh,
                                   double timestep, double cnpar, const double* ho,
                                   const double* hn, int ntracer, const double* molecular,
